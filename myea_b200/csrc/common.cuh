@@ -209,6 +209,13 @@ struct Epilogue {
   // inside the reference's per-block parameter layout: one contraction instead of four)
   long long seg_rows = 0;
   long long seg_off[4] = {0, 0, 0, 0};
+  // act_out != null (contractions from fp32 operands, direct_gemm.cu, only): the result additionally leaves as
+  // act_out[m][n] = dropout(f(result)), pitch ldc: act_mask (one byte per column, null: none) zeroes units, act_scale
+  // multiplies what is kept
+  float *act_out = nullptr;
+  uint32_t act_af = 0;
+  float act_scale = 1.f;
+  const uint8_t *act_mask = nullptr;
 };
 
 // A fp32 matrix operand given by strides: element (r, k) at ptr[r * stride_r + k * stride_k]; one of the two
@@ -277,6 +284,15 @@ void shared_panel_layout(float *mem, long long R, long long C, int role_rows, Pa
 bool epilogue_takes_stats(const Context &ctx, const Epilogue &e, long long N);
 // Launches split kernels + the tensor-core kernel (engine 0) or the FP32 FMA kernel (engine 1) on ctx.stream.
 int gemm_nt(Context &ctx, const Operand &A, const Operand &B, const Epilogue &epi, const GemmScratch &scratch);
+// Contractions of small and middle sizes straight from the fp32 operands (direct_gemm.cu): no operand panels, several
+// products per launch.  row_sum[m] += sum over k of A[m][k] rides along where it is not null (bias derivatives).
+struct DirectItem {
+  Operand A, B;
+  Epilogue epi;
+  float *row_sum = nullptr;
+};
+bool direct_gemm_suits(const Context &ctx, long long M, long long N, long long K);
+int direct_gemm(Context &ctx, const DirectItem *items, int count);
 // Optional workspace that lets the 256 x 256 tensor-core kernel split the tiles of a partial last wave along K
 // (39 MB per context); without it that kernel computes whole tiles only.
 int gemm_splitk_reserve(Context &ctx);
@@ -318,6 +334,10 @@ struct OverlapWork {
 // contraction that produced z), no pass over z is made
 int norm_forward_stats(Context &ctx, const float *z, long long rows, long long H, const NormParams &np, int training,
                        const SumHook *hook = nullptr, const OverlapWork *meanwhile = nullptr, int fused_chunks = 0);
+// statistics, activation and dropout of a normalized layer in one launch, for short batches on one GPU
+bool norm_strip_suits(long long rows, const SumHook *hook);
+int norm_activation_strip(Context &ctx, const float *z, float *out, long long rows, long long H, const NormParams &np, int training, uint32_t af,
+                          const uint8_t *mask, float keep_scale);
 // out = dropout(f(z*col_scale+col_shift)) ; col_scale null = no normalization. mask: uint8[H] or null; keep_scale = 1/p for inverted dropout
 // sink (may be null): the result is also written as operand panels of the contraction that reads it next
 bool activation_writes_panels(uint32_t af);

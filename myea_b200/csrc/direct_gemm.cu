@@ -1,0 +1,454 @@
+// Contractions of small and middle sizes straight from fp32 operands:  C[M,N] (+)= A[M,K] * B[N,K]^T, several per launch.
+//
+// The kernels of gemm.cu read operand panels that split passes have written before: three launches and two extra trips
+// through L2 per product, which is nothing beside a large product and everything beside a small one (a training step of
+// a 64-256-256-10 network on 128 rows spent 236 us in 37 launches around 0.06 GFLOP, and its tiles of 128 x 128 kept four
+// SMs busy).  Here the operands are read as they lie (rows or columns contiguous, any pitch), split in registers and
+// stored as the tensor core wants them, and the result leaves through the same fused epilogue, plus the layer's
+// activation and dropout; the weight derivatives of a whole network are one launch.
+//
+//   tile      128 x 64 per CTA of 8 warps, two CTAs per SM, 32 of K per stage, 2 stages of 48 KB.  At these sizes a
+//             product is bounded by latency, so tiles are small and the K range of a tile is cut over the CTAs of a cluster
+//             (1, 2, 4 or 8) until the grid fills the chip; partial tiles meet in distributed shared memory and are added
+//             in rank order (bitwise repeatable)
+//   stage     every thread splits 24 elements: 8 consecutive K of three rows, fetched into registers while the stage before
+//             is converted.  hi (TF32) and the cross-term group (bf16, see panel_math.cuh) go into K-major tiles with the
+//             128-byte swizzle; one thread then issues the eight tcgen05.mma of the stage.  (Warp-level mma.sync was
+//             built first: 512^3 took 12 us instead of 17 with panels; its TF32 rate on this chip is below what the
+//             precision needs - three TF32 products run no faster than plain FMAs.)
+//   sums      three rotating accumulators for hi*hi and one for the cross terms, as in the 128 x 128 kernel
+#include "common.cuh"
+#include "gemm_epilogue.cuh"
+#include "panel_math.cuh"
+#include "tcgen05.cuh"
+
+#include <algorithm>
+#include <mutex>
+
+namespace myea {
+
+constexpr int DG_M = 128, DG_N = 64, DG_THREADS = 256;
+constexpr int DG_A_BYTES = DG_M * BK * 4, DG_B_BYTES = DG_N * BK * 4;       // one panel (hi or cross) of a stage
+constexpr int DG_STAGE_BYTES = 2 * DG_A_BYTES + 2 * DG_B_BYTES;             // A hi, A cross, B hi, B cross
+constexpr int DG_STAGES = 2, DG_MAIN = 3, DG_TMEM_COLS = 256;
+static_assert((DG_MAIN + 1) * DG_N <= DG_TMEM_COLS, "accumulators exceed the allocation");
+constexpr int DG_RED_PITCH = DG_N + 4;      // partial tile [128][68], then row sums [2][128]: over the stages, which are free by then
+static_assert((DG_M * DG_RED_PITCH + 2 * DG_M) * 4 <= DG_STAGES * DG_STAGE_BYTES, "the partial tile lies over the stages");
+constexpr int DG_BAR_OFFSET = DG_STAGES * DG_STAGE_BYTES;
+constexpr int DG_SMEM = DG_BAR_OFFSET + 64 + 1024;
+constexpr int DG_MAX_ITEMS = 12;
+
+struct DirectProblem {
+  const float *a, *b;
+  long long lda, ldb;    // pitch of the non-contiguous index
+  int M, N, K;
+  int tiles_n, first_tile;
+  int a_vec, b_vec;      // 16-byte copies possible
+  int c_vec;             // 16-byte accesses possible in the epilogue
+  float *row_sum;
+  Epilogue epi;
+};
+template <int MAX> struct DirectGroup {   // kernel argument: 400 bytes for a single product, 5 KB for a group
+  int count;
+  DirectProblem p[MAX];
+};
+
+// One thread's 8 consecutive K elements of one operand row, stage after stage.  T: the rows are contiguous in memory (pitch
+// ld between K steps), a warp's lanes take consecutive rows; else K is contiguous.  Rows past the matrix repeat its last
+// row (what they produce is never stored); K elements past its end are zeros.
+template <bool T>
+struct DgReader {
+  const float *p;     // element (row, k)
+  long long ld, advance;
+  int k, K;
+  bool vec;
+  uint32_t at;        // where the group lies in a panel of a stage: rows of 128 bytes, 16-byte chunks swizzled by the row
+  __device__ __forceinline__ DgReader(const float *src, long long pitch, int tile_row, int row0, int rows, int group, int k0, int K_, bool vec16)
+      : ld(pitch), advance(T ? BK * pitch : BK), k(k0 + 8 * group), K(K_), vec(vec16) {
+    const int row = min(row0 + tile_row, rows - 1);
+    p = src + (T ? static_cast<long long>(k) * pitch + row : static_cast<long long>(row) * pitch + k);
+    at = static_cast<uint32_t>(tile_row * 128 + (((2 * group) ^ (tile_row & 7)) * 16));
+  }
+  __device__ __forceinline__ void fetch(float (&v)[8]) {
+    if (k + 8 <= K) {
+      if (T) {
+        const float *q = p;
+#pragma unroll
+        for (int j = 0; j < 8; ++j, q += ld) v[j] = *q;
+      } else if (vec) {
+        load8(v, p);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = p[j];
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = k + j < K ? p[T ? j * ld : j] : 0.f;
+    }
+    p += advance;
+    k += BK;
+  }
+};
+
+// 8 elements as a hi and a cross group into a stage
+template <int ROLE>
+__device__ __forceinline__ void dg_store8(uint8_t *hi, uint8_t *cross, uint32_t at, const float (&v)[8]) {
+  float h[8];
+  uint32_t x[8];
+  split_group(v, ROLE, 0, h, x);
+  *reinterpret_cast<float4 *>(hi + at) = make_float4(h[0], h[1], h[2], h[3]);
+  *reinterpret_cast<float4 *>(hi + (at ^ 16u)) = make_float4(h[4], h[5], h[6], h[7]);
+  *reinterpret_cast<uint4 *>(cross + at) = make_uint4(x[0], x[1], x[2], x[3]);
+  *reinterpret_cast<uint4 *>(cross + (at ^ 16u)) = make_uint4(x[4], x[5], x[6], x[7]);
+}
+
+static __device__ __noinline__ float af_fire_rare(uint32_t af, float z) { return af_fire(af, z); }
+
+// What this CTA finishes of its tile: rows [first, first + count), summed over the CTAs of the cluster in rank order, through
+// the epilogue.  A thread keeps VEC adjacent columns and takes NB rows at a time, all their loads before the first use: with
+// a row at a time this part was latency after latency and took longer than the products (29 of 31 us at K = 10).
+template <int VEC, int NB>
+__device__ __forceinline__ void dg_finish(const DirectProblem &p, const float *partial, uint32_t S, int first, int count, int m0, int n0) {
+  constexpr int LANES = DG_N / VEC, STEP = DG_THREADS / LANES;
+  using Vec = float[VEC];
+  const Epilogue &e = p.epi;
+  const int c = (static_cast<int>(threadIdx.x) % LANES) * VEC, n = n0 + c;
+  if (n >= p.N) return;
+  auto load = [](Vec &d, const float *src) {
+    if constexpr (VEC == 4) { const float4 t = *reinterpret_cast<const float4 *>(src); d[0] = t.x; d[1] = t.y; d[2] = t.z; d[3] = t.w; }
+    else d[0] = *src;
+  };
+  auto store = [](float *dst, const Vec &d) {
+    if constexpr (VEC == 4) *reinterpret_cast<float4 *>(dst) = make_float4(d[0], d[1], d[2], d[3]);
+    else *dst = d[0];
+  };
+  const bool affine = e.deriv_af != 0u && e.aux_pre != nullptr && e.col_scale != nullptr;
+  Vec bias = {}, cs, ch = {};
+#pragma unroll
+  for (int k = 0; k < VEC; ++k) cs[k] = 1.f;
+  if (e.bias != nullptr) load(bias, e.bias + n);
+  if (affine) { load(cs, e.col_scale + n); load(ch, e.col_shift + n); }
+  float factor[VEC];
+  if (e.act_out != nullptr) {
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) factor[k] = (e.act_mask != nullptr && e.act_mask[n + k] == 0) ? 0.f : e.act_scale;
+  }
+  const int end = min(first + count, p.M - m0);
+#pragma unroll 1
+  for (int r0 = first + static_cast<int>(threadIdx.x) / LANES; r0 < end; r0 += NB * STEP) {
+    Vec v[NB], add[NB], pre[NB], y[NB], old[NB];
+    float *dst[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const int r = min(r0 + b * STEP, end - 1);   // rows past the end repeat the last one and are not stored
+      const long long m = m0 + r;
+      dst[b] = e.C + c_row(e, m) + n;
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) v[b][k] = 0.f;
+      if (e.addend != nullptr) load(add[b], e.addend + m * e.ld_addend + n);
+      if (e.deriv_af != 0u && e.aux_pre != nullptr) load(pre[b], e.aux_pre + m * e.ld_aux + n);
+      if (e.deriv_af != 0u && e.aux_y != nullptr) load(y[b], e.aux_y + m * e.ld_aux + n);
+      if (e.accumulate) load(old[b], dst[b]);
+      if (S == 1) load(v[b], partial + r * DG_RED_PITCH + c);
+    }
+    if (S > 1) {
+#pragma unroll 2
+      for (uint32_t q = 0; q < S; ++q) {
+        const uint32_t base = ptx::map_to_cta(ptx::smem_u32(partial), q);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          const uint32_t at = base + (min(r0 + b * STEP, end - 1) * DG_RED_PITCH + c) * 4;
+          if constexpr (VEC == 4) {
+            const float4 t = ptx::ld_cluster_f4(at);
+            v[b][0] += t.x; v[b][1] += t.y; v[b][2] += t.z; v[b][3] += t.w;
+          } else {
+            float t;
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(t) : "r"(at) : "memory");
+            v[b][0] += t;
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) {
+        v[b][k] += bias[k];
+        if (e.addend != nullptr) v[b][k] += add[b][k];
+      }
+    }
+    if (e.deriv_af != 0u) {
+      auto derive = [&](auto f) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+          for (int k = 0; k < VEC; ++k) v[b][k] *= f(e.aux_pre != nullptr ? pre[b][k] * cs[k] + ch[k] : 0.f, e.aux_y != nullptr ? y[b][k] : 0.f);
+      };
+      switch (e.deriv_af) {
+        case MYEA_AF_TANH: derive([](float z, float w) { return af_derive(MYEA_AF_TANH, z, w); }); break;
+        case MYEA_AF_RELU: derive([](float z, float w) { return af_derive(MYEA_AF_RELU, z, w); }); break;
+        default: { const uint32_t af = e.deriv_af; derive([af](float z, float w) { return af_derive_rare(af, z, w); }); break; }
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      if (r0 + b * STEP >= end) break;
+      if (e.accumulate) {
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) v[b][k] += old[b][k];
+      }
+      store(dst[b], v[b]);
+    }
+    if (e.act_out != nullptr) {
+      auto fire = [&](auto f) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+          for (int k = 0; k < VEC; ++k) { const float t = f(v[b][k]); v[b][k] = factor[k] != 0.f ? t * factor[k] : 0.f; }
+      };
+      switch (e.act_af) {
+        case MYEA_AF_TANH: fire([](float z) { return af_fire(MYEA_AF_TANH, z); }); break;
+        case MYEA_AF_RELU: fire([](float z) { return af_fire(MYEA_AF_RELU, z); }); break;
+        case MYEA_AF_LINEAR: fire([](float z) { return z; }); break;
+        default: { const uint32_t af = e.act_af; fire([af](float z) { return af_fire_rare(af, z); }); break; }
+      }
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        if (r0 + b * STEP >= end) break;
+        store(e.act_out + (dst[b] - e.C), v[b]);
+      }
+    }
+  }
+}
+
+template <bool AT, bool BT, int MAX>
+__global__ void __launch_bounds__(DG_THREADS, 2) direct_gemm_kernel(const __grid_constant__ DirectGroup<MAX> g, int *error_flag) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint64_t *free_bar = reinterpret_cast<uint64_t *>(smem + DG_BAR_OFFSET);  // [2] the products of a stage have been computed
+  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(free_bar + DG_STAGES);
+  uint32_t S;
+  asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(S));
+  const uint32_t rank = ptx::cluster_ctarank();
+  const int tile = static_cast<int>(blockIdx.x / S);
+  int pi = 0;
+#pragma unroll 1
+  while (pi + 1 < g.count && tile >= g.p[pi + 1].first_tile) ++pi;
+  const DirectProblem &p = g.p[pi];
+  const int tl = tile - p.first_tile;
+  const int tm = tl / p.tiles_n, tn = tl - tm * p.tiles_n;
+  const int m0 = tm * DG_M, n0 = tn * DG_N;
+  const int steps = (p.K + BK - 1) / BK;
+  const int per = (steps + static_cast<int>(S) - 1) / static_cast<int>(S);
+  const int s0 = min(static_cast<int>(rank) * per, steps), n_steps = min(s0 + per, steps) - s0;
+  const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31;
+  const bool want_sum = AT && p.row_sum != nullptr && tn == 0;
+  if (tid == 0) {
+    for (int s = 0; s < DG_STAGES; ++s) ptx::mbar_init(&free_bar[s], 1);
+    ptx::fence_barrier_init();
+  }
+  if (warp == 1) {
+    ptx::tmem_alloc(tmem_holder, DG_TMEM_COLS);
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  const uint32_t tmem = *tmem_holder;
+  grid_dependency_wait();
+  grid_dependency_release();
+
+  // this thread's share of a stage: rows (a0, group ag0), (a1, ag1) of A and (b0, bg) of B
+  const int a0 = AT ? (tid & 127) : (tid >> 2), ag0 = AT ? (tid >> 7) : (tid & 3);
+  const int a1 = AT ? a0 : a0 + 64, ag1 = AT ? ag0 + 2 : ag0;
+  const int b0 = BT ? (tid & 63) : (tid >> 2), bg = BT ? (tid >> 6) : (tid & 3);
+  // two register sets: the loads of stage i + 2 leave when stage i has been stored, so that their way to L2 and back
+  // runs beside the conversion of stage i + 1
+  float va0[2][8], va1[2][8], vb[2][8];
+  DgReader<AT> ra0(p.a, p.lda, a0, m0, p.M, ag0, s0 * BK, p.K, p.a_vec != 0), ra1(p.a, p.lda, a1, m0, p.M, ag1, s0 * BK, p.K, p.a_vec != 0);
+  DgReader<BT> rb(p.b, p.ldb, b0, n0, p.N, bg, s0 * BK, p.K, p.b_vec != 0);
+  auto fetch = [&](float (&x0)[8], float (&x1)[8], float (&xb)[8]) { ra0.fetch(x0); ra1.fetch(x1); rb.fetch(xb); };
+  float rs = 0.f;   // thread: row tid & 127, half of the K groups of every stage
+  bool ok = true;
+  if (n_steps > 0) fetch(va0[0], va1[0], vb[0]);
+  if (n_steps > 1) fetch(va0[1], va1[1], vb[1]);
+#pragma unroll 1
+  for (int i2 = 0; i2 < n_steps; i2 += 2) {
+#pragma unroll
+    for (int s = 0; s < DG_STAGES; ++s) {
+      const int i = i2 + s;
+      if (i >= n_steps) break;
+      uint8_t *st = smem + s * DG_STAGE_BYTES;
+      if (i >= DG_STAGES && !ptx::mbar_wait(&free_bar[s], static_cast<uint32_t>((i >> 1) - 1) & 1u)) ok = false;
+      dg_store8<PANEL_ROLE_A>(st, st + DG_A_BYTES, ra0.at, va0[s]);
+      dg_store8<PANEL_ROLE_A>(st, st + DG_A_BYTES, ra1.at, va1[s]);
+      dg_store8<PANEL_ROLE_B>(st + 2 * DG_A_BYTES, st + 2 * DG_A_BYTES + DG_B_BYTES, rb.at, vb[s]);
+      if (want_sum) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) rs += va0[s][j] + va1[s][j];
+      }
+      if (i + 2 < n_steps) fetch(va0[s], va1[s], vb[s]);
+      ptx::fence_proxy_async();
+      __syncthreads();
+      if (tid == 0 && ok) {
+        ptx::tc_fence_after();
+        const uint32_t base = ptx::smem_u32(st);
+        const uint64_t a_hi = make_smem_desc(base), a_x = make_smem_desc(base + DG_A_BYTES);
+        const uint64_t b_hi = make_smem_desc(base + 2 * DG_A_BYTES), b_x = make_smem_desc(base + 2 * DG_A_BYTES + DG_B_BYTES);
+#pragma unroll
+        for (int k = 0; k < BK / UMMA_K; ++k) {
+          const uint64_t koff = static_cast<uint64_t>((k * UMMA_K * 4) >> 4);
+          const int step = i * (BK / UMMA_K) + k;
+          ptx::mma_bf16(tmem + DG_MAIN * DG_N, a_x + koff, b_x + koff, make_idesc_bf16(DG_M, DG_N), step > 0 ? 1u : 0u);
+          ptx::mma_tf32(tmem + static_cast<uint32_t>((step % DG_MAIN) * DG_N), a_hi + koff, b_hi + koff, make_idesc_tf32(DG_M, DG_N), step >= DG_MAIN ? 1u : 0u);
+        }
+        ptx::tc_commit(&free_bar[s]);
+      }
+    }
+  }
+  // the last commit covers everything issued before it
+  float *partial = reinterpret_cast<float *>(smem);
+  if (n_steps > 0 && !ptx::mbar_wait(&free_bar[(n_steps - 1) & 1], static_cast<uint32_t>((n_steps - 1) >> 1) & 1u)) ok = false;
+  if (!ok && lane == 0) atomicCAS(error_flag, 0, 111);
+  ptx::tc_fence_after();
+  {
+    // accumulators -> partial tile: warp = 32 rows (warp % 4) x 32 columns (warp / 4)
+    const int q = warp & 3, half = warp >> 2;
+    float sum[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) sum[j] = 0.f;
+    const int filled = min(DG_MAIN, n_steps * (BK / UMMA_K));   // 0 or all of them: a stage has four K steps
+#pragma unroll
+    for (int acc = 0; acc <= DG_MAIN; ++acc) {
+      if (filled == 0) break;
+      uint32_t r[32];
+      ptx::tmem_ld_32x32(tmem + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>((DG_MAIN - acc) * DG_N + half * 32), r);  // cross terms first
+      ptx::tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 32; ++j) sum[j] += __uint_as_float(r[j]);
+    }
+    float *d = partial + (q * 32 + lane) * DG_RED_PITCH + half * 32;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) *reinterpret_cast<float4 *>(d + 4 * j) = make_float4(sum[4 * j], sum[4 * j + 1], sum[4 * j + 2], sum[4 * j + 3]);
+  }
+  if (want_sum) partial[DG_M * DG_RED_PITCH + tid] = rs;   // [2][128]
+  ptx::tc_fence_before();
+  if (S > 1) ptx::cluster_sync_all();
+  else __syncthreads();
+  if (warp == 1) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc(tmem, DG_TMEM_COLS);
+  }
+  const int my_rows = DG_M / static_cast<int>(S), first = static_cast<int>(rank) * my_rows;
+  if (p.c_vec) dg_finish<4, 2>(p, partial, S, first, my_rows, m0, n0);
+  else dg_finish<1, 8>(p, partial, S, first, my_rows, m0, n0);
+  if (want_sum) {
+    for (int r = first + tid; r < first + my_rows; r += DG_THREADS) {
+      if (m0 + r >= p.M) continue;
+      const uint32_t at = ptx::smem_u32(partial + DG_M * DG_RED_PITCH + r);
+      float v = 0.f;
+      for (uint32_t q = 0; q < S; ++q) {
+        float x[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+          asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x[k]) : "r"(ptx::map_to_cta(at + k * DG_M * 4, q)) : "memory");
+        v += x[0] + x[1];
+      }
+      p.row_sum[m0 + r] += v;
+    }
+  }
+  if (S > 1) ptx::cluster_sync_all();  // a peer may still be reading this CTA's partial tile
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------------------------------------
+// Up to 600 M multiply-adds.  Measured against the panel kernels with their splits (us): 512^3 9.0 / 16.0, 256 x 1024 x 1024 12.1 /
+// 24.9, 512 x 2048 x 512 16.7 / 19.1, 1024^3 29.1 / 29.4, 2048 x 1024 x 512 27.4 / 22.7: conversion is repeated by every tile that
+// reads an operand, which from there on costs more than the split passes (that several contractions share).
+bool direct_gemm_suits(const Context &ctx, long long M, long long N, long long K) {
+  return ctx.gemm_engine == 0 && ctx.gemm_bn == 0 && M > 0 && N > 0 && K > 0 && M * N * K <= (600ll << 20);
+}
+
+template <bool AT, bool BT, int MAX>
+static int launch_direct(Context &ctx, const DirectGroup<MAX> &g, int tiles, int cluster) {
+  auto kernel = direct_gemm_kernel<AT, BT, MAX>;
+  static std::once_flag flags[64];
+  static bool ok[64] = {};
+  if (ctx.device < 0 || ctx.device >= 64) return MYEA_E_CUDA;
+  std::call_once(flags[ctx.device], [&] { ok[ctx.device] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM) == cudaSuccess; });
+  if (!ok[ctx.device]) return MYEA_E_CUDA;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(tiles * cluster));
+  cfg.blockDim = dim3(DG_THREADS);
+  cfg.dynamicSmemBytes = DG_SMEM;
+  cfg.stream = ctx.stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = (ctx.dependent_launch && !ctx.profiling) ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  ctx.begin(TC_GEMM);
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, g, ctx.d_error_flag);
+  ctx.end(TC_GEMM);
+  return err == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
+}
+
+static bool epilogue_is_vector(const Epilogue &e, long long N) {
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(e.C) | reinterpret_cast<uintptr_t>(e.bias) | reinterpret_cast<uintptr_t>(e.addend) |
+                         reinterpret_cast<uintptr_t>(e.aux_pre) | reinterpret_cast<uintptr_t>(e.aux_y) | reinterpret_cast<uintptr_t>(e.col_scale) |
+                         reinterpret_cast<uintptr_t>(e.col_shift) | reinterpret_cast<uintptr_t>(e.act_out);
+  return (bits & 15) == 0 && ((N | e.ldc | e.ld_addend | e.ld_aux | e.seg_off[0] | e.seg_off[1] | e.seg_off[2] | e.seg_off[3]) & 3) == 0;
+}
+
+template <int MAX>
+static int direct_gemm_launch(Context &ctx, const DirectItem *items, int n) {
+  DirectGroup<MAX> g;
+  g.count = n;
+  int tiles = 0, min_steps = 1 << 30;
+  const bool at = items[0].A.stride_k != 1, bt = items[0].B.stride_k != 1;
+  for (int i = 0; i < n; ++i) {
+    const DirectItem &it = items[i];
+    DirectProblem &p = g.p[i];
+    if (it.A.k != it.B.k || it.A.rows <= 0 || it.B.rows <= 0 || it.A.k <= 0 || (it.A.stride_k != 1) != at || (it.B.stride_k != 1) != bt) return MYEA_E_INVALID;
+    p.a = it.A.ptr; p.b = it.B.ptr;
+    p.lda = at ? it.A.stride_k : it.A.stride_r;
+    p.ldb = bt ? it.B.stride_k : it.B.stride_r;
+    p.M = static_cast<int>(it.A.rows); p.N = static_cast<int>(it.B.rows); p.K = static_cast<int>(it.A.k);
+    p.a_vec = (reinterpret_cast<uintptr_t>(p.a) & 15) == 0 && (p.lda & 3) == 0;
+    p.b_vec = (reinterpret_cast<uintptr_t>(p.b) & 15) == 0 && (p.ldb & 3) == 0;
+    p.c_vec = epilogue_is_vector(it.epi, p.N);
+    p.tiles_n = (p.N + DG_N - 1) / DG_N;
+    p.first_tile = tiles;
+    tiles += p.tiles_n * ((p.M + DG_M - 1) / DG_M);
+    p.row_sum = at ? it.row_sum : nullptr;
+    p.epi = it.epi;
+    if ((it.row_sum != nullptr && !at) || it.epi.stats_kind != 0) return MYEA_E_INVALID;
+    min_steps = std::min(min_steps, (p.K + BK - 1) / BK);
+    ctx.gemm_flops += 2.0 * p.M * p.N * static_cast<double>(p.K);
+  }
+  // K is cut in up to four while the grid stays within one CTA per SM and every CTA keeps two stages.  Measured (us per
+  // launch, cut 1 / 2 / 4 / 8): 128 x 256 x 256 9.6 / 8.0 / 6.6 / 7.2, 203 x 333 x 333 18.6 / 13.6 / 9.8 / 11.3, 512^3 15.7 / 11.2
+  // / 8.8 / 12.3, 640^3 18.7 / 12.8 / 13.1 / 24.3, 1024 x 1024 x 256 10.1 / 11.1 / 18.0: clusters of eight are placed late, and
+  // pay only for very long walks (64 x 2048 x 2048: 53.0 / 30.1 / 17.8 / 16.6)
+  int cluster = 1;
+  while (cluster < (min_steps >= 64 ? 8 : 4) && tiles * cluster * 2 <= (cluster == 4 ? 256 : 148) && min_steps >= cluster * 4) cluster *= 2;
+  if (at) return bt ? launch_direct<true, true>(ctx, g, tiles, cluster) : launch_direct<true, false>(ctx, g, tiles, cluster);
+  return bt ? launch_direct<false, true>(ctx, g, tiles, cluster) : launch_direct<false, false>(ctx, g, tiles, cluster);
+}
+
+// Items of one call share the orientation of A and of B.
+int direct_gemm(Context &ctx, const DirectItem *items, int count) {
+  for (int first = 0; first < count; first += DG_MAX_ITEMS) {
+    const int n = std::min(DG_MAX_ITEMS, count - first);
+    const int rc = n == 1 ? direct_gemm_launch<1>(ctx, items + first, n) : direct_gemm_launch<DG_MAX_ITEMS>(ctx, items + first, n);
+    if (rc != MYEA_OK) return rc;
+  }
+  return MYEA_OK;
+}
+
+}  // namespace myea

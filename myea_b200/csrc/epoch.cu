@@ -6,40 +6,59 @@
 // [T][B][width] layout from the (host-shuffled) order, so an epoch moves no example over PCIe.
 #include "net.cuh"
 
+#include <string.h>
+
+#include <algorithm>
+
 namespace myea {
 
-// dst[(t * B + b) * W + j] = src[order[first + b] * T * W + t * W + j]
-__global__ void __launch_bounds__(256) gather_batch_kernel(const float *__restrict__ src, const unsigned long long *__restrict__ order,
-                                                           long long first, long long B, long long T, long long W, float *__restrict__ dst) {
-  const long long total = T * B * W;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long j = i % W, tb = i / W, b = tb % B, t = tb / B;
-    dst[i] = src[order[first + b] * T * W + t * W + j];
-  }
+// One launch gathers the inputs and the targets of a batch straight into the network's buffers:
+//   dst[(t * pitch + b) * W + j] = b < B ? src[order[first + b] * T * W + t * W + j] : 0
+// (pitch > B: a recurrent network's short batch; its unused rows carry zeros).  V elements per thread and step.
+struct GatherSide {
+  const float *src;
+  float *dst;
+  long long W, total;   // total: T * pitch * W / V
+};
+template <typename V>
+__device__ __forceinline__ void gather_side(const GatherSide &g, const unsigned long long *__restrict__ order, long long first, long long B, long long pitch,
+                                            long long T, long long i) {
+  constexpr int n = sizeof(V) / sizeof(float);
+  const long long w = g.W / n, j = i % w, tb = i / w, b = tb % pitch, t = tb / pitch;
+  V v = {};
+  if (b < B) v = reinterpret_cast<const V *>(g.src)[(order[first + b] * T + t) * w + j];
+  reinterpret_cast<V *>(g.dst)[i] = v;
 }
-__global__ void __launch_bounds__(256) gather_batch_vec4_kernel(const float4 *__restrict__ src, const unsigned long long *__restrict__ order,
-                                                                long long first, long long B, long long T, long long W4, float4 *__restrict__ dst) {
-  const long long total = T * B * W4;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long j = i % W4, tb = i / W4, b = tb % B, t = tb / B;
-    dst[i] = src[order[first + b] * T * W4 + t * W4 + j];
+__global__ void __launch_bounds__(256) gather_batch_kernel(const GatherSide in, const GatherSide out, int in_vec, int out_vec, const unsigned long long *__restrict__ order,
+                                                           long long first, long long B, long long pitch, long long T, int in_blocks) {
+  grid_dependency_wait();
+  grid_dependency_release();
+  const bool is_in = static_cast<int>(blockIdx.x) < in_blocks;
+  const GatherSide &g = is_in ? in : out;
+  const bool vec = is_in ? in_vec != 0 : out_vec != 0;
+  const long long blocks = is_in ? in_blocks : static_cast<long long>(gridDim.x) - in_blocks, block = is_in ? blockIdx.x : static_cast<long long>(blockIdx.x) - in_blocks;
+  for (long long i = block * 256ll + threadIdx.x; i < g.total; i += blocks * 256ll) {
+    if (vec) gather_side<float4>(g, order, first, B, pitch, T, i);
+    else gather_side<float>(g, order, first, B, pitch, T, i);
   }
 }
 
-static int gather(myea_b200_net *net, const float *src, long long first, long long B, long long W, float *dst) {
+static int gather(myea_b200_net *net, long long first, long long B) {
   Context &ctx = net->ctx;
-  const long long total = net->T * B * W;
+  const long long pitch = net->full_pitch ? net->B : B;
+  auto side = [&](const float *src, float *dst, long long W, int *vec, int *blocks) {
+    GatherSide g{src, dst, W, net->T * pitch * W};
+    *vec = (W & 3) == 0;
+    if (*vec) g.total /= 4;
+    *blocks = static_cast<int>(std::max<long long>(1, std::min<long long>((g.total + 255) / 256, 148 * 8)));
+    return g;
+  };
+  int in_vec, out_vec, in_blocks, out_blocks;
+  const GatherSide in = side(net->ds_inputs, net->d_input, net->layers[0].n_out, &in_vec, &in_blocks);
+  const GatherSide out = side(net->ds_outputs, net->d_desired, net->layers.back().n_out, &out_vec, &out_blocks);
   ctx.begin(TC_ELEMENTWISE);
-  if ((W & 3) == 0) {
-    const int blocks = static_cast<int>(std::min<long long>((total / 4 + 255) / 256, 148 * 16));
-    gather_batch_vec4_kernel<<<std::max(blocks, 1), 256, 0, ctx.stream>>>(reinterpret_cast<const float4 *>(src), net->ds_order, first, B, net->T,
-                                                                          W / 4, reinterpret_cast<float4 *>(dst));
-  } else {
-    const int blocks = static_cast<int>(std::min<long long>((total + 255) / 256, 148 * 16));
-    gather_batch_kernel<<<std::max(blocks, 1), 256, 0, ctx.stream>>>(src, net->ds_order, first, B, net->T, W, dst);
-  }
+  launch_dependent(ctx, gather_batch_kernel, dim3(static_cast<unsigned>(in_blocks + out_blocks)), dim3(256), 0, in, out, in_vec, out_vec,
+                   static_cast<const unsigned long long *>(net->ds_order), first, B, pitch, net->T, in_blocks);
   ctx.end(TC_ELEMENTWISE);
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
@@ -56,6 +75,30 @@ static int set_order(myea_b200_net *net, const uint64_t *order, uint64_t n) {
   if (cudaMemcpyAsync(net->ds_order, order, n * sizeof(unsigned long long), cudaMemcpyHostToDevice, net->ctx.stream) != cudaSuccess) return MYEA_E_CUDA;
   return cudaStreamSynchronize(net->ctx.stream) == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;  // `order` is the caller's memory
 }
+
+static int reserve_loss_slots(myea_b200_net *net, uint64_t n) {
+  if (n > net->ds_loss_capacity) {
+    if (net->ds_loss != nullptr) cudaFree(net->ds_loss);
+    net->ds_loss = nullptr;
+    net->ds_loss_capacity = 0;
+    if (cudaMalloc(&net->ds_loss, 3 * n * sizeof(double)) != cudaSuccess) return MYEA_E_CUDA;
+    net->ds_loss_capacity = n;
+  }
+  return cudaMemsetAsync(net->ds_loss, 0, 3 * n * sizeof(double), net->ctx.stream) == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
+}
+// points the handle's loss accumulators at the slot of a mini-batch, and back at the end or on the way out
+struct LossSlots {
+  myea_b200_net *net;
+  double *acc;
+  unsigned long long *count;
+  explicit LossSlots(myea_b200_net *n) : net(n), acc(n->d_loss_acc), count(n->d_loss_count) {}
+  void use(uint64_t mb) {
+    net->d_loss_acc = net->ds_loss + 3 * mb;
+    net->d_loss_count = reinterpret_cast<unsigned long long *>(net->d_loss_acc + 2);
+  }
+  void restore() { net->d_loss_acc = acc; net->d_loss_count = count; }
+  ~LossSlots() { restore(); }
+};
 
 // Get__Loss(TYPE_DATASET_NONE) (Neural_Network__Loss.cpp:99-205) of the accumulators of one mini-batch
 static double reference_loss(const myea_b200_net *net, double loss_sum, uint64_t number_loss) {
@@ -75,15 +118,13 @@ extern "C" int myea_b200_dataset_set(myea_handle net, uint64_t number_examples, 
   if (net == nullptr || inputs == nullptr || outputs == nullptr || number_examples == 0) return MYEA_E_INVALID;
   if (cudaSetDevice(net->ctx.device) != cudaSuccess) return MYEA_E_CUDA;
   const size_t wi = static_cast<size_t>(net->T * net->layers[0].n_out), wo = static_cast<size_t>(net->T * net->layers.back().n_out);
-  for (float **p : {&net->ds_inputs, &net->ds_outputs, &net->ds_batch_inputs, &net->ds_batch_outputs}) {
+  for (float **p : {&net->ds_inputs, &net->ds_outputs}) {
     if (*p != nullptr) cudaFree(*p);
     *p = nullptr;
   }
   net->ds_examples = 0;
   if (cudaMalloc(&net->ds_inputs, number_examples * wi * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&net->ds_outputs, number_examples * wo * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&net->ds_batch_inputs, static_cast<size_t>(net->B) * wi * sizeof(float) + 16) != cudaSuccess ||
-      cudaMalloc(&net->ds_batch_outputs, static_cast<size_t>(net->B) * wo * sizeof(float) + 16) != cudaSuccess) {
+      cudaMalloc(&net->ds_outputs, number_examples * wo * sizeof(float)) != cudaSuccess) {
     net->ctx.error = "cudaMalloc failed (dataset)";
     return MYEA_E_CUDA;
   }
@@ -117,30 +158,51 @@ extern "C" int myea_b200_train_epoch(myea_handle net, const uint64_t *order, uin
   if (cudaSetDevice(net->ctx.device) != cudaSuccess) return MYEA_E_CUDA;
   int rc = set_order(net, order, number_examples);
   if (rc != MYEA_OK) return rc;
-  const long long wi = net->layers[0].n_out, wo = net->layers.back().n_out;
   const uint64_t mini_batches = (number_examples + mini_batch_size - 1) / mini_batch_size;
   double loss_total = 0.0, acc_total = 0.0;
+  // One GPU: every mini-batch accumulates its loss into a slot of its own, and the host reads all of them once at the end -
+  // a read per mini-batch would drain the stream each time.  (Ranks of a job add their sums up per mini-batch.)
+  const bool slots = net->comm == nullptr;
+  if (slots && (rc = reserve_loss_slots(net, mini_batches)) != MYEA_OK) return rc;
+  LossSlots slot(net);
   for (uint64_t mb = 0; mb < mini_batches; ++mb) {
     const uint64_t mb_first = mb * mini_batch_size;
     const uint64_t mb_size = std::min<uint64_t>(mini_batch_size, number_examples - mb_first);
     if (mask_seed != 0 && (rc = myea_b200_generate_masks(net, mask_seed, first_step + mb)) != MYEA_OK) return rc;
-    if ((rc = myea_b200_reset_loss(net)) != MYEA_OK) return rc;
+    if (slots) slot.use(mb);
+    else if ((rc = myea_b200_reset_loss(net)) != MYEA_OK) return rc;
     for (uint64_t done = 0; done < mb_size; done += B) {  // derivatives accumulate over the sub-batches of one mini-batch
       const uint64_t b = std::min<uint64_t>(B, mb_size - done);
       const long long first = static_cast<long long>(mb_first + done);
-      if ((rc = gather(net, net->ds_inputs, first, static_cast<long long>(b), wi, net->ds_batch_inputs)) != MYEA_OK) return rc;
-      if ((rc = gather(net, net->ds_outputs, first, static_cast<long long>(b), wo, net->ds_batch_outputs)) != MYEA_OK) return rc;
-      if ((rc = myea_b200_forward_device(net, b, net->ds_batch_inputs, 1)) != MYEA_OK) return rc;
-      if ((rc = myea_b200_compute_error_device(net, b, net->ds_batch_outputs)) != MYEA_OK) return rc;
+      if ((rc = gather(net, first, static_cast<long long>(b))) != MYEA_OK) return rc;
+      if ((rc = net_forward_staged(net, b, 1)) != MYEA_OK) return rc;
+      if ((rc = net_error_staged(net, b)) != MYEA_OK) return rc;
       if ((rc = myea_b200_backward(net, b)) != MYEA_OK) return rc;
       if ((rc = myea_b200_update_derivative_weight(net, b)) != MYEA_OK) return rc;
     }
-    double ls = 0.0, as = 0.0;
-    uint64_t nl = 0;
-    if ((rc = myea_b200_get_loss(net, &ls, &nl, &as)) != MYEA_OK) return rc;
-    loss_total += reference_loss(net, ls, nl);
-    acc_total += as;
+    if (!slots) {
+      double ls = 0.0, as = 0.0;
+      uint64_t nl = 0;
+      if ((rc = myea_b200_get_loss(net, &ls, &nl, &as)) != MYEA_OK) return rc;
+      loss_total += reference_loss(net, ls, nl);
+      acc_total += as;
+    }
     if ((rc = myea_b200_update_parameter(net, mb_size, net->ds_examples, opt)) != MYEA_OK) return rc;
+  }
+  if (slots) {
+    std::vector<double> all(3 * mini_batches);
+    slot.restore();
+    // the handle's accumulators keep the last mini-batch, as after a loop over the step functions
+    if (cudaMemcpyAsync(net->d_loss_acc, net->ds_loss + 3 * (mini_batches - 1), 3 * sizeof(double), cudaMemcpyDeviceToDevice, net->ctx.stream) != cudaSuccess ||
+        cudaMemcpyAsync(all.data(), net->ds_loss, all.size() * sizeof(double), cudaMemcpyDeviceToHost, net->ctx.stream) != cudaSuccess ||
+        cudaStreamSynchronize(net->ctx.stream) != cudaSuccess)
+      return MYEA_E_CUDA;
+    for (uint64_t mb = 0; mb < mini_batches; ++mb) {
+      uint64_t nl = 0;
+      memcpy(&nl, &all[3 * mb + 2], sizeof(nl));
+      loss_total += reference_loss(net, all[3 * mb], nl);
+      acc_total += all[3 * mb + 1];
+    }
   }
   if (mean_loss != nullptr) *mean_loss = loss_total / static_cast<double>(mini_batches);
   if (accuracy_sum != nullptr) *accuracy_sum = acc_total;
@@ -166,14 +228,12 @@ extern "C" int myea_b200_evaluate(myea_handle net, const uint64_t *order, uint64
   }
   int rc = set_order(net, order, number_examples);
   if (rc != MYEA_OK) return rc;
-  const long long wi = net->layers[0].n_out, wo = net->layers.back().n_out;
   if ((rc = myea_b200_reset_loss(net)) != MYEA_OK) return rc;
   for (uint64_t first = 0; first < number_examples; first += B) {
     const uint64_t b = std::min<uint64_t>(B, number_examples - first);
-    if ((rc = gather(net, net->ds_inputs, static_cast<long long>(first), static_cast<long long>(b), wi, net->ds_batch_inputs)) != MYEA_OK) return rc;
-    if ((rc = gather(net, net->ds_outputs, static_cast<long long>(first), static_cast<long long>(b), wo, net->ds_batch_outputs)) != MYEA_OK) return rc;
-    if ((rc = myea_b200_forward_device(net, b, net->ds_batch_inputs, 0)) != MYEA_OK) return rc;   // inference: running statistics, no masks
-    if ((rc = myea_b200_compute_error_device(net, b, net->ds_batch_outputs)) != MYEA_OK) return rc;
+    if ((rc = gather(net, static_cast<long long>(first), static_cast<long long>(b))) != MYEA_OK) return rc;
+    if ((rc = net_forward_staged(net, b, 0)) != MYEA_OK) return rc;   // inference: running statistics, no masks
+    if ((rc = net_error_staged(net, b)) != MYEA_OK) return rc;
   }
   double ls = 0.0, as = 0.0;
   uint64_t nl = 0;

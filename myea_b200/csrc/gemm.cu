@@ -1468,6 +1468,10 @@ int gemm_nt(Context &ctx, const Operand &A, const Operand &B, const Epilogue &ep
     ctx.gemm_flops += 2.0 * dims.M * dims.N * static_cast<double>(dims.K);
     return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
   }
+  if (epi.stats_kind == 0 && direct_gemm_suits(ctx, A.rows, B.rows, A.k)) {
+    const DirectItem item{A, B, epi, nullptr};
+    return direct_gemm(ctx, &item, 1);
+  }
   if (scratch.base == nullptr || scratch.floats < gemm_scratch_floats(A.rows, B.rows, A.k)) return MYEA_E_INVALID;
   float *base = reinterpret_cast<float *>((reinterpret_cast<uintptr_t>(scratch.base) + 255) & ~static_cast<uintptr_t>(255));
   Panels pa, pb;

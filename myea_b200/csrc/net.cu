@@ -262,8 +262,8 @@ static int allocate_buffers(myea_b200_net *net) {
   RC(dev_alloc(net, &net->m2hat, P + 4));
   RC(dev_alloc(net, &net->prev_delta, P + 4));
   RC(dev_alloc(net, &net->mask_reg, P + 4));
-  RC(dev_alloc(net, &net->d_loss_acc, 2));
-  RC(dev_alloc(net, &net->d_loss_count, 1));
+  RC(dev_alloc(net, &net->d_loss_acc, 3));  // loss sum, accuracy sum, number of loss terms: one reset, one read
+  net->d_loss_count = reinterpret_cast<unsigned long long *>(net->d_loss_acc + 2);
   RC(dev_alloc(net, &net->d_sumsq, 1));
   RC(dev_alloc(net, &net->d_clip_scale, 1));
   RC(dev_alloc(net, &net->d_loss_tmp, 3));
@@ -291,7 +291,8 @@ static int allocate_buffers(myea_b200_net *net) {
       if (L.has_norm) RC(dev_alloc(net, &L.errors, rows * L.n_out));
       else L.errors = L.deriv;
       if (gemm_takes_mn_major(net->ctx, rows, L.n_out) &&
-          gemm_takes_mn_major(net->ctx, rows, L.n_in) && gemm_takes_mn_major(net->ctx, L.n_out, L.n_in) && net->ctx.gemm_engine == 0) {
+          gemm_takes_mn_major(net->ctx, rows, L.n_in) && gemm_takes_mn_major(net->ctx, L.n_out, L.n_in) && net->ctx.gemm_engine == 0 &&
+          !direct_gemm_suits(net->ctx, rows, L.n_out, L.n_in)) {
         L.shared_panels = true;
         RC(dev_alloc(net, &L.in_panel_mem, shared_panel_floats(rows, L.n_in)));
         RC(dev_alloc(net, &L.w_panel_mem, shared_panel_floats(L.n_out, L.n_in)));
@@ -422,8 +423,7 @@ extern "C" void myea_b200_destroy(myea_handle net) {
   for (auto &L : net->layers) lstm_destroy(L);
   for (void *p : net->allocations) cudaFree(p);
   gemm_splitk_release(net->ctx);
-  for (void *p : {static_cast<void *>(net->ds_inputs), static_cast<void *>(net->ds_outputs), static_cast<void *>(net->ds_batch_inputs),
-                  static_cast<void *>(net->ds_batch_outputs), static_cast<void *>(net->ds_order)})
+  for (void *p : {static_cast<void *>(net->ds_inputs), static_cast<void *>(net->ds_outputs), static_cast<void *>(net->ds_order), static_cast<void *>(net->ds_loss)})
     if (p != nullptr) cudaFree(p);
   if (net->ctx.ev0) cudaEventDestroy(net->ctx.ev0);
   if (net->ctx.ev1) cudaEventDestroy(net->ctx.ev1);
@@ -574,7 +574,16 @@ int fc_product_forward(myea_b200_net *net, LayerPlan &L, const float *input, lon
   L.in_valid = L.w_valid = L.d_valid = false;
   Operand a{input, rows, L.n_in, L.n_in, 1};
   Operand b{w, L.n_out, L.n_in, L.n_in, 1};
+  if (e.act_out != nullptr) {  // only asked for where fc_runs_direct holds
+    DirectItem item{a, b, e, nullptr};
+    return direct_gemm(net->ctx, &item, 1);
+  }
   return gemm_nt(net->ctx, a, b, e, net->scratch);
+}
+
+// whether the forward product of this layer runs straight from the fp32 operands (and can carry the activation along)
+static bool fc_runs_direct(const myea_b200_net *net, const LayerPlan &L, long long rows) {
+  return !fc_uses_shared_panels(net, L, rows) && direct_gemm_suits(net->ctx, rows, L.n_out, L.n_in);
 }
 
 int fc_product_backward(myea_b200_net *net, LayerPlan &N, long long rows, const Epilogue &e) {
@@ -609,7 +618,24 @@ int fc_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long r
   // batch statistics: the contraction's epilogue leaves the column sums of every 32-row block behind, where it can
   int fused_chunks = 0;
   const bool timewise_norm = (L.has_norm && net->T > 1) || L.ind_rnn;  // a recurrent network normalizes every time step by itself
-  if (L.has_norm && norm_train && !timewise_norm) {
+  const bool direct = fc_runs_direct(net, L, rows);
+  const uint8_t *drop_mask = (drop_train && L.mask_bernoulli != nullptr) ? L.mask_bernoulli : nullptr;
+  const float drop_scale = drop_train ? (drop_mask != nullptr ? L.keep_scale : 1.f) : L.infer_scale;
+  if (direct && !timewise_norm && (drop_mask == nullptr || net->T == 1) && L.desc.type_activation_function != MYEA_AF_SOFTMAX) {
+    if (!L.has_norm) {  // the product's epilogue applies activation and dropout
+      e.act_out = L.values;
+      e.act_af = L.desc.type_activation_function;
+      e.act_scale = drop_scale;
+      e.act_mask = drop_mask;
+      return fc_product_forward(net, L, input, rows, e);
+    }
+    if (norm_strip_suits(rows, &net->hook)) {
+      RC(fc_product_forward(net, L, input, rows, e));
+      return norm_activation_strip(net->ctx, L.summations, L.values, rows, L.n_out, L.norm, norm_train ? 1 : 0, L.desc.type_activation_function, drop_mask,
+                                   drop_scale);
+    }
+  }
+  if (L.has_norm && norm_train && !timewise_norm && !direct) {
     Epilogue probe = e;
     probe.stats_kind = 1;
     probe.col_stats = L.norm.partial;
@@ -805,6 +831,7 @@ static int forward_pre_training(myea_b200_net *net, long long rows) {
   return rc;
 }
 
+// kind cudaMemcpyDefault: the batch already lies in d_input (the epoch loop gathers it there)
 static int forward_impl(myea_b200_net *net, uint64_t batch, const float *src, cudaMemcpyKind kind, int training) {
   if (net == nullptr || src == nullptr) return MYEA_E_INVALID;
   RC(batch_for_forward(net, batch));
@@ -818,7 +845,10 @@ static int forward_impl(myea_b200_net *net, uint64_t batch, const float *src, cu
   // parameters are waited for here, every fully connected layer's weights where the layer first reads them, and
   // everything that is left before any other kind of layer.
   RC(comm_wait_gathers(net, net->total_weights, net->total_parameters - net->total_weights));
-  if (kind == cudaMemcpyHostToDevice) {
+  bool panels = false;
+  for (const auto &L : net->layers) panels = panels || (L.type == MYEA_LAYER_FULLY_CONNECTED && L.n_in > 0 && fc_uses_shared_panels(net, L, rows));
+  if (kind == cudaMemcpyDefault) {
+  } else if (kind == cudaMemcpyHostToDevice && panels) {
     // inputs from the host: copy them on the side stream (once everything already queued has finished with d_input)
     // and split every large layer's weights meanwhile - the copy takes longer than all those passes together
     CK(cudaEventRecord(net->ev_input_free, net->ctx.stream));
@@ -882,7 +912,7 @@ static int compute_error_impl(myea_b200_net *net, uint64_t batch, const float *s
     const float *desired = net->layers[k - 1].values;
     if (k <= 1) {
       CK(cudaStreamWaitEvent(net->ctx.stream, net->ev_desired_free, 0));
-      CK(cudaMemcpyAsync(net->d_desired, src, rows * D.n_out * sizeof(float), kind, net->ctx.stream));
+      if (kind != cudaMemcpyDefault) CK(cudaMemcpyAsync(net->d_desired, src, rows * D.n_out * sizeof(float), kind, net->ctx.stream));
       desired = net->d_desired;
     }
     RC(output_error(net->ctx, D.summations, D.values, desired, D.errors, rows, D.n_out, D.desc.type_activation_function, net->desc.type_loss_function,
@@ -893,7 +923,8 @@ static int compute_error_impl(myea_b200_net *net, uint64_t batch, const float *s
   }
   LayerPlan &L = net->layers.back();
   const long long pitch = pitch_rows(net), rows = net->T * pitch;
-  if (kind == cudaMemcpyHostToDevice) {
+  if (kind == cudaMemcpyDefault) {
+  } else if (kind == cudaMemcpyHostToDevice && rows * L.n_out * static_cast<long long>(sizeof(float)) > (256 << 10)) {
     // host targets: copy beside the forward pass still in flight on the main stream (the last use of d_desired by an
     // error kernel is behind ev_desired_free), and let the main stream wait for the copy only now
     CK(cudaStreamWaitEvent(net->copy_stream, net->ev_desired_free, 0));
@@ -930,6 +961,11 @@ static int compute_error_impl(myea_b200_net *net, uint64_t batch, const float *s
   return MYEA_OK;
 }
 
+namespace myea {
+int net_forward_staged(myea_b200_net *net, uint64_t batch, int training) { return forward_impl(net, batch, net->d_input, cudaMemcpyDefault, training); }
+int net_error_staged(myea_b200_net *net, uint64_t batch) { return compute_error_impl(net, batch, net->d_desired, cudaMemcpyDefault); }
+}  // namespace myea
+
 extern "C" int myea_b200_compute_error(myea_handle net, uint64_t batch, const float *desired) {
   return compute_error_impl(net, batch, desired, cudaMemcpyHostToDevice);
 }
@@ -939,18 +975,17 @@ extern "C" int myea_b200_compute_error_device(myea_handle net, uint64_t batch, c
 
 extern "C" int myea_b200_reset_loss(myea_handle net) {
   if (net == nullptr) return MYEA_E_INVALID;
-  CK(cudaMemsetAsync(net->d_loss_acc, 0, 2 * sizeof(double), net->ctx.stream));
-  CK(cudaMemsetAsync(net->d_loss_count, 0, sizeof(unsigned long long), net->ctx.stream));
+  CK(cudaMemsetAsync(net->d_loss_acc, 0, 3 * sizeof(double), net->ctx.stream));
   return MYEA_OK;
 }
 
 extern "C" int myea_b200_get_loss(myea_handle net, double *loss_sum, uint64_t *number_loss, double *accuracy_sum) {
   if (net == nullptr) return MYEA_E_INVALID;
-  double acc[2] = {0, 0};
-  unsigned long long cnt = 0;
+  double acc[3] = {0, 0, 0};
   CK(cudaMemcpyAsync(acc, net->d_loss_acc, sizeof(acc), cudaMemcpyDeviceToHost, net->ctx.stream));
-  CK(cudaMemcpyAsync(&cnt, net->d_loss_count, sizeof(cnt), cudaMemcpyDeviceToHost, net->ctx.stream));
   CK(cudaStreamSynchronize(net->ctx.stream));
+  unsigned long long cnt = 0;
+  memcpy(&cnt, acc + 2, sizeof(cnt));
   if (net->comm != nullptr) {  // Merge__Post__Training across ranks: every rank must call get_loss
     double all[3] = {acc[0], acc[1], static_cast<double>(cnt)};
     CK(cudaMemcpyAsync(net->d_loss_tmp, all, sizeof(all), cudaMemcpyHostToDevice, net->ctx.stream));
@@ -1000,7 +1035,8 @@ int fc_backward_from_fc(myea_b200_net *net, LayerPlan &L, const LayerPlan &next,
       probe.col_stats = L.norm.partial;
       probe.col_mean = L.norm.mean;
       probe.stats_blocks = (rows + 31) / 32;
-      if (next_errors == next.errors && probe.stats_blocks <= L.norm.chunks && epilogue_takes_stats(net->ctx, probe, L.n_out)) {
+      const bool direct = !(next.shared_panels && next.w_valid) && direct_gemm_suits(net->ctx, rows, next.n_in, next.n_out);
+      if (!direct && next_errors == next.errors && probe.stats_blocks <= L.norm.chunks && epilogue_takes_stats(net->ctx, probe, L.n_out)) {
         e = probe;
         L.bwd_fused_chunks = static_cast<int>(probe.stats_blocks);
       }
@@ -1149,13 +1185,26 @@ extern "C" int myea_b200_backward(myea_handle net, uint64_t batch) {
 // Update_Derivative_Weight__FC (Neural_Network__Update_Derivative_Weight__OpenMP.cpp:178-216) + bias (:218-242)
 // ---------------------------------------------------------------------------------------------------------
 namespace myea {
-int fc_update_derivative_weight(myea_b200_net *net, LayerPlan &L, const float *input, long long rows) {
+static bool fc_derivative_runs_direct(const myea_b200_net *net, const LayerPlan &L, long long rows) {
+  return !(L.shared_panels && L.in_valid) && direct_gemm_suits(net->ctx, L.n_out, L.n_in, rows);
+}
+
+// `group` (may be null): collects the products of small layers so that one launch computes the derivatives of all of them
+int fc_update_derivative_weight(myea_b200_net *net, LayerPlan &L, const float *input, long long rows, std::vector<DirectItem> *group = nullptr) {
   Operand a{L.errors, L.n_out, rows, 1, L.n_out};  // delta^T: [out rows, K = batch]
   Operand b{input, L.n_in, rows, 1, L.n_in};       // input^T: [in rows, K = batch]
   Epilogue e;
   e.C = net->grads + L.idx.first_connection_index;
   e.ldc = L.n_in;
   e.accumulate = 1;
+  if (fc_derivative_runs_direct(net, L, rows)) {  // the bias derivative (row sums of delta^T) rides along
+    DirectItem item{a, b, e, L.use_bias ? net->grads + L.idx.first_bias_connection_index : nullptr};
+    if (group != nullptr) {
+      group->push_back(item);
+      return MYEA_OK;
+    }
+    return direct_gemm(net->ctx, &item, 1);
+  }
   if (L.shared_panels && L.in_valid && input == L.in_src) {
     if (!L.d_valid) {  // no error propagation below this layer (first hidden layer): only the column reading is needed
       RC(gemm_prepare_shared(net->ctx, L.errors, L.n_out, rows, L.n_out, L.d_panel_mem, PANEL_ROLE_A, nullptr, PANEL_ROLE_A, &L.d_cols));
@@ -1193,6 +1242,7 @@ extern "C" int myea_b200_update_derivative_weight(myea_handle net, uint64_t batc
   // for each layer's gather only where it reads that layer, finds the lower layers' parameters in place while the
   // upper layers' are still travelling.
   const int n_layers = static_cast<int>(net->layers.size());
+  std::vector<DirectItem> group;
   for (int step = 1; step < n_layers; ++step) {
     const int l = net->comm != nullptr ? step : n_layers - step;
     LayerPlan &L = net->layers[l];
@@ -1200,7 +1250,7 @@ extern "C" int myea_b200_update_derivative_weight(myea_handle net, uint64_t batc
       const float *input = net->layers[L.input_layer].values;
       int blk = 0;
       if (layer_in_block(net, l, &blk)) input = residual_fc_input(net, blk, l - blk);  // normalized / activated copy kept by the block
-      RC(fc_update_derivative_weight(net, L, input, rows));
+      RC(fc_update_derivative_weight(net, L, input, rows, net->comm == nullptr ? &group : nullptr));
       if (L.ind_rnn && net->T > 1) {
         // recurrent weights: dAF of step t with the output of step t - 1 (the pre-activation buffer is free by now and
         // holds the products)
@@ -1215,6 +1265,7 @@ extern "C" int myea_b200_update_derivative_weight(myea_handle net, uint64_t batc
     if (net->comm != nullptr && L.idx.last_connection_index > L.idx.first_connection_index)
       RC(comm_reduce_bucket_async(net, L.idx.first_connection_index, L.idx.last_connection_index - L.idx.first_connection_index));
   }
+  if (!group.empty()) RC(direct_gemm(net->ctx, group.data(), static_cast<int>(group.size())));
   if (net->comm != nullptr) {  // biases and normalization scales / shifts: one last bucket behind the weights
     RC(comm_reduce_bucket_async(net, net->total_weights, net->total_parameters - net->total_weights));
     net->grads_reduced = true;

@@ -59,6 +59,10 @@ struct LayerPlan {
   float *pre_af = nullptr;        // [T*B, n_out]
 };
 
+// forward / compute_error of a batch that already lies in d_input / d_desired (net.cu)
+int net_forward_staged(myea_b200_net *net, uint64_t batch, int training);
+int net_error_staged(myea_b200_net *net, uint64_t batch);
+
 // independently recurrent layers (ind_rnn.cu)
 int ind_rnn_forward_step(Context &ctx, const float *z, const float *y_prev, const float *u, float *pre, float *y, long long rows, long long H, uint32_t af,
                          const float *col_scale, const float *col_shift, const uint8_t *mask, float keep_scale);
@@ -109,7 +113,7 @@ struct myea_b200_net {
   float *d_input = nullptr;    // [T*B, inputs]
   float *d_desired = nullptr;  // [T*B, outputs]
   myea::GemmScratch scratch;
-  double *d_loss_acc = nullptr;  // [2] loss sum, accuracy sum
+  double *d_loss_acc = nullptr;  // [3] loss sum, accuracy sum, number of loss terms (an integer: d_loss_count)
   unsigned long long *d_loss_count = nullptr;
   double *d_sumsq = nullptr;
   float *d_clip_scale = nullptr;
@@ -122,10 +126,11 @@ struct myea_b200_net {
   bool grads_reduced = false;    // this step's derivative buckets have already been handed to the communicator
   bool sharded_update = true;    // the last update was element by element (no clip, no max-norm): buckets may be reduce-scattered
   double *d_loss_tmp = nullptr;  // [3] staging for the cross-GPU sum of the loss accumulators
-  // dataset kept on the device for the epoch loop (epoch.cu): rows [example][T * width], the staged batch, the order
-  float *ds_inputs = nullptr, *ds_outputs = nullptr, *ds_batch_inputs = nullptr, *ds_batch_outputs = nullptr;
+  // dataset kept on the device for the epoch loop (epoch.cu): rows [example][T * width], the order
+  float *ds_inputs = nullptr, *ds_outputs = nullptr;
   unsigned long long *ds_order = nullptr;
-  uint64_t ds_examples = 0, ds_order_capacity = 0;
+  double *ds_loss = nullptr;     // [mini-batches of an epoch][3]: every mini-batch's loss accumulators
+  uint64_t ds_examples = 0, ds_order_capacity = 0, ds_loss_capacity = 0;
   // targets arriving from the host are copied on a stream of their own, so that the copy runs under the forward pass
   // that is still executing; the two events order it against the error kernel's use of d_desired
   cudaStream_t copy_stream = nullptr;

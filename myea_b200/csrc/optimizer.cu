@@ -84,6 +84,8 @@ __device__ __forceinline__ float opt_one(const OptLaunch &o, float w, float g, f
 
 template <bool HAS_VHAT, bool HAS_PREV>
 __global__ void __launch_bounds__(256) optimizer_kernel(const OptLaunch o, const OptArrays a, size_t n) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const float scale = o.clip_scale != nullptr ? *o.clip_scale : 1.0f;
   const size_t n4 = n >> 2;
   const bool adam_like = o.type != MYEA_OPT_GD;
@@ -127,9 +129,9 @@ int optimizer_update(Context &ctx, const OptLaunch &o, float *w, float *g, float
     return MYEA_E_INVALID;
   const int blocks = static_cast<int>(std::max<size_t>(1, std::min<size_t>(((n >> 2) + 255) / 256, 148 * 16)));
   ctx.begin(TC_OPTIMIZER);
-  if (has_vhat) optimizer_kernel<true, false><<<blocks, 256, 0, ctx.stream>>>(o, a, n);
-  else if (has_prev) optimizer_kernel<false, true><<<blocks, 256, 0, ctx.stream>>>(o, a, n);
-  else optimizer_kernel<false, false><<<blocks, 256, 0, ctx.stream>>>(o, a, n);
+  if (has_vhat) launch_dependent(ctx, optimizer_kernel<true, false>, dim3(blocks), dim3(256), 0, o, a, n);
+  else if (has_prev) launch_dependent(ctx, optimizer_kernel<false, true>, dim3(blocks), dim3(256), 0, o, a, n);
+  else launch_dependent(ctx, optimizer_kernel<false, false>, dim3(blocks), dim3(256), 0, o, a, n);
   ctx.end(TC_OPTIMIZER);
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }

@@ -142,15 +142,19 @@ int residual_forward(myea_b200_net *net, int r) {
     const float *in = x;
     if (k > 1) {
       const float *prev = net->layers[r + k - 1].summations;
-      const float *cs = nullptr, *ch = nullptr;
-      if (L.has_norm) {
-        RRC(norm_forward_stats(ctx, prev, rows, L.n_in, L.norm, net->training ? 1 : 0, &net->hook));
-        cs = L.norm.col_scale;
-        ch = L.norm.col_shift;
-      }
       const uint8_t *mask = (net->training && L.mask_bernoulli != nullptr) ? L.mask_bernoulli : nullptr;
       const float scale = net->training ? (mask != nullptr ? L.keep_scale : 1.f) : L.infer_scale;
-      RRC(activation_forward(ctx, prev, L.values, rows, L.n_in, L.desc.type_activation_function, cs, ch, mask, scale));
+      if (L.has_norm && !L.shared_panels && norm_strip_suits(rows, &net->hook)) {
+        RRC(norm_activation_strip(ctx, prev, L.values, rows, L.n_in, L.norm, net->training ? 1 : 0, L.desc.type_activation_function, mask, scale));
+      } else {
+        const float *cs = nullptr, *ch = nullptr;
+        if (L.has_norm) {
+          RRC(norm_forward_stats(ctx, prev, rows, L.n_in, L.norm, net->training ? 1 : 0, &net->hook));
+          cs = L.norm.col_scale;
+          ch = L.norm.col_shift;
+        }
+        RRC(activation_forward(ctx, prev, L.values, rows, L.n_in, L.desc.type_activation_function, cs, ch, mask, scale));
+      }
       in = L.values;
     }
     Epilogue e;
