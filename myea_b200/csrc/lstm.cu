@@ -243,6 +243,18 @@ __global__ void lstm_gather_peepholes_kernel(const float *__restrict__ peep, lon
   out[2 * C + c] = peep[c * stride + 2];
 }
 
+// the input weights of the four gates, [dirs][4C][n_in], out of the blocks (w0 / w1: first block of each direction)
+__global__ void __launch_bounds__(256) lstm_gather_input_weights_kernel(const float *__restrict__ w0, const float *__restrict__ w1, long long stride, long long z_in,
+                                                                        long long i_in, long long n_in, long long C, float *__restrict__ out) {
+  const long long total = 4 * C * n_in;
+  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total; i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const long long r = i / n_in, k = i - r * n_in, g = r / C, c = r - g * C;
+    const long long at = c * stride + (g == 0 ? z_in : i_in + (g - 1) * n_in) + k;
+    out[i] = w0[at];
+    if (w1 != nullptr) out[total + i] = w1[at];
+  }
+}
+
 // ---------------------------------------------------------------------------------------------------------
 // plan
 // ---------------------------------------------------------------------------------------------------------
@@ -329,6 +341,7 @@ int lstm_create(myea_b200_net *net, LayerPlan &L) {
     LRC(two_buffers(4 * Cp, P->dg_pan));
     LRC(lstm_persistent_plan(net, L));
   }
+  LRC(lstm_resident_plan(net, L));
   // one-shot contractions use the handle's scratch: make sure it is large enough
   size_t need = 0;
   need = std::max(need, panel_floats(rows, L.n_in) + panel_floats(4 * C, L.n_in));            // input projection
@@ -337,12 +350,14 @@ int lstm_create(myea_b200_net *net, LayerPlan &L) {
   P->shared_dw = net->ctx.gemm_engine == 0 && (C % 64) == 0 && (net->B % 8) == 0 && gemm_takes_mn_major(net->ctx, C, L.n_in) &&
                  gemm_takes_mn_major(net->ctx, C, C);
   if (P->shared_dw) need = std::max(need, shared_panel_floats(rows, 4 * C) + shared_panel_floats(rows, L.n_in) + shared_panel_floats(rows, L.n_out) + 256);
+  need = std::max<size_t>(need, static_cast<size_t>(P->dirs * 4 * C * L.n_in));  // gathered input weights
   net->scratch.floats = std::max(net->scratch.floats, need + 256);
   return MYEA_OK;
 }
 
 void lstm_destroy(LayerPlan &L) {
   lstm_persistent_destroy(L.lstm);
+  lstm_resident_destroy(L.lstm);
   delete L.lstm;
   L.lstm = nullptr;
 }
@@ -411,11 +426,27 @@ int lstm_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long
   const long long T = net->T, B = net->B, rows = T * B, C = P->C, ldh = L.n_out;
   const BlockOffsets off = block_offsets(n_in, C);
   float *scratch = aligned_scratch(net);
+  const bool direct_in = direct_gemm_suits(ctx, rows, 4 * C, n_in);
+  if (direct_in) {  // the four gates (of both directions) of the input projection in one launch, straight from the blocks
+    DirectItem items[8];
+    int n = 0;
+    for (int d = 0; d < P->dirs; ++d)
+      for (int g = 0; g < 4; ++g) {
+        DirectItem &it = items[n++];
+        it.A = Operand{input, rows, n_in, n_in, 1};
+        it.B = Operand{net->params + P->d[d].w_base + (g == 0 ? off.z_in : off.in[g - 1]), C, n_in, P->stride, 1};
+        it.epi.C = P->d[d].gates_in + g * C;
+        it.epi.ldc = 4 * C;
+        it.epi.bias = net->params + P->d[d].b_base + g * C;
+      }
+    LRC(direct_gemm(ctx, items, n));
+  }
   Panels px;
-  LRC(gemm_prepare(ctx, Operand{input, rows, n_in, n_in, 1}, scratch, &px, PANEL_ROLE_A));
-  for (int d = 0; d < P->dirs; ++d) {
+  if (!direct_in) LRC(gemm_prepare(ctx, Operand{input, rows, n_in, n_in, 1}, scratch, &px, PANEL_ROLE_A));
+  for (int d = 0; d < P->dirs && !(direct_in && P->resident != nullptr); ++d) {
     LstmDir &D = P->d[d];
     const float *w = net->params + D.w_base;
+    if (!direct_in) {
     // fused input panel [4C, in], gate order z, i, f, o
     Panels pwin = panels_at(scratch + panel_floats(rows, n_in), 4 * C, n_in, PANEL_ROLE_B);
     LRC(gemm_prepare_into(ctx, Operand{w + off.z_in, C, n_in, P->stride, 1}, pwin, 0, 0));
@@ -425,6 +456,8 @@ int lstm_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long
     e.ldc = 4 * C;
     e.bias = net->params + D.b_base;
     LRC(gemm_panels(ctx, px, 0, rows, pwin, 0, 4 * C, e));
+    }
+    if (P->resident != nullptr) continue;
     // fused recurrent panel [4C, C]
     Panels pwrec = panels_at(P->panel_mem + P->off_wrec, 4 * C, C, PANEL_ROLE_B);
     float *peep_c = nullptr;
@@ -512,6 +545,10 @@ int lstm_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long
         LRC(gemm_prepare_into(ctx, Operand{h_t, B, C, ldh, 1}, P->h_pan[0], 0, 0));
     }
   }
+  if (P->resident != nullptr) {
+    const long long rec[4] = {off.z_rec, off.rec[0], off.rec[1], off.rec[2]};
+    LRC(lstm_resident_run(net, L, 1, P->zoneout && net->training, rec, off.peep));
+  }
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
 
@@ -525,6 +562,10 @@ int lstm_backward(myea_b200_net *net, LayerPlan &L) {
   const long long T = net->T, B = net->B, C = P->C, ldh = L.n_out, n_in = P->n_in;
   const long long Cp = (C + 7) & ~7ll;  // each gate's K segment starts on a group-of-8 boundary
   const BlockOffsets off = block_offsets(n_in, C);
+  if (P->resident != nullptr) {
+    const long long rec[4] = {off.z_rec, off.rec[0], off.rec[1], off.rec[2]};
+    return lstm_resident_run(net, L, 2, false, rec, off.peep);
+  }
   for (int d = 0; d < P->dirs; ++d) {
     LstmDir &D = P->d[d];
     const float *w = net->params + D.w_base;
@@ -614,9 +655,28 @@ int lstm_backward_to_input(myea_b200_net *net, LayerPlan &L, float *prev_deriv, 
   const long long Cp = (C + 7) & ~7ll;
   const BlockOffsets off = block_offsets(n_in, C);
   float *scratch = aligned_scratch(net);
+  const bool direct = direct_gemm_suits(ctx, rows, n_in, 4 * C);
+  if (direct) {  // the input weights gathered out of the blocks once (their four gate matrices are one K range then)
+    ctx.begin(TC_RECURRENT);
+    lstm_gather_input_weights_kernel<<<static_cast<unsigned>(std::min<long long>((4 * C * n_in + 255) / 256, 148 * 8)), 256, 0, ctx.stream>>>(
+        net->params + P->d[0].w_base, P->dirs > 1 ? net->params + P->d[1].w_base : nullptr, P->stride, off.z_in, off.in[0], n_in, C, scratch);
+    ctx.end(TC_RECURRENT);
+  }
   for (int d = 0; d < P->dirs; ++d) {
     LstmDir &D = P->d[d];
     const float *w = net->params + D.w_base;
+    if (direct) {
+      DirectItem it;
+      it.A = Operand{D.dgates, rows, 4 * C, 4 * C, 1};
+      it.B = Operand{scratch + d * 4 * C * n_in, n_in, 4 * C, 1, n_in};
+      if (finish != nullptr && d == P->dirs - 1) it.epi = *finish;
+      it.epi.C = prev_deriv;
+      it.epi.ldc = n_in;
+      if (d > 0 && finish != nullptr) { it.epi.addend = prev_deriv; it.epi.ld_addend = n_in; }
+      else it.epi.accumulate = d > 0 ? 1 : 0;
+      LRC(direct_gemm(ctx, &it, 1));
+      continue;
+    }
     Panels pd = panels_at(scratch, rows, 4 * Cp, PANEL_ROLE_A);
     LRC(prepare_gates(ctx, D.dgates, rows, C, Cp, pd));
     Panels pwt = panels_at(scratch + panel_floats(rows, 4 * Cp), n_in, 4 * Cp, PANEL_ROLE_B);  // [n_in, K = 4 gates]
@@ -646,7 +706,31 @@ int lstm_update_derivative_weight(myea_b200_net *net, LayerPlan &L, const float 
   for (int d = 0; d < P->dirs; ++d) {
     LstmDir &D = P->d[d];
     float *gw = net->grads + D.w_base;
-    if (P->shared_dw) {
+    if (direct_gemm_suits(ctx, 4 * C, std::max(n_in, C), rows)) {
+      // gate by gate in one launch: the gate errors against the layer's input and against its output one step earlier
+      DirectItem items[8];
+      const long long K = (T - 1) * B;
+      const float *dg0 = d == 0 ? D.dgates + B * 4 * C : D.dgates;
+      const float *h0 = d == 0 ? L.values + d * C : L.values + B * ldh + d * C;
+      int n = 0;
+      for (int g = 0; g < 4; ++g) {
+        DirectItem &it = items[n++];
+        it.A = Operand{D.dgates + g * C, C, rows, 1, 4 * C};
+        it.B = Operand{input, n_in, rows, 1, n_in};
+        it.epi.C = gw + (g == 0 ? off.z_in : off.in[g - 1]);
+        it.epi.ldc = P->stride;
+        it.epi.accumulate = 1;
+        if (T > 1) {
+          DirectItem &r = items[n++];
+          r.A = Operand{dg0 + g * C, C, K, 1, 4 * C};
+          r.B = Operand{h0, C, K, 1, ldh};
+          r.epi.C = gw + (g == 0 ? off.z_rec : off.rec[g - 1]);
+          r.epi.ldc = P->stride;
+          r.epi.accumulate = 1;
+        }
+      }
+      LRC(direct_gemm(ctx, items, n));
+    } else if (P->shared_dw) {
       // Both operands of every weight-derivative contraction are read through their columns (K = rows of the batch
       // and time axis), so one untransposed split pass per tensor serves all of them: gate errors, layer input, and
       // the layer's own outputs for the recurrent weights (a sub-range of K rows and of columns).

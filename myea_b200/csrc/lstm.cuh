@@ -18,6 +18,7 @@ struct LstmDir {
 };
 
 struct LstmPersistent;
+struct LstmResident;
 struct LstmPlan {
   int dirs = 1;
   long long C = 0, n_in = 0, stride = 0;
@@ -38,6 +39,7 @@ struct LstmPlan {
   // batch rounded up to 128, so that one tensor map covers both
   Panels h_pan[2], dg_pan[2];
   LstmPersistent *persist = nullptr;
+  LstmResident *resident = nullptr;  // the walk with resident weights (lstm_resident.cu), where it is the faster one
   // blocks of several cells (lstm_blocks.cu): K blocks of cpb cells per direction, gate rows of G = C + 3K columns
   // [z (C) | i (K) | f (K) | o (K)], weights gathered into dense matrices for the pass and their derivatives scattered back
   long long K = 0, cpb = 1;
@@ -66,5 +68,11 @@ void lstm_persistent_destroy(LstmPlan *P);
 bool lstm_persistent_ready(const LstmPlan *P);
 int lstm_persistent_forward(myea_b200_net *net, LayerPlan &L, int dir, const Panels &w_rec_interleaved, const float *peep_compact, bool zoneout);
 int lstm_persistent_backward(myea_b200_net *net, LayerPlan &L, int dir, const Panels &w_rec_transposed, const float *peep_compact);
+
+// The walk for small batches and narrow or odd layers: all time steps (and both directions) in one launch, recurrent weights
+// in shared memory, read from the parameter buffer itself.  Set by lstm_resident_plan where it is estimated to be faster.
+int lstm_resident_plan(myea_b200_net *net, LayerPlan &L);
+void lstm_resident_destroy(LstmPlan *P);
+int lstm_resident_run(myea_b200_net *net, LayerPlan &L, int kind, bool zoneout, const long long rec[4], long long peep);
 
 }  // namespace myea

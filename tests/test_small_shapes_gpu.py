@@ -1,0 +1,79 @@
+"""GPU tests of the paths small and middle networks take, at the edges of their tiles: contractions straight from fp32
+operands (128 x 64 tiles, 32 of K per stage, K cut over 1, 2, 4 or 8 CTAs), the one-launch normalization of short batches
+(8 columns per block, 4 to 32 rows per thread) and the LSTM walk with resident weights (groups of 1 to many CTAs, chunks of
+exchange data), against float64 products and the numpy restatement."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import rel_err
+from myea_b200 import capi, workloads
+from myea_b200.net import Net
+from oracle import myea_oracle
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-4
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (1, 64, 7), (3, 65, 31), (127, 63, 32), (128, 64, 33), (129, 65, 64), (130, 130, 257), (257, 10, 1000), (64, 640, 2048),
+                                   (5, 4, 4099)])
+@pytest.mark.parametrize("accumulate", [0, 1])
+def test_contraction_from_fp32_operands(M, N, K, accumulate):
+    lib = capi.load()
+    rng = np.random.default_rng(M * 7 + N * 3 + K)
+    A, B = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
+    out = rng.standard_normal((M, N), dtype=np.float32)
+    want = A.astype(np.float64) @ B.astype(np.float64).T + (out if accumulate else 0)
+    assert lib.myea_b200_gemm_nt(0, 0, M, N, K, A.ctypes.data, B.ctypes.data, out.ctypes.data, accumulate, None, 0) == 0
+    assert rel_err(out, want) < 5e-6
+
+
+def _step(wl, seed=5, rows=None):
+    """one training step and one inference pass on the GPU and on the restatement"""
+    gpu, cpu = Net(wl.desc, wl.opt), myea_oracle.OracleNet(wl.desc, wl.opt)
+    X, Y = wl.batch(seed)
+    for net in (gpu, cpu):
+        wl.materialize(net)
+        net.reset_loss(); net.forward(X); net.compute_error(Y); net.backward(); net.update_derivative_weight()
+    out = [(gpu.outputs(len(wl.layers) - 1), cpu.outputs(len(wl.layers) - 1)), (gpu.get(capi.BUF_DERIVATIVES), cpu.get(capi.BUF_DERIVATIVES))]
+    for net in (gpu, cpu):
+        net.update_parameter()
+        net.forward(X, training=False)
+    out += [(gpu.get(capi.BUF_PARAMETERS), cpu.get(capi.BUF_PARAMETERS)), (gpu.outputs(len(wl.layers) - 1), cpu.outputs(len(wl.layers) - 1))]
+    if gpu.n_norm:
+        out += [(gpu.get(b), cpu.get(b)) for b in (capi.BUF_NORM_MEAN_AVERAGE, capi.BUF_NORM_VARIANCE_AVERAGE)]
+    gpu.synchronize()
+    gpu.close()
+    for got, want in out:
+        assert rel_err(got, want) < TOL
+
+
+def _mlp(widths, B, af, norm=capi.NORM_NONE, drop=capi.DROP_NONE):
+    layers = [capi.fc(widths[0])] + [capi.fc(w, af, norm, drop, (0.7, 0, 0)) for w in widths[1:-1]] + [capi.fc(widths[-1], capi.AF_LINEAR)]
+    return workloads.Workload("edges", capi.net(layers, B, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE, r_max=3.0, d_max=5.0),
+                              capi.opt(capi.OPT_GD, gd_lr=0.01 / B, momentum=0.9), widths[0], widths[-1], False, layers)
+
+
+@pytest.mark.parametrize("widths,B", [((3, 5, 2), 1), ((31, 33, 7), 31), ((32, 64, 64), 33), ((65, 63, 129, 4), 127), ((64, 128, 256, 8), 128), ((129, 130, 65), 129),
+                                      ((300, 70, 71, 72, 73, 74, 75, 76, 77, 78, 79, 80, 81, 82), 65)])
+@pytest.mark.parametrize("af", [capi.AF_TANH, capi.AF_SINE])
+def test_plain_networks(widths, B, af):
+    _step(_mlp(widths, B, af, drop=capi.DROP_BERNOULLI))
+
+
+@pytest.mark.parametrize("B", [7, 31, 128, 129, 256, 257, 512, 513, 1024, 1025])
+@pytest.mark.parametrize("norm", [capi.NORM_BN, capi.NORM_BRN])
+def test_normalized_short_batches(B, norm):
+    _step(_mlp((9, 37, 16, 3), B, capi.AF_SIGMOID, norm, capi.DROP_BERNOULLI_INVERTED))
+
+
+@pytest.mark.parametrize("n_in,H,T,B,bidirectional,zoneout", [
+    (3, 5, 4, 3, False, 0.0), (7, 32, 3, 5, True, 0.3), (11, 37, 5, 50, False, 0.2), (16, 64, 1, 4, False, 0.0), (20, 107, 3, 9, False, 0.0), (20, 150, 4, 50, True, 0.1),
+    (9, 313, 3, 33, False, 0.0), (12, 512, 3, 70, False, 0.1), (5, 601, 3, 7, True, 0.0), (8, 1100, 2, 3, False, 0.0)])
+def test_lstm_with_resident_weights(n_in, H, T, B, bidirectional, zoneout):
+    layers = [capi.fc(n_in), capi.lstm(H, bidirectional=bidirectional, dropout=capi.DROP_ZONEOUT if zoneout else capi.DROP_NONE, p=(zoneout, zoneout, 0.0)),
+              capi.fc(H, capi.AF_LINEAR)]
+    wl = workloads.Workload("lstm edges", capi.net(layers, B, T=T, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE),
+                            capi.opt(capi.OPT_GD, gd_lr=0.01 / B, momentum=0.9), n_in, H, False, layers)
+    _step(wl)
