@@ -284,6 +284,33 @@ void shared_panel_layout(float *mem, long long R, long long C, int role_rows, Pa
 bool epilogue_takes_stats(const Context &ctx, const Epilogue &e, long long N);
 // Launches split kernels + the tensor-core kernel (engine 0) or the FP32 FMA kernel (engine 1) on ctx.stream.
 int gemm_nt(Context &ctx, const Operand &A, const Operand &B, const Epilogue &epi, const GemmScratch &scratch);
+// A tensor [R][C] as two half-precision arrays and an exponent per block of 128 x 128 (half_panels.cuh)
+struct HalfPanels {
+  uint16_t *h0 = nullptr, *h1 = nullptr;
+  long long R = 0, C = 0, pitch = 0;   // pitch in elements, a multiple of 64
+  int *exps = nullptr;                 // block (r / 128, c / 128) at exps[(r / 128) * exp_r + (c / 128) * exp_c]
+  long long exp_r = 0, exp_c = 0;      // both 0: one exponent for the whole tensor
+};
+// An operand of a contraction: rows x k elements of a tensor from (row0, k0) on, read through the tensor's rows (K along C)
+// or through its columns (K along R).  Where the tensor has an exponent per block, row0 and k0 are multiples of 128.
+struct HalfOperand {
+  HalfPanels p;
+  bool cols = false;
+  long long row0 = 0, k0 = 0, rows = 0, k = 0;
+};
+// floats of memory the panels of an [R][C] tensor take, and where they lie in it (256-byte aligned)
+size_t half_panel_floats(long long R, long long C);
+HalfPanels half_panels_at(float *mem, long long R, long long C);
+// Splits `src` (pitch stride) into panels.  seg_rows != 0: row r of the tensor is row r % seg_rows of the array that starts
+// at src + seg_off[r / seg_rows] (the four gate matrices inside an LSTM layer's parameter blocks).
+struct RowSegments {
+  long long seg_rows = 0;
+  long long seg_off[4] = {0, 0, 0, 0};
+};
+int half_split(Context &ctx, const float *src, long long stride, const HalfPanels &p, const RowSegments *seg = nullptr);
+HalfOperand half_rows(const HalfPanels &p);   // the whole tensor, read through its rows / columns
+HalfOperand half_cols(const HalfPanels &p);
+int half_gemm(Context &ctx, const HalfOperand &A, const HalfOperand &B, const Epilogue &epi);
 // Contractions of small and middle sizes straight from the fp32 operands (direct_gemm.cu): no operand panels, several
 // products per launch.  row_sum[m] += sum over k of A[m][k] rides along where it is not null (bias derivatives).
 struct DirectItem {
@@ -342,14 +369,14 @@ int norm_activation_strip(Context &ctx, const float *z, float *out, long long ro
 // sink (may be null): the result is also written as operand panels of the contraction that reads it next
 bool activation_writes_panels(uint32_t af);
 int activation_forward(Context &ctx, const float *z, float *out, long long rows, long long H, uint32_t af,
-                       const float *col_scale, const float *col_shift, const uint8_t *mask, float keep_scale, const PanelSink *sink = nullptr);
+                       const float *col_scale, const float *col_shift, const uint8_t *mask, float keep_scale, const HalfPanels *sink = nullptr);
 // in place: d *= f'(z * col_scale + col_shift, y) (col_scale null: the summation itself)
 int activation_backward(Context &ctx, float *d, const float *z, const float *y, long long rows, long long H, uint32_t af, const float *col_scale,
                         const float *col_shift);
 int softmax_forward(Context &ctx, const float *z, float *out, long long rows, long long H);
 // delta_af [rows,H] (error after the activation derivative) -> error before the normalization, plus d_gamma / d_beta
 int norm_backward(Context &ctx, const float *z, const float *delta_af, float *delta_out, long long rows, long long H,
-                  const NormParams &np, const SumHook *hook = nullptr, int fused_chunks = 0, const PanelSink *sink = nullptr);
+                  const NormParams &np, const SumHook *hook = nullptr, int fused_chunks = 0, const HalfPanels *sink = nullptr);
 // delta = f'(pre,y) * (y - desired); loss / accuracy accumulators (double[2] + uint64) on the device
 int output_error(Context &ctx, const float *pre, const float *y, const float *desired, float *delta, long long rows,
                  long long H, uint32_t af, uint32_t loss, uint32_t accuracy, float accuracy_variance, double *d_acc,

@@ -1195,14 +1195,6 @@ void shared_panel_layout(float *mem, long long R, long long C, int role_rows, Pa
   }
 }
 
-bool epilogue_takes_stats(const Context &ctx, const Epilogue &e, long long N) {
-  if (ctx.gemm_engine != 0 || (N & 31) != 0 || e.ldc != N || e.addend != nullptr || e.accumulate || e.seg_rows != 0) return false;
-  const uintptr_t bits = reinterpret_cast<uintptr_t>(e.C) | reinterpret_cast<uintptr_t>(e.bias) | reinterpret_cast<uintptr_t>(e.aux_pre) |
-                         reinterpret_cast<uintptr_t>(e.aux_y) | reinterpret_cast<uintptr_t>(e.col_scale) | reinterpret_cast<uintptr_t>(e.col_shift) |
-                         reinterpret_cast<uintptr_t>(e.col_stats) | reinterpret_cast<uintptr_t>(e.col_mean);
-  return (bits & 15) == 0 && ((e.ldc | e.ld_aux) & 3) == 0;
-}
-
 int gemm_prepare_shared(Context &ctx, const float *src, long long stride_r, long long R, long long C, float *mem, int role_rows,
                         Panels *as_rows, int role_cols, Panels *as_cols) {
   if (src == nullptr || mem == nullptr || R <= 0 || C <= 0 || (reinterpret_cast<uintptr_t>(mem) & 255) != 0) return MYEA_E_INVALID;
@@ -1224,11 +1216,6 @@ int gemm_prepare_shared(Context &ctx, const float *src, long long stride_r, long
 bool gemm_takes_mn_major(const Context &ctx, long long M, long long N) {
   if (ctx.gemm_engine == 1) return true;
   return ctx.gemm_bn == 0 ? (M > 128 && N > 128) : (ctx.gemm_bn == 3 || ctx.gemm_bn == 4);
-}
-
-size_t gemm_scratch_floats(long long M, long long N, long long K) {
-  const long long kp = round_up(K, BK);
-  return static_cast<size_t>(2 * (M + N) * kp) + 64;
 }
 
 size_t panel_floats(long long rows, long long k) { return static_cast<size_t>(2 * rows * round_up(k, BK)); }
@@ -1312,32 +1299,6 @@ static int launch_tcgen05_pair(Context &ctx, const CUtensorMap maps[4], const Ge
   dim3 grid(static_cast<unsigned>(2 * ((dims.M + 255) / 256)), static_cast<unsigned>((dims.N + 127) / 128));
   gemm3x_tf32_tcgen05_pair_kernel<<<grid, GEMM_THREADS, PairSmem::TOTAL, ctx.stream>>>(maps[0], maps[1], maps[2], maps[3], dims, epi, ctx.d_error_flag);
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
-}
-
-// Workspace of the wide kernel's split tiles: two partial-sum slots of one 256 x 256 tile per cluster and one arrival
-// counter per (split tile, warp region).  Without it the wide kernel computes whole tiles only.
-int gemm_splitk_reserve(Context &ctx) {
-  if (ctx.sk_ws != nullptr) return MYEA_OK;
-  int sms = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device) != cudaSuccess || sms < 2) return MYEA_E_CUDA;
-  const int clusters = sms / 2;
-  const size_t floats = static_cast<size_t>(clusters) * 2 * 16 * WIDE_REGION_FLOATS;
-  if (cudaMalloc(&ctx.sk_ws, floats * sizeof(float)) != cudaSuccess) { ctx.sk_ws = nullptr; return MYEA_E_CUDA; }
-  if (cudaMalloc(&ctx.sk_counters, static_cast<size_t>(clusters) * 16 * sizeof(unsigned int)) != cudaSuccess ||
-      cudaMemset(ctx.sk_counters, 0, static_cast<size_t>(clusters) * 16 * sizeof(unsigned int)) != cudaSuccess) {
-    cudaFree(ctx.sk_ws);
-    ctx.sk_ws = nullptr;
-    return MYEA_E_CUDA;
-  }
-  ctx.sk_clusters = clusters;
-  return MYEA_OK;
-}
-void gemm_splitk_release(Context &ctx) {
-  if (ctx.sk_ws != nullptr) cudaFree(ctx.sk_ws);
-  if (ctx.sk_counters != nullptr) cudaFree(ctx.sk_counters);
-  ctx.sk_ws = nullptr;
-  ctx.sk_counters = nullptr;
-  ctx.sk_clusters = 0;
 }
 
 template <bool A_MN, bool B_MN>
@@ -1455,30 +1416,6 @@ int gemm_panels(Context &ctx, const Panels &A, long long a_row0, long long M, co
   }
   ctx.gemm_flops += 2.0 * dims.M * dims.N * static_cast<double>(dims.K);
   return rc;
-}
-
-int gemm_nt(Context &ctx, const Operand &A, const Operand &B, const Epilogue &epi, const GemmScratch &scratch) {
-  if (A.k != B.k || A.rows <= 0 || B.rows <= 0 || A.k <= 0) return MYEA_E_INVALID;
-  if (ctx.gemm_engine == 1) {  // the FP32 FMA engine reads the fp32 sources directly
-    GemmDims dims{static_cast<int>(A.rows), static_cast<int>(B.rows), static_cast<int>(A.k)};
-    ctx.begin(TC_GEMM);
-    dim3 grid(static_cast<unsigned>((dims.N + 63) / 64), static_cast<unsigned>((dims.M + 63) / 64));
-    gemm_fp32_fma_kernel<<<grid, 256, 0, ctx.stream>>>(A, B, dims, epi);
-    ctx.end(TC_GEMM);
-    ctx.gemm_flops += 2.0 * dims.M * dims.N * static_cast<double>(dims.K);
-    return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
-  }
-  if (epi.stats_kind == 0 && direct_gemm_suits(ctx, A.rows, B.rows, A.k)) {
-    const DirectItem item{A, B, epi, nullptr};
-    return direct_gemm(ctx, &item, 1);
-  }
-  if (scratch.base == nullptr || scratch.floats < gemm_scratch_floats(A.rows, B.rows, A.k)) return MYEA_E_INVALID;
-  float *base = reinterpret_cast<float *>((reinterpret_cast<uintptr_t>(scratch.base) + 255) & ~static_cast<uintptr_t>(255));
-  Panels pa, pb;
-  int rc = gemm_prepare(ctx, A, base, &pa, PANEL_ROLE_A);
-  if (rc == MYEA_OK) rc = gemm_prepare(ctx, B, base + panel_floats(A.rows, A.k), &pb, PANEL_ROLE_B);
-  if (rc != MYEA_OK) return rc;
-  return gemm_panels(ctx, pa, 0, A.rows, pb, 0, B.rows, epi);
 }
 
 }  // namespace myea

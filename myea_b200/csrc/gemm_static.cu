@@ -13,11 +13,10 @@
 // Limit: the hi/lo K-major panels of both operands must fit: 2 * (M + N) * round_up(K, 32) + 64 floats <= 8 Mi floats;
 // larger problems are refused with MYEA_E_INVALID and a message, never truncated.
 // Sharing: all calls on a device use the same array, which keeps whatever the previous call left in it.  Nothing in
-// it has to start at zero except the status word, which each call clears first: a call rewrites columns
-// [0, round_up(K, 8)) of every panel row it uses, and what an earlier, larger call left beyond that is never read,
-// because the tensor maps the kernel loads through end at round_up(K, 8) and the hardware fills the rest of a tile
-// with zeros.  Two calls that overlap on the GPU (different streams, or different host threads) would overwrite each
-// other's panels: callers must serialise them.
+// it has to start at zero except the status word, which each call clears first: a call writes every element of the panels
+// it reads, and the tensor maps the kernel loads through end where the operands end (the hardware fills the rest of a
+// tile with zeros).  Two calls that overlap on the GPU (different streams, or different host threads) would overwrite
+// each other's panels: callers must serialise them.
 // Set-up: the device address of the array is looked up once per device, on the first call for that device, with that
 // device current.
 // The call is synchronous: it waits for the result and reads the status word back, so it must never be made on a
@@ -34,7 +33,9 @@ namespace {
 constexpr size_t kStaticScratchFloats = size_t(8) << 20;  // 32 MiB
 constexpr int kMaxDevices = 64;
 
-static __device__ __align__(256) float g_static_scratch[kStaticScratchFloats];
+// (the panels of the largest problems that fit the documented limit are a few hundred floats longer: block exponents and
+// alignment)
+static __device__ __align__(256) float g_static_scratch[kStaticScratchFloats + (size_t(64) << 10)];
 static __device__ __align__(256) int g_static_status[64];
 
 struct StaticSetup {
@@ -63,7 +64,7 @@ extern "C" int myea_b200_gemm_nt_static(int device, uint64_t M, uint64_t N, uint
     say(error_message, error_capacity, "gemm_nt_static: device index out of range");
     return MYEA_E_INVALID;
   }
-  const size_t need = gemm_scratch_floats(static_cast<long long>(M), static_cast<long long>(N), static_cast<long long>(K));
+  const size_t need = 2 * (M + N) * ((K + 31) / 32 * 32) + 64;
   if (M > (1u << 30) || N > (1u << 30) || K > (1u << 30) || need > kStaticScratchFloats) {
     char msg[200];
     snprintf(msg, sizeof(msg),
@@ -115,7 +116,7 @@ extern "C" int myea_b200_gemm_nt_static(int device, uint64_t M, uint64_t N, uint
   e.C = device_C;
   e.ldc = static_cast<long long>(N);
   e.accumulate = accumulate;
-  GemmScratch gs{su.scratch, kStaticScratchFloats};
+  GemmScratch gs{su.scratch, kStaticScratchFloats + (size_t(64) << 10)};
   int rc = gemm_nt(ctx, a, b, e, gs);
   if (rc != MYEA_OK) {
     say(error_message, error_capacity, "gemm_nt_static: kernel launch failed");

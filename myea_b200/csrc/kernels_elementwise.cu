@@ -3,7 +3,7 @@
 // for the bias derivatives.  All of them stream [rows, H] row-major fp32 tensors with 128-bit accesses where the
 // shape allows and reduce over rows with per-thread partial sums, a shared-memory tree and a second small pass.
 #include "common.cuh"
-#include "panel_math.cuh"
+#include "half_panels.cuh"
 
 #include <algorithm>
 
@@ -170,6 +170,8 @@ __device__ __forceinline__ void norm_stats_of_column(const NormParams &np, long 
 // then, partial = the reduced [2][H] sums).
 __global__ void __launch_bounds__(256) norm_stats_finalize_kernel(const float *__restrict__ partial, int chunks, long long rows, long long H,
                                                                   NormParams np, int training) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const long long j = blockIdx.x * 32ll + (threadIdx.x & 31);
   float s = 0.f, q = 0.f;
   if (training) chunk_sums(partial, chunks, H, j, s, q);
@@ -214,7 +216,7 @@ int norm_forward_stats(Context &ctx, const float *z, long long rows, long long H
       rows_total = rows * hook->world;
     }
   }
-  norm_stats_finalize_kernel<<<static_cast<unsigned>((H + 31) / 32), 256, 0, ctx.stream>>>(sums, chunks, rows_total, H, np, training);
+  launch_dependent(ctx, norm_stats_finalize_kernel, dim3(static_cast<unsigned>((H + 31) / 32)), dim3(256), 0, sums, chunks, rows_total, H, np, training);
   ctx.end(TC_NORM, launches);
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
@@ -299,96 +301,64 @@ __global__ void __launch_bounds__(256) activation_forward_cols_kernel(const floa
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Producers that also write their result as operand panels (see PanelSink): the contraction that reads the tensor next
-// then needs no split pass of its own.  A thread keeps EIGHT columns (one group of the cross panels) and walks rows.
+// Producers that also write their result as operand panels (half_panels.cuh): the contractions that read the tensor next then
+// need no split pass of their own
 // ---------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void write_panels8(const PanelSink &s, long long r, long long c, const float (&v)[8]) {
-  float h[8];
-  uint32_t x[8];
-  split_group(v, s.role_k, 0, h, x);
-  store8(s.hi + r * s.kp + c, h);
-  if (s.cross_k != nullptr) {
-    uint4 *px = reinterpret_cast<uint4 *>(s.cross_k + r * s.kp + c);
-    px[0] = make_uint4(x[0], x[1], x[2], x[3]);
-    px[1] = make_uint4(x[4], x[5], x[6], x[7]);
-  }
-  if (s.cross_mn != nullptr) {
-    // x[0..3] / x[4..7] are the packed lo and hi values of these 8 columns in the order of role_k; the column reading
-    // wants, per 8 source rows, 8 panel rows of lo and 8 of hi (role A) or hi then lo (role B)
-    const uint4 lo4 = s.role_k ? make_uint4(x[4], x[5], x[6], x[7]) : make_uint4(x[0], x[1], x[2], x[3]);
-    const uint4 hi4 = s.role_k ? make_uint4(x[0], x[1], x[2], x[3]) : make_uint4(x[4], x[5], x[6], x[7]);
-    const long long g16 = (r >> 3) * 16 + (r & 7);
-    const long long row_lo = g16 + (s.role_mn ? 8 : 0), row_hi = g16 + (s.role_mn ? 0 : 8);
-    *reinterpret_cast<uint4 *>(s.cross_mn + row_lo * s.kp + c) = lo4;
-    *reinterpret_cast<uint4 *>(s.cross_mn + row_hi * s.kp + c) = hi4;
-  }
-}
-
 template <uint32_t AF>
-__global__ void __launch_bounds__(256) activation_forward_panels_kernel(const float *__restrict__ z, float *__restrict__ out, long long rows,
-                                                                        long long H, const float *__restrict__ col_scale,
-                                                                        const float *__restrict__ col_shift, const uint8_t *__restrict__ mask,
-                                                                        float keep_scale, const PanelSink sink) {
-  const long long c = (blockIdx.x * 256ll + threadIdx.x) * 8;
-  if (c >= H) return;
-  const bool affine = col_scale != nullptr;
-  float cs[8], ch[8];
+struct ActivationProducer {
+  const float *z;
+  float *out;
+  long long H;
+  const float *col_scale, *col_shift;
+  const uint8_t *mask;
+  float keep_scale;
+  bool vec;
+  struct Cols { float cs[8], ch[8], f[8]; };
+  __device__ __forceinline__ void columns(Cols &k, long long c, int n) const {
 #pragma unroll
-  for (int k = 0; k < 8; ++k) { cs[k] = affine ? col_scale[c + k] : 1.f; ch[k] = affine ? col_shift[c + k] : 0.f; }
-  const bool masked = mask != nullptr;
-  const unsigned long long keep = masked ? *reinterpret_cast<const unsigned long long *>(mask + c) : ~0ull;
-  const bool scale = masked || keep_scale != 1.0f;
-  for (long long r0 = blockIdx.y * 2ll; r0 < rows; r0 += gridDim.y * 2ll) {
-    float v[2][8];
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-      if (r0 + u < rows) load8(v[u], z + (r0 + u) * H + c);
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      if (r0 + u >= rows) break;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        float y = af_fire(AF, affine ? v[u][k] * cs[k] + ch[k] : v[u][k]);
-        if (scale) y *= keep_scale;
-        if (((keep >> (8 * k)) & 0xFFull) == 0ull) y = 0.f;
-        v[u][k] = y;
-      }
-      store8(out + (r0 + u) * H + c, v[u]);
-      write_panels8(sink, r0 + u, c, v[u]);
+    for (int j = 0; j < 8; ++j) {
+      k.cs[j] = col_scale != nullptr && j < n ? col_scale[c + j] : 1.f;
+      k.ch[j] = col_scale != nullptr && j < n ? col_shift[c + j] : 0.f;
+      k.f[j] = mask != nullptr && j < n && mask[c + j] == 0 ? 0.f : keep_scale;
     }
   }
-}
-
-__global__ void __launch_bounds__(256) norm_backward_apply_panels_kernel(const float *__restrict__ z, const float *__restrict__ delta,
-                                                                         float *__restrict__ out, long long rows, long long H,
-                                                                         const float *__restrict__ mean, const float *__restrict__ coef,
-                                                                         const PanelSink sink) {
-  const long long c = (blockIdx.x * 256ll + threadIdx.x) * 8;
-  if (c >= H) return;
-  float mu[8], k0[8], k1[8], k2[8];
-  load8(mu, mean + c); load8(k0, coef + c); load8(k1, coef + H + c); load8(k2, coef + 2 * H + c);
-  for (long long r0 = blockIdx.y * 2ll; r0 < rows; r0 += gridDim.y * 2ll) {
-    float t[2][8], u[2][8];
+  __device__ __forceinline__ void row(const Cols &k, long long r, long long c, int n, float (&v)[8]) const {
+    ld8(v, z + r * H + c, n, vec);
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-      if (r0 + i < rows) { load8(t[i], z + (r0 + i) * H + c); load8(u[i], delta + (r0 + i) * H + c); }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      if (r0 + i >= rows) break;
-      float d[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) d[k] = u[i][k] * k0[k] + (t[i][k] - mu[k]) * k1[k] + k2[k];
-      store8(out + (r0 + i) * H + c, d);
-      write_panels8(sink, r0 + i, c, d);
+    for (int j = 0; j < 8; ++j) {
+      const float y = af_fire(AF, v[j] * k.cs[j] + k.ch[j]);
+      v[j] = j < n && k.f[j] != 0.f ? y * k.f[j] : 0.f;
     }
   }
-}
+  __device__ __forceinline__ void keep(long long r, long long c, int n, const float (&v)[8]) const { st8(out + r * H + c, v, n, vec); }
+};
 
-static dim3 column_walk_grid8(long long rows, long long H) {
-  const unsigned gx = static_cast<unsigned>((H / 8 + 255) / 256);
-  const long long walkers = std::max<long long>(1, (148 * 8) / gx);
-  return dim3(gx, static_cast<unsigned>(std::max<long long>(1, std::min<long long>((rows + 1) / 2, walkers))));
-}
+// error = delta * k0 + (z - mean) * k1 + k2
+struct NormBackwardProducer {
+  const float *z, *delta;
+  float *out;
+  long long H;
+  const float *mean, *coef;
+  bool vec;
+  struct Cols { float mu[8], k0[8], k1[8], k2[8]; };
+  __device__ __forceinline__ void columns(Cols &k, long long c, int n) const {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      k.mu[j] = j < n ? mean[c + j] : 0.f;
+      k.k0[j] = j < n ? coef[c + j] : 0.f;
+      k.k1[j] = j < n ? coef[H + c + j] : 0.f;
+      k.k2[j] = j < n ? coef[2 * H + c + j] : 0.f;
+    }
+  }
+  __device__ __forceinline__ void row(const Cols &k, long long r, long long c, int n, float (&v)[8]) const {
+    float t[8];
+    ld8(t, z + r * H + c, n, vec);
+    ld8(v, delta + r * H + c, n, vec);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = v[j] * k.k0[j] + (t[j] - k.mu[j]) * k.k1[j] + k.k2[j];
+  }
+  __device__ __forceinline__ void keep(long long r, long long c, int n, const float (&v)[8]) const { st8(out + r * H + c, v, n, vec); }
+};
 
 static dim3 column_walk_grid(long long rows, long long H) {
   const unsigned gx = static_cast<unsigned>((H / 4 + 255) / 256);
@@ -405,14 +375,13 @@ bool activation_writes_panels(uint32_t af) {
 }
 
 int activation_forward(Context &ctx, const float *z, float *out, long long rows, long long H, uint32_t af, const float *col_scale,
-                       const float *col_shift, const uint8_t *mask, float keep_scale, const PanelSink *sink) {
+                       const float *col_shift, const uint8_t *mask, float keep_scale, const HalfPanels *sink) {
   ctx.begin(TC_ELEMENTWISE);
   const bool vec4 = (H % 4 == 0) && ((reinterpret_cast<uintptr_t>(z) & 15) == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0) &&
                     ((reinterpret_cast<uintptr_t>(col_scale) & 15) == 0) && ((reinterpret_cast<uintptr_t>(col_shift) & 15) == 0);
   if (sink != nullptr) {
-    if (!vec4 || (H & 7) != 0 || (rows & 7) != 0) return MYEA_E_INVALID;
-    const dim3 grid = column_walk_grid8(rows, H);
-#define MYEA_AF_CASE(A) case A: activation_forward_panels_kernel<A><<<grid, 256, 0, ctx.stream>>>(z, out, rows, H, col_scale, col_shift, mask, keep_scale, *sink); break
+    cudaError_t err;
+#define MYEA_AF_CASE(A) case A: err = half_produce(ctx, ActivationProducer<A>{z, out, H, col_scale, col_shift, mask, keep_scale, vec4}, *sink); break
     switch (af) {
       MYEA_AF_CASE(MYEA_AF_TANH);
       MYEA_AF_CASE(MYEA_AF_SIGMOID);
@@ -420,12 +389,12 @@ int activation_forward(Context &ctx, const float *z, float *out, long long rows,
       MYEA_AF_CASE(MYEA_AF_LEAKY_RELU);
       MYEA_AF_CASE(MYEA_AF_ELU);
       MYEA_AF_CASE(MYEA_AF_SELU);
-      case MYEA_AF_LINEAR: activation_forward_panels_kernel<MYEA_AF_LINEAR><<<grid, 256, 0, ctx.stream>>>(z, out, rows, H, col_scale, col_shift, mask, keep_scale, *sink); break;
+      MYEA_AF_CASE(MYEA_AF_LINEAR);
       default: return MYEA_E_INVALID;  // activation_writes_panels(af) is false: the caller asks for plain arrays
     }
 #undef MYEA_AF_CASE
     ctx.end(TC_ELEMENTWISE);
-    return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
+    return err == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
   }
   const long long total = rows * (vec4 ? H / 4 : H);
   const int blocks = static_cast<int>(std::max<long long>(1, std::min<long long>((total + 255) / 256, 148 * 16)));
@@ -652,6 +621,8 @@ __device__ __forceinline__ void norm_backward_coefficients(const NormParams &np,
 // (the derivative buffers are summed over ranks later), d_mean / d_sigma and `rows` are those of the whole batch.
 __global__ void __launch_bounds__(256) norm_backward_finalize_kernel(const float *__restrict__ partial, int chunks, const float *__restrict__ global,
                                                                      long long rows, long long H, NormParams np, float *__restrict__ coef) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const long long j = blockIdx.x * 32ll + (threadIdx.x & 31);
   float s1, s2;
   chunk_sums(partial, chunks, H, j, s1, s2);
@@ -759,7 +730,7 @@ __global__ void __launch_bounds__(256) norm_backward_strip_kernel(const float *_
 }
 
 int norm_backward(Context &ctx, const float *z, const float *delta_af, float *delta_out, long long rows, long long H,
-                  const NormParams &np, const SumHook *hook, int fused_chunks, const PanelSink *sink) {
+                  const NormParams &np, const SumHook *hook, int fused_chunks, const HalfPanels *sink) {
   ctx.begin(TC_NORM);
   if (fused_chunks <= 0 && sink == nullptr && norm_strip_suits(rows, hook)) {
     const dim3 grid(static_cast<unsigned>((H + 7) / 8));
@@ -786,15 +757,14 @@ int norm_backward(Context &ctx, const float *z, const float *delta_af, float *de
     global = g;
     rows_total = rows * hook->world;
   }
-  norm_backward_finalize_kernel<<<static_cast<unsigned>((H + 31) / 32), 256, 0, ctx.stream>>>(np.partial, chunks, global, rows_total, H, np, coef);
+  launch_dependent(ctx, norm_backward_finalize_kernel, dim3(static_cast<unsigned>((H + 31) / 32)), dim3(256), 0, static_cast<const float *>(np.partial), chunks, global, rows_total, H, np, coef);
   const bool vec4 = (H % 4 == 0) && ((reinterpret_cast<uintptr_t>(z) & 15) == 0) && ((reinterpret_cast<uintptr_t>(delta_af) & 15) == 0) &&
                     ((reinterpret_cast<uintptr_t>(delta_out) & 15) == 0);
   const long long total = rows * (vec4 ? H / 4 : H);
   const int blocks = static_cast<int>(std::max<long long>(1, std::min<long long>((total + 255) / 256, 148 * 16)));
   const bool cols_ok = vec4 && (reinterpret_cast<uintptr_t>(np.mean) & 15) == 0 && (reinterpret_cast<uintptr_t>(coef) & 15) == 0;
-  if (sink != nullptr && !(cols_ok && (H & 7) == 0 && (rows & 7) == 0)) return MYEA_E_INVALID;
   if (sink != nullptr)
-    norm_backward_apply_panels_kernel<<<column_walk_grid8(rows, H), 256, 0, ctx.stream>>>(z, delta_af, delta_out, rows, H, np.mean, coef, *sink);
+    half_produce(ctx, NormBackwardProducer{z, delta_af, delta_out, H, np.mean, coef, vec4}, *sink);
   else if (cols_ok)
     norm_backward_apply_cols_kernel<<<column_walk_grid(rows, H), 256, 0, ctx.stream>>>(z, delta_af, delta_out, rows, H, np.mean, coef);
   else if (vec4)

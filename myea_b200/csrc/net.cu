@@ -290,13 +290,12 @@ static int allocate_buffers(myea_b200_net *net) {
       RC(dev_alloc(net, &L.deriv, rows * wide));
       if (L.has_norm) RC(dev_alloc(net, &L.errors, rows * L.n_out));
       else L.errors = L.deriv;
-      if (gemm_takes_mn_major(net->ctx, rows, L.n_out) &&
-          gemm_takes_mn_major(net->ctx, rows, L.n_in) && gemm_takes_mn_major(net->ctx, L.n_out, L.n_in) && net->ctx.gemm_engine == 0 &&
-          !direct_gemm_suits(net->ctx, rows, L.n_out, L.n_in)) {
+      if (net->ctx.gemm_engine == 0 && !direct_gemm_suits(net->ctx, rows, L.n_out, L.n_in)) {
         L.shared_panels = true;
-        RC(dev_alloc(net, &L.in_panel_mem, shared_panel_floats(rows, L.n_in)));
-        RC(dev_alloc(net, &L.w_panel_mem, shared_panel_floats(L.n_out, L.n_in)));
-        RC(dev_alloc(net, &L.d_panel_mem, shared_panel_floats(rows, L.n_out)));
+        RC(dev_alloc(net, &L.in_panel_mem, half_panel_floats(rows, L.n_in), false));
+        RC(dev_alloc(net, &L.w_panel_mem, half_panel_floats(L.n_out, L.n_in), false));
+        RC(dev_alloc(net, &L.d_panel_mem, half_panel_floats(rows, L.n_out), false));
+        L.w_pan = half_panels_at(L.w_panel_mem, L.n_out, L.n_in);
       }
       scratch = std::max(scratch, gemm_scratch_floats(rows, L.n_out, L.n_in));   // forward
       scratch = std::max(scratch, gemm_scratch_floats(rows, L.n_in, L.n_out));   // backward data
@@ -535,20 +534,33 @@ namespace myea {
 
 // One fully connected layer on `rows` rows: z = x W^T (+ b); normalization statistics; activation; dropout.
 // Forward_Pass__FC (Neural_Network__Forward_Pass__Loop.cpp:350-790 is the per-layer driver).
-// (a short last batch may fall below the 256 x 256 kernel's shapes: then the layer goes the per-contraction way)
+// (a short last batch may be small enough for the products that need no panels)
 static bool fc_uses_shared_panels(const myea_b200_net *net, const LayerPlan &L, long long rows) {
-  return L.shared_panels && gemm_takes_mn_major(net->ctx, rows, L.n_out) && gemm_takes_mn_major(net->ctx, rows, L.n_in);
+  return L.shared_panels && !direct_gemm_suits(net->ctx, rows, L.n_out, L.n_in);
 }
 
 // The weight panels of a layer depend on no activation: a forward pass whose inputs come from the host makes them all
 // while the inputs are still on their way (see forward_impl).
 static int fc_prepare_weights(myea_b200_net *net, LayerPlan &L) {
-  const bool tr = net->training;
   RC(comm_wait_gathers(net, L.idx.first_connection_index, L.idx.last_connection_index - L.idx.first_connection_index));
-  RC(gemm_prepare_shared(net->ctx, net->params + L.idx.first_connection_index, L.n_in, L.n_out, L.n_in, L.w_panel_mem, PANEL_ROLE_B, &L.w_rows,
-                         PANEL_ROLE_B, tr ? &L.w_cols : nullptr));
+  RC(half_split(net->ctx, net->params + L.idx.first_connection_index, L.n_in, L.w_pan));
   L.w_prepared = true;
   return MYEA_OK;
+}
+
+HalfPanels *fc_input_sink(myea_b200_net *net, LayerPlan &L, const float *input, long long rows) {
+  if (L.type != MYEA_LAYER_FULLY_CONNECTED || !fc_uses_shared_panels(net, L, rows)) return nullptr;
+  L.in_pan = half_panels_at(L.in_panel_mem, rows, L.n_in);
+  L.in_ready_src = input;
+  L.in_ready_rows = rows;
+  return &L.in_pan;
+}
+
+HalfPanels *fc_error_sink(myea_b200_net *net, LayerPlan &L, long long rows) {
+  if (!L.shared_panels || !L.in_valid || !fc_uses_shared_panels(net, L, rows)) return nullptr;
+  L.d_pan = half_panels_at(L.d_panel_mem, rows, L.n_out);
+  L.d_valid = true;
+  return &L.d_pan;
 }
 
 int fc_product_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long rows, const Epilogue &e) {
@@ -556,12 +568,10 @@ int fc_product_forward(myea_b200_net *net, LayerPlan &L, const float *input, lon
   // the other ranks' slices of this layer's updated weights (a sharded update gathers them layer by layer)
   RC(comm_wait_gathers(net, L.idx.first_connection_index, L.idx.last_connection_index - L.idx.first_connection_index));
   if (fc_uses_shared_panels(net, L, rows)) {
-    // while training, the same pass also writes the column readings the backward contractions will want
     const bool tr = net->training;
-    if (L.in_ready_src == input && L.in_ready_rows == rows) {
-      // the kernel that produced `input` has written these panels already (fc_forward of the layer before)
-    } else {
-      RC(gemm_prepare_shared(net->ctx, input, L.n_in, rows, L.n_in, L.in_panel_mem, PANEL_ROLE_A, &L.in_rows, PANEL_ROLE_B, tr ? &L.in_cols : nullptr));
+    if (!(L.in_ready_src == input && L.in_ready_rows == rows)) {  // else the kernel that produced `input` has written these panels already
+      L.in_pan = half_panels_at(L.in_panel_mem, rows, L.n_in);
+      RC(half_split(net->ctx, input, L.n_in, L.in_pan));
     }
     L.in_ready_src = nullptr;
     if (!L.w_prepared) RC(fc_prepare_weights(net, L));
@@ -569,7 +579,7 @@ int fc_product_forward(myea_b200_net *net, LayerPlan &L, const float *input, lon
     L.in_valid = L.w_valid = tr;
     L.in_src = input;
     L.d_valid = false;
-    return gemm_panels(net->ctx, L.in_rows, 0, rows, L.w_rows, 0, L.n_out, e);
+    return half_gemm(net->ctx, half_rows(L.in_pan), half_rows(L.w_pan), e);
   }
   L.in_valid = L.w_valid = L.d_valid = false;
   Operand a{input, rows, L.n_in, L.n_in, 1};
@@ -588,10 +598,12 @@ static bool fc_runs_direct(const myea_b200_net *net, const LayerPlan &L, long lo
 
 int fc_product_backward(myea_b200_net *net, LayerPlan &N, long long rows, const Epilogue &e) {
   if (N.shared_panels && N.w_valid) {
-    if (!N.d_valid)  // (the normalization backward of N may have written them already)
-      RC(gemm_prepare_shared(net->ctx, N.errors, N.n_out, rows, N.n_out, N.d_panel_mem, PANEL_ROLE_A, &N.d_rows, PANEL_ROLE_A, &N.d_cols));
+    if (!N.d_valid) {  // (the kernel that produced N's errors may have written them already)
+      N.d_pan = half_panels_at(N.d_panel_mem, rows, N.n_out);
+      RC(half_split(net->ctx, N.errors, N.n_out, N.d_pan));
+    }
     N.d_valid = true;
-    return gemm_panels(net->ctx, N.d_rows, 0, rows, N.w_cols, 0, N.n_in, e);
+    return half_gemm(net->ctx, half_rows(N.d_pan), half_cols(N.w_pan), e);
   }
   Operand a{N.errors, rows, N.n_out, N.n_out, 1};
   Operand b{net->params + N.idx.first_connection_index, N.n_in, N.n_out, 1, N.n_in};  // W[out,in] read as [in rows, K=out]
@@ -648,17 +660,13 @@ int fc_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long r
   RC(fc_product_forward(net, L, input, rows, e));
   const size_t li = static_cast<size_t>(&L - net->layers.data());
   // the layer that reads this one's output from shared operand panels gets them from the activation kernel
-  PanelSink sink;
-  bool use_sink = false;
-  if (li + 1 < net->layers.size() && !timewise_norm && activation_writes_panels(L.desc.type_activation_function) && (rows & 7) == 0 && (L.n_out & 7) == 0 &&
-      net->ctx.gemm_engine == 0) {
-    LayerPlan &N = net->layers[li + 1];
-    if (N.type == MYEA_LAYER_FULLY_CONNECTED && N.input_layer == static_cast<int>(li) && fc_uses_shared_panels(net, N, rows)) {
-      shared_panel_layout(N.in_panel_mem, rows, N.n_in, PANEL_ROLE_A, &N.in_rows, PANEL_ROLE_B, net->training ? &N.in_cols : nullptr, &sink);
-      N.in_ready_src = L.values;
-      N.in_ready_rows = rows;
-      use_sink = true;
-    }
+  const HalfPanels *sink = nullptr;
+  const bool masks_per_step = drop_mask != nullptr && net->T > 1;  // one activation pass per time step
+  if (!timewise_norm && !masks_per_step && activation_writes_panels(L.desc.type_activation_function)) {
+    // (behind a layer the next one may be a residual block, whose first layer reads this output)
+    size_t reader = li + 1;
+    if (reader < net->layers.size() && net->layers[reader].type == MYEA_LAYER_RESIDUAL) ++reader;
+    if (reader < net->layers.size() && net->layers[reader].input_layer == static_cast<int>(li)) sink = fc_input_sink(net, net->layers[reader], L.values, rows);
   }
   if (L.ind_rnn) {
     // the recurrence runs step by step on the summations of all steps (one contraction above): per step the statistics of
@@ -724,18 +732,13 @@ int fc_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long r
   if (mask != nullptr && net->T > 1) {
     // a recurrent network draws one mask per time step (mask[t][unit], Forward_Pass__Dropout__Bernoulli__Training__Loop,
     // Neural_Network__Forward_Pass__Loop.cpp:4947-4970): one activation pass per step, each with its own mask row
-    if (use_sink) net->layers[li + 1].in_ready_src = nullptr;
     const long long step_rows = rows / net->T;
     for (long long t = 0; t < net->T; ++t)
       RC(activation_forward(net->ctx, L.summations + t * step_rows * L.n_out, L.values + t * step_rows * L.n_out, step_rows, L.n_out,
                             L.desc.type_activation_function, cs, ch, mask + t * L.n_out, scale, nullptr));
     return MYEA_OK;
   }
-  if (use_sink && ((reinterpret_cast<uintptr_t>(cs) | reinterpret_cast<uintptr_t>(ch)) & 15) != 0) {  // unaligned coefficients: the plain kernel, and the reader splits
-    use_sink = false;
-    net->layers[li + 1].in_ready_src = nullptr;
-  }
-  RC(activation_forward(net->ctx, L.summations, L.values, rows, L.n_out, L.desc.type_activation_function, cs, ch, mask, scale, use_sink ? &sink : nullptr));
+  RC(activation_forward(net->ctx, L.summations, L.values, rows, L.n_out, L.desc.type_activation_function, cs, ch, mask, scale, sink));
   return MYEA_OK;
 }
 
@@ -1054,18 +1057,9 @@ int fc_finish_backward(myea_b200_net *net, LayerPlan &L, long long rows) {
   if (!L.has_norm) return MYEA_OK;
   // the layer's errors are read next by the error propagation below it (rows) and by its weight derivative (columns),
   // both from shared operand panels: the kernel that writes the errors writes those panels as well
-  PanelSink sink;
-  // (the panel-writing kernel reads the layer's statistics eight columns at a time: they lie behind those of the
-  // normalized layers before this one, whose unit counts need not be multiples of four - then the plain kernel runs and
-  // the readers of the errors split them themselves, as the forward pass does with unaligned coefficients)
-  const uintptr_t stat_bits = reinterpret_cast<uintptr_t>(L.norm.mean) | reinterpret_cast<uintptr_t>(L.norm.partial) |
-                              reinterpret_cast<uintptr_t>(L.summations) | reinterpret_cast<uintptr_t>(L.deriv) | reinterpret_cast<uintptr_t>(L.errors);
-  const bool use_sink = L.shared_panels && L.in_valid && net->ctx.gemm_engine == 0 && (rows & 7) == 0 && (L.n_out & 7) == 0 && (stat_bits & 15) == 0 &&
-                        gemm_takes_mn_major(net->ctx, rows, L.n_out) && gemm_takes_mn_major(net->ctx, rows, L.n_in);
-  if (use_sink) shared_panel_layout(L.d_panel_mem, rows, L.n_out, PANEL_ROLE_A, &L.d_rows, PANEL_ROLE_A, &L.d_cols, &sink);
-  RC(norm_backward(net->ctx, L.summations, L.deriv, L.errors, rows, L.n_out, L.norm, &net->hook, L.bwd_fused_chunks, use_sink ? &sink : nullptr));
+  const HalfPanels *sink = fc_error_sink(net, L, rows);
+  RC(norm_backward(net->ctx, L.summations, L.deriv, L.errors, rows, L.n_out, L.norm, &net->hook, L.bwd_fused_chunks, sink));
   L.bwd_fused_chunks = 0;
-  if (use_sink) L.d_valid = true;
   return MYEA_OK;
 }
 
@@ -1206,10 +1200,11 @@ int fc_update_derivative_weight(myea_b200_net *net, LayerPlan &L, const float *i
     return direct_gemm(net->ctx, &item, 1);
   }
   if (L.shared_panels && L.in_valid && input == L.in_src) {
-    if (!L.d_valid) {  // no error propagation below this layer (first hidden layer): only the column reading is needed
-      RC(gemm_prepare_shared(net->ctx, L.errors, L.n_out, rows, L.n_out, L.d_panel_mem, PANEL_ROLE_A, nullptr, PANEL_ROLE_A, &L.d_cols));
+    if (!L.d_valid) {  // no error propagation below this layer (first hidden layer)
+      L.d_pan = half_panels_at(L.d_panel_mem, rows, L.n_out);
+      RC(half_split(net->ctx, L.errors, L.n_out, L.d_pan));
     }
-    RC(gemm_panels(net->ctx, L.d_cols, 0, L.n_out, L.in_cols, 0, L.n_in, e));
+    RC(half_gemm(net->ctx, half_cols(L.d_pan), half_cols(L.in_pan), e));
     L.d_valid = false;  // the errors of the next step will differ
   } else {
     RC(gemm_nt(net->ctx, a, b, e, net->scratch));

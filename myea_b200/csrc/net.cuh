@@ -36,13 +36,12 @@ struct LayerPlan {
   uint8_t *shake_mask = nullptr;      // [B]
   float *shake_alpha = nullptr, *shake_beta = nullptr;  // [B, n_out]
   long long norm_unit_offset = 0;     // units of earlier layers in the normalized-unit run
-  // Operand panels shared by the three contractions of a large fully connected layer (all on the 256 x 256 kernel):
-  // one split pass per tensor and step serves both of its readings.  input: forward (rows, role A) and dW (columns,
-  // role B); weights: forward (rows, role B) and error propagation (columns, role B); errors: error propagation
-  // (rows, role A) and dW (columns, role A).
+  // Operand panels shared by the three contractions of a large fully connected layer: one set per tensor and step serves
+  // both of its readings.  input: forward (rows) and dW (columns); weights: forward (rows) and error propagation (columns);
+  // errors: error propagation (rows) and dW (columns).
   bool shared_panels = false;
   float *in_panel_mem = nullptr, *w_panel_mem = nullptr, *d_panel_mem = nullptr;
-  Panels in_rows, in_cols, w_rows, w_cols, d_rows, d_cols;
+  HalfPanels in_pan, w_pan, d_pan;  // as of the step in flight (a short batch has fewer rows)
   bool in_valid = false, w_valid = false, d_valid = false;
   bool w_prepared = false;  // the weight panels have already been made in this forward pass (hoisted under the input copy)
   const float *in_src = nullptr;  // the array the input panels were made from
@@ -80,6 +79,10 @@ int pooling_backward(myea_b200_net *net, LayerPlan &L, float *d_input, long long
 
 // z = input * W^T of a fully connected layer and D = errors * W (error on the layer's inputs), from the layer's shared
 // operand panels when it has them, else through gemm_nt; `e` carries destination and fused extras (net.cu)
+// Where a kernel that produces the input of layer L (the array `input`), or the errors of layer L, leaves the operand panels
+// its contractions will read; null when the layer reads none.  The panels count as made from then on.
+HalfPanels *fc_input_sink(myea_b200_net *net, LayerPlan &L, const float *input, long long rows);
+HalfPanels *fc_error_sink(myea_b200_net *net, LayerPlan &L, long long rows);
 int fc_product_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long rows, const Epilogue &e);
 int fc_product_backward(myea_b200_net *net, LayerPlan &N, long long rows, const Epilogue &e);
 

@@ -17,6 +17,7 @@
 // masked rows, to s_D; layer k > 1 sends W_k^T delta_k through f_k' and the normalization backward to s_{k-1}; the layer
 // feeding the block receives skip error + W_1^T delta_1, with its own activation derivative fused when it is a fully
 // connected layer.  ShakeDrop's alpha, beta and row mask are inputs (the reference draws them on the fly).
+#include "half_panels.cuh"
 #include "net.cuh"
 
 #include <algorithm>
@@ -99,10 +100,49 @@ __global__ void __launch_bounds__(256) shakedrop_pad_backward_kernel(const float
   }
 }
 
+// the same as producers of operand panels: forward for the layer that reads the block's output next, backward for the
+// block's last layer
+struct ShakeDropProducer {
+  const float *x, *s;
+  float *out;
+  const uint8_t *mask;
+  const float *coef;
+  float scale;
+  long long H;
+  bool vec;
+  struct Cols {};
+  __device__ __forceinline__ void columns(Cols &, long long, int) const {}
+  __device__ __forceinline__ void row(const Cols &, long long r, long long c, int n, float (&v)[8]) const {
+    ld8(v, s + r * H + c, n, vec);
+    if (mask != nullptr && mask[r] != 0) {
+      float w[8];
+      ld8(w, coef + r * H + c, n, vec);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] *= w[j];
+    }
+    if (scale != 1.0f) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] *= scale;
+    }
+    if (x != nullptr) {
+      float u[8];
+      ld8(u, x + r * H + c, n, vec);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] += u[j];
+    }
+  }
+  __device__ __forceinline__ void keep(long long r, long long c, int n, const float (&v)[8]) const { st8(out + r * H + c, v, n, vec); }
+};
+
 static int launch_shakedrop(Context &ctx, const float *x, const float *s, float *out, const uint8_t *mask, const float *coef, float scale,
-                            long long rows, long long H) {
+                            long long rows, long long H, const HalfPanels *sink = nullptr) {
   ctx.begin(TC_ELEMENTWISE);
   const bool vec4 = (H % 4 == 0);
+  if (sink != nullptr) {
+    half_produce(ctx, ShakeDropProducer{x, s, out, mask, coef, scale, H, vec4}, *sink);
+    ctx.end(TC_ELEMENTWISE);
+    return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
+  }
   const long long total = rows * (vec4 ? H / 4 : H);
   const int blocks = static_cast<int>(std::max<long long>(1, std::min<long long>((total + 255) / 256, 148 * 16)));
   if (vec4) shakedrop_kernel<4><<<blocks, 256, 0, ctx.stream>>>(x, s, out, mask, coef, scale, rows, H);
@@ -153,7 +193,8 @@ int residual_forward(myea_b200_net *net, int r) {
           cs = L.norm.col_scale;
           ch = L.norm.col_shift;
         }
-        RRC(activation_forward(ctx, prev, L.values, rows, L.n_in, L.desc.type_activation_function, cs, ch, mask, scale));
+        const HalfPanels *sink = activation_writes_panels(L.desc.type_activation_function) ? fc_input_sink(net, L, L.values, rows) : nullptr;
+        RRC(activation_forward(ctx, prev, L.values, rows, L.n_in, L.desc.type_activation_function, cs, ch, mask, scale, sink));
       }
       in = L.values;
     }
@@ -176,7 +217,12 @@ int residual_forward(myea_b200_net *net, int r) {
     RRC(activation_forward(ctx, last.summations, R.summations, rows, W, MYEA_AF_LINEAR, R.norm.col_scale, R.norm.col_shift, nullptr, 1.f));
     s = R.summations;
   }
-  if (A == W) return launch_shakedrop(ctx, x, s, R.values, mask, R.shake_alpha, scale, rows, R.n_out);
+  if (A == W) {
+    size_t reader = static_cast<size_t>(r + R.block_depth + 1);
+    if (reader < net->layers.size() && net->layers[reader].type == MYEA_LAYER_RESIDUAL) ++reader;
+    const HalfPanels *sink = reader < net->layers.size() && net->layers[reader].input_layer == r ? fc_input_sink(net, net->layers[reader], R.values, rows) : nullptr;
+    return launch_shakedrop(ctx, x, s, R.values, mask, R.shake_alpha, scale, rows, R.n_out, sink);
+  }
   const long long pad = residual_padding(A, W);
   ctx.begin(TC_ELEMENTWISE);
   const long long total = rows * R.n_out;
@@ -201,7 +247,8 @@ int residual_backward(myea_b200_net *net, int r) {
     const long long A = R.n_in, W = last.n_out;
     float *dst = R.has_norm ? R.summations : last.errors;  // R.summations: the normalized copy is not needed any more
     if (A == W) {
-      RRC(launch_shakedrop(ctx, nullptr, R.deriv, dst, shake ? R.shake_mask : nullptr, R.shake_beta, 1.0f, rows, R.n_out));
+      RRC(launch_shakedrop(ctx, nullptr, R.deriv, dst, shake ? R.shake_mask : nullptr, R.shake_beta, 1.0f, rows, R.n_out,
+                           R.has_norm ? nullptr : fc_error_sink(net, last, rows)));
     } else {
       ctx.begin(TC_ELEMENTWISE);
       const long long total = rows * W;
@@ -210,7 +257,7 @@ int residual_backward(myea_b200_net *net, int r) {
                                                                     R.shake_beta, rows);
       ctx.end(TC_ELEMENTWISE);
     }
-    if (R.has_norm) RRC(norm_backward(ctx, last.summations, dst, last.errors, rows, W, R.norm, &net->hook));
+    if (R.has_norm) RRC(norm_backward(ctx, last.summations, dst, last.errors, rows, W, R.norm, &net->hook, 0, fc_error_sink(net, last, rows)));
   }
   for (int k = R.block_depth; k > 1; --k) {
     LayerPlan &L = net->layers[r + k];
@@ -224,7 +271,7 @@ int residual_backward(myea_b200_net *net, int r) {
     e.ld_aux = L.n_in;
     if (L.has_norm) { e.col_scale = L.norm.col_scale; e.col_shift = L.norm.col_shift; }
     RRC(fc_product_backward(net, L, rows, e));
-    if (L.has_norm) RRC(norm_backward(ctx, below.summations, L.deriv, below.errors, rows, L.n_in, L.norm, &net->hook));
+    if (L.has_norm) RRC(norm_backward(ctx, below.summations, L.deriv, below.errors, rows, L.n_in, L.norm, &net->hook, 0, fc_error_sink(net, below, rows)));
   }
   // the layer feeding the block: skip error + W_1^T delta_1, then its own activation derivative / normalization
   LayerPlan &first = net->layers[r + 1];

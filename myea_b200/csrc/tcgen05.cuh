@@ -319,5 +319,9 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int m, int n, bool a_mn =
   return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn ? (1u << 15) : 0u) | (b_mn ? (1u << 16) : 0u) | (static_cast<uint32_t>(n >> 3) << 17) |
          (static_cast<uint32_t>(m >> 4) << 24);
 }
+// the same with half inputs (format 0)
+__host__ __device__ constexpr uint32_t make_idesc_f16(int m, int n, bool a_mn = false, bool b_mn = false) {
+  return (1u << 4) | (a_mn ? (1u << 15) : 0u) | (b_mn ? (1u << 16) : 0u) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
+}
 
 }  // namespace myea
