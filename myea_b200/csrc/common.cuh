@@ -31,8 +31,8 @@ struct Context {
   double gemm_flops = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::string error;
-  int gemm_engine = 0;  // 0 = tcgen05 3xTF32, 1 = FP32 FMA
-  int gemm_bn = 0;      // forced N tile of the tcgen05 kernel (0 = heuristic)
+  int gemm_engine = 0;  // 0 = tcgen05 split precision, 1 = FP32 FMA
+  int gemm_bn = 0;      // kernel-level tests: not 0 = operand panels whatever the size, 4 = the same with tiles never split along K
   bool dependent_launch = true;  // programmatic dependent launch for the kernels that support it
   float *sk_ws = nullptr;               // partial sums of tiles split along K (gemm_splitk_reserve)
   unsigned int *sk_counters = nullptr;  // arrival counters of those tiles, all zero between launches
@@ -224,62 +224,14 @@ struct Operand {
   const float *ptr = nullptr;
   long long rows = 0, k = 0;
   long long stride_r = 0, stride_k = 0;
-  const float *lo = nullptr;  // optional second addend with the same strides (value = ptr[..] + lo[..]); FMA engine only
 };
 
-// K-major hi / lo panels of one operand, pitch kp floats (a multiple of 32): what the tensor-core kernel reads with TMA.
-// `hi`: TF32-rounded values in fp32 containers.  `lo`: the CROSS panel, per 8 K elements 16 bf16 = [lo x8 | hi x8] for the
-// left operand (role A) and [hi x8 | lo x8] for the right operand (role B), so that one K = 16 BF16 MMA of an A group with
-// a B group yields lo_a*hi_b + hi_a*lo_b.
-enum { PANEL_ROLE_A = 0, PANEL_ROLE_B = 1 };
-// An MN-major panel set (major == PANEL_MN) describes the operand TRANSPOSED: the arrays are [k][kp] (hi, fp32) and
-// [2 * round_up(k, 8)][kp] (cross, bf16; per 8 K rows 16 panel rows, lo rows / hi rows ordered by role), the operand's
-// `rows` run along the contiguous axis.  Only the 256 x 256 kernel reads this form; it needs kp to be a multiple of 64.
-enum { PANEL_K = 0, PANEL_MN = 1 };
-struct Panels {
-  float *hi = nullptr, *lo = nullptr;
-  long long rows = 0, k = 0, kp = 0;
-  int role = PANEL_ROLE_A;
-  int major = PANEL_K;
-};
-
-struct GemmScratch {   // hi/lo K-major panels of both operands, reused by every contraction of a handle
+struct GemmScratch {   // operand panels of contractions that have none of their own, and other working memory of a handle
   float *base = nullptr;
   size_t floats = 0;
 };
 
 size_t gemm_scratch_floats(long long M, long long N, long long K);
-size_t panel_floats(long long rows, long long k);
-Panels panels_at(float *mem, long long rows, long long k, int role);
-int gemm_prepare(Context &ctx, const Operand &op, float *mem, Panels *out, int role);
-int gemm_prepare_into(Context &ctx, const Operand &op, const Panels &dst, long long row_offset, long long k_offset);
-// The same with the source rows landing on every `row_step`-th panel row starting at row_offset (interleaving several
-// matrices row by row into one panel set); K-major sources only.
-int gemm_prepare_interleaved(Context &ctx, const Operand &op, const Panels &dst, long long row_offset, long long row_step);
-int gemm_panels(Context &ctx, const Panels &A, long long a_row0, long long M, const Panels &B, long long b_row0, long long N,
-                const Epilogue &epi);
-// TMA descriptor of a K-major panel [rows][kp] (hi, or cross seen as 32-bit words): boxes of 32 floats of K x box_rows
-// rows, 128-byte swizzle; K ends at round_up(k, 8) and rows at `rows` (the hardware fills the rest of a box with zeros)
-bool make_panel_map(CUtensorMap *map, const float *panel, long long rows, long long k, long long kp, int box_rows);
-// One pass over a row-major source S[R][C] that serves BOTH readings of it: `as_rows` is the K-major operand
-// (rows = R, K = C) and `as_cols` the MN-major operand (rows = C, K = R); they share the hi panel.  Either output may
-// be null.  `mem` needs shared_panel_floats(R, C) floats.
-size_t shared_panel_floats(long long R, long long C);
-int gemm_prepare_shared(Context &ctx, const float *src, long long stride_r, long long R, long long C, float *mem, int role_rows,
-                        Panels *as_rows, int role_cols, Panels *as_cols);
-// true when a contraction of this shape runs on the 256 x 256 kernel (the only one that takes MN-major operands)
-bool gemm_takes_mn_major(const Context &ctx, long long M, long long N);
-// The Panels of gemm_prepare_shared's layout in `mem` without writing them (for a producer kernel that writes them itself),
-// and what such a producer needs to know: where the three panels lie and which cross-term order each reading wants.
-// Only for R and C that are multiples of 8 (no padding rows or columns to clear).
-struct PanelSink {
-  float *hi = nullptr;            // [R][kp] TF32-rounded values
-  float *cross_k = nullptr;       // [R][kp] cross panel of the row reading (null: not wanted)
-  uint16_t *cross_mn = nullptr;   // [2 R][kp] bf16 cross panel of the column reading (null: not wanted)
-  long long kp = 0;
-  int role_k = 0, role_mn = 0;    // PANEL_ROLE_A / _B of the two readings
-};
-void shared_panel_layout(float *mem, long long R, long long C, int role_rows, Panels *as_rows, int role_cols, Panels *as_cols, PanelSink *sink);
 // whether the epilogue of a tensor-core contraction with this description can emit column statistics (stats_kind)
 bool epilogue_takes_stats(const Context &ctx, const Epilogue &e, long long N);
 // Launches split kernels + the tensor-core kernel (engine 0) or the FP32 FMA kernel (engine 1) on ctx.stream.
@@ -311,6 +263,8 @@ int half_split(Context &ctx, const float *src, long long stride, const HalfPanel
 HalfOperand half_rows(const HalfPanels &p);   // the whole tensor, read through its rows / columns
 HalfOperand half_cols(const HalfPanels &p);
 int half_gemm(Context &ctx, const HalfOperand &A, const HalfOperand &B, const Epilogue &epi);
+// TMA descriptor of one half array of an operand: boxes of 64 of K x box_rows operand rows, 128-byte swizzle
+bool make_half_map(CUtensorMap *map, const HalfOperand &o, const uint16_t *h, int box_rows);
 // Contractions of small and middle sizes straight from the fp32 operands (direct_gemm.cu): no operand panels, several
 // products per launch.  row_sum[m] += sum over k of A[m][k] rides along where it is not null (bias derivatives).
 struct DirectItem {

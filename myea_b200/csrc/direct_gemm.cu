@@ -38,6 +38,17 @@ constexpr int DG_BAR_OFFSET = DG_STAGES * DG_STAGE_BYTES;
 constexpr int DG_SMEM = DG_BAR_OFFSET + 64 + 1024;
 constexpr int DG_MAX_ITEMS = 12;
 
+// x rounded to TF32, half away from zero, on the integer pipe: cvt.rna.tf32 gives the same bits at a quarter of the rate
+// (it and single bf16 conversions kept the pipe of special functions busy: 14 instructions per split element, now 4).
+// A NaN leaves its trace in the low part x - round_tf32(x).
+__device__ __forceinline__ float round_tf32(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
+// two values as a bf16 pair, a in the lower half
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+  return r;
+}
+
 struct DirectProblem {
   const float *a, *b;
   long long lda, ldb;    // pitch of the non-contiguous index
@@ -90,12 +101,30 @@ struct DgReader {
   }
 };
 
+// One group of 8 K elements as 8 TF32 values and the 8 words of a cross-term group: 16 bf16, [lo x8 | hi x8] for operand A
+// (ROLE 0) and [hi x8 | lo x8] for operand B (ROLE 1), so that one bf16 instruction (K = 16) of an A group with a B group gives
+// lo_a*hi_b + hi_a*lo_b
+template <int ROLE>
+__device__ __forceinline__ void split_group(const float (&v)[8], float (&hi)[8], uint32_t (&cross)[8]) {
+  float lo[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    hi[j] = round_tf32(v[j]);
+    lo[j] = v[j] - hi[j];
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t l = pack_bf16(lo[2 * j], lo[2 * j + 1]), h = pack_bf16(hi[2 * j], hi[2 * j + 1]);
+    cross[j] = ROLE ? h : l;
+    cross[4 + j] = ROLE ? l : h;
+  }
+}
 // 8 elements as a hi and a cross group into a stage
 template <int ROLE>
 __device__ __forceinline__ void dg_store8(uint8_t *hi, uint8_t *cross, uint32_t at, const float (&v)[8]) {
   float h[8];
   uint32_t x[8];
-  split_group(v, ROLE, 0, h, x);
+  split_group<ROLE>(v, h, x);
   *reinterpret_cast<float4 *>(hi + at) = make_float4(h[0], h[1], h[2], h[3]);
   *reinterpret_cast<float4 *>(hi + (at ^ 16u)) = make_float4(h[4], h[5], h[6], h[7]);
   *reinterpret_cast<uint4 *>(cross + at) = make_uint4(x[0], x[1], x[2], x[3]);
@@ -280,9 +309,9 @@ __global__ void __launch_bounds__(DG_THREADS, 2) direct_gemm_kernel(const __grid
       if (i >= n_steps) break;
       uint8_t *st = smem + s * DG_STAGE_BYTES;
       if (i >= DG_STAGES && !ptx::mbar_wait(&free_bar[s], static_cast<uint32_t>((i >> 1) - 1) & 1u)) ok = false;
-      dg_store8<PANEL_ROLE_A>(st, st + DG_A_BYTES, ra0.at, va0[s]);
-      dg_store8<PANEL_ROLE_A>(st, st + DG_A_BYTES, ra1.at, va1[s]);
-      dg_store8<PANEL_ROLE_B>(st + 2 * DG_A_BYTES, st + 2 * DG_A_BYTES + DG_B_BYTES, rb.at, vb[s]);
+      dg_store8<0>(st, st + DG_A_BYTES, ra0.at, va0[s]);
+      dg_store8<0>(st, st + DG_A_BYTES, ra1.at, va1[s]);
+      dg_store8<1>(st + 2 * DG_A_BYTES, st + 2 * DG_A_BYTES + DG_B_BYTES, rb.at, vb[s]);
       if (want_sum) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) rs += va0[s][j] + va1[s][j];

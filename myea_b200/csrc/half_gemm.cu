@@ -399,7 +399,7 @@ struct SplitSource {
 // ---------------------------------------------------------------------------------------------------------
 // FP32 FMA engine: 64x64 tile, 16 of K per step, 256 threads x (4x4) outputs, arbitrary strides
 // ---------------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) fma_gemm_kernel(const Operand A, const Operand B, const GemmDims dims, const Epilogue epi) {
+__global__ void __launch_bounds__(256) gemm_fp32_fma_kernel(const Operand A, const Operand B, const GemmDims dims, const Epilogue epi) {
   __shared__ float sa[16][64 + 4];
   __shared__ float sb[16][64 + 4];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -410,10 +410,10 @@ __global__ void __launch_bounds__(256) fma_gemm_kernel(const Operand A, const Op
       int r, kk;
       if (A.stride_k == 1) { r = i >> 4; kk = i & 15; } else { kk = i >> 6; r = i & 63; }
       const long long m = m0 + r, k = k0 + kk;
-      sa[kk][r] = (m < dims.M && k < dims.K) ? A.ptr[m * A.stride_r + k * A.stride_k] + (A.lo ? A.lo[m * A.stride_r + k * A.stride_k] : 0.f) : 0.f;
+      sa[kk][r] = (m < dims.M && k < dims.K) ? A.ptr[m * A.stride_r + k * A.stride_k] : 0.f;
       if (B.stride_k == 1) { r = i >> 4; kk = i & 15; } else { kk = i >> 6; r = i & 63; }
       const long long n = n0 + r;
-      sb[kk][r] = (n < dims.N && k0 + kk < dims.K) ? B.ptr[n * B.stride_r + (k0 + kk) * B.stride_k] + (B.lo ? B.lo[n * B.stride_r + (k0 + kk) * B.stride_k] : 0.f) : 0.f;
+      sb[kk][r] = (n < dims.N && k0 + kk < dims.K) ? B.ptr[n * B.stride_r + (k0 + kk) * B.stride_k] : 0.f;
     }
     __syncthreads();
 #pragma unroll
@@ -684,7 +684,7 @@ int gemm_nt(Context &ctx, const Operand &A, const Operand &B, const Epilogue &ep
     GemmDims dims{static_cast<int>(A.rows), static_cast<int>(B.rows), static_cast<int>(A.k)};
     ctx.begin(TC_GEMM);
     dim3 grid(static_cast<unsigned>((dims.N + 63) / 64), static_cast<unsigned>((dims.M + 63) / 64));
-    fma_gemm_kernel<<<grid, 256, 0, ctx.stream>>>(A, B, dims, epi);
+    gemm_fp32_fma_kernel<<<grid, 256, 0, ctx.stream>>>(A, B, dims, epi);
     ctx.end(TC_GEMM);
     ctx.gemm_flops += 2.0 * dims.M * dims.N * static_cast<double>(dims.K);
     return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;

@@ -19,6 +19,7 @@
 // contraction plus one fused cell kernel (gate nonlinearities, peepholes, cell-state recurrence, zoneout select), each
 // BPTT step is one [B, 4C] x [4C, C] contraction accumulated into the output error plus one fused cell-backward kernel,
 // and the weight derivatives are contractions over K = T*B.  Bias and peephole derivatives are column reductions.
+#include "half_panels.cuh"
 #include "lstm.cuh"
 #include "panel_math.cuh"
 
@@ -58,6 +59,8 @@ struct CellFwd {
 };
 
 __global__ void __launch_bounds__(256) lstm_cell_forward_kernel(const CellFwd p) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const long long total = p.B * p.C;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -103,6 +106,8 @@ struct CellBwd {
 };
 
 __global__ void __launch_bounds__(256) lstm_cell_backward_kernel(const CellBwd p) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const long long total = p.B * p.C;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -203,37 +208,6 @@ __global__ void __launch_bounds__(256) lstm_bias_peephole_finalize_kernel(const 
   d_peep[c * stride + 2] += t[6];
 }
 
-// Cell kernels of the steps that have a predecessor / successor, 8 consecutive cells of one batch row per thread: the
-// arithmetic of lstm_cell_forward_kernel / lstm_cell_backward_kernel, and the results also leave as the operand panels
-// of the next step's contraction (no separate split pass).  p.kind selects; s_rec / rec_dh is the contraction's output.
-__global__ void __launch_bounds__(256) lstm_cells8_forward_kernel(const LstmStep p, const float *__restrict__ s_rec, long long B) {
-  grid_dependency_wait();
-  grid_dependency_release();
-  const long long groups = p.C >> 3, total = B * groups;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long b = i / groups, c0 = (i - b * groups) << 3;
-    float gz[8], gi[8], gf[8], go[8], rec[32];
-    const float *r = s_rec + b * 4 * p.C + c0;
-    load8(gz, r); load8(gi, r + p.C); load8(gf, r + 2 * p.C); load8(go, r + 3 * p.C);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { rec[4 * k] = gz[k]; rec[4 * k + 1] = gi[k]; rec[4 * k + 2] = gf[k]; rec[4 * k + 3] = go[k]; }
-    lstm_forward_cells8(p, rec, b, c0);
-  }
-}
-// the error through time has already been added into p.dh by the contraction (accumulate epilogue): rec = 0
-__global__ void __launch_bounds__(256) lstm_cells8_backward_kernel(const LstmStep p, long long B) {
-  grid_dependency_wait();
-  grid_dependency_release();
-  const long long groups = p.C >> 3, total = B * groups;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long b = i / groups, c0 = (i - b * groups) << 3;
-    const float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    lstm_backward_cells8(p, zero, b, c0);
-  }
-}
-
 // peepholes p_i, p_f, p_o of every cell, gathered from the blocks of the parameter buffer into [3][C]
 __global__ void lstm_gather_peepholes_kernel(const float *__restrict__ peep, long long stride, long long C, float *__restrict__ out) {
   const long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
@@ -243,13 +217,14 @@ __global__ void lstm_gather_peepholes_kernel(const float *__restrict__ peep, lon
   out[2 * C + c] = peep[c * stride + 2];
 }
 
-// the input weights of the four gates, [dirs][4C][n_in], out of the blocks (w0 / w1: first block of each direction)
-__global__ void __launch_bounds__(256) lstm_gather_input_weights_kernel(const float *__restrict__ w0, const float *__restrict__ w1, long long stride, long long z_in,
-                                                                        long long i_in, long long n_in, long long C, float *__restrict__ out) {
-  const long long total = 4 * C * n_in;
+// the input (recurrent) weights of the four gates, [dirs][4C][width], out of the blocks (w0 / w1: first block of each
+// direction; the cell input's row lies at off_z, the three gates' rows at off_gates, one after the other)
+__global__ void __launch_bounds__(256) lstm_gather_weights_kernel(const float *__restrict__ w0, const float *__restrict__ w1, long long stride, long long off_z,
+                                                                  long long off_gates, long long width, long long C, float *__restrict__ out) {
+  const long long total = 4 * C * width;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total; i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long r = i / n_in, k = i - r * n_in, g = r / C, c = r - g * C;
-    const long long at = c * stride + (g == 0 ? z_in : i_in + (g - 1) * n_in) + k;
+    const long long r = i / width, k = i - r * width, g = r / C, c = r - g * C;
+    const long long at = c * stride + (g == 0 ? off_z : off_gates + (g - 1) * width) + k;
     out[i] = w0[at];
     if (w1 != nullptr) out[total + i] = w1[at];
   }
@@ -312,45 +287,45 @@ int lstm_create(myea_b200_net *net, LayerPlan &L) {
   LRC(lalloc(net, &L.values, rows * L.n_out));
   LRC(lalloc(net, &L.deriv, rows * L.n_out));
   L.errors = L.deriv;
-  LRC(lalloc(net, &P->s_rec, net->B * 4 * C));
-  P->off_wrec = 0;
-  const long long Cp = (C + 7) & ~7ll;
-  P->off_wrect = P->off_wrec + panel_floats(4 * C, C) + 64;
-  P->off_step = P->off_wrect + panel_floats(C, 4 * Cp) + 64;
-  LRC(lalloc(net, &P->panel_mem, P->off_step + panel_floats(net->B, 4 * Cp) + 64));
   LRC(lalloc(net, &P->partial, static_cast<size_t>(7) * net->reduce_chunks * C));
-  P->fuse = (C % 8 == 0) && net->ctx.gemm_engine == 0;
-  if (P->fuse) {
-    LRC(lalloc(net, &P->peep_compact, static_cast<size_t>(P->dirs) * 3 * C));
-    // ping-pong operand panels, rows padded to whole 128-row tiles and zero (rows past the batch stay zero for ever)
-    const long long prow = (net->B + 127) / 128 * 128;
-    auto two_buffers = [&](long long k, Panels (&pan)[2]) -> int {
-      const long long kp = (k + 31) / 32 * 32;
-      float *mem = nullptr;
-      LRC(lalloc(net, &mem, static_cast<size_t>(4 * prow * kp) + 64));
-      for (int i = 0; i < 2; ++i) {
-        pan[i] = Panels{};
-        pan[i].hi = mem + i * prow * kp;
-        pan[i].lo = mem + (2 + i) * prow * kp;
-        pan[i].rows = net->B; pan[i].k = k; pan[i].kp = kp;
-        pan[i].role = PANEL_ROLE_A; pan[i].major = PANEL_K;
-      }
-      return MYEA_OK;
-    };
-    LRC(two_buffers(C, P->h_pan));
-    LRC(two_buffers(4 * Cp, P->dg_pan));
-    LRC(lstm_persistent_plan(net, L));
-  }
+  P->G = (C + 15) / 16 * 64;
+  size_t need = static_cast<size_t>(P->dirs) * 4 * C * std::max<long long>(L.n_in, C);  // gathered weights
+  LRC(lstm_persistent_plan(net, L));
   LRC(lstm_resident_plan(net, L));
-  // one-shot contractions use the handle's scratch: make sure it is large enough
-  size_t need = 0;
-  need = std::max(need, panel_floats(rows, L.n_in) + panel_floats(4 * C, L.n_in));            // input projection
-  need = std::max(need, panel_floats(rows, 4 * Cp) + panel_floats(L.n_in, 4 * Cp));          // error to the previous layer
-  need = std::max(need, panel_floats(4 * C, rows) + panel_floats(std::max(L.n_in, C), rows));  // weight derivatives
-  P->shared_dw = net->ctx.gemm_engine == 0 && (C % 64) == 0 && (net->B % 8) == 0 && gemm_takes_mn_major(net->ctx, C, L.n_in) &&
-                 gemm_takes_mn_major(net->ctx, C, C);
-  if (P->shared_dw) need = std::max(need, shared_panel_floats(rows, 4 * C) + shared_panel_floats(rows, L.n_in) + shared_panel_floats(rows, L.n_out) + 256);
-  need = std::max<size_t>(need, static_cast<size_t>(P->dirs * 4 * C * L.n_in));  // gathered input weights
+  const bool tensor = net->ctx.gemm_engine == 0;
+  if (tensor && P->resident == nullptr && lstm_persistent_ready(P)) {
+    LRC(lalloc(net, &P->peep_compact, static_cast<size_t>(P->dirs) * 3 * C));
+    const long long a_rows = (net->B + 127) / 128 * 128;
+    float *mem = nullptr;
+    LRC(lalloc(net, &mem, half_panel_floats(2 * a_rows, C)));       // zero: rows past the batch stay zero for ever
+    P->h_pan = half_panels_at(mem, 2 * a_rows, C);
+    LRC(lalloc(net, &mem, half_panel_floats(2 * a_rows, P->G)));
+    P->dg_pan = half_panels_at(mem, 2 * a_rows, P->G);
+    LRC(lalloc(net, &P->dg_exps, static_cast<size_t>(2 * (a_rows / 128) * (P->G / 64))));
+    for (int d = 0; d < P->dirs; ++d) {
+      LRC(lalloc(net, &P->w_rec_mem[d], half_panel_floats(P->G, C)));
+      P->w_rec[d] = half_panels_at(P->w_rec_mem[d], P->G, C);
+    }
+  } else if (P->resident == nullptr) {
+    LRC(lalloc(net, &P->s_rec, net->B * 4 * C));
+    if (tensor && !direct_gemm_suits(net->ctx, net->B, 4 * C, C)) {
+      for (int d = 0; d < P->dirs; ++d) {
+        LRC(lalloc(net, &P->w_rec_mem[d], half_panel_floats(4 * C, C)));
+        P->w_rec[d] = half_panels_at(P->w_rec_mem[d], 4 * C, C);
+      }
+      LRC(lalloc(net, &P->step_mem, half_panel_floats(net->B, 4 * C)));
+    } else {
+      for (int d = 0; d < P->dirs; ++d) LRC(lalloc(net, &P->w_rec_mem[d], static_cast<size_t>(4 * C * C)));
+    }
+  }
+  const bool in_panels = tensor && !direct_gemm_suits(net->ctx, rows, 4 * C, L.n_in);
+  const bool dw_panels = tensor && !direct_gemm_suits(net->ctx, 4 * C, std::max(L.n_in, C), rows);
+  if (in_panels || dw_panels) LRC(lalloc(net, &P->x_mem, half_panel_floats(rows, L.n_in)));
+  for (int d = 0; d < P->dirs; ++d) {
+    if (in_panels) LRC(lalloc(net, &P->w_in_mem[d], half_panel_floats(4 * C, L.n_in)));
+    if (in_panels || dw_panels) LRC(lalloc(net, &P->dg_all_mem[d], half_panel_floats(rows, 4 * C)));
+    if (dw_panels) LRC(lalloc(net, &P->h_shift_mem[d], half_panel_floats(rows, C)));
+  }
   net->scratch.floats = std::max(net->scratch.floats, need + 256);
   return MYEA_OK;
 }
@@ -392,42 +367,68 @@ void lstm_zoneout_arrays(LayerPlan &L, int dir, uint8_t **state, uint8_t **outpu
   *p_output = L.desc.dropout_values[1];
 }
 
-static float *aligned_scratch(myea_b200_net *net) {
-  return reinterpret_cast<float *>((reinterpret_cast<uintptr_t>(net->scratch.base) + 255) & ~static_cast<uintptr_t>(255));
-}
-
-// [rows, 4C] gate matrix -> panel [rows, K = 4*Cp]: gate g occupies K columns [g*Cp, g*Cp + C); one pass when C is a
-// multiple of 8, else one pass per gate (the panel builder zero-fills each gate's tail up to its group boundary)
-static int prepare_gates(Context &ctx, const float *gates, long long rows, long long C, long long Cp, const Panels &dst) {
-  if (Cp == C) return gemm_prepare_into(ctx, Operand{gates, rows, 4 * C, 4 * C, 1}, dst, 0, 0);
-  for (int g = 0; g < 4; ++g) {
-    int rc = gemm_prepare_into(ctx, Operand{gates + g * C, rows, C, 4 * C, 1}, dst, 0, g * Cp);
-    if (rc != MYEA_OK) return rc;
-  }
-  return MYEA_OK;
-}
-
-// the 8-cell kernels: 128-thread blocks while 256-thread ones would leave SMs without a block (a 256 x 1024 step has
-// 32768 threads: 128 blocks of 256 for 148 SMs), 256-thread blocks otherwise
-static int cell_threads8(long long total) { return (total + 255) / 256 < 148 ? 128 : 256; }
-static int cell_blocks8(long long total) {
-  const long long t = cell_threads8(total);
-  return static_cast<int>(std::max<long long>(1, std::min<long long>((total + t - 1) / t, 148 * 8)));
-}
 static int cell_blocks(long long total) { return static_cast<int>(std::max<long long>(1, std::min<long long>((total + 255) / 256, 148 * 8))); }
+
+// gate rows of the recurrent weights in the order (group of 16 cells, gate, cell): the tensor the persistent walk reads
+struct GroupedGateRows {
+  const float *w;
+  long long stride, rec[4], C;
+  bool vec;
+  struct Cols {};
+  __device__ __forceinline__ void columns(Cols &, long long, int) const {}
+  __device__ __forceinline__ void row(const Cols &, long long r, long long c, int n, float (&v)[8]) const {
+    const long long cell = (r >> 6) * 16 + (r & 15);
+    const int g = static_cast<int>(r >> 4) & 3;
+    if (cell < C) {
+      ld8(v, w + cell * stride + rec[g] + c, n, vec);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = 0.f;
+    }
+  }
+  __device__ __forceinline__ void keep(long long, long long, int, const float (&)[8]) const {}
+};
+// rows of `src` shifted by `shift` rows, zeros where there is none
+struct ShiftedRows {
+  const float *src;
+  long long pitch, shift, rows;
+  bool vec;
+  struct Cols {};
+  __device__ __forceinline__ void columns(Cols &, long long, int) const {}
+  __device__ __forceinline__ void row(const Cols &, long long r, long long c, int n, float (&v)[8]) const {
+    const long long s = r - shift;
+    if (s >= 0 && s < rows) {
+      ld8(v, src + s * pitch + c, n, vec);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = 0.f;
+    }
+  }
+  __device__ __forceinline__ void keep(long long, long long, int, const float (&)[8]) const {}
+};
+static bool vec8(const float *p, long long a, long long b = 0) { return ((reinterpret_cast<uintptr_t>(p) & 15) == 0) && ((a | b) & 3) == 0; }
 
 // ---------------------------------------------------------------------------------------------------------
 // forward
 // ---------------------------------------------------------------------------------------------------------
+static int prepare_input(myea_b200_net *net, LstmPlan *P, const float *input, long long rows, long long n_in) {
+  if (P->x_src == input) return MYEA_OK;
+  P->x = half_panels_at(P->x_mem, rows, n_in);
+  LRC(half_split(net->ctx, input, n_in, P->x));
+  P->x_src = input;
+  return MYEA_OK;
+}
+
 int lstm_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long n_in) {
   LstmPlan *P = L.lstm;
   if (P->cpb != 1) return lstm_blocks_forward(net, L, input, n_in);
   Context &ctx = net->ctx;
   const long long T = net->T, B = net->B, rows = T * B, C = P->C, ldh = L.n_out;
   const BlockOffsets off = block_offsets(n_in, C);
-  float *scratch = aligned_scratch(net);
-  const bool direct_in = direct_gemm_suits(ctx, rows, 4 * C, n_in);
-  if (direct_in) {  // the four gates (of both directions) of the input projection in one launch, straight from the blocks
+  P->x_src = nullptr;
+  P->dg_all_valid[0] = P->dg_all_valid[1] = false;
+  // input projection of all steps: gates_in = x W_in^T + b, columns [z | i | f | o]
+  if (P->w_in_mem[0] == nullptr) {  // the four gates (of both directions) in one launch, straight from the blocks
     DirectItem items[8];
     int n = 0;
     for (int d = 0; d < P->dirs; ++d)
@@ -439,91 +440,77 @@ int lstm_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long
         it.epi.ldc = 4 * C;
         it.epi.bias = net->params + P->d[d].b_base + g * C;
       }
-    LRC(direct_gemm(ctx, items, n));
+    if (ctx.gemm_engine == 0) {
+      LRC(direct_gemm(ctx, items, n));
+    } else {
+      for (int i = 0; i < n; ++i) LRC(gemm_nt(ctx, items[i].A, items[i].B, items[i].epi, net->scratch));
+    }
+  } else {
+    LRC(prepare_input(net, P, input, rows, n_in));
+    for (int d = 0; d < P->dirs; ++d) {
+      RowSegments seg;
+      seg.seg_rows = C;
+      seg.seg_off[0] = off.z_in;
+      for (int g = 0; g < 3; ++g) seg.seg_off[g + 1] = off.in[g];
+      P->w_in[d] = half_panels_at(P->w_in_mem[d], 4 * C, n_in);
+      LRC(half_split(ctx, net->params + P->d[d].w_base, P->stride, P->w_in[d], &seg));
+      Epilogue e;
+      e.C = P->d[d].gates_in;
+      e.ldc = 4 * C;
+      e.bias = net->params + P->d[d].b_base;
+      LRC(half_gemm(ctx, half_rows(P->x), half_rows(P->w_in[d]), e));
+    }
   }
-  Panels px;
-  if (!direct_in) LRC(gemm_prepare(ctx, Operand{input, rows, n_in, n_in, 1}, scratch, &px, PANEL_ROLE_A));
-  for (int d = 0; d < P->dirs && !(direct_in && P->resident != nullptr); ++d) {
+  const bool zone = P->zoneout && net->training;
+  const long long rec[4] = {off.z_rec, off.rec[0], off.rec[1], off.rec[2]};
+  if (P->resident != nullptr) return lstm_resident_run(net, L, 1, zone, rec, off.peep);
+  if (lstm_persistent_ready(P)) {
+    for (int d = 0; d < P->dirs; ++d) {
+      const float *w = net->params + P->d[d].w_base;
+      ctx.begin(TC_RECURRENT);
+      lstm_gather_peepholes_kernel<<<static_cast<unsigned>((C + 255) / 256), 256, 0, ctx.stream>>>(w + off.peep, P->stride, C, P->peep_compact + static_cast<size_t>(d) * 3 * C);
+      ctx.end(TC_RECURRENT);
+      ctx.begin(TC_SPLIT);
+      GroupedGateRows src{w, P->stride, {rec[0], rec[1], rec[2], rec[3]}, C, vec8(w, P->stride, rec[0] | rec[1] | rec[2] | rec[3])};
+      half_produce(ctx, src, P->w_rec[d]);
+      ctx.end(TC_SPLIT);
+      LRC(lstm_persistent_forward(net, L, d, zone));
+    }
+    return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
+  }
+  // the walk by launches: per step the recurrent product and the cell kernel
+  for (int d = 0; d < P->dirs; ++d) {
     LstmDir &D = P->d[d];
     const float *w = net->params + D.w_base;
-    if (!direct_in) {
-    // fused input panel [4C, in], gate order z, i, f, o
-    Panels pwin = panels_at(scratch + panel_floats(rows, n_in), 4 * C, n_in, PANEL_ROLE_B);
-    LRC(gemm_prepare_into(ctx, Operand{w + off.z_in, C, n_in, P->stride, 1}, pwin, 0, 0));
-    for (int g = 0; g < 3; ++g) LRC(gemm_prepare_into(ctx, Operand{w + off.in[g], C, n_in, P->stride, 1}, pwin, (g + 1) * C, 0));
-    Epilogue e;
-    e.C = D.gates_in;
-    e.ldc = 4 * C;
-    e.bias = net->params + D.b_base;
-    LRC(gemm_panels(ctx, px, 0, rows, pwin, 0, 4 * C, e));
-    }
-    if (P->resident != nullptr) continue;
-    // fused recurrent panel [4C, C]
-    Panels pwrec = panels_at(P->panel_mem + P->off_wrec, 4 * C, C, PANEL_ROLE_B);
-    float *peep_c = nullptr;
-    if (P->fuse) {
-      peep_c = P->peep_compact + static_cast<size_t>(d) * 3 * C;
+    if (P->step_mem != nullptr) {
+      RowSegments seg;
+      seg.seg_rows = C;
+      for (int g = 0; g < 4; ++g) seg.seg_off[g] = rec[g];
+      LRC(half_split(ctx, w, P->stride, P->w_rec[d], &seg));
+    } else {
       ctx.begin(TC_RECURRENT);
-      lstm_gather_peepholes_kernel<<<static_cast<unsigned>((C + 255) / 256), 256, 0, ctx.stream>>>(w + off.peep, P->stride, C, peep_c);
+      lstm_gather_weights_kernel<<<static_cast<unsigned>(std::min<long long>((4 * C * C + 255) / 256, 148 * 8)), 256, 0, ctx.stream>>>(w, nullptr, P->stride, rec[0], rec[1], C, C,
+                                                                                                                                   P->w_rec_mem[d]);
       ctx.end(TC_RECURRENT);
     }
-    const bool persistent = lstm_persistent_ready(P);
-    if (persistent) {
-      // rows interleaved cell by cell (row 4 * cell + gate): the 128 columns of a tile of the step's product then hold the
-      // four gate sums of 32 cells side by side and the kernel finishes whole cells from its share of the tile
-      LRC(gemm_prepare_interleaved(ctx, Operand{w + off.z_rec, C, C, P->stride, 1}, pwrec, 0, 4));
-      for (int g = 0; g < 3; ++g) LRC(gemm_prepare_interleaved(ctx, Operand{w + off.rec[g], C, C, P->stride, 1}, pwrec, g + 1, 4));
-    } else {
-      LRC(gemm_prepare_into(ctx, Operand{w + off.z_rec, C, C, P->stride, 1}, pwrec, 0, 0));
-      for (int g = 0; g < 3; ++g) LRC(gemm_prepare_into(ctx, Operand{w + off.rec[g], C, C, P->stride, 1}, pwrec, (g + 1) * C, 0));
-    }
-    const bool zone = P->zoneout && net->training;
     for (long long s = 0; s < T; ++s) {
       const long long t = d == 0 ? s : T - 1 - s;
       const long long tp = d == 0 ? t - 1 : t + 1;
-      float *h_t = L.values + t * B * ldh + d * C;
-      if (persistent && s > 0) {  // one launch walks steps 1 .. T-1
-        LRC(lstm_persistent_forward(net, L, d, pwrec, peep_c, zone));
-        break;
-      }
-      if (P->fuse && s > 0) {
-        // recurrent contraction on the panels the previous step left, then the cell kernel; h_t leaves as the layer
-        // output and as the operand panels of step s + 1
-        const Panels &ph_prev = P->h_pan[(s - 1) & 1];
-        const Panels &ph_next = P->h_pan[s & 1];
-        Epilogue e;
-        LstmStep f;
-        f.C = C; f.ldh = ldh; f.kp = ph_next.kp;
-        f.peep = peep_c;
-        if (s + 1 < T) { f.p_hi = ph_next.hi; f.p_cross = ph_next.lo; }
-        f.gates_in = D.gates_in + t * B * 4 * C;
-        f.c_prev = D.cstate + tp * B * C;
-        f.h_prev = L.values + tp * B * ldh + d * C;
-        f.act = D.act + t * B * 4 * C;
-        f.cstate = D.cstate + t * B * C;
-        f.cact = D.cact + t * B * C;
-        f.h = h_t;
-        f.zone_state = zone ? D.zone_state + t * C : nullptr;
-        f.zone_output = zone ? D.zone_output + t * C : nullptr;
-        e.C = P->s_rec;
-        e.ldc = 4 * C;
-        LRC(gemm_panels(ctx, ph_prev, 0, B, pwrec, 0, 4 * C, e));
-        ctx.begin(TC_RECURRENT);
-        launch_dependent(ctx, lstm_cells8_forward_kernel, dim3(cell_blocks8(B * C / 8)), dim3(cell_threads8(B * C / 8)), 0, f, static_cast<const float *>(P->s_rec), B);
-        ctx.end(TC_RECURRENT);
-        continue;
-      }
       CellFwd cf;
       cf.gates_in = D.gates_in + t * B * 4 * C;
       cf.s_rec = nullptr; cf.c_prev = nullptr; cf.h_prev = nullptr;
       if (s > 0) {
         const float *h_prev = L.values + tp * B * ldh + d * C;
-        Panels ph;
-        LRC(gemm_prepare(ctx, Operand{h_prev, B, C, ldh, 1}, P->panel_mem + P->off_step, &ph, PANEL_ROLE_A));
         Epilogue er;
         er.C = P->s_rec;
         er.ldc = 4 * C;
-        LRC(gemm_panels(ctx, ph, 0, B, pwrec, 0, 4 * C, er));
+        if (P->step_mem != nullptr) {
+          const HalfPanels ph = half_panels_at(P->step_mem, B, C);
+          LRC(half_split(ctx, h_prev, ldh, ph));
+          LRC(half_gemm(ctx, half_rows(ph), half_rows(P->w_rec[d]), er));
+        } else {
+          LRC(gemm_nt(ctx, Operand{h_prev, B, C, ldh, 1}, Operand{P->w_rec_mem[d], 4 * C, C, C, 1}, er, net->scratch));
+        }
         cf.s_rec = P->s_rec;
         cf.c_prev = D.cstate + tp * B * C;
         cf.h_prev = h_prev;
@@ -533,21 +520,15 @@ int lstm_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long
       cf.act = D.act + t * B * 4 * C;
       cf.cstate = D.cstate + t * B * C;
       cf.cact = D.cact + t * B * C;
-      cf.h = h_t;
+      cf.h = L.values + t * B * ldh + d * C;
       cf.ldh = ldh;
       cf.zone_state = zone ? D.zone_state + t * C : nullptr;
       cf.zone_output = zone ? D.zone_output + t * C : nullptr;
       cf.B = B; cf.C = C;
       ctx.begin(TC_RECURRENT);
-      lstm_cell_forward_kernel<<<cell_blocks(B * C), 256, 0, ctx.stream>>>(cf);
+      launch_dependent(ctx, lstm_cell_forward_kernel, dim3(cell_blocks(B * C)), dim3(256), 0, cf);
       ctx.end(TC_RECURRENT);
-      if (P->fuse && T > 1)  // first step: its output becomes the operand of the second step
-        LRC(gemm_prepare_into(ctx, Operand{h_t, B, C, ldh, 1}, P->h_pan[0], 0, 0));
     }
-  }
-  if (P->resident != nullptr) {
-    const long long rec[4] = {off.z_rec, off.rec[0], off.rec[1], off.rec[2]};
-    LRC(lstm_resident_run(net, L, 1, P->zoneout && net->training, rec, off.peep));
   }
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
@@ -560,64 +541,36 @@ int lstm_backward(myea_b200_net *net, LayerPlan &L) {
   if (P->cpb != 1) return lstm_blocks_backward(net, L);
   Context &ctx = net->ctx;
   const long long T = net->T, B = net->B, C = P->C, ldh = L.n_out, n_in = P->n_in;
-  const long long Cp = (C + 7) & ~7ll;  // each gate's K segment starts on a group-of-8 boundary
   const BlockOffsets off = block_offsets(n_in, C);
+  P->dg_all_valid[0] = P->dg_all_valid[1] = false;
   if (P->resident != nullptr) {
     const long long rec[4] = {off.z_rec, off.rec[0], off.rec[1], off.rec[2]};
     return lstm_resident_run(net, L, 2, false, rec, off.peep);
   }
   for (int d = 0; d < P->dirs; ++d) {
     LstmDir &D = P->d[d];
-    const float *w = net->params + D.w_base;
-    // transposed recurrent panel [C (unit j of h), K = 4C (gate, cell)]
-    Panels pwt = panels_at(P->panel_mem + P->off_wrect, C, 4 * Cp, PANEL_ROLE_B);
-    LRC(gemm_prepare_into(ctx, Operand{w + off.z_rec, C, C, 1, P->stride}, pwt, 0, 0));
-    for (int g = 0; g < 3; ++g) LRC(gemm_prepare_into(ctx, Operand{w + off.rec[g], C, C, 1, P->stride}, pwt, 0, (g + 1) * Cp));
+    if (lstm_persistent_ready(P)) {
+      LRC(lstm_persistent_backward(net, L, d));
+      continue;
+    }
     for (long long s = 0; s < T; ++s) {
       const long long t = d == 0 ? T - 1 - s : s;      // walk against the layer's direction
       const long long tn = d == 0 ? t + 1 : t - 1;     // the step after t in the layer's direction
       const long long tp = d == 0 ? t - 1 : t + 1;     // the step before t
       float *dh_t = L.deriv + t * B * ldh + d * C;
-      if (lstm_persistent_ready(P) && s > 0) {  // one launch walks the remaining steps
-        LRC(lstm_persistent_backward(net, L, d, pwt, P->peep_compact + static_cast<size_t>(d) * 3 * C));
-        break;
-      }
-      if (P->fuse && s > 0) {
-        // error through time (gate errors of the next step times W_rec) on the panels the previous step left, then the
-        // cell's backward arithmetic; the gate errors of step t leave as arrays and as the next operand panels
-        const Panels &pd_prev = P->dg_pan[(s - 1) & 1];
-        const Panels &pd_next = P->dg_pan[s & 1];
-        Epilogue e;
-        LstmStep f;
-        f.C = C; f.ldh = ldh; f.kp = pd_next.kp; f.Cp = Cp;
-        f.peep = P->peep_compact + static_cast<size_t>(d) * 3 * C;
-        if (s + 1 < T) { f.p_hi = pd_next.hi; f.p_cross = pd_next.lo; }
-        f.dh = dh_t;
-        f.b_act = D.act + t * B * 4 * C;
-        f.b_cact = D.cact + t * B * C;
-        f.b_c_prev = (tp >= 0 && tp < T) ? D.cstate + tp * B * C : nullptr;
-        f.act_next = D.act + tn * B * 4 * C;
-        f.dgates_next = D.dgates + tn * B * 4 * C;
-        f.dc_next = D.dcstate + tn * B * C;
-        f.dgates = D.dgates + t * B * 4 * C;
-        f.dcstate = D.dcstate + t * B * C;
-        e.C = dh_t;
-        e.ldc = ldh;
-        e.accumulate = 1;
-        LRC(gemm_panels(ctx, pd_prev, 0, B, pwt, 0, C, e));
-        ctx.begin(TC_RECURRENT);
-        launch_dependent(ctx, lstm_cells8_backward_kernel, dim3(cell_blocks8(B * C / 8)), dim3(cell_threads8(B * C / 8)), 0, f, B);
-        ctx.end(TC_RECURRENT);
-        continue;
-      }
-      if (s > 0) {
-        Panels pd = panels_at(P->panel_mem + P->off_step, B, 4 * Cp, PANEL_ROLE_A);
-        LRC(prepare_gates(ctx, D.dgates + tn * B * 4 * C, B, C, Cp, pd));
+      if (s > 0) {  // error through time: the gate errors of the step after times the recurrent weights
+        const float *dg = D.dgates + tn * B * 4 * C;
         Epilogue e;
         e.C = dh_t;
         e.ldc = ldh;
         e.accumulate = 1;
-        LRC(gemm_panels(ctx, pd, 0, B, pwt, 0, C, e));
+        if (P->step_mem != nullptr) {
+          const HalfPanels pd = half_panels_at(P->step_mem, B, 4 * C);
+          LRC(half_split(ctx, dg, 4 * C, pd));
+          LRC(half_gemm(ctx, half_rows(pd), half_cols(P->w_rec[d]), e));
+        } else {
+          LRC(gemm_nt(ctx, Operand{dg, B, 4 * C, 4 * C, 1}, Operand{P->w_rec_mem[d], C, 4 * C, 1, C}, e, net->scratch));
+        }
       }
       CellBwd cb;
       cb.dh = dh_t;
@@ -628,19 +581,27 @@ int lstm_backward(myea_b200_net *net, LayerPlan &L) {
       cb.act_next = s > 0 ? D.act + tn * B * 4 * C : nullptr;
       cb.dgates_next = s > 0 ? D.dgates + tn * B * 4 * C : nullptr;
       cb.dc_next = s > 0 ? D.dcstate + tn * B * C : nullptr;
-      cb.peep = w + off.peep;
+      cb.peep = net->params + D.w_base + off.peep;
       cb.stride = P->stride;
       cb.dgates = D.dgates + t * B * 4 * C;
       cb.dcstate = D.dcstate + t * B * C;
       cb.B = B; cb.C = C;
       ctx.begin(TC_RECURRENT);
-      lstm_cell_backward_kernel<<<cell_blocks(B * C), 256, 0, ctx.stream>>>(cb);
+      launch_dependent(ctx, lstm_cell_backward_kernel, dim3(cell_blocks(B * C)), dim3(256), 0, cb);
       ctx.end(TC_RECURRENT);
-      if (P->fuse && T > 1)  // last time step (first of the walk): its gate errors are the operand of the next contraction
-        LRC(prepare_gates(ctx, D.dgates + t * B * 4 * C, B, C, Cp, P->dg_pan[0]));
     }
   }
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
+}
+
+// the gate errors of all steps as panels: read through their rows by the error to the layer below, through their columns by
+// the weight derivatives
+static int prepare_gate_errors(myea_b200_net *net, LstmPlan *P, int d, long long rows) {
+  if (P->dg_all_valid[d]) return MYEA_OK;
+  P->dg_all[d] = half_panels_at(P->dg_all_mem[d], rows, 4 * P->C);
+  LRC(half_split(net->ctx, P->d[d].dgates, 4 * P->C, P->dg_all[d]));
+  P->dg_all_valid[d] = true;
+  return MYEA_OK;
 }
 
 // error of the LSTM layer L propagated to the outputs of the layer feeding it: prev_deriv [T*B, n_in] = sum over
@@ -652,43 +613,30 @@ int lstm_backward_to_input(myea_b200_net *net, LayerPlan &L, float *prev_deriv, 
   Context &ctx = net->ctx;
   const long long rows = net->T * net->B, C = P->C, n_in = P->n_in;
   if (prev.n_out != n_in) return MYEA_E_INVALID;
-  const long long Cp = (C + 7) & ~7ll;
   const BlockOffsets off = block_offsets(n_in, C);
-  float *scratch = aligned_scratch(net);
-  const bool direct = direct_gemm_suits(ctx, rows, n_in, 4 * C);
-  if (direct) {  // the input weights gathered out of the blocks once (their four gate matrices are one K range then)
+  const bool gathered = P->w_in_mem[0] == nullptr;
+  if (gathered) {  // the input weights gathered out of the blocks once (their four gate matrices are one K range then)
     ctx.begin(TC_RECURRENT);
-    lstm_gather_input_weights_kernel<<<static_cast<unsigned>(std::min<long long>((4 * C * n_in + 255) / 256, 148 * 8)), 256, 0, ctx.stream>>>(
-        net->params + P->d[0].w_base, P->dirs > 1 ? net->params + P->d[1].w_base : nullptr, P->stride, off.z_in, off.in[0], n_in, C, scratch);
+    lstm_gather_weights_kernel<<<static_cast<unsigned>(std::min<long long>((4 * C * n_in + 255) / 256, 148 * 8)), 256, 0, ctx.stream>>>(
+        net->params + P->d[0].w_base, P->dirs > 1 ? net->params + P->d[1].w_base : nullptr, P->stride, off.z_in, off.in[0], n_in, C, net->scratch.base);
     ctx.end(TC_RECURRENT);
   }
   for (int d = 0; d < P->dirs; ++d) {
     LstmDir &D = P->d[d];
-    const float *w = net->params + D.w_base;
-    if (direct) {
-      DirectItem it;
-      it.A = Operand{D.dgates, rows, 4 * C, 4 * C, 1};
-      it.B = Operand{scratch + d * 4 * C * n_in, n_in, 4 * C, 1, n_in};
-      if (finish != nullptr && d == P->dirs - 1) it.epi = *finish;
-      it.epi.C = prev_deriv;
-      it.epi.ldc = n_in;
-      if (d > 0 && finish != nullptr) { it.epi.addend = prev_deriv; it.epi.ld_addend = n_in; }
-      else it.epi.accumulate = d > 0 ? 1 : 0;
-      LRC(direct_gemm(ctx, &it, 1));
-      continue;
-    }
-    Panels pd = panels_at(scratch, rows, 4 * Cp, PANEL_ROLE_A);
-    LRC(prepare_gates(ctx, D.dgates, rows, C, Cp, pd));
-    Panels pwt = panels_at(scratch + panel_floats(rows, 4 * Cp), n_in, 4 * Cp, PANEL_ROLE_B);  // [n_in, K = 4 gates]
-    LRC(gemm_prepare_into(ctx, Operand{w + off.z_in, n_in, C, 1, P->stride}, pwt, 0, 0));
-    for (int g = 0; g < 3; ++g) LRC(gemm_prepare_into(ctx, Operand{w + off.in[g], n_in, C, 1, P->stride}, pwt, 0, (g + 1) * Cp));
     Epilogue e;
     if (finish != nullptr && d == P->dirs - 1) e = *finish;
     e.C = prev_deriv;
     e.ldc = n_in;
     if (d > 0 && finish != nullptr) { e.addend = prev_deriv; e.ld_addend = n_in; }  // the addend enters before the derivative
     else e.accumulate = d > 0 ? 1 : 0;
-    LRC(gemm_panels(ctx, pd, 0, rows, pwt, 0, n_in, e));
+    if (gathered) {
+      const DirectItem it{Operand{D.dgates, rows, 4 * C, 4 * C, 1}, Operand{net->scratch.base + d * 4 * C * n_in, n_in, 4 * C, 1, n_in}, e, nullptr};
+      if (ctx.gemm_engine == 0) LRC(direct_gemm(ctx, &it, 1));
+      else LRC(gemm_nt(ctx, it.A, it.B, e, GemmScratch{}));
+    } else {
+      LRC(prepare_gate_errors(net, P, d, rows));
+      LRC(half_gemm(ctx, half_rows(P->dg_all[d]), half_cols(P->w_in[d]), e));
+    }
   }
   return MYEA_OK;
 }
@@ -702,11 +650,11 @@ int lstm_update_derivative_weight(myea_b200_net *net, LayerPlan &L, const float 
   Context &ctx = net->ctx;
   const long long T = net->T, B = net->B, rows = T * B, C = P->C, ldh = L.n_out;
   const BlockOffsets off = block_offsets(n_in, C);
-  float *scratch = aligned_scratch(net);
   for (int d = 0; d < P->dirs; ++d) {
     LstmDir &D = P->d[d];
     float *gw = net->grads + D.w_base;
-    if (direct_gemm_suits(ctx, 4 * C, std::max(n_in, C), rows)) {
+    const long long shift = d == 0 ? B : -B;   // rows of time step t against the outputs one step earlier in the direction
+    if (P->h_shift_mem[0] == nullptr) {
       // gate by gate in one launch: the gate errors against the layer's input and against its output one step earlier
       DirectItem items[8];
       const long long K = (T - 1) * B;
@@ -729,85 +677,39 @@ int lstm_update_derivative_weight(myea_b200_net *net, LayerPlan &L, const float 
           r.epi.accumulate = 1;
         }
       }
-      LRC(direct_gemm(ctx, items, n));
-    } else if (P->shared_dw) {
-      // Both operands of every weight-derivative contraction are read through their columns (K = rows of the batch
-      // and time axis), so one untransposed split pass per tensor serves all of them: gate errors, layer input, and
-      // the layer's own outputs for the recurrent weights (a sub-range of K rows and of columns).
-      float *mem_d = scratch;
-      float *mem_x = mem_d + ((shared_panel_floats(rows, 4 * C) + 63) & ~static_cast<size_t>(63));
-      float *mem_h = mem_x + ((shared_panel_floats(rows, n_in) + 63) & ~static_cast<size_t>(63));
-      Panels pd, px, ph;
-      LRC(gemm_prepare_shared(ctx, D.dgates, 4 * C, rows, 4 * C, mem_d, PANEL_ROLE_A, nullptr, PANEL_ROLE_A, &pd));
-      LRC(gemm_prepare_shared(ctx, input, n_in, rows, n_in, mem_x, PANEL_ROLE_B, nullptr, PANEL_ROLE_B, &px));
-      const long long in_off[4] = {off.z_in, off.in[0], off.in[1], off.in[2]};
-      {  // the four gates in one contraction: row g*C + c of the product lands in block c at gate g's offset
-        Epilogue e;
-        e.C = gw;
-        e.ldc = P->stride;
-        e.accumulate = 1;
-        e.seg_rows = C;
-        for (int g = 0; g < 4; ++g) e.seg_off[g] = in_off[g];
-        LRC(gemm_panels(ctx, pd, 0, 4 * C, px, 0, n_in, e));
-      }
-      if (T > 1) {
-        LRC(gemm_prepare_shared(ctx, L.values, ldh, rows, ldh, mem_h, PANEL_ROLE_B, nullptr, PANEL_ROLE_B, &ph));
-        const long long K = (T - 1) * B;
-        // K rows of steps 1..T-1 of the gate errors against steps 0..T-2 of the outputs (forward direction), the
-        // other way round for the backward direction: a K offset of B rows on one side
-        Panels pdk = pd, phk = ph;
-        const long long kd = d == 0 ? B : 0, kh = d == 0 ? 0 : B;
-        pdk.hi += kd * pd.kp;
-        pdk.lo = reinterpret_cast<float *>(reinterpret_cast<uint16_t *>(pd.lo) + 2 * kd * pd.kp);
-        pdk.k = K;
-        phk.hi += kh * ph.kp;
-        phk.lo = reinterpret_cast<float *>(reinterpret_cast<uint16_t *>(ph.lo) + 2 * kh * ph.kp);
-        phk.k = K;
-        const long long rec_off[4] = {off.z_rec, off.rec[0], off.rec[1], off.rec[2]};
-        Epilogue e;
-        e.C = gw;
-        e.ldc = P->stride;
-        e.accumulate = 1;
-        e.seg_rows = C;
-        for (int g = 0; g < 4; ++g) e.seg_off[g] = rec_off[g];
-        LRC(gemm_panels(ctx, pdk, 0, 4 * C, phk, d * C, C, e));
+      if (ctx.gemm_engine == 0) {
+        LRC(direct_gemm(ctx, items, n));
+      } else {
+        for (int i = 0; i < n; ++i) LRC(gemm_nt(ctx, items[i].A, items[i].B, items[i].epi, GemmScratch{}));
       }
     } else {
-    // input weights: K = all T*B rows
-    Panels pdt, pxt;
-    LRC(gemm_prepare(ctx, Operand{D.dgates, 4 * C, rows, 1, 4 * C}, scratch, &pdt, PANEL_ROLE_A));                        // dgates^T [4C, rows]
-    LRC(gemm_prepare(ctx, Operand{input, n_in, rows, 1, n_in}, scratch + panel_floats(4 * C, rows), &pxt, PANEL_ROLE_B));  // x^T [n_in, rows]
-    const long long in_off[4] = {off.z_in, off.in[0], off.in[1], off.in[2]};
-    for (int g = 0; g < 4; ++g) {
+      // the four gates in one contraction: row g*C + c of the product lands in block c at gate g's offset
+      LRC(prepare_input(net, P, input, rows, n_in));
+      LRC(prepare_gate_errors(net, P, d, rows));
       Epilogue e;
-      e.C = gw + in_off[g];
+      e.C = gw;
       e.ldc = P->stride;
       e.accumulate = 1;
-      LRC(gemm_panels(ctx, pdt, g * C, C, pxt, 0, n_in, e));
-    }
-    // recurrent weights: pairs (gate error of the next step in the layer's direction, output of this step)
-    if (T > 1) {
-      const long long K = (T - 1) * B;
-      const float *dg0 = d == 0 ? D.dgates + B * 4 * C : D.dgates;              // rows of steps 1..T-1 (forward) / 0..T-2 (backward)
-      const float *h0 = d == 0 ? L.values + d * C : L.values + B * ldh + d * C;  // rows of steps 0..T-2 (forward) / 1..T-1 (backward)
-      Panels pdr, pht;
-      LRC(gemm_prepare(ctx, Operand{dg0, 4 * C, K, 1, 4 * C}, scratch, &pdr, PANEL_ROLE_A));
-      LRC(gemm_prepare(ctx, Operand{h0, C, K, 1, ldh}, scratch + panel_floats(4 * C, K), &pht, PANEL_ROLE_B));
-      const long long rec_off[4] = {off.z_rec, off.rec[0], off.rec[1], off.rec[2]};
-      for (int g = 0; g < 4; ++g) {
-        Epilogue e;
-        e.C = gw + rec_off[g];
-        e.ldc = P->stride;
-        e.accumulate = 1;
-        LRC(gemm_panels(ctx, pdr, g * C, C, pht, 0, C, e));
+      e.seg_rows = C;
+      e.seg_off[0] = off.z_in;
+      for (int g = 0; g < 3; ++g) e.seg_off[g + 1] = off.in[g];
+      LRC(half_gemm(ctx, half_cols(P->dg_all[d]), half_cols(P->x), e));
+      if (T > 1) {
+        // recurrent weights over all rows too: the outputs shifted by one step, zeros at the direction's first step
+        const HalfPanels hs = half_panels_at(P->h_shift_mem[d], rows, C);
+        ctx.begin(TC_SPLIT);
+        half_produce(ctx, ShiftedRows{L.values + d * C, ldh, shift, rows, vec8(L.values, ldh, C)}, hs);
+        ctx.end(TC_SPLIT);
+        e.seg_off[0] = off.z_rec;
+        for (int g = 0; g < 3; ++g) e.seg_off[g + 1] = off.rec[g];
+        LRC(half_gemm(ctx, half_cols(P->dg_all[d]), half_cols(hs), e));
       }
-    }
     }
     // biases and peepholes
     const int chunks = static_cast<int>(std::max<long long>(1, std::min<long long>(net->reduce_chunks, rows / 8)));
     ctx.begin(TC_RECURRENT);
     dim3 grid(static_cast<unsigned>((C + 31) / 32), chunks);
-    lstm_bias_peephole_reduce_kernel<<<grid, 256, 0, ctx.stream>>>(D.dgates, D.cstate, rows, C, d == 0 ? B : -B, chunks, P->partial);
+    lstm_bias_peephole_reduce_kernel<<<grid, 256, 0, ctx.stream>>>(D.dgates, D.cstate, rows, C, shift, chunks, P->partial);
     lstm_bias_peephole_finalize_kernel<<<static_cast<unsigned>((C + 31) / 32), 256, 0, ctx.stream>>>(P->partial, chunks, C, net->grads + D.b_base,
                                                                                                     gw + off.peep, P->stride);
     ctx.end(TC_RECURRENT, 2);

@@ -24,20 +24,26 @@ struct LstmPlan {
   long long C = 0, n_in = 0, stride = 0;
   bool zoneout = false;
   LstmDir d[2];
-  float *s_rec = nullptr;      // [B, 4C] recurrent projection of the current step
-  float *panel_mem = nullptr;  // W_rec panels, their transpose, per-step operand panels
-  size_t off_wrec = 0, off_wrect = 0, off_step = 0;
+  float *s_rec = nullptr;      // [B, 4C] recurrent projection of the current step (walk by launches)
   float *partial = nullptr;    // [7][chunks][C]
-  bool shared_dw = false;  // weight derivatives from untransposed (column-read) operand panels
-  // `fuse` (C a multiple of 8, tensor-core engine): the cell arithmetic of a step also writes the next step's operand
-  // panels - ping-pong panels of h (forward) and of the gate errors (backward) - and reads compact peepholes
-  // [dirs][3][C].  All steps but the first then run in one persistent launch (`persist`, lstm_persistent.cu) when the
-  // layer's tiles fit the device at once, else as a contraction plus an 8-cells-per-thread cell kernel per step.
-  bool fuse = false;
-  float *peep_compact = nullptr;
-  // both buffers of a ping-pong pair lie in one allocation, hi [2][rows][kp] then cross [2][rows][kp] with rows = the
-  // batch rounded up to 128, so that one tensor map covers both
-  Panels h_pan[2], dg_pan[2];
+  float *peep_compact = nullptr;  // [dirs][3][C]
+  // Operand panels (half_panels.cuh) of contractions too large for the products straight from fp32.  x: layer input [T*B, in];
+  // w_in: the four gates' input weights [4C, in]; dg_all: gate errors [T*B, 4C]; h_shift: the layer's outputs one step
+  // earlier in the direction [T*B, C] (zeros at its first step).
+  float *x_mem = nullptr, *w_in_mem[2] = {nullptr, nullptr}, *dg_all_mem[2] = {nullptr, nullptr}, *h_shift_mem[2] = {nullptr, nullptr};
+  HalfPanels x, w_in[2], dg_all[2];
+  const float *x_src = nullptr;   // the array the x panels were made from in this step
+  bool dg_all_valid[2] = {false, false};
+  // Recurrent weights as panels: for the persistent walk [G, C] with the gate rows in the order (group of 16 cells, gate,
+  // cell), G = 64 * ceil(C / 16); for the walk by launches [4C, C] gate after gate, or (small products) gathered in fp32.
+  long long G = 0;
+  float *w_rec_mem[2] = {nullptr, nullptr};
+  HalfPanels w_rec[2];
+  // Ping-pong operand panels of the persistent walk, both buffers in one tensor of 2 * a_rows rows (a_rows: the batch rounded up to
+  // 128): h [.., C] with a fixed exponent, gate errors [.., G] with exponents [2][rows / 128][G / 64]
+  HalfPanels h_pan, dg_pan;
+  int *dg_exps = nullptr;
+  float *step_mem = nullptr;   // walk by launches: panels of one step's operand
   LstmPersistent *persist = nullptr;
   LstmResident *resident = nullptr;  // the walk with resident weights (lstm_resident.cu), where it is the faster one
   // blocks of several cells (lstm_blocks.cu): K blocks of cpb cells per direction, gate rows of G = C + 3K columns
@@ -55,19 +61,18 @@ int lstm_blocks_backward_to_input(myea_b200_net *net, LayerPlan &L, float *prev_
 int lstm_blocks_update_derivative_weight(myea_b200_net *net, LayerPlan &L, const float *input, long long n_in);
 
 
-// One launch that walks ALL remaining time steps of one layer and direction (lstm_persistent.cu): the recurrent
+// One launch that walks ALL time steps of one layer and direction (lstm_persistent.cu): the recurrent
 // contraction of every step on the tensor cores, the cell arithmetic in its epilogue, the step's results written as the
-// next step's operand panels, and a bounded grid-wide barrier between steps.  The first step of a walk has no predecessor
-// and is computed by the per-step kernels, which leave its panels behind.
-//   forward: steps s = 1 .. T-1 of direction `dir` (step s reads the h panels of buffer (s - 1) & 1)
-//   backward: steps s = 1 .. T-1 of the walk against the direction (step s reads the gate-error panels of (s - 1) & 1)
+// next step's operand panels, and a bounded grid-wide barrier between steps.
+//   forward: steps s = 0 .. T-1 of direction `dir` (step s reads the h panels of buffer (s - 1) & 1)
+//   backward: steps s = 0 .. T-1 of the walk against the direction (step s reads the gate-error panels of (s - 1) & 1)
 // lstm_persistent_plan decides at creation whether the layer's shapes fit (every tile resident at once); the step
 // functions return MYEA_E_UNSUPPORTED when they do not apply and the caller takes the per-step path.
 int lstm_persistent_plan(myea_b200_net *net, LayerPlan &L);
 void lstm_persistent_destroy(LstmPlan *P);
 bool lstm_persistent_ready(const LstmPlan *P);
-int lstm_persistent_forward(myea_b200_net *net, LayerPlan &L, int dir, const Panels &w_rec_interleaved, const float *peep_compact, bool zoneout);
-int lstm_persistent_backward(myea_b200_net *net, LayerPlan &L, int dir, const Panels &w_rec_transposed, const float *peep_compact);
+int lstm_persistent_forward(myea_b200_net *net, LayerPlan &L, int dir, bool zoneout);
+int lstm_persistent_backward(myea_b200_net *net, LayerPlan &L, int dir);
 
 // The walk for small batches and narrow or odd layers: all time steps (and both directions) in one launch, recurrent weights
 // in shared memory, read from the parameter buffer itself.  Set by lstm_resident_plan where it is estimated to be faster.

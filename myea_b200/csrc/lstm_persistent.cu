@@ -9,24 +9,30 @@
 //   grid      one cluster of SPLIT CTAs per 128 x BN tile of the step's product; the CTAs of a cluster share the tile and
 //             split its K range (forward: BN = 128 gate columns, K = cells in 2 slices; backward: BN = 64 cells, K = 4 x
 //             cells in 4 slices: 8-CTA clusters would halve the weight traffic per SM, but a B200 holds only 15 of the 16
-//             the benchmark layer needs), so that every SM streams a small share of the recurrent weights per step
+//             a layer of 1024 cells needs), so that every SM streams a small share of the recurrent weights per step
 //             (they do not fit shared memory; they stay in L2)
+//   operands  half panels (half_panels.cuh): 4 bytes per element.  The gate rows of the weights are ordered (group of 16
+//             cells, gate, cell), one tensor for both passes: forward reads its rows, backward its columns.  h is at most 1 in
+//             magnitude and has a fixed exponent; the gate errors have one exponent per 128 batch rows and group of 16 cells -
+//             the 64 of K that one CTA produces and that one stage of a later step consumes
 //   warp 0    TMA producer: waits until the operand panels of the previous step are complete (step barrier), then
 //             loads its K slice of the step's operand (h of step s-1, or the gate errors of step s-1 of the walk) and
-//             of the recurrent weight panels, 32 floats of K per stage, hi and cross panels
-//   warp 1    one lane issues tcgen05.mma (TF32 hi*hi + one BF16 K=16 instruction for both cross terms) into tensor memory
-//   warps 4-11 take the partial sums out of tensor memory and exchange them inside the cluster: every thread pushes the
-//             columns that other CTAs finish into those CTAs' shared memory (distributed shared memory) and keeps its
-//             own; the sums are added in slice order (bitwise repeatable).  Each thread then finishes 8 cells of one batch
-//             row: gates, peepholes, cell state, zoneout keep (forward) or the gate errors (backward).  The operand
-//             panels of the next step are stored before the step barrier; the layer's arrays, which only later kernels
-//             read, after it.  What the cell needs from global memory is fetched before the wait for the tensor cores.
+//             of the recurrent weights, 64 of K per stage
+//   warp 1    one lane issues tcgen05.mma (h1*h0 + h0*h1 + h0*h0 per 16 of K) into a ring of accumulators in tensor memory
+//   warps 4-11 take the partial sums out of tensor memory, times the power of two of their operands' exponents, and exchange
+//             them inside the cluster: every thread pushes the columns that other CTAs finish into those CTAs' shared
+//             memory (distributed shared memory) and keeps its own; the sums are added in slice order (bitwise
+//             repeatable).  Each thread then finishes 8 cells of one batch row: gates, peepholes, cell state, zoneout keep
+//             (forward) or the gate errors (backward).  The operand panels of the next step are stored before the step
+//             barrier; the layer's arrays, which only later kernels read, after it.  What the cell needs from global
+//             memory is fetched before the wait for the tensor cores.
 //   step barrier: every CTA of a row of tiles counts itself in on a global counter when its results of step s are
 //             written; producers poll it before they load step s + 1.  Every wait in the kernel is bounded (about a
 //             second of SM clock): a wait that runs out sets the handle's error flag and an abort word that makes all
 //             other waits give up, the CTAs meet at their final barriers, free tensor memory and return.
 // The launch needs all its CTAs resident at once (they wait for each other): lstm_persistent_plan checks the tile count
 // against cudaOccupancyMaxActiveClusters and the layer falls back to one launch pair per step otherwise.
+#include "half_panels.cuh"
 #include "lstm.cuh"
 #include "panel_math.cuh"
 #include "tcgen05.cuh"
@@ -44,25 +50,25 @@ namespace myea {
 constexpr int PS_THREADS = 384;
 constexpr int PS_EPI_WARP0 = 4;
 constexpr int PS_EPI_THREADS = 256;
-constexpr int PS_TILE_BYTES = 128 * BK * 4;          // 128 operand rows x 128 bytes
-// shapes of the two kernels: BN columns per tile, SPLIT K slices (= CTAs per cluster)
+constexpr int PS_BK = 64;                            // K per stage
+constexpr int PS_A_BYTES = 128 * 128;                // 128 operand rows x 64 halves
+// shapes of the two kernels: BN columns per tile, SPLIT K slices (= CTAs per cluster), CHUNK stages per accumulator (the
+// K range over which all exponents are the same)
 template <int KIND> struct PsShape;
-template <> struct PsShape<1> { static constexpr int BN = 128, SPLIT = 2, STAGES = 3; };
-template <> struct PsShape<2> { static constexpr int BN = 64, SPLIT = 4, STAGES = 4; };
+template <> struct PsShape<1> { static constexpr int BN = 128, SPLIT = 2, STAGES = 3, CHUNK = 2; };
+template <> struct PsShape<2> { static constexpr int BN = 64, SPLIT = 4, STAGES = 4, CHUNK = 1; };
 template <int KIND> struct PsSmem {
   static constexpr int BN = PsShape<KIND>::BN, STAGES = PsShape<KIND>::STAGES;
-  static constexpr int B_BYTES = BN * BK * 4;
-  static constexpr int STAGE_BYTES = 2 * PS_TILE_BYTES + 2 * B_BYTES;  // A hi, A cross, B hi, B cross
+  static constexpr int B_BYTES = BN * 128;
+  static constexpr int STAGE_BYTES = 2 * PS_A_BYTES + 2 * B_BYTES;     // A h0, A h1, B h0, B h1
   static constexpr int RECV_OFFSET = STAGES * STAGE_BYTES;
   static constexpr int RECV_BYTES = (PsShape<KIND>::SPLIT - 1) * 128 * (BN / PsShape<KIND>::SPLIT) * 4;  // one slot per peer
   static constexpr int BAR_OFFSET = RECV_OFFSET + RECV_BYTES;
   static constexpr int TOTAL = BAR_OFFSET + 512 + 1024;                // barriers, peepholes, slack to align the base
-  // Accumulators in tensor memory, BN columns each, filled one after the other: every one takes the products of
-  // ACC_KB K blocks (or more when the K slice is longer than MAX_ACC of them), hi*hi and cross terms alike.  The tensor
-  // core truncates when it adds into an accumulator, so a chain of adds is kept to 64 instructions where the slice
-  // allows; and the exchange warps read an accumulator while the tensor core fills the next one.
+  // Accumulators in tensor memory, BN columns each, used as a ring: the exchange warps read one while the tensor core
+  // fills the next ones.
   static constexpr int TMEM_COLS = 512;
-  static constexpr int MAX_ACC = TMEM_COLS / BN, ACC_KB = 8;
+  static constexpr int ACCS = TMEM_COLS / BN;
   static_assert(TOTAL <= 227 * 1024, "shared memory of one SM");
   static_assert(STAGE_BYTES % 1024 == 0 && B_BYTES % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
 };
@@ -72,12 +78,14 @@ struct LstmSeq {
   int reverse = 0;              // the direction's time runs from T-1 down to 0
   int tiles_m = 0, tiles_n = 0;
   int split = 1;                // CTAs per cluster = K slices per tile
-  int kb_per = 0, num_kb = 0;   // 32-float K blocks per slice / in all
+  int kb_per = 0, num_kb = 0;   // stages of K per slice / in all
   long long ldh = 0;            // pitch of the layer's output / error rows
   long long a_rows = 0;         // rows of one of the two operand-panel buffers (a multiple of 128)
   long long kpa = 0;            // pitch of the operand panels
-  long long Cp = 0;
-  float *a_hi = nullptr, *a_cross = nullptr;  // [2][a_rows][kpa]: step s reads buffer (s-1)&1 and writes buffer s&1
+  uint16_t *a0 = nullptr, *a1 = nullptr;      // [2][a_rows][kpa]: step s reads buffer (s-1)&1 and writes buffer s&1
+  int *a_exp = nullptr;                       // backward: [2][tiles_m][num_kb] exponents of the gate errors
+  const int *w_exp = nullptr;                 // exponents of the weights, [gate rows / 128][cells / 128]
+  long long w_exp_pitch = 0;
   const float *peep = nullptr;                // [3][C]
   const float *gates_in = nullptr;            // [T*B, 4C]
   float *act = nullptr, *cstate = nullptr, *cact = nullptr;
@@ -94,11 +102,11 @@ template <int KIND>
 __device__ __forceinline__ LstmStep step_view(const LstmSeq &q, int s) {
   LstmStep p;
   const long long B = q.B, C = q.C, T = q.T;
-  p.C = C; p.ldh = q.ldh; p.kp = q.kpa; p.Cp = q.Cp;
+  p.C = C; p.ldh = q.ldh; p.kp = q.kpa;
   p.peep = q.peep;
   if (s + 1 < q.T) {
-    p.p_hi = q.a_hi + static_cast<long long>(s & 1) * q.a_rows * q.kpa;
-    p.p_cross = q.a_cross + static_cast<long long>(s & 1) * q.a_rows * q.kpa;
+    p.p_h0 = q.a0 + static_cast<long long>(s & 1) * q.a_rows * q.kpa;
+    p.p_h1 = q.a1 + static_cast<long long>(s & 1) * q.a_rows * q.kpa;
   }
   if (KIND == 1) {
     const long long t = q.reverse ? T - 1 - s : s, tp = q.reverse ? t + 1 : t - 1;
@@ -119,7 +127,7 @@ __device__ __forceinline__ LstmStep step_view(const LstmSeq &q, int s) {
     p.b_act = q.act + t * B * 4 * C;
     p.b_cact = q.cact + t * B * C;
     p.b_c_prev = (tp >= 0 && tp < T) ? q.cstate + tp * B * C : nullptr;
-    p.act_next = q.act + tn * B * 4 * C;
+    p.act_next = (tn >= 0 && tn < T) ? q.act + tn * B * 4 * C : nullptr;
     p.dgates_next = q.dgates + tn * B * 4 * C;
     p.dc_next = q.dcstate + tn * B * C;
     p.dgates = q.dgates + t * B * 4 * C;
@@ -158,10 +166,10 @@ __device__ __forceinline__ bool wait_step_counter(const unsigned int *counter, u
 
 template <int KIND>
 __global__ void __launch_bounds__(PS_THREADS, 1)
-lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ CUtensorMap tm_a_x,
-                       const __grid_constant__ CUtensorMap tm_b_hi, const __grid_constant__ CUtensorMap tm_b_x, const LstmSeq q) {
+lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_constant__ CUtensorMap tm_a1,
+                       const __grid_constant__ CUtensorMap tm_b0, const __grid_constant__ CUtensorMap tm_b1, const LstmSeq q) {
   using SM = PsSmem<KIND>;
-  constexpr int STAGES = SM::STAGES, BN = SM::BN, S = PsShape<KIND>::SPLIT;
+  constexpr int STAGES = SM::STAGES, BN = SM::BN, S = PsShape<KIND>::SPLIT, CHUNK = PsShape<KIND>::CHUNK, ACCS = SM::ACCS;
   constexpr int W = BN / S;   // columns of the tile this CTA finishes: 16 cells (x 4 gates forward)
   extern __shared__ uint8_t smem_raw[];
   // the dynamic shared-memory window starts at the same offset in every CTA of the cluster, so the aligned offsets
@@ -170,13 +178,14 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid
   float *recv = reinterpret_cast<float *>(smem + SM::RECV_OFFSET);  // [S - 1 peers][128 rows][W]: partial sums pushed by the peers
   uint64_t *full_bar = reinterpret_cast<uint64_t *>(smem + SM::BAR_OFFSET);
   uint64_t *empty_bar = full_bar + STAGES;
-  uint64_t *acc_full = empty_bar + STAGES;   // [MAX_ACC] accumulator a of the step is complete
-  uint64_t *acc_empty = acc_full + SM::MAX_ACC;  // the 8 exchange warps have read tensor memory
-  uint64_t *red_ready = acc_empty + 1;       // every exchange warp of every peer has pushed its partial sums for this CTA
+  uint64_t *acc_full = empty_bar + STAGES;   // [ACCS] an accumulator is complete
+  uint64_t *acc_empty = acc_full + ACCS;     // [ACCS] the 8 exchange warps have read it
+  uint64_t *red_ready = acc_empty + ACCS;    // every exchange warp of every peer has pushed its partial sums for this CTA
   uint64_t *step_go = red_ready + 1;         // the producer has passed the step barrier
   uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(step_go + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
-  float *peep_s = reinterpret_cast<float *>(smem + SM::BAR_OFFSET + 256);  // [3][16] peepholes of this CTA's cells
+  int *amax_s = reinterpret_cast<int *>(tmem_holder + 2);                  // backward: largest gate error of each warp (bits of a float)
+  float *peep_s = reinterpret_cast<float *>(smem + SM::BAR_OFFSET + 320);  // [3][16] peepholes of this CTA's cells
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = ptx::cluster_ctarank();
@@ -185,8 +194,7 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid
   const int m0 = tile_m * 128, n0 = tile_n * BN;
   const int kb0 = min(static_cast<int>(rank) * q.kb_per, q.num_kb), kb1 = min(kb0 + q.kb_per, q.num_kb);
   const int my_kb = kb1 - kb0;
-  const int acc_kb = max(SM::ACC_KB, (q.kb_per + SM::MAX_ACC - 1) / SM::MAX_ACC);  // K blocks per accumulator
-  const int nacc = (my_kb + acc_kb - 1) / acc_kb;                                    // accumulators this CTA fills per step
+  const int nacc = (my_kb + CHUNK - 1) / CHUNK;   // accumulators this CTA fills per step
   unsigned int *counter = q.sync + tile_m;
   unsigned int *abort_word = q.sync + q.tiles_m;
   const unsigned int per_step = static_cast<unsigned int>(q.tiles_n * S);  // CTAs that complete a row of tiles
@@ -196,8 +204,10 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid
       ptx::mbar_init(&full_bar[s], 1);
       ptx::mbar_init(&empty_bar[s], 1);
     }
-    for (int a = 0; a < SM::MAX_ACC; ++a) ptx::mbar_init(&acc_full[a], 1);
-    ptx::mbar_init(acc_empty, 8);
+    for (int a = 0; a < ACCS; ++a) {
+      ptx::mbar_init(&acc_full[a], 1);
+      ptx::mbar_init(&acc_empty[a], 8);
+    }
     ptx::mbar_init(red_ready, static_cast<uint32_t>(8 * (S - 1)));
     ptx::mbar_init(step_go, 1);
     *abort_flag = 0;
@@ -221,11 +231,8 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid
     if (lane == 0) {
       bool ok = true;
       for (int s = 1; s < q.T && ok; ++s) {
-        // the panels this step reads: left by the kernels before this launch (s == 1) or by step s - 1 of this launch
-        if (s > 1) {
-          if (!wait_step_counter(counter, per_step * static_cast<unsigned int>(s - 1), abort_word, abort_flag)) { ok = false; break; }
-          ptx::mbar_arrive_local(step_go);
-        }
+        if (!wait_step_counter(counter, per_step * static_cast<unsigned int>(s), abort_word, abort_flag)) { ok = false; break; }
+        ptx::mbar_arrive_local(step_go);
         ptx::fence_proxy_async_global();  // the other CTAs wrote them with ordinary stores; TMA reads through the async proxy
         const int a_row = ((s - 1) & 1) * static_cast<int>(q.a_rows) + m0;
         for (int kb = kb0; kb < kb1; ++kb, ++issued) {
@@ -234,10 +241,16 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid
           if (!ptx::mbar_wait_or_abort(&empty_bar[st], ph ^ 1u, abort_flag)) { ok = false; break; }
           uint8_t *dst = smem + st * SM::STAGE_BYTES;
           ptx::mbar_arrive_expect_tx(&full_bar[st], SM::STAGE_BYTES);
-          ptx::tma_load_2d(dst, &tm_a_hi, &full_bar[st], kb * BK, a_row);
-          ptx::tma_load_2d(dst + PS_TILE_BYTES, &tm_a_x, &full_bar[st], kb * BK, a_row);
-          ptx::tma_load_2d(dst + 2 * PS_TILE_BYTES, &tm_b_hi, &full_bar[st], kb * BK, n0);
-          ptx::tma_load_2d(dst + 2 * PS_TILE_BYTES + SM::B_BYTES, &tm_b_x, &full_bar[st], kb * BK, n0);
+          ptx::tma_load_2d(dst, &tm_a0, &full_bar[st], kb * PS_BK, a_row);
+          ptx::tma_load_2d(dst + PS_A_BYTES, &tm_a1, &full_bar[st], kb * PS_BK, a_row);
+          uint8_t *dst_b = dst + 2 * PS_A_BYTES;
+          if constexpr (KIND == 1) {
+            ptx::tma_load_2d(dst_b, &tm_b0, &full_bar[st], kb * PS_BK, n0);
+            ptx::tma_load_2d(dst_b + SM::B_BYTES, &tm_b1, &full_bar[st], kb * PS_BK, n0);
+          } else {
+            ptx::tma_load_3d(dst_b, &tm_b0, &full_bar[st], 0, kb * PS_BK, n0 >> 6);
+            ptx::tma_load_3d(dst_b + SM::B_BYTES, &tm_b1, &full_bar[st], 0, kb * PS_BK, n0 >> 6);
+          }
         }
       }
       if (!ok) {
@@ -250,36 +263,37 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid
     ptx::reg_release<40>();
     if (lane == 0) {
       bool ok = true;
-      constexpr uint32_t idesc_main = make_idesc_tf32(128, BN);
-      constexpr uint32_t idesc_cross = make_idesc_bf16(128, BN);
-      uint32_t it = 0;
+      constexpr uint32_t idesc = make_idesc_f16(128, BN, false, KIND == 2);
+      constexpr uint64_t b_step = KIND == 2 ? 128 : 2;
+      uint32_t it = 0, n = 0;  // stages consumed, accumulators filled
       for (int s = 1; s < q.T && ok; ++s) {
-        if (s > 1) {  // tensor memory still holds step s - 1 until the exchange warps have read it
-          if (!ptx::mbar_wait_or_abort(acc_empty, static_cast<uint32_t>(s - 2) & 1u, abort_flag)) { ok = false; break; }
-          ptx::tc_fence_after();
-        }
-        int in_acc = 0, acc = 0;  // K blocks issued into the current accumulator, its index
-        for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
-          const int st = static_cast<int>(it % STAGES);
-          const uint32_t ph = (it / STAGES) & 1u;
-          if (!ptx::mbar_wait_or_abort(&full_bar[st], ph, abort_flag)) { ok = false; break; }
-          ptx::tc_fence_after();
-          const uint32_t base = ptx::smem_u32(smem + st * SM::STAGE_BYTES);
-          const uint64_t a_hi = make_smem_desc(base), a_x = make_smem_desc(base + PS_TILE_BYTES);
-          const uint64_t b_hi = make_smem_desc(base + 2 * PS_TILE_BYTES), b_x = make_smem_desc(base + 2 * PS_TILE_BYTES + SM::B_BYTES);
-          const uint32_t t_acc = tmem_base + static_cast<uint32_t>(acc * BN);
+        for (int c = 0; c < nacc && ok; ++c, ++n) {
+          const uint32_t a = n % ACCS, use = n / ACCS;
+          if (use > 0) {
+            if (!ptx::mbar_wait_or_abort(&acc_empty[a], (use - 1u) & 1u, abort_flag)) { ok = false; break; }
+            ptx::tc_fence_after();
+          }
+          const uint32_t t_acc = tmem_base + a * static_cast<uint32_t>(BN);
+          const int kb_end = min(kb0 + (c + 1) * CHUNK, kb1);
+          for (int kb = kb0 + c * CHUNK; kb < kb_end; ++kb, ++it) {
+            const int st = static_cast<int>(it % STAGES);
+            const uint32_t ph = (it / STAGES) & 1u;
+            if (!ptx::mbar_wait_or_abort(&full_bar[st], ph, abort_flag)) { ok = false; break; }
+            ptx::tc_fence_after();
+            const uint32_t base = ptx::smem_u32(smem + st * SM::STAGE_BYTES), base_b = base + 2 * PS_A_BYTES;
+            const uint64_t a0 = make_smem_desc(base), a1 = make_smem_desc(base + PS_A_BYTES);
+            const uint64_t b0 = KIND == 2 ? make_smem_desc_mn(base_b, 8192, false) : make_smem_desc(base_b);
+            const uint64_t b1 = KIND == 2 ? make_smem_desc_mn(base_b + SM::B_BYTES, 8192, false) : make_smem_desc(base_b + SM::B_BYTES);
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            const uint64_t koff = static_cast<uint64_t>((k * UMMA_K * 4) >> 4);
-            ptx::mma_bf16(t_acc, a_x + koff, b_x + koff, idesc_cross, (in_acc > 0 || k > 0) ? 1u : 0u);  // lo*hi + hi*lo
-            ptx::mma_tf32(t_acc, a_hi + koff, b_hi + koff, idesc_main, 1u);                                  // hi*hi
+            for (int k = 0; k < PS_BK / 16; ++k) {
+              const uint64_t ka = static_cast<uint64_t>(k) * 2, kbo = static_cast<uint64_t>(k) * b_step;
+              ptx::mma_bf16(t_acc, a1 + ka, b0 + kbo, idesc, (kb > kb0 + c * CHUNK || k > 0) ? 1u : 0u);
+              ptx::mma_bf16(t_acc, a0 + ka, b1 + kbo, idesc, 1u);
+              ptx::mma_bf16(t_acc, a0 + ka, b0 + kbo, idesc, 1u);
+            }
+            ptx::tc_commit(&empty_bar[st]);
           }
-          ptx::tc_commit(&empty_bar[st]);
-          if (++in_acc == acc_kb || kb + 1 == kb1) {
-            ptx::tc_commit(&acc_full[acc]);
-            ++acc;
-            in_acc = 0;
-          }
+          if (ok) ptx::tc_commit(&acc_full[a]);
         }
       }
       if (!ok) {
@@ -314,120 +328,150 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid
     using Out = typename std::conditional<KIND == 1, LstmForwardOut, LstmBackwardOut>::type;
     Out out;               // results of the step before; its arrays are written once the step barrier has been passed
     bool pending = false;
+    uint32_t n = 0;        // accumulators read so far
     auto store_arrays = [&](int step) {
       const LstmStep pp = step_view<KIND>(q, step);
       if constexpr (KIND == 1) lstm_forward_store_arrays8(pp, out, b, cell0);
       else lstm_backward_store_arrays8(pp, out, b, cell0);
     };
-    for (int s = 1; s < q.T; ++s) {
+    for (int s = 0; s < q.T; ++s) {
       bool ok = true;
       const LstmStep p = step_view<KIND>(q, s);
       In in;
       if (active) {
         // what the cell needs from global memory goes out before any wait; what this thread computed itself in the step
         // before (and has not written yet) comes from its registers
-        if (!pending) {
-          if constexpr (KIND == 1) lstm_forward_load8<true, false>(p, in, b, cell0);
-          else lstm_backward_load8<true, false>(p, in, b, cell0);
+        if constexpr (KIND == 1) {
+          lstm_forward_load8<false, false>(p, in, b, cell0);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) { in.cp[i] = s > 0 ? out.cs[i] : 0.f; in.hp[i] = s > 0 ? out.h[i] : 0.f; }
         } else {
-          if constexpr (KIND == 1) {
-            lstm_forward_load8<false, false>(p, in, b, cell0);
+          lstm_backward_load8<false, false>(p, in, b, cell0);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) { in.cp[i] = out.cs[i]; in.hp[i] = out.h[i]; }
-          } else {
-            lstm_backward_load8<false, false>(p, in, b, cell0);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) { in.dni[i] = out.di[i]; in.dnf[i] = out.df[i]; in.dcn[i] = out.dc[i]; }
-          }
+          for (int i = 0; i < 8; ++i) { in.dni[i] = s > 0 ? out.di[i] : 0.f; in.dnf[i] = s > 0 ? out.df[i] : 0.f; in.dcn[i] = s > 0 ? out.dc[i] : 0.f; }
         }
       }
       if (pending) {
         // the arrays of step s - 1 (read by later kernels only) leave now, beside this step's operand stream, and not
         // while the step barrier is in flight: 128 CTAs storing at once slowed the barrier down by microseconds
-        if (!ptx::mbar_wait_or_abort(step_go, static_cast<uint32_t>(s - 2) & 1u, abort_flag)) ok = false;
+        if (!ptx::mbar_wait_or_abort(step_go, static_cast<uint32_t>(s - 1) & 1u, abort_flag)) ok = false;
         if (ok && active) store_arrays(s - 1);
         pending = false;
       }
-      // Partial sums of this CTA's K slice: for every CTA d of the cluster the columns of d's cells that belong to this
-      // thread's (row, half), added up over the accumulators as the tensor core completes them (part[S - 1] is this
-      // CTA's own share, the others go to the peers in the order rank + 1, rank + 2, ...)
-      float part[S][HW];
+      float rec[HW];
 #pragma unroll
-      for (int dd = 0; dd < S; ++dd)
+      for (int i = 0; i < HW; ++i) rec[i] = 0.f;
+      if (s > 0) {
+        // Partial sums of this CTA's K slice: for every CTA d of the cluster the columns of d's cells that belong to this
+        // thread's (row, half), added up over the accumulators as the tensor core completes them (part[S - 1] is this
+        // CTA's own share, the others go to the peers in the order rank + 1, rank + 2, ...).  Forward: column g * 16 + cell
+        // of a CTA's 64, kept as [gate][8 cells].
+        float part[S][HW];
 #pragma unroll
-        for (int j = 0; j < HW; ++j) part[dd][j] = 0.f;
-      for (int a = 0; a < nacc && ok; ++a) {
-        if (!ptx::mbar_wait_or_abort(&acc_full[a], static_cast<uint32_t>(s - 1) & 1u, abort_flag)) { ok = false; break; }
-        ptx::tc_fence_after();
+        for (int dd = 0; dd < S; ++dd)
 #pragma unroll
-        for (int dd = 1; dd <= S; ++dd) {
-          const int d = (static_cast<int>(rank) + dd) % S;
-          uint32_t r[HW];
-          const uint32_t t0 = tmem_base + (static_cast<uint32_t>(qd * 32) << 16) + static_cast<uint32_t>(a * BN + d * W + half * HW);
-          if constexpr (HW == 32) ptx::tmem_ld_32x32(t0, r);
-          else ptx::tmem_ld_32x8(t0, r);
-          ptx::tmem_ld_wait();
+          for (int j = 0; j < HW; ++j) part[dd][j] = 0.f;
+        for (int c = 0; c < nacc && ok; ++c, ++n) {
+          const uint32_t a = n % ACCS;
+          const int kb = kb0 + c * CHUNK;
+          int e;
+          if constexpr (KIND == 1) e = LSTM_H_EXPONENT + __ldg(q.w_exp + tile_n * q.w_exp_pitch + (kb >> 1));
+          else e = __ldcg(q.a_exp + (static_cast<long long>((s - 1) & 1) * q.tiles_m + tile_m) * q.num_kb + kb) + __ldg(q.w_exp + (kb >> 1) * q.w_exp_pitch + (tile_n >> 1));
+          if (!ptx::mbar_wait_or_abort(&acc_full[a], (n / ACCS) & 1u, abort_flag)) { ok = false; break; }
+          ptx::tc_fence_after();
+          const int e1 = max(-126, min(127, e)), e2 = max(-126, min(127, e - e1));
+          const float s1 = pow2(e1), s2 = pow2(e2);
+          const uint32_t tq = tmem_base + (static_cast<uint32_t>(qd * 32) << 16) + a * static_cast<uint32_t>(BN);
 #pragma unroll
-          for (int j = 0; j < HW; ++j) part[dd - 1][j] += __uint_as_float(r[j]);
+          for (int dd = 1; dd <= S; ++dd) {
+            const int d = (static_cast<int>(rank) + dd) % S;
+            uint32_t r[HW / 8][8];
+#pragma unroll
+            for (int k = 0; k < HW / 8; ++k) ptx::tmem_ld_32x8(tq + static_cast<uint32_t>(d * W + k * 16 + half * 8), r[k]);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < HW; ++j) {
+              const float x = __uint_as_float(r[j / 8][j % 8]);
+              part[dd - 1][j] = fmaf(e2 == 0 ? x : x * s2, s1, part[dd - 1][j]);
+            }
+          }
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive_local(&acc_empty[a]);
         }
-      }
-      if (ok) {
-        // the peers' shares are pushed into their receive slots, this CTA's own share stays in registers
+        if (ok) {
+          // the peers' shares are pushed into their receive slots, this CTA's own share stays in registers
 #pragma unroll
-        for (int dd = 1; dd < S; ++dd) {
-          const int d = (static_cast<int>(rank) + dd) % S;
-          const int slot = static_cast<int>(rank) < d ? static_cast<int>(rank) : static_cast<int>(rank) - 1;
-          const uint32_t dst = ptx::map_to_cta(recv_addr + static_cast<uint32_t>((slot * 128 + row) * W * 4), static_cast<uint32_t>(d));
+          for (int dd = 1; dd < S; ++dd) {
+            const int d = (static_cast<int>(rank) + dd) % S;
+            const int slot = static_cast<int>(rank) < d ? static_cast<int>(rank) : static_cast<int>(rank) - 1;
+            const uint32_t dst = ptx::map_to_cta(recv_addr + static_cast<uint32_t>((slot * 128 + row) * W * 4), static_cast<uint32_t>(d));
 #pragma unroll
-          for (int i = 0; i < HW / 4; ++i)
-            ptx::st_cluster_f4(dst + (static_cast<uint32_t>((half * (HW / 4) + i) ^ swz) << 4),
-                               make_float4(part[dd - 1][4 * i], part[dd - 1][4 * i + 1], part[dd - 1][4 * i + 2], part[dd - 1][4 * i + 3]));
+            for (int i = 0; i < HW / 4; ++i)
+              ptx::st_cluster_f4(dst + (static_cast<uint32_t>((half * (HW / 4) + i) ^ swz) << 4),
+                                 make_float4(part[dd - 1][4 * i], part[dd - 1][4 * i + 1], part[dd - 1][4 * i + 2], part[dd - 1][4 * i + 3]));
+          }
+          __syncwarp();
+          if (lane == 0) {
+#pragma unroll
+            for (int dd = 1; dd < S; ++dd) ptx::mbar_arrive_release_cluster(red_ready, (rank + static_cast<uint32_t>(dd)) % S);
+          }
+          if (!ptx::mbar_wait_cluster_or_abort(red_ready, static_cast<uint32_t>(s - 1) & 1u, abort_flag)) ok = false;
         }
-        ptx::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) {
-          ptx::mbar_arrive_local(acc_empty);
+        if (ok) {
+          // the sums over the K slices, added in slice order whichever CTA adds them (bitwise repeatable)
 #pragma unroll
-          for (int dd = 1; dd < S; ++dd) ptx::mbar_arrive_release_cluster(red_ready, (rank + static_cast<uint32_t>(dd)) % S);
-        }
-        if (!ptx::mbar_wait_cluster_or_abort(red_ready, static_cast<uint32_t>(s - 1) & 1u, abort_flag)) ok = false;
-      }
-      if (ok) {
-        // the sums over the K slices, added in slice order whichever CTA adds them (bitwise repeatable)
-        float rec[HW];
+          for (int j = 0; j < S; ++j) {
+            if (j == static_cast<int>(rank)) {
 #pragma unroll
-        for (int i = 0; i < HW; ++i) rec[i] = 0.f;
+              for (int i = 0; i < HW; ++i) rec[i] += part[S - 1][i];
+            } else {
+              const int slot = j < static_cast<int>(rank) ? j : j - 1;
+              const float *src = recv + (slot * 128 + row) * W;
+              float4 v[HW / 4];
 #pragma unroll
-        for (int j = 0; j < S; ++j) {
-          if (j == static_cast<int>(rank)) {
+              for (int i = 0; i < HW / 4; ++i) v[i] = *reinterpret_cast<const float4 *>(src + (((half * (HW / 4) + i) ^ swz) << 2));
 #pragma unroll
-            for (int i = 0; i < HW; ++i) rec[i] += part[S - 1][i];
-          } else {
-            const int slot = j < static_cast<int>(rank) ? j : j - 1;
-            const float *src = recv + (slot * 128 + row) * W;
-            float4 v[HW / 4];
-#pragma unroll
-            for (int i = 0; i < HW / 4; ++i) v[i] = *reinterpret_cast<const float4 *>(src + (((half * (HW / 4) + i) ^ swz) << 2));
-#pragma unroll
-            for (int i = 0; i < HW / 4; ++i) { rec[4 * i] += v[i].x; rec[4 * i + 1] += v[i].y; rec[4 * i + 2] += v[i].z; rec[4 * i + 3] += v[i].w; }
+              for (int i = 0; i < HW / 4; ++i) { rec[4 * i] += v[i].x; rec[4 * i + 1] += v[i].y; rec[4 * i + 2] += v[i].z; rec[4 * i + 3] += v[i].w; }
+            }
           }
         }
+      }
+      float m = 0.f;   // backward: this thread's largest gate error
+      if (ok) {
         if (active) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) { in.pi[i] = peep_s[half * 8 + i]; in.pf[i] = peep_s[16 + half * 8 + i]; in.po[i] = peep_s[32 + half * 8 + i]; }
-          // the cell; only what the NEXT step's contraction reads (the operand panels) leaves before the step barrier
-          if constexpr (KIND == 1) {
-            lstm_forward_compute8(in, rec, out);
-            lstm_forward_store_panels8(p, out, b, cell0);
-          } else {
-            lstm_backward_compute8(in, rec, p.b_c_prev != nullptr, out);
-            lstm_backward_store_panels8(p, out, b, cell0);
-          }
         }
-        // this thread's panel stores come before the TMA copies that the step barrier lets loose (generic -> async proxy)
-        ptx::fence_proxy_async_global();
+        // the cell; only what the NEXT step's contraction reads (the operand panels) leaves before the step barrier
+        if constexpr (KIND == 1) {
+          if (active) {
+            lstm_forward_compute8(in, rec, s == 0, out);
+            if (p.p_h0 != nullptr) lstm_store_h_panels8(p, out.h, b, cell0);
+          }
+        } else if (active) {
+          lstm_backward_compute8(in, rec, p.b_c_prev != nullptr, out);
+          m = amax8(out.dz, amax8(out.di, amax8(out.df, amax8(out.d_o, 0.f))));
+        }
         pending = true;
       }
+      if constexpr (KIND == 2) {
+        if (p.p_h0 != nullptr) {
+          // one exponent for this CTA's 128 rows x 16 cells x 4 gates (a warp that gave up takes part: the barrier is for all)
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+          if (lane == 0) amax_s[warp - PS_EPI_WARP0] = __float_as_int(m);
+          ptx::named_barrier_sync(1, PS_EPI_THREADS);
+#pragma unroll
+          for (int w = 0; w < 8; ++w) m = fmaxf(m, __int_as_float(amax_s[w]));
+          const int e = half_exponent(m);
+          const int group = static_cast<int>(cta_cell0 >> 4);
+          if (warp == PS_EPI_WARP0 && lane == 0 && group < q.num_kb) q.a_exp[(static_cast<long long>(s & 1) * q.tiles_m + tile_m) * q.num_kb + group] = e;
+          if (active && ok) lstm_store_gate_panels8(p, out, pow2(-e), b, static_cast<long long>(group) * 64 + half * 8);
+        }
+      }
+      // this thread's panel stores come before the TMA copies that the step barrier lets loose (generic -> async proxy)
+      ptx::fence_proxy_async_global();
       if (!ok && lane == 0) {
         atomicCAS(q.error_flag, 0, 403);
         atomicExch(abort_word, 1u);
@@ -507,10 +551,10 @@ static int resident_clusters(int device) {
 int lstm_persistent_plan(myea_b200_net *net, LayerPlan &L) {
   LstmPlan *P = L.lstm;
   P->persist = nullptr;
-  if (!P->fuse || net->T < 2) return MYEA_OK;
+  if (P->C % 8 != 0 || net->ctx.gemm_engine != 0 || net->T < 2) return MYEA_OK;
   const long long B = net->B, C = P->C;
   const int tiles_m = static_cast<int>((B + 127) / 128);
-  const long long fwd_clusters = tiles_m * ((4 * C + PsShape<1>::BN - 1) / PsShape<1>::BN), bwd_clusters = tiles_m * ((C + PsShape<2>::BN - 1) / PsShape<2>::BN);
+  const long long fwd_clusters = tiles_m * ((P->G + PsShape<1>::BN - 1) / PsShape<1>::BN), bwd_clusters = tiles_m * ((C + PsShape<2>::BN - 1) / PsShape<2>::BN);
   const int fit_f = resident_clusters<1>(net->ctx.device), fit_b = resident_clusters<2>(net->ctx.device);
   if (fwd_clusters > fit_f || bwd_clusters > fit_b) return MYEA_OK;  // the CTAs of a launch wait for each other: all of them have to fit
   LstmPersistent *ps = new LstmPersistent();
@@ -532,13 +576,16 @@ void lstm_persistent_destroy(LstmPlan *P) {
 bool lstm_persistent_ready(const LstmPlan *P) { return P != nullptr && P->persist != nullptr && P->persist->ready; }
 
 template <int KIND>
-static int launch(myea_b200_net *net, LstmSeq &q, const float *a_hi, const float *a_cross, long long K, const Panels &w) {
+static int launch(myea_b200_net *net, LstmSeq &q, long long K, const HalfPanels &w) {
   Context &ctx = net->ctx;
+  // operand panels: both ping-pong buffers in one map (row coordinate = buffer * a_rows + tile row)
+  HalfOperand a;
+  a.p.h0 = q.a0; a.p.h1 = q.a1; a.p.R = 2 * q.a_rows; a.p.C = K; a.p.pitch = q.kpa;
+  a.rows = a.p.R; a.k = K;
+  const HalfOperand b = KIND == 1 ? half_rows(w) : half_cols(w);
   CUtensorMap maps[4];
-  // operand panels: both ping-pong buffers in one map (row coordinate = buffer * a_rows + tile row); weights: one box of
-  // 128 panel rows per tile of output columns
-  if (!make_panel_map(&maps[0], a_hi, 2 * q.a_rows, K, q.kpa, 128) || !make_panel_map(&maps[1], a_cross, 2 * q.a_rows, K, q.kpa, 128) ||
-      !make_panel_map(&maps[2], w.hi, w.rows, w.k, w.kp, PsShape<KIND>::BN) || !make_panel_map(&maps[3], w.lo, w.rows, w.k, w.kp, PsShape<KIND>::BN))
+  if (!make_half_map(&maps[0], a, a.p.h0, 128) || !make_half_map(&maps[1], a, a.p.h1, 128) || !make_half_map(&maps[2], b, w.h0, PsShape<KIND>::BN) ||
+      !make_half_map(&maps[3], b, w.h1, PsShape<KIND>::BN))
     return MYEA_E_CUDA;
   if (cudaMemsetAsync(q.sync, 0, (q.tiles_m + 1) * sizeof(unsigned int), ctx.stream) != cudaSuccess) return MYEA_E_CUDA;
   cudaLaunchConfig_t cfg = {};
@@ -560,57 +607,56 @@ static int launch(myea_b200_net *net, LstmSeq &q, const float *a_hi, const float
   return err == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
 
-int lstm_persistent_forward(myea_b200_net *net, LayerPlan &L, int dir, const Panels &w_rec_interleaved, const float *peep_compact, bool zoneout) {
+static void common_args(myea_b200_net *net, LayerPlan &L, int dir, LstmSeq &q) {
+  LstmPlan *P = L.lstm;
+  q.T = static_cast<int>(net->T); q.B = static_cast<int>(net->B); q.C = static_cast<int>(P->C);
+  q.reverse = dir;
+  q.tiles_m = P->persist->tiles_m;
+  q.ldh = L.n_out;
+  q.a_rows = P->persist->a_rows;
+  q.w_exp = P->w_rec[dir].exps;
+  q.w_exp_pitch = P->w_rec[dir].exp_r;
+  q.peep = P->peep_compact + static_cast<size_t>(dir) * 3 * P->C;
+  q.sync = P->persist->sync;
+  q.error_flag = net->ctx.d_error_flag;
+}
+
+int lstm_persistent_forward(myea_b200_net *net, LayerPlan &L, int dir, bool zoneout) {
   LstmPlan *P = L.lstm;
   if (!lstm_persistent_ready(P)) return MYEA_E_UNSUPPORTED;
   const LstmDir &D = P->d[dir];
   LstmSeq q;
-  q.T = static_cast<int>(net->T); q.B = static_cast<int>(net->B); q.C = static_cast<int>(P->C);
-  q.reverse = dir;
-  q.tiles_m = P->persist->tiles_m;
-  q.tiles_n = static_cast<int>((4 * P->C + PsShape<1>::BN - 1) / PsShape<1>::BN);
+  common_args(net, L, dir, q);
+  q.tiles_n = static_cast<int>((P->G + PsShape<1>::BN - 1) / PsShape<1>::BN);
   q.split = PsShape<1>::SPLIT;
-  q.num_kb = static_cast<int>((P->C + BK - 1) / BK);
-  q.kb_per = (q.num_kb + q.split - 1) / q.split;
-  q.ldh = L.n_out;
-  q.a_rows = P->persist->a_rows;
-  q.kpa = P->h_pan[0].kp;
-  q.a_hi = P->h_pan[0].hi; q.a_cross = P->h_pan[0].lo;
-  q.peep = peep_compact;
+  q.num_kb = static_cast<int>((P->C + PS_BK - 1) / PS_BK);
+  q.kb_per = ((q.num_kb + q.split - 1) / q.split + 1) / 2 * 2;   // slices start on the weights' blocks of 128
+  q.kpa = P->h_pan.pitch;
+  q.a0 = P->h_pan.h0; q.a1 = P->h_pan.h1;
   q.gates_in = D.gates_in; q.act = D.act; q.cstate = D.cstate; q.cact = D.cact;
   q.values = L.values + dir * P->C;
   q.zone_state = zoneout ? D.zone_state : nullptr;
   q.zone_output = zoneout ? D.zone_output : nullptr;
-  q.sync = P->persist->sync;
-  q.error_flag = net->ctx.d_error_flag;
-  return launch<1>(net, q, q.a_hi, q.a_cross, P->C, w_rec_interleaved);
+  return launch<1>(net, q, P->C, P->w_rec[dir]);
 }
 
-int lstm_persistent_backward(myea_b200_net *net, LayerPlan &L, int dir, const Panels &w_rec_transposed, const float *peep_compact) {
+int lstm_persistent_backward(myea_b200_net *net, LayerPlan &L, int dir) {
   LstmPlan *P = L.lstm;
   if (!lstm_persistent_ready(P)) return MYEA_E_UNSUPPORTED;
   const LstmDir &D = P->d[dir];
-  const long long Cp = (P->C + 7) & ~7ll;
   LstmSeq q;
-  q.T = static_cast<int>(net->T); q.B = static_cast<int>(net->B); q.C = static_cast<int>(P->C);
-  q.reverse = dir;
-  q.tiles_m = P->persist->tiles_m;
+  common_args(net, L, dir, q);
   q.tiles_n = static_cast<int>((P->C + PsShape<2>::BN - 1) / PsShape<2>::BN);
   q.split = PsShape<2>::SPLIT;
-  q.num_kb = static_cast<int>((4 * Cp + BK - 1) / BK);
+  q.num_kb = static_cast<int>(P->G / PS_BK);
   q.kb_per = (q.num_kb + q.split - 1) / q.split;
-  q.ldh = L.n_out;
-  q.a_rows = P->persist->a_rows;
-  q.kpa = P->dg_pan[0].kp;
-  q.Cp = Cp;
-  q.a_hi = P->dg_pan[0].hi; q.a_cross = P->dg_pan[0].lo;
-  q.peep = peep_compact;
+  q.kpa = P->dg_pan.pitch;
+  q.a0 = P->dg_pan.h0; q.a1 = P->dg_pan.h1;
+  q.a_exp = P->dg_exps;
   q.act = D.act; q.cstate = D.cstate; q.cact = D.cact;
   q.deriv = L.deriv + dir * P->C;
   q.dgates = D.dgates; q.dcstate = D.dcstate;
-  q.sync = P->persist->sync;
-  q.error_flag = net->ctx.d_error_flag;
-  return launch<2>(net, q, q.a_hi, q.a_cross, 4 * Cp, w_rec_transposed);
+  return launch<2>(net, q, P->G, P->w_rec[dir]);
 }
 
 }  // namespace myea
