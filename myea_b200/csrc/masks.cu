@@ -35,10 +35,18 @@ struct DrawStream {
   uint32_t seed_lo, seed_hi, step_lo, step_hi, stream;
 };
 
-__device__ __forceinline__ float draw_uniform(const DrawStream &s, unsigned long long element) {
-  uint32_t c[4] = {static_cast<uint32_t>(element >> 2), s.step_lo, s.step_hi, s.stream};
+// the four numbers of one block of the counter: elements 4 * block .. 4 * block + 3
+__device__ __forceinline__ float4 draw_uniform4(const DrawStream &s, uint32_t stream, unsigned long long block) {
+  uint32_t c[4] = {static_cast<uint32_t>(block), s.step_lo, s.step_hi, stream};
   philox4x32_10(c, s.seed_lo, s.seed_hi);
-  return static_cast<float>(c[element & 3ull] >> 8) * (1.0f / 16777216.0f);
+  constexpr float scale = 1.0f / 16777216.0f;
+  return make_float4(static_cast<float>(c[0] >> 8) * scale, static_cast<float>(c[1] >> 8) * scale, static_cast<float>(c[2] >> 8) * scale,
+                     static_cast<float>(c[3] >> 8) * scale);
+}
+__device__ __forceinline__ float draw_uniform(const DrawStream &s, unsigned long long element) {
+  const float4 u = draw_uniform4(s, s.stream, element >> 2);
+  const unsigned k = static_cast<unsigned>(element & 3ull);
+  return k == 0 ? u.x : k == 1 ? u.y : k == 2 ? u.z : u.w;
 }
 
 // out[i] = u(element(i)) < p ? below : other;  element(i) = (i / inner) * outer_pitch + offset + i % inner lets one
@@ -51,10 +59,24 @@ __global__ void draw_mask_kernel(uint8_t *__restrict__ out, long long n, float p
   out[i] = draw_uniform(s, static_cast<unsigned long long>(e)) < p ? below : other;
 }
 
-__global__ void draw_coefficient_kernel(float *__restrict__ out, long long n, float scale, float shift, const DrawStream s) {
+// All draws of one ShakeDrop layer: out_a = 2u - 1 and out_b = u per (sample, unit), the mask u < p per sample.  Bound by the
+// stores, so a thread makes whole counter blocks: 4 elements of both arrays per 2 Philox blocks and one 16-byte store each.
+// 2 x 4 Mi elements: 10 us in one launch (one block and one 4-byte store per element took three launches and 43 us).
+__global__ void draw_shakedrop_kernel(float *__restrict__ out_a, float *__restrict__ out_b, long long n, uint32_t stream_a, uint32_t stream_b,
+                                      uint8_t *__restrict__ mask, long long rows, float p, const DrawStream s) {
   const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-  if (i >= n) return;
-  out[i] = __fmaf_rn(scale, draw_uniform(s, static_cast<unsigned long long>(i)), shift);
+  if (i < rows) mask[i] = draw_uniform(s, static_cast<unsigned long long>(i)) < p ? 1 : 0;
+  if (4 * i >= n) return;
+  float4 a = draw_uniform4(s, stream_a, static_cast<unsigned long long>(i));
+  const float4 b = draw_uniform4(s, stream_b, static_cast<unsigned long long>(i));
+  a = make_float4(__fmaf_rn(2.0f, a.x, -1.0f), __fmaf_rn(2.0f, a.y, -1.0f), __fmaf_rn(2.0f, a.z, -1.0f), __fmaf_rn(2.0f, a.w, -1.0f));
+  if (4 * i + 4 <= n) {
+    reinterpret_cast<float4 *>(out_a)[i] = a;
+    reinterpret_cast<float4 *>(out_b)[i] = b;
+  } else {
+    const float va[4] = {a.x, a.y, a.z, a.w}, vb[4] = {b.x, b.y, b.z, b.w};
+    for (int k = 0; 4 * i + k < n; ++k) { out_a[4 * i + k] = va[k]; out_b[4 * i + k] = vb[k]; }
+  }
 }
 
 static unsigned blocks_for(long long n) { return static_cast<unsigned>((n + 255) / 256); }
@@ -100,12 +122,10 @@ extern "C" int myea_b200_generate_masks(myea_handle net, uint64_t seed, uint64_t
       const long long n = net->B * L.n_out;
       ctx.begin(TC_ELEMENTWISE);
       s.stream = static_cast<uint32_t>(8 * l + MYEA_MASK_SHAKEDROP);
-      draw_mask_kernel<<<blocks_for(net->B), 256, 0, ctx.stream>>>(L.shake_mask, net->B, L.desc.dropout_values[0], 1, 0, net->B, 0, 0, s);
-      s.stream = static_cast<uint32_t>(8 * l + MYEA_MASK_SHAKEDROP_ALPHA);
-      draw_coefficient_kernel<<<blocks_for(n), 256, 0, ctx.stream>>>(L.shake_alpha, n, 2.0f, -1.0f, s);
-      s.stream = static_cast<uint32_t>(8 * l + MYEA_MASK_SHAKEDROP_BETA);
-      draw_coefficient_kernel<<<blocks_for(n), 256, 0, ctx.stream>>>(L.shake_beta, n, 1.0f, 0.0f, s);
-      ctx.end(TC_ELEMENTWISE, 3);
+      draw_shakedrop_kernel<<<blocks_for(std::max((n + 3) / 4, net->B)), 256, 0, ctx.stream>>>(
+          L.shake_alpha, L.shake_beta, n, static_cast<uint32_t>(8 * l + MYEA_MASK_SHAKEDROP_ALPHA), static_cast<uint32_t>(8 * l + MYEA_MASK_SHAKEDROP_BETA),
+          L.shake_mask, net->B, L.desc.dropout_values[0], s);
+      ctx.end(TC_ELEMENTWISE);
     }
   }
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
