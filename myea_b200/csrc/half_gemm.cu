@@ -222,21 +222,27 @@ half_gemm_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_constan
       constexpr uint64_t a_step = A_COLS ? 128 : 2, b_step = B_COLS ? 128 : 2;
       uint32_t it = 0;  // k-blocks consumed so far
       uint32_t g = 0;   // K chunks issued so far: chunk g goes into buffer g & 1
+      // the barriers of the next K block are asked before this one's instructions are issued: while the tensor core reads its
+      // operands a look at shared memory takes hundreds of cycles, which would drain the short instruction queue
+      bool full_ok = false, acc_ok = false;
       WideSegments seg(work, cluster_id, num_clusters, num_chunks);
       while (ok && seg.next()) {
         for (int c = seg.c0; c < seg.c1 && ok; ++c, ++g) {
           const uint32_t b = g & 1u;
           if (g >= 2) {
-            if (!ptx::mbar_wait_or_abort(&acc_empty_bar[b], ((g >> 1) - 1u) & 1u, abort_flag)) { ok = false; break; }
+            if (!acc_ok && !ptx::mbar_wait_or_abort(&acc_empty_bar[b], ((g >> 1) - 1u) & 1u, abort_flag)) { ok = false; break; }
             ptx::tc_fence_after();
           }
+          acc_ok = false;
           const uint32_t acc = tmem_base + b * static_cast<uint32_t>(BN);
           const int kb_end = min(num_kb, (c + 1) * HG_KC);
           for (int kb = c * HG_KC; kb < kb_end; ++kb, ++it) {
             const int s = static_cast<int>(it % STAGES);
             const uint32_t ph = (it / STAGES) & 1u;
-            if (!ptx::mbar_wait_or_abort(&full_bar[s], ph, abort_flag)) { ok = false; break; }
+            if (!full_ok && !ptx::mbar_wait_or_abort(&full_bar[s], ph, abort_flag)) { ok = false; break; }
             ptx::tc_fence_after();
+            full_ok = ptx::mbar_test(&full_bar[(it + 1) % STAGES], ((it + 1) / STAGES) & 1u);
+            if (kb + 1 == kb_end && g >= 1) acc_ok = ptx::mbar_test(&acc_empty_bar[b ^ 1u], (((g + 1) >> 1) - 1u) & 1u);
             const uint32_t st = ptx::smem_u32(smem + s * S::STAGE_BYTES);
             const uint32_t sb = st + 2 * S::A_BYTES;
             const uint64_t a0 = A_COLS ? make_smem_desc_mn(st, 8192, false) : make_smem_desc(st);

@@ -225,32 +225,51 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
   const uint32_t tmem_base = *tmem_holder;
 
   uint32_t issued = 0;  // producer: K blocks staged so far (for the final drain)
+  int ahead_issued = 0; // of the next step: stages whose weights are on their way (not 0 only when a wait has given up)
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     ptx::reg_release<40>();
     if (lane == 0) {
       bool ok = true;
+      auto load_a = [&](uint32_t u, int kb, int a_row) {
+        uint8_t *dst = smem + (u % STAGES) * SM::STAGE_BYTES;
+        ptx::tma_load_2d(dst, &tm_a0, &full_bar[u % STAGES], kb * PS_BK, a_row);
+        ptx::tma_load_2d(dst + PS_A_BYTES, &tm_a1, &full_bar[u % STAGES], kb * PS_BK, a_row);
+      };
+      auto load_b = [&](uint32_t u, int kb) {
+        uint8_t *dst = smem + (u % STAGES) * SM::STAGE_BYTES + 2 * PS_A_BYTES;
+        if constexpr (KIND == 1) {
+          ptx::tma_load_2d(dst, &tm_b0, &full_bar[u % STAGES], kb * PS_BK, n0);
+          ptx::tma_load_2d(dst + SM::B_BYTES, &tm_b1, &full_bar[u % STAGES], kb * PS_BK, n0);
+        } else {
+          ptx::tma_load_3d(dst, &tm_b0, &full_bar[u % STAGES], 0, kb * PS_BK, n0 >> 6);
+          ptx::tma_load_3d(dst + SM::B_BYTES, &tm_b1, &full_bar[u % STAGES], 0, kb * PS_BK, n0 >> 6);
+        }
+      };
       for (int s = 1; s < q.T && ok; ++s) {
-        if (!wait_step_counter(counter, per_step * static_cast<unsigned int>(s), abort_word, abort_flag)) { ok = false; break; }
-        ptx::mbar_arrive_local(step_go);
+        // the weights of the step's first stages do not depend on the step before: they are on their way before the barrier
+        const int ahead = min(STAGES, my_kb);
+        for (int i = 0; i < ahead; ++i) {
+          const uint32_t u = issued + static_cast<uint32_t>(i);
+          if (!ptx::mbar_wait_or_abort(&empty_bar[u % STAGES], ((u / STAGES) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+          ptx::mbar_arrive_expect_tx(&full_bar[u % STAGES], SM::STAGE_BYTES);
+          load_b(u, kb0 + i);
+          ++ahead_issued;
+        }
+        if (!ok || !wait_step_counter(counter, per_step * static_cast<unsigned int>(s), abort_word, abort_flag)) { ok = false; break; }
         ptx::fence_proxy_async_global();  // the other CTAs wrote them with ordinary stores; TMA reads through the async proxy
         const int a_row = ((s - 1) & 1) * static_cast<int>(q.a_rows) + m0;
-        for (int kb = kb0; kb < kb1; ++kb, ++issued) {
-          const int st = static_cast<int>(issued % STAGES);
-          const uint32_t ph = (issued / STAGES) & 1u;
-          if (!ptx::mbar_wait_or_abort(&empty_bar[st], ph ^ 1u, abort_flag)) { ok = false; break; }
-          uint8_t *dst = smem + st * SM::STAGE_BYTES;
+        for (int i = 0; i < ahead; ++i) load_a(issued + static_cast<uint32_t>(i), kb0 + i, a_row);
+        issued += static_cast<uint32_t>(ahead);
+        ahead_issued = 0;
+        // only now may the other warps store the arrays of the step before: their stores would keep these copies waiting
+        ptx::mbar_arrive_local(step_go);
+        for (int kb = kb0 + ahead; kb < kb1; ++kb, ++issued) {
+          const uint32_t st = issued % STAGES;
+          if (!ptx::mbar_wait_or_abort(&empty_bar[st], ((issued / STAGES) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
           ptx::mbar_arrive_expect_tx(&full_bar[st], SM::STAGE_BYTES);
-          ptx::tma_load_2d(dst, &tm_a0, &full_bar[st], kb * PS_BK, a_row);
-          ptx::tma_load_2d(dst + PS_A_BYTES, &tm_a1, &full_bar[st], kb * PS_BK, a_row);
-          uint8_t *dst_b = dst + 2 * PS_A_BYTES;
-          if constexpr (KIND == 1) {
-            ptx::tma_load_2d(dst_b, &tm_b0, &full_bar[st], kb * PS_BK, n0);
-            ptx::tma_load_2d(dst_b + SM::B_BYTES, &tm_b1, &full_bar[st], kb * PS_BK, n0);
-          } else {
-            ptx::tma_load_3d(dst_b, &tm_b0, &full_bar[st], 0, kb * PS_BK, n0 >> 6);
-            ptx::tma_load_3d(dst_b + SM::B_BYTES, &tm_b1, &full_bar[st], 0, kb * PS_BK, n0 >> 6);
-          }
+          load_a(issued, kb, a_row);
+          load_b(issued, kb);
         }
       }
       if (!ok) {
@@ -266,20 +285,25 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
       constexpr uint32_t idesc = make_idesc_f16(128, BN, false, KIND == 2);
       constexpr uint64_t b_step = KIND == 2 ? 128 : 2;
       uint32_t it = 0, n = 0;  // stages consumed, accumulators filled
+      // the barriers of the next stage are asked before this one's instructions are issued (see half_gemm.cu)
+      bool full_ok = false, acc_ok = false;
       for (int s = 1; s < q.T && ok; ++s) {
         for (int c = 0; c < nacc && ok; ++c, ++n) {
           const uint32_t a = n % ACCS, use = n / ACCS;
           if (use > 0) {
-            if (!ptx::mbar_wait_or_abort(&acc_empty[a], (use - 1u) & 1u, abort_flag)) { ok = false; break; }
+            if (!acc_ok && !ptx::mbar_wait_or_abort(&acc_empty[a], (use - 1u) & 1u, abort_flag)) { ok = false; break; }
             ptx::tc_fence_after();
           }
+          acc_ok = false;
           const uint32_t t_acc = tmem_base + a * static_cast<uint32_t>(BN);
           const int kb_end = min(kb0 + (c + 1) * CHUNK, kb1);
           for (int kb = kb0 + c * CHUNK; kb < kb_end; ++kb, ++it) {
             const int st = static_cast<int>(it % STAGES);
             const uint32_t ph = (it / STAGES) & 1u;
-            if (!ptx::mbar_wait_or_abort(&full_bar[st], ph, abort_flag)) { ok = false; break; }
+            if (!full_ok && !ptx::mbar_wait_or_abort(&full_bar[st], ph, abort_flag)) { ok = false; break; }
             ptx::tc_fence_after();
+            full_ok = ptx::mbar_test(&full_bar[(it + 1) % STAGES], ((it + 1) / STAGES) & 1u);
+            if (kb + 1 == kb_end && n + 1 >= ACCS) acc_ok = ptx::mbar_test(&acc_empty[(n + 1) % ACCS], ((n + 1) / ACCS - 1u) & 1u);
             const uint32_t base = ptx::smem_u32(smem + st * SM::STAGE_BYTES), base_b = base + 2 * PS_A_BYTES;
             const uint64_t a0 = make_smem_desc(base), a1 = make_smem_desc(base + PS_A_BYTES);
             const uint64_t b0 = KIND == 2 ? make_smem_desc_mn(base_b, 8192, false) : make_smem_desc(base_b);
@@ -334,9 +358,16 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
       if constexpr (KIND == 1) lstm_forward_store_arrays8(pp, out, b, cell0);
       else lstm_backward_store_arrays8(pp, out, b, cell0);
     };
+    // power of two of the product of accumulator c's operands; asked for one accumulator ahead
+    auto exponent_of = [&](int step, int c) {
+      const int kb = kb0 + c * CHUNK;
+      if constexpr (KIND == 1) return LSTM_H_EXPONENT + __ldg(q.w_exp + tile_n * q.w_exp_pitch + (kb >> 1));
+      else return __ldcg(q.a_exp + (static_cast<long long>((step - 1) & 1) * q.tiles_m + tile_m) * q.num_kb + kb) + __ldg(q.w_exp + (kb >> 1) * q.w_exp_pitch + (tile_n >> 1));
+    };
     for (int s = 0; s < q.T; ++s) {
       bool ok = true;
       const LstmStep p = step_view<KIND>(q, s);
+      int e_next = 0;
       In in;
       if (active) {
         // what the cell needs from global memory goes out before any wait; what this thread computed itself in the step
@@ -355,6 +386,7 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
         // the arrays of step s - 1 (read by later kernels only) leave now, beside this step's operand stream, and not
         // while the step barrier is in flight: 128 CTAs storing at once slowed the barrier down by microseconds
         if (!ptx::mbar_wait_or_abort(step_go, static_cast<uint32_t>(s - 1) & 1u, abort_flag)) ok = false;
+        if (ok && nacc > 0) e_next = exponent_of(s, 0);
         if (ok && active) store_arrays(s - 1);
         pending = false;
       }
@@ -373,10 +405,8 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
           for (int j = 0; j < HW; ++j) part[dd][j] = 0.f;
         for (int c = 0; c < nacc && ok; ++c, ++n) {
           const uint32_t a = n % ACCS;
-          const int kb = kb0 + c * CHUNK;
-          int e;
-          if constexpr (KIND == 1) e = LSTM_H_EXPONENT + __ldg(q.w_exp + tile_n * q.w_exp_pitch + (kb >> 1));
-          else e = __ldcg(q.a_exp + (static_cast<long long>((s - 1) & 1) * q.tiles_m + tile_m) * q.num_kb + kb) + __ldg(q.w_exp + (kb >> 1) * q.w_exp_pitch + (tile_n >> 1));
+          const int e = e_next;
+          if (c + 1 < nacc) e_next = exponent_of(s, c + 1);
           if (!ptx::mbar_wait_or_abort(&acc_full[a], (n / ACCS) & 1u, abort_flag)) { ok = false; break; }
           ptx::tc_fence_after();
           const int e1 = max(-126, min(127, e)), e2 = max(-126, min(127, e - e1));
@@ -493,6 +523,13 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
     const uint32_t first = issued > static_cast<uint32_t>(STAGES) ? issued - STAGES : 0u;
     for (uint32_t i = first; i < issued; ++i) {
       if (!ptx::mbar_wait(&full_bar[i % STAGES], (i / STAGES) & 1u)) break;
+    }
+    // weights of a step that never began: their barriers cannot complete (the operand's bytes are missing), and copies of this
+    // GPU's own memory land within microseconds
+    if (ahead_issued > 0) {
+      const long long t0 = clock64();
+      while (clock64() - t0 < (1ll << 20)) {
+      }
     }
   }
   // peers may still be pushing into this CTA's receive slots or signalling its barriers: the cluster stays together until

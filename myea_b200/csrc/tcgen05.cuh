@@ -40,6 +40,22 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
   return ok != 0;
 }
 
+// Has the phase completed?  Never suspends: the answer is fetched ahead of the work that precedes the wait, so that the wait
+// itself costs nothing when the phase was complete by then.
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait: gives up after ~2^31 SM cycles (about a second). Returns false on timeout.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return true;
@@ -225,8 +241,8 @@ __device__ __forceinline__ bool mbar_try_wait_acquire_cluster(uint64_t *bar, uin
 }
 // bounded like mbar_wait; gives up at once when another wait of this CTA has already failed
 __device__ __forceinline__ bool mbar_wait_cluster_or_abort(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
-  if (*abort_flag) return false;
   if (mbar_try_wait_acquire_cluster(bar, parity)) return true;
+  if (*abort_flag) return false;
   const long long t0 = clock64();
   while (!mbar_try_wait_acquire_cluster(bar, parity)) {
     if (*abort_flag) return false;
@@ -269,6 +285,7 @@ __device__ __forceinline__ bool named_barrier_or(int id, int threads, bool pred)
 
 // Bounded wait that gives up at once when another wait of this CTA has already failed (keeps the worst case short).
 __device__ __forceinline__ bool mbar_wait_or_abort(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
+  if (mbar_try_wait(bar, parity)) return true;
   if (*abort_flag) return false;
   if (mbar_wait(bar, parity)) return true;
   *abort_flag = 1;
