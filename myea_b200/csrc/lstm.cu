@@ -72,17 +72,17 @@ __global__ void __launch_bounds__(256) lstm_cell_forward_kernel(const CellFwd p)
     const float cp = first ? 0.f : p.c_prev[b * p.C + c];
     const float sz = gi[c] + (first ? 0.f : sr[c]);
     const float si = gi[p.C + c] + (first ? 0.f : sr[p.C + c] + pi * cp);
-    const float z = tanh_ref(sz);
-    const float ig = sigmoid_ref(si);
+    const float z = tanh_cell(sz);
+    const float ig = sigmoid_cell(si);
     float fg = 0.f;
     float cs = z * ig;
     if (!first) {
-      fg = sigmoid_ref(gi[2 * p.C + c] + sr[2 * p.C + c] + pf * cp);
+      fg = sigmoid_cell(gi[2 * p.C + c] + sr[2 * p.C + c] + pf * cp);
       cs += fg * cp;
     }
     if (p.zone_state != nullptr && !p.zone_state[c]) cs = cp;  // cp is 0 at the first step
-    const float a = tanh_ref(cs);
-    const float og = sigmoid_ref(gi[3 * p.C + c] + (first ? 0.f : sr[3 * p.C + c]) + po * cs);
+    const float a = tanh_cell(cs);
+    const float og = sigmoid_cell(gi[3 * p.C + c] + (first ? 0.f : sr[3 * p.C + c]) + po * cs);
     float h = a * og;
     if (p.zone_output != nullptr && !p.zone_output[c]) h = first ? 0.f : p.h_prev[b * p.ldh + c];
     float *act = p.act + b * 4 * p.C;

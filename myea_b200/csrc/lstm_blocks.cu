@@ -87,20 +87,20 @@ __global__ void __launch_bounds__(128) lstm_blocks_forward_kernel(const BlocksFw
         sf = fmaf(p.peep[p.C + j], cp[j], sf);
       }
     }
-    const float ig = sigmoid_ref(si), fg = first ? 0.f : sigmoid_ref(sf);
+    const float ig = sigmoid_cell(si), fg = first ? 0.f : sigmoid_cell(sf);
     float *act = p.act + b * G;
     for (long long j = j0; j < j0 + p.cpb; ++j) {
-      const float z = tanh_ref(gi[j] + (first ? 0.f : sr[j]));
+      const float z = tanh_cell(gi[j] + (first ? 0.f : sr[j]));
       const float c_old = first ? 0.f : cp[j];
       float cs = z * ig;
       if (!first) cs += fg * c_old;
       if (p.zone_state != nullptr && !p.zone_state[j]) cs = c_old;
       act[j] = z;
       p.cstate[b * p.C + j] = cs;
-      p.cact[b * p.C + j] = tanh_ref(cs);
+      p.cact[b * p.C + j] = tanh_cell(cs);
       so = fmaf(p.peep[2 * p.C + j], cs, so);
     }
-    const float og = sigmoid_ref(so);
+    const float og = sigmoid_cell(so);
     act[p.C + k] = ig; act[p.C + p.K + k] = fg; act[p.C + 2 * p.K + k] = og;
     for (long long j = j0; j < j0 + p.cpb; ++j) {
       float h = p.cact[b * p.C + j] * og;

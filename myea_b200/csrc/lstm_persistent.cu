@@ -21,7 +21,7 @@
 //   warp 1    one lane issues tcgen05.mma (h1*h0 + h0*h1 + h0*h0 per 16 of K) into a ring of accumulators in tensor memory
 //   warps 4-11 take the partial sums out of tensor memory, times the power of two of their operands' exponents, and exchange
 //             them inside the cluster: every thread pushes the columns that other CTAs finish into those CTAs' shared
-//             memory (distributed shared memory) and keeps its own; the sums are added in slice order (bitwise
+//             memory (st.async: the receiver's barrier counts the bytes, the sender waits for nothing) and keeps its own; the sums are added in slice order (bitwise
 //             repeatable).  Each thread then finishes 8 cells of one batch row: gates, peepholes, cell state, zoneout keep
 //             (forward) or the gate errors (backward).  The operand panels of the next step are stored before the step
 //             barrier; the layer's arrays, which only later kernels read, after it.  What the cell needs from global
@@ -52,11 +52,15 @@ constexpr int PS_EPI_WARP0 = 4;
 constexpr int PS_EPI_THREADS = 256;
 constexpr int PS_BK = 64;                            // K per stage
 constexpr int PS_A_BYTES = 128 * 128;                // 128 operand rows x 64 halves
-// shapes of the two kernels: BN columns per tile, SPLIT K slices (= CTAs per cluster), CHUNK stages per accumulator (the
-// K range over which all exponents are the same)
+// shapes of the two kernels: BN columns per tile, SPLIT K slices (= CTAs per cluster), SETS of columns per accumulator: with
+// two, a0 * [b0 b1] is one instruction of twice the width (the two halves of the weights lie one behind the other in a stage),
+// so that a0 is read from shared memory once for both.  Shared memory is what these narrow tiles wait for: 128 bytes per clock
+// make 6 KB of operands per 128 x 64 x 16 product last 48 clocks where the product takes 32 (backward stage 1530 -> 1230
+// clocks).  At 128 columns operands and product take 64 alike, and two sets leave a ring of two accumulators that the exchange
+// warps do not empty in time (forward stage 1450 -> 1560 clocks).
 template <int KIND> struct PsShape;
-template <> struct PsShape<1> { static constexpr int BN = 128, SPLIT = 2, STAGES = 3, CHUNK = 2; };
-template <> struct PsShape<2> { static constexpr int BN = 64, SPLIT = 4, STAGES = 4, CHUNK = 1; };
+template <> struct PsShape<1> { static constexpr int BN = 128, SPLIT = 2, STAGES = 3, SETS = 1; };
+template <> struct PsShape<2> { static constexpr int BN = 64, SPLIT = 4, STAGES = 4, SETS = 2; };
 template <int KIND> struct PsSmem {
   static constexpr int BN = PsShape<KIND>::BN, STAGES = PsShape<KIND>::STAGES;
   static constexpr int B_BYTES = BN * 128;
@@ -65,10 +69,12 @@ template <int KIND> struct PsSmem {
   static constexpr int RECV_BYTES = (PsShape<KIND>::SPLIT - 1) * 128 * (BN / PsShape<KIND>::SPLIT) * 4;  // one slot per peer
   static constexpr int BAR_OFFSET = RECV_OFFSET + RECV_BYTES;
   static constexpr int TOTAL = BAR_OFFSET + 512 + 1024;                // barriers, peepholes, slack to align the base
-  // Accumulators in tensor memory, BN columns each, used as a ring: the exchange warps read one while the tensor core
-  // fills the next ones.
+  // Accumulators in tensor memory, used as a ring: the exchange warps read one while the tensor core fills the next ones.
+  // Two sets: h0 * h0 and the cross products.
   static constexpr int TMEM_COLS = 512;
-  static constexpr int ACCS = TMEM_COLS / BN;
+  static constexpr int ACC_COLS = PsShape<KIND>::SETS * BN;
+  static constexpr int ACCS = TMEM_COLS / ACC_COLS;
+  static_assert(STAGES <= 4, "a stage's done barrier is not reused before the stage is");
   static_assert(TOTAL <= 227 * 1024, "shared memory of one SM");
   static_assert(STAGE_BYTES % 1024 == 0 && B_BYTES % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
 };
@@ -103,16 +109,13 @@ __device__ __forceinline__ LstmStep step_view(const LstmSeq &q, int s) {
   LstmStep p;
   const long long B = q.B, C = q.C, T = q.T;
   p.C = C; p.ldh = q.ldh; p.kp = q.kpa;
-  p.peep = q.peep;
   if (s + 1 < q.T) {
     p.p_h0 = q.a0 + static_cast<long long>(s & 1) * q.a_rows * q.kpa;
     p.p_h1 = q.a1 + static_cast<long long>(s & 1) * q.a_rows * q.kpa;
   }
   if (KIND == 1) {
-    const long long t = q.reverse ? T - 1 - s : s, tp = q.reverse ? t + 1 : t - 1;
+    const long long t = q.reverse ? T - 1 - s : s;
     p.gates_in = q.gates_in + t * B * 4 * C;
-    p.c_prev = q.cstate + tp * B * C;
-    p.h_prev = q.values + tp * B * q.ldh;
     p.act = q.act + t * B * 4 * C;
     p.cstate = q.cstate + t * B * C;
     p.cact = q.cact + t * B * C;
@@ -121,15 +124,11 @@ __device__ __forceinline__ LstmStep step_view(const LstmSeq &q, int s) {
     p.zone_output = q.zone_output != nullptr ? q.zone_output + t * C : nullptr;
   } else {
     const long long t = q.reverse ? s : T - 1 - s;        // the walk goes against the direction
-    const long long tn = q.reverse ? t - 1 : t + 1;       // the step after t in the layer's direction (done before)
     const long long tp = q.reverse ? t + 1 : t - 1;       // the step before t
     p.dh = q.deriv + t * B * q.ldh;
     p.b_act = q.act + t * B * 4 * C;
     p.b_cact = q.cact + t * B * C;
     p.b_c_prev = (tp >= 0 && tp < T) ? q.cstate + tp * B * C : nullptr;
-    p.act_next = (tn >= 0 && tn < T) ? q.act + tn * B * 4 * C : nullptr;
-    p.dgates_next = q.dgates + tn * B * 4 * C;
-    p.dc_next = q.dcstate + tn * B * C;
     p.dgates = q.dgates + t * B * 4 * C;
     p.dcstate = q.dcstate + t * B * C;
   }
@@ -150,18 +149,18 @@ __device__ __forceinline__ void red_release_gpu_add(unsigned int *p, unsigned in
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Bounded wait for a step counter; gives up when any CTA has raised the abort word or after about a second.
+// Bounded wait for a step counter; gives up when any CTA has raised the abort word or after about a second.  The counter is
+// polled alone (the abort word every 64 looks: a second round trip per look delayed every step by half of it).
 __device__ __forceinline__ bool wait_step_counter(const unsigned int *counter, unsigned int target, const unsigned int *abort_word, volatile int *abort_flag) {
   if (*abort_flag) return false;
-  if (ld_acquire_gpu(counter) >= target) return true;
   const long long t0 = clock64();
-  for (;;) {
-    if (ld_acquire_gpu(counter) >= target) return true;
-    if (ld_relaxed_gpu(abort_word) != 0u || clock64() - t0 > (1ll << 31)) {
+  for (int look = 0; ld_relaxed_gpu(counter) < target; ++look) {
+    if ((look & 63) == 63 && (ld_relaxed_gpu(abort_word) != 0u || clock64() - t0 > (1ll << 31))) {
       *abort_flag = 1;
       return false;
     }
   }
+  return ld_acquire_gpu(counter) >= target;   // (orders what follows after the other CTAs' stores)
 }
 
 template <int KIND>
@@ -169,7 +168,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
 lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_constant__ CUtensorMap tm_a1,
                        const __grid_constant__ CUtensorMap tm_b0, const __grid_constant__ CUtensorMap tm_b1, const LstmSeq q) {
   using SM = PsSmem<KIND>;
-  constexpr int STAGES = SM::STAGES, BN = SM::BN, S = PsShape<KIND>::SPLIT, CHUNK = PsShape<KIND>::CHUNK, ACCS = SM::ACCS;
+  constexpr int STAGES = SM::STAGES, BN = SM::BN, S = PsShape<KIND>::SPLIT, ACCS = SM::ACCS, DONE = 4, SETS = PsShape<KIND>::SETS;
   constexpr int W = BN / S;   // columns of the tile this CTA finishes: 16 cells (x 4 gates forward)
   extern __shared__ uint8_t smem_raw[];
   // the dynamic shared-memory window starts at the same offset in every CTA of the cluster, so the aligned offsets
@@ -177,10 +176,9 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   float *recv = reinterpret_cast<float *>(smem + SM::RECV_OFFSET);  // [S - 1 peers][128 rows][W]: partial sums pushed by the peers
   uint64_t *full_bar = reinterpret_cast<uint64_t *>(smem + SM::BAR_OFFSET);
-  uint64_t *empty_bar = full_bar + STAGES;
-  uint64_t *acc_full = empty_bar + STAGES;   // [ACCS] an accumulator is complete
-  uint64_t *acc_empty = acc_full + ACCS;     // [ACCS] the 8 exchange warps have read it
-  uint64_t *red_ready = acc_empty + ACCS;    // every exchange warp of every peer has pushed its partial sums for this CTA
+  uint64_t *done_bar = full_bar + STAGES;    // [DONE] the products of a stage are done: its accumulator is complete, the stage free
+  uint64_t *acc_empty = done_bar + DONE;     // [ACCS] the 8 exchange warps have read the accumulator
+  uint64_t *red_ready = acc_empty + ACCS;    // the peers' partial sums for this CTA have landed
   uint64_t *step_go = red_ready + 1;         // the producer has passed the step barrier
   uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(step_go + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
@@ -194,21 +192,15 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
   const int m0 = tile_m * 128, n0 = tile_n * BN;
   const int kb0 = min(static_cast<int>(rank) * q.kb_per, q.num_kb), kb1 = min(kb0 + q.kb_per, q.num_kb);
   const int my_kb = kb1 - kb0;
-  const int nacc = (my_kb + CHUNK - 1) / CHUNK;   // accumulators this CTA fills per step
   unsigned int *counter = q.sync + tile_m;
   unsigned int *abort_word = q.sync + q.tiles_m;
   const unsigned int per_step = static_cast<unsigned int>(q.tiles_n * S);  // CTAs that complete a row of tiles
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      ptx::mbar_init(&full_bar[s], 1);
-      ptx::mbar_init(&empty_bar[s], 1);
-    }
-    for (int a = 0; a < ACCS; ++a) {
-      ptx::mbar_init(&acc_full[a], 1);
-      ptx::mbar_init(&acc_empty[a], 8);
-    }
-    ptx::mbar_init(red_ready, static_cast<uint32_t>(8 * (S - 1)));
+    for (int s = 0; s < STAGES; ++s) ptx::mbar_init(&full_bar[s], 1);
+    for (int s = 0; s < DONE; ++s) ptx::mbar_init(&done_bar[s], 1);
+    for (int a = 0; a < ACCS; ++a) ptx::mbar_init(&acc_empty[a], 8);
+    ptx::mbar_init(red_ready, 1);
     ptx::mbar_init(step_go, 1);
     *abort_flag = 0;
     ptx::fence_barrier_init();
@@ -225,12 +217,15 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
   const uint32_t tmem_base = *tmem_holder;
 
   uint32_t issued = 0;  // producer: K blocks staged so far (for the final drain)
-  int ahead_issued = 0; // of the next step: stages whose weights are on their way (not 0 only when a wait has given up)
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     ptx::reg_release<40>();
     if (lane == 0) {
       bool ok = true;
+      auto wait_free = [&](uint32_t u) {   // the stage's last products are done
+        const uint32_t v = u - static_cast<uint32_t>(STAGES);
+        return u < static_cast<uint32_t>(STAGES) || ptx::mbar_wait_or_abort(&done_bar[v % DONE], (v / DONE) & 1u, abort_flag);
+      };
       auto load_a = [&](uint32_t u, int kb, int a_row) {
         uint8_t *dst = smem + (u % STAGES) * SM::STAGE_BYTES;
         ptx::tma_load_2d(dst, &tm_a0, &full_bar[u % STAGES], kb * PS_BK, a_row);
@@ -251,23 +246,20 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
         const int ahead = min(STAGES, my_kb);
         for (int i = 0; i < ahead; ++i) {
           const uint32_t u = issued + static_cast<uint32_t>(i);
-          if (!ptx::mbar_wait_or_abort(&empty_bar[u % STAGES], ((u / STAGES) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+          if (!wait_free(u)) { ok = false; break; }
           ptx::mbar_arrive_expect_tx(&full_bar[u % STAGES], SM::STAGE_BYTES);
           load_b(u, kb0 + i);
-          ++ahead_issued;
         }
         if (!ok || !wait_step_counter(counter, per_step * static_cast<unsigned int>(s), abort_word, abort_flag)) { ok = false; break; }
         ptx::fence_proxy_async_global();  // the other CTAs wrote them with ordinary stores; TMA reads through the async proxy
         const int a_row = ((s - 1) & 1) * static_cast<int>(q.a_rows) + m0;
         for (int i = 0; i < ahead; ++i) load_a(issued + static_cast<uint32_t>(i), kb0 + i, a_row);
         issued += static_cast<uint32_t>(ahead);
-        ahead_issued = 0;
         // only now may the other warps store the arrays of the step before: their stores would keep these copies waiting
         ptx::mbar_arrive_local(step_go);
         for (int kb = kb0 + ahead; kb < kb1; ++kb, ++issued) {
-          const uint32_t st = issued % STAGES;
-          if (!ptx::mbar_wait_or_abort(&empty_bar[st], ((issued / STAGES) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
-          ptx::mbar_arrive_expect_tx(&full_bar[st], SM::STAGE_BYTES);
+          if (!wait_free(issued)) { ok = false; break; }
+          ptx::mbar_arrive_expect_tx(&full_bar[issued % STAGES], SM::STAGE_BYTES);
           load_a(issued, kb, a_row);
           load_b(issued, kb);
         }
@@ -282,42 +274,41 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
     ptx::reg_release<40>();
     if (lane == 0) {
       bool ok = true;
-      constexpr uint32_t idesc = make_idesc_f16(128, BN, false, KIND == 2);
+      constexpr uint32_t idesc = make_idesc_f16(128, BN, false, KIND == 2), idesc2 = make_idesc_f16(128, SETS * BN, false, KIND == 2);
       constexpr uint64_t b_step = KIND == 2 ? 128 : 2;
-      uint32_t it = 0, n = 0;  // stages consumed, accumulators filled
+      uint32_t it = 0;  // stages consumed = accumulators filled
       // the barriers of the next stage are asked before this one's instructions are issued (see half_gemm.cu)
       bool full_ok = false, acc_ok = false;
       for (int s = 1; s < q.T && ok; ++s) {
-        for (int c = 0; c < nacc && ok; ++c, ++n) {
-          const uint32_t a = n % ACCS, use = n / ACCS;
-          if (use > 0) {
-            if (!acc_ok && !ptx::mbar_wait_or_abort(&acc_empty[a], (use - 1u) & 1u, abort_flag)) { ok = false; break; }
-            ptx::tc_fence_after();
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+          const uint32_t a = it % ACCS, st = it % STAGES;
+          if (it >= ACCS) {
+            if (!acc_ok && !ptx::mbar_wait_or_abort(&acc_empty[a], (it / ACCS - 1u) & 1u, abort_flag)) { ok = false; break; }
           }
-          acc_ok = false;
-          const uint32_t t_acc = tmem_base + a * static_cast<uint32_t>(BN);
-          const int kb_end = min(kb0 + (c + 1) * CHUNK, kb1);
-          for (int kb = kb0 + c * CHUNK; kb < kb_end; ++kb, ++it) {
-            const int st = static_cast<int>(it % STAGES);
-            const uint32_t ph = (it / STAGES) & 1u;
-            if (!full_ok && !ptx::mbar_wait_or_abort(&full_bar[st], ph, abort_flag)) { ok = false; break; }
-            ptx::tc_fence_after();
-            full_ok = ptx::mbar_test(&full_bar[(it + 1) % STAGES], ((it + 1) / STAGES) & 1u);
-            if (kb + 1 == kb_end && n + 1 >= ACCS) acc_ok = ptx::mbar_test(&acc_empty[(n + 1) % ACCS], ((n + 1) / ACCS - 1u) & 1u);
-            const uint32_t base = ptx::smem_u32(smem + st * SM::STAGE_BYTES), base_b = base + 2 * PS_A_BYTES;
-            const uint64_t a0 = make_smem_desc(base), a1 = make_smem_desc(base + PS_A_BYTES);
-            const uint64_t b0 = KIND == 2 ? make_smem_desc_mn(base_b, 8192, false) : make_smem_desc(base_b);
-            const uint64_t b1 = KIND == 2 ? make_smem_desc_mn(base_b + SM::B_BYTES, 8192, false) : make_smem_desc(base_b + SM::B_BYTES);
+          if (!full_ok && !ptx::mbar_wait_or_abort(&full_bar[st], (it / STAGES) & 1u, abort_flag)) { ok = false; break; }
+          ptx::tc_fence_after();
+          full_ok = ptx::mbar_test(&full_bar[(it + 1) % STAGES], ((it + 1) / STAGES) & 1u);
+          acc_ok = it + 1 >= ACCS && ptx::mbar_test(&acc_empty[(it + 1) % ACCS], ((it + 1) / ACCS - 1u) & 1u);
+          const uint32_t t_acc = tmem_base + a * static_cast<uint32_t>(SM::ACC_COLS);
+          const uint32_t base = ptx::smem_u32(smem + st * SM::STAGE_BYTES), base_b = base + 2 * PS_A_BYTES;
+          const uint64_t a0 = make_smem_desc(base), a1 = make_smem_desc(base + PS_A_BYTES);
+          const uint64_t b0 = KIND == 2 ? make_smem_desc_mn(base_b, 8192, false) : make_smem_desc(base_b);
 #pragma unroll
-            for (int k = 0; k < PS_BK / 16; ++k) {
-              const uint64_t ka = static_cast<uint64_t>(k) * 2, kbo = static_cast<uint64_t>(k) * b_step;
-              ptx::mma_bf16(t_acc, a1 + ka, b0 + kbo, idesc, (kb > kb0 + c * CHUNK || k > 0) ? 1u : 0u);
+          for (int k = 0; k < PS_BK / 16; ++k) {
+            const uint64_t ka = static_cast<uint64_t>(k) * 2, kbo = static_cast<uint64_t>(k) * b_step;
+            if constexpr (SETS == 2) {
+              ptx::mma_bf16(t_acc, a0 + ka, b0 + kbo, idesc2, k > 0 ? 1u : 0u);   // a0 * b0 and a0 * b1
+              ptx::mma_bf16(t_acc + BN, a1 + ka, b0 + kbo, idesc, 1u);            // a1 * b0 onto a0 * b1
+            } else {
+              const uint64_t b1 = make_smem_desc(base_b + SM::B_BYTES);
+              ptx::mma_bf16(t_acc, a1 + ka, b0 + kbo, idesc, k > 0 ? 1u : 0u);
               ptx::mma_bf16(t_acc, a0 + ka, b1 + kbo, idesc, 1u);
               ptx::mma_bf16(t_acc, a0 + ka, b0 + kbo, idesc, 1u);
             }
-            ptx::tc_commit(&empty_bar[st]);
           }
-          if (ok) ptx::tc_commit(&acc_full[a]);
+          // one commit per stage: the accumulator is complete and the stage free (a second one right behind it stalls the
+          // issuer for 600 cycles)
+          ptx::tc_commit(&done_bar[it % DONE]);
         }
       }
       if (!ok) {
@@ -351,16 +342,24 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
     using In = typename std::conditional<KIND == 1, LstmForwardIn, LstmBackwardIn>::type;
     using Out = typename std::conditional<KIND == 1, LstmForwardOut, LstmBackwardOut>::type;
     Out out;               // results of the step before; its arrays are written once the step barrier has been passed
+    float fn[8];           // backward: the forget gates of the step of the walk before
+#pragma unroll
+    for (int i = 0; i < 8; ++i) fn[i] = 0.f;
     bool pending = false;
     uint32_t n = 0;        // accumulators read so far
-    auto store_arrays = [&](int step) {
+    constexpr int ARRAYS = KIND == 1 ? LSTM_FORWARD_ARRAYS : LSTM_BACKWARD_ARRAYS;
+    auto store_arrays = [&](int step, int first, int last) {
       const LstmStep pp = step_view<KIND>(q, step);
-      if constexpr (KIND == 1) lstm_forward_store_arrays8(pp, out, b, cell0);
-      else lstm_backward_store_arrays8(pp, out, b, cell0);
+#pragma unroll
+      for (int k = 0; k < ARRAYS; ++k) {
+        if (k < first || k >= last) continue;
+        if constexpr (KIND == 1) lstm_forward_store_array8(pp, out, b, cell0, k);
+        else lstm_backward_store_array8(pp, out, b, cell0, k);
+      }
     };
     // power of two of the product of accumulator c's operands; asked for one accumulator ahead
     auto exponent_of = [&](int step, int c) {
-      const int kb = kb0 + c * CHUNK;
+      const int kb = kb0 + c;
       if constexpr (KIND == 1) return LSTM_H_EXPONENT + __ldg(q.w_exp + tile_n * q.w_exp_pitch + (kb >> 1));
       else return __ldcg(q.a_exp + (static_cast<long long>((step - 1) & 1) * q.tiles_m + tile_m) * q.num_kb + kb) + __ldg(q.w_exp + (kb >> 1) * q.w_exp_pitch + (tile_n >> 1));
     };
@@ -373,22 +372,21 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
         // what the cell needs from global memory goes out before any wait; what this thread computed itself in the step
         // before (and has not written yet) comes from its registers
         if constexpr (KIND == 1) {
-          lstm_forward_load8<false, false>(p, in, b, cell0);
+          lstm_forward_load8(p, in, b, cell0);
 #pragma unroll
           for (int i = 0; i < 8; ++i) { in.cp[i] = s > 0 ? out.cs[i] : 0.f; in.hp[i] = s > 0 ? out.h[i] : 0.f; }
         } else {
-          lstm_backward_load8<false, false>(p, in, b, cell0);
+          lstm_backward_load8(p, in, b, cell0);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) { in.dni[i] = s > 0 ? out.di[i] : 0.f; in.dnf[i] = s > 0 ? out.df[i] : 0.f; in.dcn[i] = s > 0 ? out.dc[i] : 0.f; }
+          for (int i = 0; i < 8; ++i) { in.dni[i] = s > 0 ? out.di[i] : 0.f; in.dnf[i] = s > 0 ? out.df[i] : 0.f; in.dcn[i] = s > 0 ? out.dc[i] : 0.f; in.fn[i] = fn[i]; fn[i] = in.fg[i]; }
         }
       }
       if (pending) {
-        // the arrays of step s - 1 (read by later kernels only) leave now, beside this step's operand stream, and not
-        // while the step barrier is in flight: 128 CTAs storing at once slowed the barrier down by microseconds
+        // the arrays of step s - 1 (read by later kernels only) leave from here on, two per accumulator beside this step's
+        // operand stream: all at once, the 128 CTAs' stores kept its first copies waiting (4 of a forward step's 30 kcycles), and
+        // stored while the step barrier is in flight they slowed the barrier down
         if (!ptx::mbar_wait_or_abort(step_go, static_cast<uint32_t>(s - 1) & 1u, abort_flag)) ok = false;
-        if (ok && nacc > 0) e_next = exponent_of(s, 0);
-        if (ok && active) store_arrays(s - 1);
-        pending = false;
+        if (ok && my_kb > 0) e_next = exponent_of(s, 0);
       }
       float rec[HW];
 #pragma unroll
@@ -403,32 +401,45 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
         for (int dd = 0; dd < S; ++dd)
 #pragma unroll
           for (int j = 0; j < HW; ++j) part[dd][j] = 0.f;
-        for (int c = 0; c < nacc && ok; ++c, ++n) {
+        for (int c = 0; c < my_kb; ++c, ++n) {
           const uint32_t a = n % ACCS;
           const int e = e_next;
-          if (c + 1 < nacc) e_next = exponent_of(s, c + 1);
-          if (!ptx::mbar_wait_or_abort(&acc_full[a], (n / ACCS) & 1u, abort_flag)) { ok = false; break; }
+          if (c + 1 < my_kb) e_next = exponent_of(s, c + 1);
+          if (!ptx::mbar_wait_or_abort(&done_bar[n % DONE], (n / DONE) & 1u, abort_flag)) { ok = false; break; }
           ptx::tc_fence_after();
           const int e1 = max(-126, min(127, e)), e2 = max(-126, min(127, e - e1));
           const float s1 = pow2(e1), s2 = pow2(e2);
-          const uint32_t tq = tmem_base + (static_cast<uint32_t>(qd * 32) << 16) + a * static_cast<uint32_t>(BN);
+          const uint32_t tq = tmem_base + (static_cast<uint32_t>(qd * 32) << 16) + a * static_cast<uint32_t>(SM::ACC_COLS);
 #pragma unroll
           for (int dd = 1; dd <= S; ++dd) {
             const int d = (static_cast<int>(rank) + dd) % S;
-            uint32_t r[HW / 8][8];
+            constexpr int BATCH = HW / 8;   // 8-column groups per round trip
 #pragma unroll
-            for (int k = 0; k < HW / 8; ++k) ptx::tmem_ld_32x8(tq + static_cast<uint32_t>(d * W + k * 16 + half * 8), r[k]);
-            ptx::tmem_ld_wait();
+            for (int k0 = 0; k0 < HW / 8; k0 += BATCH) {
+              uint32_t r[BATCH][8], x[BATCH][8];
 #pragma unroll
-            for (int j = 0; j < HW; ++j) {
-              const float x = __uint_as_float(r[j / 8][j % 8]);
-              part[dd - 1][j] = fmaf(e2 == 0 ? x : x * s2, s1, part[dd - 1][j]);
+              for (int k = 0; k < BATCH; ++k) {
+                const uint32_t col = tq + static_cast<uint32_t>(d * W + (k0 + k) * 16 + half * 8);
+                ptx::tmem_ld_32x8(col, r[k]);
+                if constexpr (SETS == 2) ptx::tmem_ld_32x8(col + BN, x[k]);
+              }
+              ptx::tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < BATCH * 8; ++j) {
+                float v = __uint_as_float(r[j / 8][j % 8]);
+                if constexpr (SETS == 2) v += __uint_as_float(x[j / 8][j % 8]);
+                float &t = part[dd - 1][k0 * 8 + j];
+                t = fmaf(e2 == 0 ? v : v * s2, s1, t);
+              }
             }
           }
           ptx::tc_fence_before();
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive_local(&acc_empty[a]);
+          if (active && 2 * c < ARRAYS) store_arrays(s - 1, 2 * c, 2 * c + 2);
         }
+        if (ok && active && 2 * my_kb < ARRAYS) store_arrays(s - 1, 2 * my_kb, ARRAYS);
+        pending = false;
         if (ok) {
           // the peers' shares are pushed into their receive slots, this CTA's own share stays in registers
 #pragma unroll
@@ -436,16 +447,13 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
             const int d = (static_cast<int>(rank) + dd) % S;
             const int slot = static_cast<int>(rank) < d ? static_cast<int>(rank) : static_cast<int>(rank) - 1;
             const uint32_t dst = ptx::map_to_cta(recv_addr + static_cast<uint32_t>((slot * 128 + row) * W * 4), static_cast<uint32_t>(d));
+            const uint32_t bar = ptx::map_to_cta(ptx::smem_u32(red_ready), static_cast<uint32_t>(d));
 #pragma unroll
             for (int i = 0; i < HW / 4; ++i)
-              ptx::st_cluster_f4(dst + (static_cast<uint32_t>((half * (HW / 4) + i) ^ swz) << 4),
-                                 make_float4(part[dd - 1][4 * i], part[dd - 1][4 * i + 1], part[dd - 1][4 * i + 2], part[dd - 1][4 * i + 3]));
+              ptx::st_async_f4(dst + (static_cast<uint32_t>((half * (HW / 4) + i) ^ swz) << 4),
+                               make_float4(part[dd - 1][4 * i], part[dd - 1][4 * i + 1], part[dd - 1][4 * i + 2], part[dd - 1][4 * i + 3]), bar);
           }
-          __syncwarp();
-          if (lane == 0) {
-#pragma unroll
-            for (int dd = 1; dd < S; ++dd) ptx::mbar_arrive_release_cluster(red_ready, (rank + static_cast<uint32_t>(dd)) % S);
-          }
+          if (warp == PS_EPI_WARP0 && lane == 0) ptx::mbar_arrive_expect_tx(red_ready, static_cast<uint32_t>(SM::RECV_BYTES));
           if (!ptx::mbar_wait_cluster_or_abort(red_ready, static_cast<uint32_t>(s - 1) & 1u, abort_flag)) ok = false;
         }
         if (ok) {
@@ -513,7 +521,7 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
       // the GPU together with the count
       if (warp == PS_EPI_WARP0 && lane == 0) red_release_gpu_add(counter, 1u);
     }
-    if (pending && active) store_arrays(q.T - 1);
+    if (pending && active) store_arrays(q.T - 1, 0, ARRAYS);
   } else {
     ptx::reg_release<40>();  // warps 2-3: no role, but the whole warpgroup has to give its registers back
   }
@@ -524,12 +532,13 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
     for (uint32_t i = first; i < issued; ++i) {
       if (!ptx::mbar_wait(&full_bar[i % STAGES], (i / STAGES) & 1u)) break;
     }
-    // weights of a step that never began: their barriers cannot complete (the operand's bytes are missing), and copies of this
-    // GPU's own memory land within microseconds
-    if (ahead_issued > 0) {
-      const long long t0 = clock64();
-      while (clock64() - t0 < (1ll << 20)) {
-      }
+  }
+  // A wait has given up: copies whose barriers will never complete - weights of a step that did not begin, partial sums that
+  // nobody waits for - may be on their way into this CTA's shared memory.  They land within microseconds; half a millisecond
+  // passes before the CTA goes on to its end.
+  if (*abort_flag != 0) {
+    const long long t0 = clock64();
+    while (clock64() - t0 < (1ll << 20)) {
     }
   }
   // peers may still be pushing into this CTA's receive slots or signalling its barriers: the cluster stays together until
@@ -667,7 +676,7 @@ int lstm_persistent_forward(myea_b200_net *net, LayerPlan &L, int dir, bool zone
   q.tiles_n = static_cast<int>((P->G + PsShape<1>::BN - 1) / PsShape<1>::BN);
   q.split = PsShape<1>::SPLIT;
   q.num_kb = static_cast<int>((P->C + PS_BK - 1) / PS_BK);
-  q.kb_per = ((q.num_kb + q.split - 1) / q.split + 1) / 2 * 2;   // slices start on the weights' blocks of 128
+  q.kb_per = (q.num_kb + q.split - 1) / q.split;
   q.kpa = P->h_pan.pitch;
   q.a0 = P->h_pan.h0; q.a1 = P->h_pan.h1;
   q.gates_in = D.gates_in; q.act = D.act; q.cstate = D.cstate; q.cact = D.cact;

@@ -263,16 +263,16 @@ __global__ void __launch_bounds__(LR_THREADS, 1) lstm_resident_kernel(const __gr
               r4[0] += v.x; r4[1] += v.y; r4[2] += v.z; r4[3] += v.w;
             }
           }
-          const float z = tanh_ref(in.g[0] + r4[0]);
-          const float ig = sigmoid_ref(in.g[1] + (has_rec ? r4[1] + in.p_i * in.cp : 0.f));
+          const float z = tanh_cell(in.g[0] + r4[0]);
+          const float ig = sigmoid_cell(in.g[1] + (has_rec ? r4[1] + in.p_i * in.cp : 0.f));
           float fg = 0.f, cs = z * ig;
           if (has_rec) {
-            fg = sigmoid_ref(in.g[2] + r4[2] + in.p_f * in.cp);
+            fg = sigmoid_cell(in.g[2] + r4[2] + in.p_f * in.cp);
             cs += fg * in.cp;
           }
           if (!in.zs) cs = in.cp;
-          const float a = tanh_ref(cs);
-          const float og = sigmoid_ref(in.g[3] + r4[3] + in.p_o * cs);
+          const float a = tanh_cell(cs);
+          const float og = sigmoid_cell(in.g[3] + r4[3] + in.p_o * cs);
           float h = a * og;
           if (!in.zo) h = in.hp;
           dst[cell * q.Rp + rg] = h;

@@ -15,19 +15,43 @@ __device__ __forceinline__ void store8(float *p, const float (&d)[8]) {
   *reinterpret_cast<float4 *>(p) = make_float4(d[0], d[1], d[2], d[3]);
   *reinterpret_cast<float4 *>(p + 4) = make_float4(d[4], d[5], d[6], d[7]);
 }
+// 32 aligned bytes in one access
+__device__ __forceinline__ void load32(float (&d)[8], const float *p) {
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]), "=f"(d[4]), "=f"(d[5]), "=f"(d[6]), "=f"(d[7])
+               : "l"(p)
+               : "memory");
+}
+__device__ __forceinline__ void store32(float *p, const float (&d)[8]) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(d[0]), "f"(d[1]), "f"(d[2]), "f"(d[3]), "f"(d[4]), "f"(d[5]), "f"(d[6]),
+               "f"(d[7])
+               : "memory");
+}
+// 1 / d for d in [1, inf]: the hardware's approximation and one Newton-Raphson step in fused arithmetic, which rounds the
+// result correctly (P. Markstein, IA-64 and Elementary Functions, 2000) as the division does, without its branch: the eight
+// cells of a thread interleave.  Past 2^126 the approximation stands (0: the division gives at most 1.2e-38 there).
+__device__ __forceinline__ float reciprocal_from_one(float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float n = fmaf(r, fmaf(-d, r, 1.0f), r);
+  return d < 8.507059e37f ? n : r;
+}
+// the gates' functions as common.cuh has them: 1 / (1 + e^-x), 2 / (1 + e^-2x) - 1
+__device__ __forceinline__ float sigmoid_cell(float x) { return reciprocal_from_one(1.0f + expf(-x)); }
+__device__ __forceinline__ float tanh_cell(float x) { return 2.0f * reciprocal_from_one(1.0f + expf(-2.0f * x)) - 1.0f; }
+
 // One time step of an LSTM layer as the cell arithmetic sees it: the arrays of step t, of the step before / after it in
 // the layer's direction, and where the results also leave as operand panels of the next step's contraction.
 struct LstmStep {
   long long C = 0, ldh = 0, kp = 0;
-  const float *peep = nullptr;  // compact peepholes [3][C]: p_i, p_f, p_o
   uint16_t *p_h0 = nullptr, *p_h1 = nullptr;  // operand panels written for the next step (pitch kp), or null
   // forward (rows of step t unless said otherwise)
-  const float *gates_in = nullptr, *c_prev = nullptr, *h_prev = nullptr;
+  const float *gates_in = nullptr;
   float *act = nullptr, *cstate = nullptr, *cact = nullptr, *h = nullptr;
   const uint8_t *zone_state = nullptr, *zone_output = nullptr;
   // backward
   float *dh = nullptr;  // [B, ldh] error on h of step t from above; the error through time is added in place
-  const float *b_act = nullptr, *b_cact = nullptr, *b_c_prev = nullptr, *act_next = nullptr, *dgates_next = nullptr, *dc_next = nullptr;
+  const float *b_act = nullptr, *b_cact = nullptr, *b_c_prev = nullptr;
   float *dgates = nullptr, *dcstate = nullptr;
 };
 
@@ -39,18 +63,13 @@ struct LstmForwardIn {
   float gz[8], gi[8], gf[8], go[8], cp[8], hp[8], pi[8], pf[8], po[8];
   unsigned long long zs, zo;
 };
-// SELF: also fetch what this same cell wrote in the step before (cell state, output); a caller that still holds those
-// values in registers passes false and fills in.cp / in.hp itself.  PEEP: fetch the peepholes.
-template <bool SELF = true, bool PEEP = true>
+// (what this same cell computed in the step before, in.cp and in.hp, and the peepholes stay with the caller)
 __device__ __forceinline__ void lstm_forward_load8(const LstmStep &p, LstmForwardIn &in, long long b, long long c0) {
   const long long C = p.C;
   const float *g = p.gates_in + b * 4 * C + c0;
-  load8(in.gz, g); load8(in.gi, g + C); load8(in.gf, g + 2 * C); load8(in.go, g + 3 * C);
-  if (SELF) load8(in.cp, p.c_prev + b * C + c0);
-  if (PEEP) { load8(in.pi, p.peep + c0); load8(in.pf, p.peep + C + c0); load8(in.po, p.peep + 2 * C + c0); }
+  load32(in.gz, g); load32(in.gi, g + C); load32(in.gf, g + 2 * C); load32(in.go, g + 3 * C);
   in.zs = p.zone_state != nullptr ? *reinterpret_cast<const unsigned long long *>(p.zone_state + c0) : ~0ull;
   in.zo = p.zone_output != nullptr ? *reinterpret_cast<const unsigned long long *>(p.zone_output + c0) : ~0ull;
-  if (SELF && p.zone_output != nullptr) load8(in.hp, p.h_prev + b * p.ldh + c0);
 }
 struct LstmForwardOut {
   float z[8], ig[8], fg[8], og[8], cs[8], a[8], h[8];
@@ -58,15 +77,15 @@ struct LstmForwardOut {
 __device__ __forceinline__ void lstm_forward_compute8(const LstmForwardIn &in, const float (&rec)[32], bool first, LstmForwardOut &o) {
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    o.z[i] = tanh_ref(in.gz[i] + rec[i]);
-    o.ig[i] = sigmoid_ref(in.gi[i] + (rec[8 + i] + in.pi[i] * in.cp[i]));
-    o.fg[i] = first ? 0.f : sigmoid_ref(in.gf[i] + rec[16 + i] + in.pf[i] * in.cp[i]);
+    o.z[i] = tanh_cell(in.gz[i] + rec[i]);
+    o.ig[i] = sigmoid_cell(in.gi[i] + (rec[8 + i] + in.pi[i] * in.cp[i]));
+    o.fg[i] = first ? 0.f : sigmoid_cell(in.gf[i] + rec[16 + i] + in.pf[i] * in.cp[i]);
     float c = o.z[i] * o.ig[i];
     c += o.fg[i] * in.cp[i];
     if (((in.zs >> (8 * i)) & 0xFFull) == 0ull) c = in.cp[i];
     o.cs[i] = c;
-    o.a[i] = tanh_ref(c);
-    o.og[i] = sigmoid_ref(in.go[i] + rec[24 + i] + in.po[i] * c);
+    o.a[i] = tanh_cell(c);
+    o.og[i] = sigmoid_cell(in.go[i] + rec[24 + i] + in.po[i] * c);
     float hh = o.a[i] * o.og[i];
     if (((in.zo >> (8 * i)) & 0xFFull) == 0ull) hh = in.hp[i];
     o.h[i] = hh;
@@ -85,41 +104,33 @@ __device__ __forceinline__ void lstm_store_h_panels8(const LstmStep &p, const fl
   *reinterpret_cast<uint4 *>(p.p_h1 + b * p.kp + c0) = h1;
 }
 // what the backward pass and the layers above read
-__device__ __forceinline__ void lstm_forward_store_arrays8(const LstmStep &p, const LstmForwardOut &o, long long b, long long c0) {
+constexpr int LSTM_FORWARD_ARRAYS = 7, LSTM_BACKWARD_ARRAYS = 6;
+__device__ __forceinline__ void lstm_forward_store_array8(const LstmStep &p, const LstmForwardOut &o, long long b, long long c0, int k) {
   const long long C = p.C;
   float *act = p.act + b * 4 * C + c0;
-  store8(act, o.z); store8(act + C, o.ig); store8(act + 2 * C, o.fg); store8(act + 3 * C, o.og);
-  store8(p.cstate + b * C + c0, o.cs);
-  store8(p.cact + b * C + c0, o.a);
-  store8(p.h + b * p.ldh + c0, o.h);
+  switch (k) {
+    case 0: store32(act, o.z); break;
+    case 1: store32(act + C, o.ig); break;
+    case 2: store32(act + 2 * C, o.fg); break;
+    case 3: store32(act + 3 * C, o.og); break;
+    case 4: store32(p.cstate + b * C + c0, o.cs); break;
+    case 5: store32(p.cact + b * C + c0, o.a); break;
+    default: store32(p.h + b * p.ldh + c0, o.h); break;
+  }
 }
 // LSTM backward cell for batch row b, cells [c0, c0 + 8): rec[i] is the error arriving on h of cell c0 + i through time.
 // Same arithmetic as lstm_cell_backward_kernel on a step that has a successor; load8 / finish8 as above.
 struct LstmBackwardIn {
   float dh[8], z[8], ig[8], fg[8], og[8], a[8], pi[8], pf[8], po[8], cp[8], dni[8], dnf[8], dcn[8], fn[8];
 };
-// SELF: also fetch what this same cell wrote in the step of the walk before (input / forget gate errors, cell-state
-// error); PEEP: fetch the peepholes (see lstm_forward_load8)
-template <bool SELF = true, bool PEEP = true>
+// (dni, dnf, dcn and fn, the step of the walk before, and the peepholes stay with the caller)
 __device__ __forceinline__ void lstm_backward_load8(const LstmStep &p, LstmBackwardIn &in, long long b, long long c0) {
   const long long C = p.C;
-  load8(in.dh, p.dh + b * p.ldh + c0);
+  load32(in.dh, p.dh + b * p.ldh + c0);
   const float *act = p.b_act + b * 4 * C + c0;
-  load8(in.z, act); load8(in.ig, act + C); load8(in.fg, act + 2 * C); load8(in.og, act + 3 * C);
-  load8(in.a, p.b_cact + b * C + c0);
-  if (PEEP) { load8(in.pi, p.peep + c0); load8(in.pf, p.peep + C + c0); load8(in.po, p.peep + 2 * C + c0); }
-  if (p.b_c_prev != nullptr) load8(in.cp, p.b_c_prev + b * C + c0);
-  if (SELF) {
-    const float *dn = p.dgates_next + b * 4 * C + c0;
-    load8(in.dni, dn + C); load8(in.dnf, dn + 2 * C);
-    load8(in.dcn, p.dc_next + b * C + c0);
-  }
-  if (p.act_next != nullptr) {
-    load8(in.fn, p.act_next + b * 4 * C + 2 * C + c0);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) in.fn[i] = 0.f;
-  }
+  load32(in.z, act); load32(in.ig, act + C); load32(in.fg, act + 2 * C); load32(in.og, act + 3 * C);
+  load32(in.a, p.b_cact + b * C + c0);
+  if (p.b_c_prev != nullptr) load32(in.cp, p.b_c_prev + b * C + c0);
 }
 struct LstmBackwardOut {
   float dh[8], dz[8], di[8], df[8], d_o[8], dc[8];
@@ -153,11 +164,16 @@ __device__ __forceinline__ void lstm_store_gate_panels8(const LstmStep &p, const
   };
   put(o.dz, 0); put(o.di, 1); put(o.df, 2); put(o.d_o, 3);
 }
-__device__ __forceinline__ void lstm_backward_store_arrays8(const LstmStep &p, const LstmBackwardOut &o, long long b, long long c0) {
+__device__ __forceinline__ void lstm_backward_store_array8(const LstmStep &p, const LstmBackwardOut &o, long long b, long long c0, int k) {
   const long long C = p.C;
-  store8(p.dh + b * p.ldh + c0, o.dh);
   float *dg = p.dgates + b * 4 * C + c0;
-  store8(dg, o.dz); store8(dg + C, o.di); store8(dg + 2 * C, o.df); store8(dg + 3 * C, o.d_o);
-  store8(p.dcstate + b * C + c0, o.dc);
+  switch (k) {
+    case 0: store32(p.dh + b * p.ldh + c0, o.dh); break;
+    case 1: store32(dg, o.dz); break;
+    case 2: store32(dg + C, o.di); break;
+    case 3: store32(dg + 2 * C, o.df); break;
+    case 4: store32(dg + 3 * C, o.d_o); break;
+    default: store32(p.dcstate + b * C + c0, o.dc); break;
+  }
 }
 }  // namespace myea

@@ -218,11 +218,6 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t cta)
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(cta));
   return r;
 }
-// arrive (release at cluster scope: this thread's earlier shared-memory writes become visible to whoever acquires the
-// barrier) on the mbarrier at this offset in CTA `cta`
-__device__ __forceinline__ void mbar_arrive_release_cluster(uint64_t *bar, uint32_t cta) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(map_to_cta(smem_u32(bar), cta)) : "memory");
-}
 __device__ __forceinline__ void mbar_arrive_local(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -255,8 +250,12 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_cluster_f4(uint32_t cluster_addr, float4 v) {
-  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+// 16 bytes into another CTA's shared memory; the mbarrier there (its address in that CTA) counts them as they land.  Nothing
+// here waits for them, and the wait on that barrier makes them visible.
+__device__ __forceinline__ void st_async_f4(uint32_t cluster_addr, float4 v, uint32_t cluster_bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(cluster_addr), "f"(v.x), "f"(v.y),
+               "f"(v.z), "f"(v.w), "r"(cluster_bar)
+               : "memory");
 }
 // orders this thread's generic-proxy accesses (global and shared memory) against async-proxy (TMA) ones
 __device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
