@@ -349,8 +349,21 @@ struct OptLaunch {
   int rprop_error_is_worse = 0;
   const float *clip_scale = nullptr;  // device float: multiply the gradient by it first (global-norm clip), may be null
 };
-int optimizer_update(Context &ctx, const OptLaunch &o, float *w, float *g, float *m, float *v, float *vhat,
-                     float *prev_delta, const float *mask, size_t n);
+// parameters, derivatives, moments, previous update, regularization mask: element i of each belongs together
+struct OptArrays {
+  float *w, *g, *m, *v, *vhat, *prev;
+  const float *mask;
+  OptArrays at(size_t off) const { return {w + off, g + off, m + off, v + off, vhat + off, prev + off, mask + off}; }
+};
+int optimizer_update(Context &ctx, const OptLaunch &o, const OptArrays &a, size_t n);
+// The same for the weights [R][C] (of p, C a multiple of 8) of layers that start at element `offset`: leaves the new weights as
+// arrays and as the panels p, and does NOT zero the derivatives.
+struct OptPanelLayer {
+  size_t offset;
+  HalfPanels p;
+  int first_block;   // (filled in by the call)
+};
+int optimizer_update_panels(Context &ctx, const OptLaunch &o, const OptArrays &a, const OptPanelLayer *layers, int n);
 // every row of w[rows][cols] whose Euclidean norm is >= max_norm is scaled to norm max_norm (Euclidean_Norm__Loop,
 // Neural_Network__Regularization__Max_Norm_Constraints.cpp:48-88)
 int row_max_norm(Context &ctx, float *w, long long rows, long long cols, float max_norm);

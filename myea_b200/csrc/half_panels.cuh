@@ -51,14 +51,15 @@ __device__ __forceinline__ void half_split8(const float (&v)[8], uint4 &h0, uint
 // A block of 256 threads holds a 128 x 128 block of the tensor: thread = 8 columns (tid % 16) of rows tid / 16 + 16 i.
 // half_block_finish: the block's exponent from every thread's largest magnitude (all threads of the block call it).
 constexpr int HP_THREADS = 256;
+template <int THREADS = HP_THREADS>
 __device__ __forceinline__ int half_block_exponent(float amax) {
-  __shared__ float sh[HP_THREADS / 32];
+  __shared__ float sh[THREADS / 32];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = amax;
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < HP_THREADS / 32; ++w) amax = fmaxf(amax, sh[w]);
+  for (int w = 0; w < THREADS / 32; ++w) amax = fmaxf(amax, sh[w]);
   return half_exponent(amax);
 }
 __device__ __forceinline__ float amax8(const float (&v)[8], float m) {

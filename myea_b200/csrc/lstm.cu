@@ -448,12 +448,14 @@ int lstm_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long
   } else {
     LRC(prepare_input(net, P, input, rows, n_in));
     for (int d = 0; d < P->dirs; ++d) {
-      RowSegments seg;
-      seg.seg_rows = C;
-      seg.seg_off[0] = off.z_in;
-      for (int g = 0; g < 3; ++g) seg.seg_off[g + 1] = off.in[g];
-      P->w_in[d] = half_panels_at(P->w_in_mem[d], 4 * C, n_in);
-      LRC(half_split(ctx, net->params + P->d[d].w_base, P->stride, P->w_in[d], &seg));
+      if (!L.w_fresh) {
+        RowSegments seg;
+        seg.seg_rows = C;
+        seg.seg_off[0] = off.z_in;
+        for (int g = 0; g < 3; ++g) seg.seg_off[g + 1] = off.in[g];
+        P->w_in[d] = half_panels_at(P->w_in_mem[d], 4 * C, n_in);
+        LRC(half_split(ctx, net->params + P->d[d].w_base, P->stride, P->w_in[d], &seg));
+      }
       Epilogue e;
       e.C = P->d[d].gates_in;
       e.ldc = 4 * C;
@@ -463,9 +465,15 @@ int lstm_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long
   }
   const bool zone = P->zoneout && net->training;
   const long long rec[4] = {off.z_rec, off.rec[0], off.rec[1], off.rec[2]};
+  const bool fresh = L.w_fresh;
+  L.w_fresh = true;   // (what is laid out from the weights below stays until the parameters change)
   if (P->resident != nullptr) return lstm_resident_run(net, L, 1, zone, rec, off.peep);
   if (lstm_persistent_ready(P)) {
     for (int d = 0; d < P->dirs; ++d) {
+      if (fresh) {
+        LRC(lstm_persistent_forward(net, L, d, zone));
+        continue;
+      }
       const float *w = net->params + P->d[d].w_base;
       ctx.begin(TC_RECURRENT);
       lstm_gather_peepholes_kernel<<<static_cast<unsigned>((C + 255) / 256), 256, 0, ctx.stream>>>(w + off.peep, P->stride, C, P->peep_compact + static_cast<size_t>(d) * 3 * C);
@@ -482,7 +490,8 @@ int lstm_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long
   for (int d = 0; d < P->dirs; ++d) {
     LstmDir &D = P->d[d];
     const float *w = net->params + D.w_base;
-    if (P->step_mem != nullptr) {
+    if (fresh) {
+    } else if (P->step_mem != nullptr) {
       RowSegments seg;
       seg.seg_rows = C;
       for (int g = 0; g < 4; ++g) seg.seg_off[g] = rec[g];

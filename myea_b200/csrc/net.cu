@@ -452,6 +452,17 @@ extern "C" int myea_b200_layer_index(myea_handle net, uint32_t layer, myea_layer
   return MYEA_OK;
 }
 
+// The update leaves the weight derivatives of large layers unzeroed: the next accumulation writes them instead of adding to
+// them.  Whoever else looks at the buffer first sets them to the zeros that they stand for.
+static int settle_derivatives(myea_b200_net *net) {
+  for (auto &L : net->layers) {
+    if (!L.dw_stale) continue;
+    CK(cudaMemsetAsync(net->grads + L.idx.first_connection_index, 0, static_cast<size_t>(L.n_out * L.n_in) * sizeof(float), net->ctx.stream));
+    L.dw_stale = false;
+  }
+  return MYEA_OK;
+}
+
 static float *select_buffer(myea_b200_net *net, int which, size_t *count) {
   *count = net->total_parameters;
   switch (which) {
@@ -475,10 +486,11 @@ extern "C" int myea_b200_upload(myea_handle net, int which, const float *host, u
   if (dst == nullptr || offset > n || count > n - offset) return fail(net, MYEA_E_INVALID, "upload: buffer selector or range out of bounds");
   CK(cudaSetDevice(net->ctx.device));
   RC(comm_gather_join(net));
+  if (which == MYEA_BUF_DERIVATIVES) RC(settle_derivatives(net));
   CK(cudaMemcpyAsync(dst + offset, host, count * sizeof(float), cudaMemcpyHostToDevice, net->ctx.stream));
   CK(cudaStreamSynchronize(net->ctx.stream));
   if (dst == net->params) {
-    for (auto &L : net->layers) L.w_valid = false;  // weight panels of the last forward pass no longer match
+    for (auto &L : net->layers) L.w_valid = L.w_fresh = false;  // weight panels of the last forward pass no longer match
   }
   return MYEA_OK;
 }
@@ -492,6 +504,7 @@ extern "C" int myea_b200_download(myea_handle net, int which, float *host, uint6
   // under a sharded update every rank keeps the optimizer state of its slices only: reading such a buffer back gathers
   // the slices first (collective: every rank has to make the call)
   RC(comm_gather_join(net));
+  if (which == MYEA_BUF_DERIVATIVES) RC(settle_derivatives(net));
   if (net->comm != nullptr && (src == net->m1 || src == net->m2 || src == net->m2hat || src == net->prev_delta)) RC(comm_gather_state(net, src));
   CK(cudaMemcpyAsync(host, src + offset, count * sizeof(float), cudaMemcpyDeviceToHost, net->ctx.stream));
   CK(cudaStreamSynchronize(net->ctx.stream));
@@ -540,11 +553,12 @@ static bool fc_uses_shared_panels(const myea_b200_net *net, const LayerPlan &L, 
 }
 
 // The weight panels of a layer depend on no activation: a forward pass whose inputs come from the host makes them all
-// while the inputs are still on their way (see forward_impl).
+// while the inputs are still on their way (see forward_impl).  They stay until the parameters change, and an update writes them
+// along (optimizer_update_panels): inference passes and most training steps find them in place.
 static int fc_prepare_weights(myea_b200_net *net, LayerPlan &L) {
   RC(comm_wait_gathers(net, L.idx.first_connection_index, L.idx.last_connection_index - L.idx.first_connection_index));
   RC(half_split(net->ctx, net->params + L.idx.first_connection_index, L.n_in, L.w_pan));
-  L.w_prepared = true;
+  L.w_fresh = true;
   return MYEA_OK;
 }
 
@@ -574,8 +588,7 @@ int fc_product_forward(myea_b200_net *net, LayerPlan &L, const float *input, lon
       RC(half_split(net->ctx, input, L.n_in, L.in_pan));
     }
     L.in_ready_src = nullptr;
-    if (!L.w_prepared) RC(fc_prepare_weights(net, L));
-    L.w_prepared = false;
+    if (!L.w_fresh) RC(fc_prepare_weights(net, L));
     L.in_valid = L.w_valid = tr;
     L.in_src = input;
     L.d_valid = false;
@@ -713,7 +726,7 @@ int fc_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long r
     struct Next { myea_b200_net *net; LayerPlan *layer; } next{net, nullptr};
     if (li + 1 < net->layers.size()) {
       LayerPlan &N = net->layers[li + 1];
-      if (N.type == MYEA_LAYER_FULLY_CONNECTED && !N.w_prepared && fc_uses_shared_panels(net, N, rows)) next.layer = &N;
+      if (N.type == MYEA_LAYER_FULLY_CONNECTED && !N.w_fresh && fc_uses_shared_panels(net, N, rows)) next.layer = &N;
     }
     OverlapWork work;
     work.arg = &next;
@@ -843,7 +856,7 @@ static int forward_impl(myea_b200_net *net, uint64_t batch, const float *src, cu
   net->active_B = static_cast<long long>(batch);
   const long long rows = step_rows_total(net);
   const int n = static_cast<int>(net->layers.size());
-  for (auto &L : net->layers) { L.w_prepared = false; L.in_ready_src = nullptr; }
+  for (auto &L : net->layers) L.in_ready_src = nullptr;
   // After a sharded update the gathers of the updated parameters may still be travelling.  Biases and normalization
   // parameters are waited for here, every fully connected layer's weights where the layer first reads them, and
   // everything that is left before any other kind of layer.
@@ -860,7 +873,7 @@ static int forward_impl(myea_b200_net *net, uint64_t batch, const float *src, cu
     CK(cudaEventRecord(net->ev_input_ready, net->copy_stream));
     for (int l = 1; l < n; ++l) {
       LayerPlan &L = net->layers[l];
-      if (L.type == MYEA_LAYER_FULLY_CONNECTED && fc_uses_shared_panels(net, L, rows)) RC(fc_prepare_weights(net, L));
+      if (L.type == MYEA_LAYER_FULLY_CONNECTED && !L.w_fresh && fc_uses_shared_panels(net, L, rows)) RC(fc_prepare_weights(net, L));
     }
     CK(cudaStreamWaitEvent(net->ctx.stream, net->ev_input_ready, 0));
   } else {
@@ -1190,7 +1203,8 @@ int fc_update_derivative_weight(myea_b200_net *net, LayerPlan &L, const float *i
   Epilogue e;
   e.C = net->grads + L.idx.first_connection_index;
   e.ldc = L.n_in;
-  e.accumulate = 1;
+  e.accumulate = L.dw_stale ? 0 : 1;
+  L.dw_stale = false;
   if (fc_derivative_runs_direct(net, L, rows)) {  // the bias derivative (row sums of delta^T) rides along
     DirectItem item{a, b, e, L.use_bias ? net->grads + L.idx.first_bias_connection_index : nullptr};
     if (group != nullptr) {
@@ -1276,6 +1290,7 @@ extern "C" int myea_b200_update_parameter(myea_handle net, uint64_t batch, uint6
   if (net == nullptr || opt == nullptr || training_size == 0) return MYEA_E_INVALID;
   CK(cudaSetDevice(net->ctx.device));
   RC(comm_gather_join(net));
+  RC(settle_derivatives(net));
   const size_t P = net->total_parameters;
   // The update is element by element, so each derivative bucket can be applied as soon as ITS sum over the ranks has
   // arrived, while the later buckets are still on the wire - and only on this rank's slice of it where the bucket was
@@ -1293,7 +1308,7 @@ extern "C" int myea_b200_update_parameter(myea_handle net, uint64_t batch, uint6
     else RC(comm_all_reduce_sum(net, net->grads, P));      // nothing was issued: reduce everything now
     net->grads_reduced = false;
   }
-  for (auto &L : net->layers) L.w_valid = false;  // the weights change below
+  for (auto &L : net->layers) L.w_valid = L.w_fresh = false;  // the weights change below
   OptLaunch o;
   o.type = opt->type_optimizer_function;
   struct ReadyBucket { size_t i, n, off, slice; };
@@ -1381,8 +1396,8 @@ extern "C" int myea_b200_update_parameter(myea_handle net, uint64_t batch, uint6
       if (!ready.empty()) { i = ready[k].i; n = ready[k].n; off = ready[k].off; slice = ready[k].slice; }
       else RC(comm_bucket_wait(net, i, &bucket_off, &n, &off, &slice));
       if ((off & 3) != 0) return fail(net, MYEA_E_INVALID, "derivative bucket does not start on a 16-byte boundary");
-      RC(optimizer_update(net->ctx, o, net->params + off, net->grads + off, net->m1 + off, net->m2 + off, net->m2hat + off, net->prev_delta + off,
-                          net->mask_reg + off, slice));
+      const OptArrays all{net->params, net->grads, net->m1, net->m2, net->m2hat, net->prev_delta, net->mask_reg};
+      RC(optimizer_update(net->ctx, o, all.at(off), slice));
       RC(comm_bucket_gather(net, i));  // the other ranks' slices of the updated parameters (nothing for an all-reduced bucket)
       covered += n;
     }
@@ -1390,7 +1405,23 @@ extern "C" int myea_b200_update_parameter(myea_handle net, uint64_t batch, uint6
     net->grads_reduced = false;
     if (covered != P) return fail(net, MYEA_E_INVALID, "derivative buckets do not cover the parameter buffer");
   } else {
-    RC(optimizer_update(net->ctx, o, net->params, net->grads, net->m1, net->m2, net->m2hat, net->prev_delta, net->mask_reg, P));
+    const OptArrays all{net->params, net->grads, net->m1, net->m2, net->m2hat, net->prev_delta, net->mask_reg};
+    // One GPU: the weights of layers that work on operand panels are updated block by block, and the new panels leave with
+    // them (a rank of a job holds a slice of the new weights only; the max-norm constraint changes them once more).
+    std::vector<OptPanelLayer> blocks;
+    std::vector<std::pair<size_t, size_t>> rest;   // [begin, end) of what the plain kernel updates
+    size_t done = 0;
+    for (auto &L : net->layers) {
+      const size_t first = L.idx.first_connection_index, count = static_cast<size_t>(L.n_out * L.n_in);
+      if (net->comm != nullptr || max_norm != 0.f || !L.shared_panels || L.ind_rnn || (L.n_in & 7) != 0 || (first & 3) != 0 || first < done) continue;
+      if (first > done) rest.emplace_back(done, first);
+      blocks.push_back(OptPanelLayer{first, L.w_pan, 0});
+      done = first + count;
+      L.w_fresh = L.dw_stale = true;
+    }
+    if (done < P) rest.emplace_back(done, P);
+    if (!blocks.empty()) RC(optimizer_update_panels(net->ctx, o, all, blocks.data(), static_cast<int>(blocks.size())));
+    for (const auto &r : rest) RC(optimizer_update(net->ctx, o, all.at(r.first), r.second - r.first));
   }
   // independently recurrent layers keep their recurrent weights inside their bound (Update_Parameter: Use__Regularization__Constraint_Recurrent_Weight)
   for (const auto &L : net->layers)
@@ -1415,6 +1446,7 @@ extern "C" int myea_b200_clear_training_arrays(myea_handle net) {
   if (net == nullptr) return MYEA_E_INVALID;
   const size_t bytes = (net->total_parameters + 4) * sizeof(float);
   CK(cudaMemsetAsync(net->grads, 0, bytes, net->ctx.stream));
+  for (auto &L : net->layers) L.dw_stale = false;
   CK(cudaMemsetAsync(net->m1, 0, bytes, net->ctx.stream));
   CK(cudaMemsetAsync(net->m2, 0, bytes, net->ctx.stream));
   CK(cudaMemsetAsync(net->m2hat, 0, bytes, net->ctx.stream));

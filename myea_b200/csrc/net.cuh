@@ -43,7 +43,8 @@ struct LayerPlan {
   float *in_panel_mem = nullptr, *w_panel_mem = nullptr, *d_panel_mem = nullptr;
   HalfPanels in_pan, w_pan, d_pan;  // as of the step in flight (a short batch has fewer rows)
   bool in_valid = false, w_valid = false, d_valid = false;
-  bool w_prepared = false;  // the weight panels have already been made in this forward pass (hoisted under the input copy)
+  bool w_fresh = false;   // the weight panels (of an LSTM layer: all that its forward pass lays out from its weights) match the parameters
+  bool dw_stale = false;  // the weight derivatives are zero by the interface; their memory still holds the values of the last update
   const float *in_src = nullptr;  // the array the input panels were made from
   const float *in_ready_src = nullptr;  // set by the producer of this layer's input when IT has written the input panels
   long long in_ready_rows = 0;

@@ -6,15 +6,11 @@
 // Clip_Gradient / Euclidean_Norm (Neural_Network__Clip_Gradient.cpp:82-94, …Regularization__Max_Norm_Constraints.cpp:48-87).
 // Pure HBM streaming: every array is read and written once with 128-bit accesses; the optimizer is a uniform branch.
 #include "common.cuh"
+#include "half_panels.cuh"
 
 #include <algorithm>
 
 namespace myea {
-
-struct OptArrays {
-  float *w, *g, *m, *v, *vhat, *prev;
-  const float *mask;
-};
 
 __device__ __forceinline__ float opt_one(const OptLaunch &o, float w, float g, float &m, float &v, float &vhat, float &prev, float mask) {
   const float decay = (o.weight_decay != 0.f) ? mask * o.weight_decay * w : 0.f;
@@ -120,19 +116,115 @@ __global__ void __launch_bounds__(256) optimizer_kernel(const OptLaunch o, const
   }
 }
 
-int optimizer_update(Context &ctx, const OptLaunch &o, float *w, float *g, float *m, float *v, float *vhat, float *prev_delta,
-                     const float *mask, size_t n) {
-  OptArrays a{w, g, m, v, vhat, prev_delta, mask};
-  const bool has_vhat = (o.type == MYEA_OPT_AMSGRAD || o.type == MYEA_OPT_AMSBOUND);
-  const bool has_prev = (o.type == MYEA_OPT_GD && o.momentum != 0.f) || o.type == MYEA_OPT_IRPROP_PLUS;
-  if ((has_vhat && vhat == nullptr) || (has_prev && prev_delta == nullptr) || (o.type != MYEA_OPT_GD && (m == nullptr || v == nullptr)))
-    return MYEA_E_INVALID;
+static bool opt_arrays(const OptLaunch &o, const OptArrays &a, bool &has_vhat, bool &has_prev) {
+  has_vhat = (o.type == MYEA_OPT_AMSGRAD || o.type == MYEA_OPT_AMSBOUND);
+  has_prev = (o.type == MYEA_OPT_GD && o.momentum != 0.f) || o.type == MYEA_OPT_IRPROP_PLUS;
+  return !((has_vhat && a.vhat == nullptr) || (has_prev && a.prev == nullptr) || (o.type != MYEA_OPT_GD && (a.m == nullptr || a.v == nullptr)));
+}
+
+int optimizer_update(Context &ctx, const OptLaunch &o, const OptArrays &a, size_t n) {
+  bool has_vhat, has_prev;
+  if (!opt_arrays(o, a, has_vhat, has_prev)) return MYEA_E_INVALID;
   const int blocks = static_cast<int>(std::max<size_t>(1, std::min<size_t>(((n >> 2) + 255) / 256, 148 * 16)));
   ctx.begin(TC_OPTIMIZER);
   if (has_vhat) launch_dependent(ctx, optimizer_kernel<true, false>, dim3(blocks), dim3(256), 0, o, a, n);
   else if (has_prev) launch_dependent(ctx, optimizer_kernel<false, true>, dim3(blocks), dim3(256), 0, o, a, n);
   else launch_dependent(ctx, optimizer_kernel<false, false>, dim3(blocks), dim3(256), 0, o, a, n);
   ctx.end(TC_OPTIMIZER);
+  return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
+}
+
+// The update of weights that contractions read as operand panels: a CTA updates a block of 128 x 128 weights, keeps the new
+// values, finds their exponent and writes the panels of the next step along, which otherwise cost a pass of their own over the
+// weights (4 bytes read and 4 written per weight); the derivatives are not zeroed (4 bytes less), the next accumulation
+// overwrites them instead of adding to them (4 bytes less again).  Bound by HBM, so by loads in flight: a thread has 8 elements
+// of all arrays on the way, 1024 threads per SM; the new weights wait in shared memory (64 KB) because in registers they leave
+// room for half the threads (134 M weights, Adam: 686 us, 6.26 TB/s, where update and splits were 720 + 200 us; with the
+// weights in registers and 512 threads per SM 1770 us).
+constexpr int OPT_LAYERS = 32;
+constexpr int OPT_THREADS = 512;
+constexpr int OPT_ROWS = HP_BLOCK * 16 / OPT_THREADS;   // rows per thread: 8 columns of rows tid / 16 + 32 i
+constexpr int OPT_SMEM = HP_BLOCK * HP_BLOCK * 4;
+struct OptPanelTable {
+  OptPanelLayer l[OPT_LAYERS];
+  int n;
+};
+template <bool HAS_VHAT, bool HAS_PREV>
+__global__ void __launch_bounds__(OPT_THREADS, 2) optimizer_panels_kernel(const OptLaunch o, const OptArrays a, const __grid_constant__ OptPanelTable t) {
+  extern __shared__ float4 kept[];   // [row][2][thread]
+  grid_dependency_wait();
+  grid_dependency_release();
+  const float scale = o.clip_scale != nullptr ? *o.clip_scale : 1.0f;
+  const bool adam_like = o.type != MYEA_OPT_GD, decays = o.weight_decay != 0.f && a.mask != nullptr;
+  int k = 0;
+  while (k + 1 < t.n && static_cast<int>(blockIdx.x) >= t.l[k + 1].first_block) ++k;
+  const HalfPanels &p = t.l[k].p;
+  const int block = static_cast<int>(blockIdx.x) - t.l[k].first_block;
+  const int across = static_cast<int>((p.C + HP_BLOCK - 1) / HP_BLOCK), by = block / across, bx = block - by * across;
+  const long long c = bx * static_cast<long long>(HP_BLOCK) + (threadIdx.x & 15) * 8;
+  const long long r0 = by * static_cast<long long>(HP_BLOCK) + (threadIdx.x >> 4);
+  float amax = 0.f;
+#pragma unroll 1
+  for (int i = 0; i < OPT_ROWS; ++i) {
+    const long long r = r0 + OPT_THREADS / 16 * i;
+    float w[8] = {};
+    if (r < p.R && c < p.C) {
+      const size_t at = t.l[k].offset + static_cast<size_t>(r * p.C + c);
+      float g[8], m[8] = {}, v[8] = {}, vh[8] = {}, pv[8] = {}, mk[8] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
+      ld8(w, a.w + at, 8, true);
+      ld8(g, a.g + at, 8, true);
+      if (adam_like) { ld8(m, a.m + at, 8, true); ld8(v, a.v + at, 8, true); }
+      if (HAS_VHAT) ld8(vh, a.vhat + at, 8, true);
+      if (HAS_PREV) ld8(pv, a.prev + at, 8, true);
+      if (decays) ld8(mk, a.mask + at, 8, true);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) w[j] = opt_one(o, w[j], g[j] * scale, m[j], v[j], vh[j], pv[j], mk[j]);
+      st8(a.w + at, w, 8, true);
+      if (adam_like) { st8(a.m + at, m, 8, true); st8(a.v + at, v, 8, true); }
+      if (HAS_VHAT) st8(a.vhat + at, vh, 8, true);
+      if (HAS_PREV) st8(a.prev + at, pv, 8, true);
+      amax = amax8(w, amax);
+    }
+    kept[(2 * i) * OPT_THREADS + threadIdx.x] = make_float4(w[0], w[1], w[2], w[3]);
+    kept[(2 * i + 1) * OPT_THREADS + threadIdx.x] = make_float4(w[4], w[5], w[6], w[7]);
+  }
+  const int e = half_block_exponent<OPT_THREADS>(amax);
+  if (threadIdx.x == 0) p.exps[by * p.exp_r + bx * p.exp_c] = e;
+  if (c >= p.pitch) return;
+  const float s = pow2(-e);
+#pragma unroll
+  for (int i = 0; i < OPT_ROWS; ++i) {
+    const long long r = r0 + OPT_THREADS / 16 * i;
+    const float4 x = kept[(2 * i) * OPT_THREADS + threadIdx.x], y = kept[(2 * i + 1) * OPT_THREADS + threadIdx.x];
+    const float w[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+    if (r < p.R) half_store8(p, r, c, w, s);
+  }
+}
+template <bool HAS_VHAT, bool HAS_PREV>
+static int launch_optimizer_panels(Context &ctx, int blocks, const OptLaunch &o, const OptArrays &a, const OptPanelTable &t) {
+  auto kernel = optimizer_panels_kernel<HAS_VHAT, HAS_PREV>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OPT_SMEM) != cudaSuccess) return MYEA_E_CUDA;
+  return launch_dependent(ctx, kernel, dim3(blocks), dim3(OPT_THREADS), OPT_SMEM, o, a, t) == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
+}
+
+int optimizer_update_panels(Context &ctx, const OptLaunch &o, const OptArrays &a, const OptPanelLayer *layers, int n) {
+  bool has_vhat, has_prev;
+  if (!opt_arrays(o, a, has_vhat, has_prev)) return MYEA_E_INVALID;
+  for (int first = 0; first < n; first += OPT_LAYERS) {
+    OptPanelTable t = {};
+    t.n = std::min(OPT_LAYERS, n - first);
+    int blocks = 0;
+    for (int k = 0; k < t.n; ++k) {
+      t.l[k] = layers[first + k];
+      t.l[k].first_block = blocks;
+      blocks += static_cast<int>(((t.l[k].p.R + HP_BLOCK - 1) / HP_BLOCK) * ((t.l[k].p.C + HP_BLOCK - 1) / HP_BLOCK));
+    }
+    ctx.begin(TC_OPTIMIZER);
+    const int rc = has_vhat ? launch_optimizer_panels<true, false>(ctx, blocks, o, a, t)
+                 : has_prev ? launch_optimizer_panels<false, true>(ctx, blocks, o, a, t) : launch_optimizer_panels<false, false>(ctx, blocks, o, a, t);
+    ctx.end(TC_OPTIMIZER);
+    if (rc != MYEA_OK) return rc;
+  }
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
 

@@ -77,3 +77,40 @@ def test_lstm_with_resident_weights(n_in, H, T, B, bidirectional, zoneout):
     wl = workloads.Workload("lstm edges", capi.net(layers, B, T=T, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE),
                             capi.opt(capi.OPT_GD, gd_lr=0.01 / B, momentum=0.9), n_in, H, False, layers)
     _step(wl)
+
+
+@pytest.mark.parametrize("widths,B", [((1000, 904, 1100, 130), 700), ((1004, 1000, 1096), 640)])   # multiples of 8 and not, ragged blocks of 128
+@pytest.mark.parametrize("opt", [dict(t=capi.OPT_ADAM, eps=1.0), dict(t=capi.OPT_AMSGRAD, eps=1.0, weight_decay=1e-3), dict(t=capi.OPT_GD, gd_lr=1e-5, momentum=0.9, nesterov=True, clip=0.5)])
+def test_update_writes_operand_panels(widths, B, opt):
+    """updates that leave the next step's weight panels and unzeroed derivatives: accumulation over two batches, derivatives read
+    back, an update without any, parameters replaced from the host, inference between the steps"""
+    kw = dict(opt)
+    layers = [capi.fc(widths[0])] + [capi.fc(w, capi.AF_TANH) for w in widths[1:-1]] + [capi.fc(widths[-1], capi.AF_LINEAR)]
+    wl = workloads.Workload("panels", capi.net(layers, B, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE), capi.opt(kw.pop("t"), **kw), widths[0], widths[-1], False, layers)
+    gpu, cpu = Net(wl.desc, wl.opt), myea_oracle.OracleNet(wl.desc, wl.opt)
+    out = []
+    for net in (gpu, cpu):
+        wl.materialize(net)
+        got = []
+        if opt.get("weight_decay"):
+            mask = np.ones(gpu.P, np.float32)
+            mask[::3] = 0
+            net.set(capi.BUF_MASK_REGULARIZED, mask)
+        for batches in (1, 2, 0, 1):
+            for k in range(batches):
+                X, Y = wl.batch(7 + k)
+                net.reset_loss(); net.forward(X); net.compute_error(Y); net.backward(); net.update_derivative_weight()
+            got.append(net.get(capi.BUF_DERIVATIVES) if batches == 2 else None)
+            net.update_parameter()
+            got.append(net.get(capi.BUF_PARAMETERS))
+        assert not np.any(net.get(capi.BUF_DERIVATIVES))
+        net.forward(X, training=False)
+        got.append(net.outputs(len(widths) - 1))
+        net.set(capi.BUF_PARAMETERS, got[1])
+        net.forward(X, training=False)
+        got.append(net.outputs(len(widths) - 1))
+        out.append([g for g in got if g is not None])
+    gpu.synchronize()
+    gpu.close()
+    for got, want in zip(*out):
+        assert rel_err(got, want) < TOL
