@@ -51,7 +51,7 @@ template <int BN> struct HalfSmem {
   static constexpr int B_BYTES = BN / 2 * 128;
   static constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;  // A h0, A h1, B h0, B h1
   static constexpr int BAR_OFFSET = HG_STAGES * STAGE_BYTES;
-  static constexpr int TR_OFFSET = BAR_OFFSET + 512;        // epilogue staging: 8 warps x 16 x 36 floats (the stages stay busy)
+  static constexpr int TR_OFFSET = BAR_OFFSET + 512;        // epilogue staging: 8 warps x 32 x 32 floats (the stages stay busy)
   static constexpr int TOTAL = TR_OFFSET + 8 * TR_WARP_FLOATS * 4 + 1024;
 };
 

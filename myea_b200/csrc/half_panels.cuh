@@ -48,9 +48,10 @@ __device__ __forceinline__ void half_split8(const float (&v)[8], uint4 &h0, uint
   h1 = make_uint4(b[0], b[1], b[2], b[3]);
 }
 
-// A block of 256 threads holds a 128 x 128 block of the tensor: thread = 8 columns (tid % 16) of rows tid / 16 + 16 i.
+// A block of 512 threads holds a 128 x 128 block of the tensor: thread = 8 columns (tid % 16) of rows tid / 16 + 32 i.
 // half_block_finish: the block's exponent from every thread's largest magnitude (all threads of the block call it).
-constexpr int HP_THREADS = 256;
+constexpr int HP_THREADS = 512;
+constexpr int HP_ROWS = HP_BLOCK * 16 / HP_THREADS;   // rows per thread
 template <int THREADS = HP_THREADS>
 __device__ __forceinline__ int half_block_exponent(float amax) {
   __shared__ float sh[THREADS / 32];
@@ -80,7 +81,9 @@ __device__ __forceinline__ void half_store8(const HalfPanels &p, long long r, lo
 
 // ---------------------------------------------------------------------------------------------------------
 // A producer computes an fp32 tensor and leaves it both as an array and as panels for the contractions that read it next:
-// one block of 128 x 128 per CTA, read once, its largest magnitude found in registers, everything written once.
+// one block of 128 x 128 per CTA, read once, its largest magnitude found in registers, everything written once.  Bound by HBM
+// at 4096 x 4096 (26 us for the 128 MB of a split) and by the chain load - maximum - store of the one block an SM gets at 512 rows:
+// 512 threads of 4 rows (activation of 512 x 4096 11.3 us, with 256 threads of 8 rows 13.1).
 // F: struct Cols; columns(Cols &, c, n): what belongs to this thread's columns c .. c + n - 1; row(cols, r, c, n, v): the
 // values of row r (zeros in v[n] ..); keep(r, c, n, v): stores the fp32 result (may do nothing).
 // ---------------------------------------------------------------------------------------------------------
@@ -113,10 +116,10 @@ __global__ void __launch_bounds__(HP_THREADS, 2) half_produce_kernel(const F f, 
   const int n = static_cast<int>(max(0ll, min(8ll, p.C - c)));
   typename F::Cols cols;
   f.columns(cols, c, n);
-  float v[8][8], m = 0.f;
+  float v[HP_ROWS][8], m = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const long long r = r0 + 16 * i;
+  for (int i = 0; i < HP_ROWS; ++i) {
+    const long long r = r0 + HP_THREADS / 16 * i;
     if (r < p.R) {
       f.row(cols, r, c, n, v[i]);
     } else {
@@ -125,14 +128,14 @@ __global__ void __launch_bounds__(HP_THREADS, 2) half_produce_kernel(const F f, 
     }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) m = amax8(v[i], m);
+  for (int i = 0; i < HP_ROWS; ++i) m = amax8(v[i], m);
   const int e = half_block_exponent(m);
   if (threadIdx.x == 0) p.exps[blockIdx.y * p.exp_r + blockIdx.x * p.exp_c] = e;
   if (c >= p.pitch) return;
   const float scale = pow2(-e);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const long long r = r0 + 16 * i;
+  for (int i = 0; i < HP_ROWS; ++i) {
+    const long long r = r0 + HP_THREADS / 16 * i;
     if (r >= p.R) continue;
     f.keep(r, c, n, v[i]);
     half_store8(p, r, c, v[i], scale);
