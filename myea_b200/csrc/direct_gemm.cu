@@ -37,6 +37,8 @@ static_assert((DG_M * DG_RED_PITCH + 2 * DG_M) * 4 <= DG_STAGES * DG_STAGE_BYTES
 constexpr int DG_BAR_OFFSET = DG_STAGES * DG_STAGE_BYTES;
 constexpr int DG_SMEM = DG_BAR_OFFSET + 64 + 1024;
 constexpr int DG_MAX_ITEMS = 12;
+constexpr int FG_M = 32, FG_N = 32;          // tile of the kernel that multiplies with plain FMAs
+constexpr int FG_K = 256;                    // K it holds in shared memory at a time
 
 // x rounded to TF32, half away from zero, on the integer pipe: cvt.rna.tf32 gives the same bits at a quarter of the rate
 // (it and single bf16 conversions kept the pipe of special functions busy: 14 instructions per split element, now 4).
@@ -136,9 +138,10 @@ static __device__ __noinline__ float af_fire_rare(uint32_t af, float z) { return
 // What this CTA finishes of its tile: rows [first, first + count), summed over the CTAs of the cluster in rank order, through
 // the epilogue.  A thread keeps VEC adjacent columns and takes NB rows at a time, all their loads before the first use: with
 // a row at a time this part was latency after latency and took longer than the products (29 of 31 us at K = 10).
-template <int VEC, int NB>
+// TN: columns of the tile; PARTS: partial tiles of FG_M rows in this CTA's own shared memory, one behind the other (S == 1).
+template <int TN, int PARTS, int VEC, int NB>
 __device__ __forceinline__ void dg_finish(const DirectProblem &p, const float *partial, uint32_t S, int first, int count, int m0, int n0) {
-  constexpr int LANES = DG_N / VEC, STEP = DG_THREADS / LANES;
+  constexpr int LANES = TN / VEC, STEP = DG_THREADS / LANES, PITCH = TN + 4;
   using Vec = float[VEC];
   const Epilogue &e = p.epi;
   const int c = (static_cast<int>(threadIdx.x) % LANES) * VEC, n = n0 + c;
@@ -178,15 +181,23 @@ __device__ __forceinline__ void dg_finish(const DirectProblem &p, const float *p
       if (e.deriv_af != 0u && e.aux_pre != nullptr) load(pre[b], e.aux_pre + m * e.ld_aux + n);
       if (e.deriv_af != 0u && e.aux_y != nullptr) load(y[b], e.aux_y + m * e.ld_aux + n);
       if (e.accumulate) load(old[b], dst[b]);
-      if (S == 1) load(v[b], partial + r * DG_RED_PITCH + c);
+      if (S == 1) {
+#pragma unroll
+        for (int q = 0; q < PARTS; ++q) {
+          Vec t;
+          load(t, partial + (q * FG_M + r) * PITCH + c);   // (one part: row r of it)
+#pragma unroll
+          for (int k = 0; k < VEC; ++k) v[b][k] += t[k];
+        }
+      }
     }
-    if (S > 1) {
+    if (PARTS == 1 && S > 1) {
 #pragma unroll 2
       for (uint32_t q = 0; q < S; ++q) {
         const uint32_t base = ptx::map_to_cta(ptx::smem_u32(partial), q);
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
-          const uint32_t at = base + (min(r0 + b * STEP, end - 1) * DG_RED_PITCH + c) * 4;
+          const uint32_t at = base + (min(r0 + b * STEP, end - 1) * PITCH + c) * 4;
           if constexpr (VEC == 4) {
             const float4 t = ptx::ld_cluster_f4(at);
             v[b][0] += t.x; v[b][1] += t.y; v[b][2] += t.z; v[b][3] += t.w;
@@ -369,8 +380,8 @@ __global__ void __launch_bounds__(DG_THREADS, 2) direct_gemm_kernel(const __grid
     ptx::tmem_dealloc(tmem, DG_TMEM_COLS);
   }
   const int my_rows = DG_M / static_cast<int>(S), first = static_cast<int>(rank) * my_rows;
-  if (p.c_vec) dg_finish<4, 2>(p, partial, S, first, my_rows, m0, n0);
-  else dg_finish<1, 8>(p, partial, S, first, my_rows, m0, n0);
+  if (p.c_vec) dg_finish<DG_N, 1, 4, 2>(p, partial, S, first, my_rows, m0, n0);
+  else dg_finish<DG_N, 1, 1, 8>(p, partial, S, first, my_rows, m0, n0);
   if (want_sum) {
     for (int r = first + tid; r < first + my_rows; r += DG_THREADS) {
       if (m0 + r >= p.M) continue;
@@ -387,6 +398,161 @@ __global__ void __launch_bounds__(DG_THREADS, 2) direct_gemm_kernel(const __grid
     }
   }
   if (S > 1) ptx::cluster_sync_all();  // a peer may still be reading this CTA's partial tile
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// The smallest products with plain FMAs.  A tensor-core tile pays for tensor memory, barriers, conversion, a cluster and its
+// exchange before anything else: 128 x 256 x 256 takes it 6.8 us (here 5.4), of which the products are a tenth.  Here a CTA owns
+// 32 x 32 outputs, fetches both operands' rows for up to 256 of K at once (16 loads of 16 bytes per thread in flight: one trip
+// to L2), and its 8 warps walk interleaved groups of four K each with 4 x 8 sums per lane; the 8 partial tiles are added in warp
+// order in shared memory (bitwise repeatable).  Bound by latency, from about K = 512 on by shared-memory reads and FMA issue.
+// Operand rows contiguous in K lie as [row][FG_K + 4] (lanes read rows rg + 8 i: eight different 16-byte chunks), operands
+// read through their columns as [k][32].
+// ---------------------------------------------------------------------------------------------------------
+constexpr int FG_PITCH = FG_K + 4;
+constexpr int FG_OP_FLOATS = 32 * FG_PITCH;               // one operand
+constexpr int FG_RED_FLOATS = 8 * FG_M * (FG_N + 4) + 8 * FG_M;   // partial tiles, then the warps' row sums; over the operands
+constexpr int FG_SMEM = (2 * FG_OP_FLOATS > FG_RED_FLOATS ? 2 * FG_OP_FLOATS : FG_RED_FLOATS) * 4;
+
+// rows row0 .. row0 + 31 (past `rows`: the last one again), K elements k0 .. k0 + kc - 1 (zeros up to a multiple of 4)
+template <bool T>
+__device__ __forceinline__ void fg_fetch(float *s, const float *src, long long ld, int row0, int rows, int k0, int kc, bool vec) {
+  const int tid = static_cast<int>(threadIdx.x), kz = (kc + 3) & ~3;
+  if (T) {
+    // [k][32]: lanes take consecutive rows
+    if (vec && row0 + 32 <= rows) {
+      const int c = (tid & 7) * 4, kk0 = tid >> 3;   // 32 K rows per round
+      float4 v[8];
+#pragma unroll
+      for (int i = 0; i < FG_K / 32; ++i) {
+        const int kk = kk0 + 32 * i;
+        if (kk < kc) v[i] = *reinterpret_cast<const float4 *>(src + static_cast<long long>(k0 + kk) * ld + row0 + c);
+        else v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int i = 0; i < FG_K / 32; ++i) {
+        const int kk = kk0 + 32 * i;
+        if (kk < kz) *reinterpret_cast<float4 *>(s + kk * 32 + c) = v[i];
+      }
+    } else {
+      const int r = tid & 31, row = min(row0 + r, rows - 1);
+      const float *q = src + static_cast<long long>(k0) * ld + row;
+      for (int base = 0; base < kz; base += 64) {
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int kk = base + (tid >> 5) + 8 * i;
+          v[i] = kk < kc ? q[static_cast<long long>(kk) * ld] : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int kk = base + (tid >> 5) + 8 * i;
+          if (kk < kz) s[kk * 32 + r] = v[i];
+        }
+      }
+    }
+  } else if (vec && (kc & 3) == 0) {
+    // [row][FG_PITCH]: lanes take consecutive 16-byte chunks of a row (a whole row of 256 by two warps)
+    const int c = (tid & 63) * 4, r0 = tid >> 6;
+    float4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = min(row0 + r0 + 4 * i, rows - 1);
+      if (c < kc) v[i] = *reinterpret_cast<const float4 *>(src + static_cast<long long>(row) * ld + k0 + c);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (c < kc) *reinterpret_cast<float4 *>(s + (r0 + 4 * i) * FG_PITCH + c) = v[i];
+  } else {
+    const int lane = tid & 31, r0 = tid >> 5;
+#pragma unroll 2
+    for (int i = 0; i < 4; ++i) {
+      const int row = min(row0 + r0 + 8 * i, rows - 1);
+      const float *q = src + static_cast<long long>(row) * ld + k0;
+      float v[FG_K / 32];
+#pragma unroll
+      for (int j = 0; j < FG_K / 32; ++j) v[j] = lane + 32 * j < kc ? q[lane + 32 * j] : 0.f;
+#pragma unroll
+      for (int j = 0; j < FG_K / 32; ++j)
+        if (lane + 32 * j < kz) s[(r0 + 8 * i) * FG_PITCH + lane + 32 * j] = v[j];
+    }
+  }
+}
+
+template <bool AT, bool BT, int MAX>
+__global__ void __launch_bounds__(DG_THREADS, 2) fma_gemm_kernel(const __grid_constant__ DirectGroup<MAX> g) {
+  extern __shared__ float fg_smem[];
+  float *sa = fg_smem, *sb = fg_smem + FG_OP_FLOATS;
+  const int tile = static_cast<int>(blockIdx.x);
+  int pi = 0;
+#pragma unroll 1
+  while (pi + 1 < g.count && tile >= g.p[pi + 1].first_tile) ++pi;
+  const DirectProblem &p = g.p[pi];
+  const int tl = tile - p.first_tile;
+  const int tm = tl / p.tiles_n, tn = tl - tm * p.tiles_n;
+  const int m0 = tm * FG_M, n0 = tn * FG_N;
+  const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31;
+  const int rg = lane >> 2, cg = lane & 3;   // rows rg + 8 i or 4 rg + i, columns cg + 4 j or 8 cg + j
+  const bool want_sum = AT && p.row_sum != nullptr && tn == 0;
+  float acc[4][8] = {};
+  float rs = 0.f;
+  grid_dependency_wait();
+  grid_dependency_release();
+#pragma unroll 1
+  for (int k0 = 0; k0 < p.K; k0 += FG_K) {
+    const int kc = min(FG_K, p.K - k0);
+    if (k0 > 0) __syncthreads();
+    fg_fetch<AT>(sa, p.a, p.lda, m0, p.M, k0, kc, p.a_vec != 0);
+    fg_fetch<BT>(sb, p.b, p.ldb, n0, p.N, k0, kc, p.b_vec != 0);
+    __syncthreads();
+    if (want_sum)
+      for (int k = warp; k < kc; k += 8) rs += sa[k * 32 + lane];
+#pragma unroll 2
+    for (int k = warp * 4; k < kc; k += 32) {
+      float a[4][4], b[4][8];   // [row][k], [k][column]
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 t = *reinterpret_cast<const float4 *>(AT ? sa + (k + i) * 32 + rg * 4 : sa + (rg + 8 * i) * FG_PITCH + k);
+        if (AT) { a[0][i] = t.x; a[1][i] = t.y; a[2][i] = t.z; a[3][i] = t.w; }
+        else { a[i][0] = t.x; a[i][1] = t.y; a[i][2] = t.z; a[i][3] = t.w; }
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (BT) {
+          const float4 t = *reinterpret_cast<const float4 *>(sb + (k + (i >> 1)) * 32 + cg * 8 + (i & 1) * 4);
+          b[i >> 1][(i & 1) * 4] = t.x; b[i >> 1][(i & 1) * 4 + 1] = t.y; b[i >> 1][(i & 1) * 4 + 2] = t.z; b[i >> 1][(i & 1) * 4 + 3] = t.w;
+        } else {
+          const float4 t = *reinterpret_cast<const float4 *>(sb + (cg + 4 * i) * FG_PITCH + k);
+          b[0][i] = t.x; b[1][i] = t.y; b[2][i] = t.z; b[3][i] = t.w;
+        }
+      }
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i][kk], b[kk][j], acc[i][j]);
+    }
+  }
+  __syncthreads();   // the operands have been read: the partial tiles take their place
+  float *part = fg_smem + warp * FG_M * (FG_N + 4);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float *d = part + (AT ? rg * 4 + i : rg + 8 * i) * (FG_N + 4);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) d[BT ? cg * 8 + j : cg + 4 * j] = acc[i][j];
+  }
+  float *sums = fg_smem + 8 * FG_M * (FG_N + 4);
+  if (want_sum) sums[tid] = rs;
+  __syncthreads();
+  if (p.c_vec) dg_finish<FG_N, 8, 4, 1>(p, fg_smem, 1, 0, FG_M, m0, n0);
+  else dg_finish<FG_N, 8, 1, 4>(p, fg_smem, 1, 0, FG_M, m0, n0);
+  if (want_sum && tid < FG_M && m0 + tid < p.M) {
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) v += sums[w * 32 + tid];
+    p.row_sum[m0 + tid] += v;
+  }
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -434,12 +600,45 @@ static bool epilogue_is_vector(const Epilogue &e, long long N) {
   return (bits & 15) == 0 && ((N | e.ldc | e.ld_addend | e.ld_aux | e.seg_off[0] | e.seg_off[1] | e.seg_off[2] | e.seg_off[3]) & 3) == 0;
 }
 
+template <bool AT, bool BT, int MAX>
+static int launch_fma(Context &ctx, const DirectGroup<MAX> &g, int tiles) {
+  auto kernel = fma_gemm_kernel<AT, BT, MAX>;
+  static std::once_flag flags[64];
+  static bool ok[64] = {};
+  if (ctx.device < 0 || ctx.device >= 64) return MYEA_E_CUDA;
+  std::call_once(flags[ctx.device], [&] { ok[ctx.device] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FG_SMEM) == cudaSuccess; });
+  if (!ok[ctx.device]) return MYEA_E_CUDA;
+  ctx.begin(TC_GEMM);
+  const cudaError_t err = launch_dependent(ctx, kernel, dim3(static_cast<unsigned>(tiles)), dim3(DG_THREADS), FG_SMEM, g);
+  ctx.end(TC_GEMM);
+  return err == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
+}
+
+// One tile per SM at most: two of these CTAs take all registers of an SM, so that the next launch cannot set itself up beside
+// them (a 256 x 1024 x 10 product alone took 3.4 us instead of 4.6, and the training step around it 5 us more).  Then the walk over
+// K decides: about 2.6 us and 11 ns per K, where the tensor-core tile takes 5.2 us at K = 64, 6.8 at 256 and 8.5 at 512, and 3 us
+// more where its operands' rows are not 16-byte aligned.  Measured (us, FMAs / tensor cores): 128 x 256 x 64 3.5 / 5.3,
+// 128 x 256 x 256 5.4 / 6.8, 256 x 512 x 256 5.6 / 6.9, 384^3 8.0 / 7.8; unaligned 203 x 333 x 75 4.1 / 9.7, 203 x 333 x 333 8.2 / 9.7.
+static bool fma_suits(const DirectItem *items, int n) {
+  long long tiles = 0, longest = 0;
+  bool aligned = true;
+  for (int i = 0; i < n; ++i) {
+    tiles += (items[i].A.rows + FG_M - 1) / FG_M * ((items[i].B.rows + FG_N - 1) / FG_N);
+    longest = std::max(longest, items[i].A.k);
+    for (const Operand *o : {&items[i].A, &items[i].B})
+      aligned = aligned && (reinterpret_cast<uintptr_t>(o->ptr) & 15) == 0 && ((o->stride_k != 1 ? o->stride_k : o->stride_r) & 3) == 0;
+  }
+  return tiles <= 148 && longest <= (aligned ? 280 : 360);
+}
+
 template <int MAX>
 static int direct_gemm_launch(Context &ctx, const DirectItem *items, int n) {
   DirectGroup<MAX> g;
   g.count = n;
   int tiles = 0, min_steps = 1 << 30;
   const bool at = items[0].A.stride_k != 1, bt = items[0].B.stride_k != 1;
+  const bool fma = fma_suits(items, n);
+  const int tile_m = fma ? FG_M : DG_M, tile_n = fma ? FG_N : DG_N;
   for (int i = 0; i < n; ++i) {
     const DirectItem &it = items[i];
     DirectProblem &p = g.p[i];
@@ -451,14 +650,18 @@ static int direct_gemm_launch(Context &ctx, const DirectItem *items, int n) {
     p.a_vec = (reinterpret_cast<uintptr_t>(p.a) & 15) == 0 && (p.lda & 3) == 0;
     p.b_vec = (reinterpret_cast<uintptr_t>(p.b) & 15) == 0 && (p.ldb & 3) == 0;
     p.c_vec = epilogue_is_vector(it.epi, p.N);
-    p.tiles_n = (p.N + DG_N - 1) / DG_N;
+    p.tiles_n = (p.N + tile_n - 1) / tile_n;
     p.first_tile = tiles;
-    tiles += p.tiles_n * ((p.M + DG_M - 1) / DG_M);
+    tiles += p.tiles_n * ((p.M + tile_m - 1) / tile_m);
     p.row_sum = at ? it.row_sum : nullptr;
     p.epi = it.epi;
     if ((it.row_sum != nullptr && !at) || it.epi.stats_kind != 0) return MYEA_E_INVALID;
     min_steps = std::min(min_steps, (p.K + BK - 1) / BK);
     ctx.gemm_flops += 2.0 * p.M * p.N * static_cast<double>(p.K);
+  }
+  if (fma) {
+    if (at) return bt ? launch_fma<true, true>(ctx, g, tiles) : launch_fma<true, false>(ctx, g, tiles);
+    return bt ? launch_fma<false, true>(ctx, g, tiles) : launch_fma<false, false>(ctx, g, tiles);
   }
   // K is cut in up to four while the grid stays within one CTA per SM and every CTA keeps two stages.  Measured (us per
   // launch, cut 1 / 2 / 4 / 8): 128 x 256 x 256 9.6 / 8.0 / 6.6 / 7.2, 203 x 333 x 333 18.6 / 13.6 / 9.8 / 11.3, 512^3 15.7 / 11.2

@@ -114,3 +114,17 @@ def test_update_writes_operand_panels(widths, B, opt):
     gpu.close()
     for got, want in zip(*out):
         assert rel_err(got, want) < TOL
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (31, 33, 3), (32, 32, 4), (33, 65, 255), (64, 96, 256), (65, 31, 257), (128, 256, 280), (100, 37, 360), (96, 128, 281), (90, 50, 361)])
+@pytest.mark.parametrize("columns", [0, 1 << 18, 3 << 17])   # both operands by rows, B by columns, both by columns
+def test_contraction_with_fmas(M, N, K, columns):
+    """the 32 x 32 FMA tile and the sizes where the tensor-core tile takes over"""
+    lib = capi.load()
+    rng = np.random.default_rng(M + N + K)
+    A, B = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
+    out = rng.standard_normal((M, N), dtype=np.float32)
+    want = A.astype(np.float64) @ B.astype(np.float64).T + out
+    a, b = np.ascontiguousarray(A.T if columns & (1 << 17) else A), np.ascontiguousarray(B.T if columns & (1 << 18) else B)
+    assert lib.myea_b200_gemm_nt(0, columns, M, N, K, a.ctypes.data, b.ctypes.data, out.ctypes.data, 1, None, 0) == 0
+    assert rel_err(out, want) < 5e-6
