@@ -27,7 +27,7 @@
 namespace myea {
 
 constexpr int LR_THREADS = 512, LR_WARPS = LR_THREADS / 32;
-constexpr int LR_IN_FLOATS = 10240;                // exchange data of a step (or two chunks of it) in shared memory
+constexpr int LR_RED_FLOATS = 4 * LR_WARPS * 32;     // partial sums: KW * RB * NOp floats, 4 rows x 32 outputs per warp at most
 constexpr int LR_SMEM_MAX = 225 * 1024;
 
 struct ResidentDir {
@@ -42,6 +42,7 @@ struct ResidentArgs {
   int G = 1, groups = 1, R = 0, Rp = 0;   // CTAs per group, groups per direction, rows per group, the same rounded up to 4
   int cpc = 0, NOp = 0, K = 0;            // cells per CTA, outputs per CTA (padded to 4), length of the products
   int RB = 0, KC = 0, KW = 1;             // rows per pass, K per chunk of exchange data, warps that share an output's K range
+  int in_floats = 0;                      // exchange data of a step (or two chunks of it) in shared memory
   long long stride = 0, ldh = 0;
   long long rec[4] = {0, 0, 0, 0}, peep = 0;  // offsets inside a block: recurrent rows of z, i, f, o and the peepholes
   ResidentDir d[2];
@@ -77,9 +78,9 @@ template <int KIND>
 __global__ void __launch_bounds__(LR_THREADS, 1) lstm_resident_kernel(const __grid_constant__ ResidentArgs q) {
   extern __shared__ __align__(16) float lr_smem[];
   __shared__ int s_ok;
-  float *w_s = lr_smem;                                  // [K][NOp]
+  float *red_s = lr_smem;                                // [KW][RB][NOp]
+  float *w_s = lr_smem + LR_RED_FLOATS;                  // [K][NOp]
   float *in_s = w_s + static_cast<size_t>(q.K) * q.NOp;  // G == 1: [2][K][Rp]; else one or two chunks [KC][RB]
-  float *red_s = in_s + LR_IN_FLOATS;                    // [KW][RB][NOp]
   const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31;
   const int per_dir = q.groups * q.G;
   const int dir = static_cast<int>(blockIdx.x) / per_dir, in_dir = static_cast<int>(blockIdx.x) - dir * per_dir;
@@ -344,21 +345,28 @@ static bool resident_shape(int kind, long long B, long long C, int dirs, int sms
   q->RB = std::min(q->Rp, 4 * (LR_WARPS / tiles_c));
   const int tasks = tiles_c * (q->RB / 4);
   q->KW = LR_WARPS / tasks;
+  // The whole exchange data of a pass where it fits: every chunk more is another trip to L2 within the step (1024 cells,
+  // 16 rows: four chunks of 20 KB 11.3 us per step, one of 64 KB 9.7).
+  const long long room = LR_SMEM_MAX / static_cast<long long>(sizeof(float)) - static_cast<long long>(q->K) * q->NOp - LR_RED_FLOATS;
   if (G == 1) {
-    if (2ll * q->K * q->Rp > LR_IN_FLOATS) return false;
+    if (2ll * q->K * q->Rp > room) return false;
     q->KC = q->K;
+    q->in_floats = 2 * q->K * q->Rp;
+  } else if (static_cast<long long>(q->K) * q->RB <= room) {
+    q->KC = q->K;
+    q->in_floats = q->K * q->RB;
   } else {
-    q->KC = q->K * q->RB <= LR_IN_FLOATS ? q->K : LR_IN_FLOATS / 2 / q->RB;
-    if (q->KC < 4 * q->KW) return false;
-    if (q->KC < q->K) q->KC = q->KC / (4 * q->KW) * (4 * q->KW);
+    if (room / 2 / q->RB < 4 * q->KW) return false;
+    q->KC = static_cast<int>(room / 2 / q->RB / (4 * q->KW)) * (4 * q->KW);
+    q->in_floats = 2 * q->KC * q->RB;
   }
-  *smem = (static_cast<size_t>(q->K) * q->NOp + LR_IN_FLOATS + static_cast<size_t>(q->KW) * q->RB * q->NOp) * sizeof(float);
-  if (*smem > LR_SMEM_MAX) return false;
+  *smem = (static_cast<size_t>(q->K) * q->NOp + static_cast<size_t>(q->in_floats) + LR_RED_FLOATS) * sizeof(float);
   const double passes = static_cast<double>((q->Rp + q->RB - 1) / q->RB);
   const double reads = passes * tasks * (q->K / 4.0) * 5.0;                        // shared-memory wavefronts
   const double issue = passes * (q->K / (4.0 * q->KW)) * 20.0;                     // one warp's share, instruction by instruction
   const double exchange = G == 1 ? 0.0 : 3000.0 + 6.0 * G + q->K * static_cast<double>(q->Rp) * 4.0 / 40.0;
-  *clocks = std::max(reads, issue) + exchange + 900.0 * passes + 300.0;
+  const double chunks = (q->K + q->KC - 1) / q->KC;
+  *clocks = std::max(reads, issue) + exchange + 900.0 * passes + 1000.0 * passes * (chunks - 1.0) + 300.0;
   return true;
 }
 
