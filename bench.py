@@ -343,7 +343,7 @@ def run_ours(args):
             "metric": "train samples/sec (fwd+bwd+update)", "value": value, "unit": "samples/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": per_step, "higher_is_better": True,
             "scaling": "strong", "vs_baseline": None,
-            "dtype": "f32 (split-precision tensor-core products: TF32 hi*hi + BF16 cross terms, fp32 accumulate)",
+            "dtype": "f32 (split-precision tensor-core products: operands as two half-precision terms and a power of two per block, fp32 accumulate)",
             "data": "synthetic",
             "config": {"workload": wl.name, "global_batch": global_batch, "per_gpu_batch": wl.B,
                        "parallelism": "dp%d" % world, "l2": "per-step working set (> 6 GB at one GPU) far exceeds the 126 MB L2"},
@@ -355,14 +355,14 @@ def run_ours(args):
                          "frac": gemm_tflops / peak if peak else None,
                          # DRAM bytes of ONE launch of the dominant kernel on the 4096^3 contraction of this workload
                          # (dram__bytes_read.sum + dram__bytes_write.sum of the ncu capture summarised under profiles/;
-                         # algorithmic: 335 MB)
-                         "traffic": 704.7e6 if args.workload == "c2" else None,
-                         "traffic_source": "profiles/gemm3x_tf32_tcgen05_wide_4096x4096x4096.md" if args.workload == "c2" else None,
-                         "kernel": "gemm3x_tf32_tcgen05_wide_kernel", "peak_source": peaks["source"] + " bf16 sustained",
-                         # every fp32 product costs one TF32 and one BF16 K=16 instruction of equal duration: the
-                         # scheme's own ceiling is a quarter of the bf16 peak (sustained: inside a step; burst: alone)
-                         "scheme_ceiling": peak / 4.0, "frac_of_scheme_ceiling": gemm_tflops / (peak / 4.0),
-                         "scheme_ceiling_burst": burst / 4.0, "frac_of_scheme_ceiling_burst": gemm_tflops / (burst / 4.0),
+                         # algorithmic: 201 MB of operands and result, read and written once)
+                         "traffic": 364.6e6 if args.workload == "c2" else None,
+                         "traffic_source": "profiles/half_gemm_4096x4096x4096.md" if args.workload == "c2" else None,
+                         "kernel": "half_gemm_kernel", "peak_source": peaks["source"] + " bf16 sustained",
+                         # every fp32 product costs three half-precision ones: the
+                         # scheme's own ceiling is a third of the bf16 peak (sustained: inside a step; burst: alone)
+                         "scheme_ceiling": peak / 3.0, "frac_of_scheme_ceiling": gemm_tflops / (peak / 3.0),
+                         "scheme_ceiling_burst": burst / 3.0, "frac_of_scheme_ceiling_burst": gemm_tflops / (burst / 3.0),
                          "step_tflops": wl.flops_per_step * world / (per_step / 1e3) / 1e12},
             "kernel_classes_ms_per_step": {n: m / cls_steps for n, m in zip(CLASS_NAMES, cls_ms) if m > 0},
         }

@@ -348,11 +348,10 @@ void *myea_b200_stream(myea_handle h);
 uint64_t myea_b200_kernel_launches(myea_handle h);
 
 /* Stand-alone dense contraction used by the step, exposed for kernel-level tests and roofline timing:
- * C[M,N] (+)= A[M,K] · B[N,K]^T, fp32 in HOST memory, computed on tcgen05 with split precision (TF32 main
- * product + bf16 cross terms; bit 0 of `engine` clear) or with the FP32 FMA kernel (bit 0 set).  Bits 8..16 of
- * `engine` force a tile shape (0 heuristic, 128 single CTA, 2 CTA pair 256x128, 3 CTA pair 256x256, 4 the same
- * without splitting tiles along K); bit 17 / bit 18: A / B is handed over transposed, [K][M] / [K][N] row-major,
- * and read as it lies (256x256 kernel only); bit 19: C = (A·B^T) .* relu'(C on entry), the fused activation-derivative
+ * C[M,N] (+)= A[M,K] · B[N,K]^T, fp32 in HOST memory, computed in split precision on tcgen05 or, where
+ * small, with FMAs (bit 0 of `engine` clear) or with the FP32 FMA engine (bit 0 set).  Bits 8..16 of `engine`: 0 chosen by
+ * size, 4 operand panels without splitting tiles along K, any other value operand panels; bit 17 / bit 18: A / B is handed
+ * over transposed, [K][M] / [K][N] row-major, and read as it lies; bit 19: C = (A·B^T) .* relu'(C on entry), the fused activation-derivative
  * epilogue of the error-propagation product, for kernel-level tests (bits 20 / 21: timing variants of it).  `elapsed_ms` (may be null) receives the mean device time of `repeats`
  * extra runs.  Replaces the triple loops
  * Forward_Pass__FC / Backward_Pass__FC / Update_Derivative_Weight__FC
@@ -363,7 +362,7 @@ int myea_b200_gemm_nt(int device, int engine, uint64_t M, uint64_t N, uint64_t K
 /* No counterpart in the reference.  The same contraction for callers that cannot allocate device memory in the call
  * path (a host that reserved all GPU memory up front, a tick-driven trading loop that cannot absorb cudaMalloc's
  * device-wide synchronisation or its failure): C[M,N] (+)= A[M,K] * B[N,K]^T with A, B, C DEVICE pointers owned by
- * the caller and the operand-panel scratch in a fixed 32 MiB array inside the library image, so the call performs no
+ * the caller and the operand-panel scratch in a fixed array of a little over 32 MiB inside the library image, so the call performs no
  * cudaMalloc / cudaFree.  Limit: 2*(M+N)*round_up(K,32)+64 floats <= 8 Mi floats, else MYEA_E_INVALID with a message in
  * error_message (optional, error_capacity bytes).  Every GPU that loads the library holds the array until exit.  All
  * calls share it: calls that overlap on the GPU race and must be serialised by the caller.  The first call on a
