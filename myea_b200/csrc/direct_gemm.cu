@@ -1,6 +1,6 @@
 // Contractions of small and middle sizes straight from fp32 operands:  C[M,N] (+)= A[M,K] * B[N,K]^T, several per launch.
 //
-// The kernels of gemm.cu read operand panels that split passes have written before: three launches and two extra trips
+// The kernels of half_gemm.cu read operand panels that split passes have written before: three launches and two extra trips
 // through L2 per product, which is nothing beside a large product and everything beside a small one (a training step of
 // a 64-256-256-10 network on 128 rows spent 236 us in 37 launches around 0.06 GFLOP, and its tiles of 128 x 128 kept four
 // SMs busy).  Here the operands are read as they lie (rows or columns contiguous, any pitch), split in registers and
@@ -16,7 +16,7 @@
 //             128-byte swizzle; one thread then issues the eight tcgen05.mma of the stage.  (Warp-level mma.sync was
 //             built first: 512^3 took 12 us instead of 17 with panels; its TF32 rate on this chip is below what the
 //             precision needs - three TF32 products run no faster than plain FMAs.)
-//   sums      three rotating accumulators for hi*hi and one for the cross terms, as in the 128 x 128 kernel
+//   sums      three rotating accumulators for hi*hi and one for the cross terms
 #include "common.cuh"
 #include "gemm_epilogue.cuh"
 #include "panel_math.cuh"

@@ -1,5 +1,5 @@
 // Inline-PTX wrappers for the Blackwell tensor-core path (tcgen05 / tensor memory / TMA / mbarrier / clusters) and the
-// shared-memory and instruction descriptors of tcgen05.mma, shared by the contraction kernels (gemm.cu) and the
+// shared-memory and instruction descriptors of tcgen05.mma, shared by the contraction kernels (half_gemm.cu, direct_gemm.cu) and the
 // persistent LSTM step kernels (lstm_persistent.cu).
 #pragma once
 
