@@ -405,13 +405,15 @@ __global__ void __launch_bounds__(DG_THREADS, 2) direct_gemm_kernel(const __grid
 // exchange before anything else: 128 x 256 x 256 takes it 6.8 us (here 5.4), of which the products are a tenth.  Here a CTA owns
 // 32 x 32 outputs, fetches both operands' rows for up to 256 of K at once (16 loads of 16 bytes per thread in flight: one trip
 // to L2), and its 8 warps walk interleaved groups of four K each with 4 x 8 sums per lane; the 8 partial tiles are added in warp
-// order in shared memory (bitwise repeatable).  Bound by latency, from about K = 512 on by shared-memory reads and FMA issue.
+// order in shared memory (bitwise repeatable).  Bound by latency, then by shared-memory reads and FMA issue (11 ns per K): a long K of
+// few tiles is cut over the CTAs of a cluster, whose tiles are added in rank order through distributed shared memory.
 // Operand rows contiguous in K lie as [row][FG_K + 4] (lanes read rows rg + 8 i: eight different 16-byte chunks), operands
 // read through their columns as [k][32].
 // ---------------------------------------------------------------------------------------------------------
 constexpr int FG_PITCH = FG_K + 4;
 constexpr int FG_OP_FLOATS = 32 * FG_PITCH;               // one operand
-constexpr int FG_RED_FLOATS = 8 * FG_M * (FG_N + 4) + 8 * FG_M;   // partial tiles, then the warps' row sums; over the operands
+constexpr int FG_TILE_FLOATS = FG_M * (FG_N + 4);
+constexpr int FG_RED_FLOATS = 9 * FG_TILE_FLOATS + 9 * FG_M;   // the warps' partial tiles and their sum, the warps' row sums and theirs; over the operands
 constexpr int FG_SMEM = (2 * FG_OP_FLOATS > FG_RED_FLOATS ? 2 * FG_OP_FLOATS : FG_RED_FLOATS) * 4;
 
 // rows row0 .. row0 + 31 (past `rows`: the last one again), K elements k0 .. k0 + kc - 1 (zeros up to a multiple of 4)
@@ -465,7 +467,7 @@ __device__ __forceinline__ void fg_fetch(float *s, const float *src, long long l
       if (c < kc) *reinterpret_cast<float4 *>(s + (r0 + 4 * i) * FG_PITCH + c) = v[i];
   } else {
     const int lane = tid & 31, r0 = tid >> 5;
-#pragma unroll 2
+#pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int row = min(row0 + r0 + 8 * i, rows - 1);
       const float *q = src + static_cast<long long>(row) * ld + k0;
@@ -479,11 +481,17 @@ __device__ __forceinline__ void fg_fetch(float *s, const float *src, long long l
   }
 }
 
-template <bool AT, bool BT, int MAX>
+// CUT: the CTAs of a cluster share a tile
+template <bool AT, bool BT, int MAX, bool CUT>
 __global__ void __launch_bounds__(DG_THREADS, 2) fma_gemm_kernel(const __grid_constant__ DirectGroup<MAX> g) {
   extern __shared__ float fg_smem[];
   float *sa = fg_smem, *sb = fg_smem + FG_OP_FLOATS;
-  const int tile = static_cast<int>(blockIdx.x);
+  uint32_t S = 1, rank = 0;
+  if constexpr (CUT) {
+    asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(S));
+    rank = ptx::cluster_ctarank();
+  }
+  const int tile = static_cast<int>(CUT ? blockIdx.x / S : blockIdx.x);
   int pi = 0;
 #pragma unroll 1
   while (pi + 1 < g.count && tile >= g.p[pi + 1].first_tile) ++pi;
@@ -498,10 +506,16 @@ __global__ void __launch_bounds__(DG_THREADS, 2) fma_gemm_kernel(const __grid_co
   float rs = 0.f;
   grid_dependency_wait();
   grid_dependency_release();
+  int k_begin = 0, k_end = p.K;
+  if constexpr (CUT) {
+    const int share = ((p.K + static_cast<int>(S) - 1) / static_cast<int>(S) + 3) & ~3;
+    k_begin = min(static_cast<int>(rank) * share, p.K);
+    k_end = min(k_begin + share, p.K);
+  }
 #pragma unroll 1
-  for (int k0 = 0; k0 < p.K; k0 += FG_K) {
-    const int kc = min(FG_K, p.K - k0);
-    if (k0 > 0) __syncthreads();
+  for (int k0 = k_begin; k0 < k_end; k0 += FG_K) {
+    const int kc = min(FG_K, k_end - k0);
+    if (k0 > k_begin) __syncthreads();
     fg_fetch<AT>(sa, p.a, p.lda, m0, p.M, k0, kc, p.a_vec != 0);
     fg_fetch<BT>(sb, p.b, p.ldb, n0, p.N, k0, kc, p.b_vec != 0);
     __syncthreads();
@@ -535,23 +549,54 @@ __global__ void __launch_bounds__(DG_THREADS, 2) fma_gemm_kernel(const __grid_co
     }
   }
   __syncthreads();   // the operands have been read: the partial tiles take their place
-  float *part = fg_smem + warp * FG_M * (FG_N + 4);
+  float *part = fg_smem + warp * FG_TILE_FLOATS;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     float *d = part + (AT ? rg * 4 + i : rg + 8 * i) * (FG_N + 4);
 #pragma unroll
     for (int j = 0; j < 8; ++j) d[BT ? cg * 8 + j : cg + 4 * j] = acc[i][j];
   }
-  float *sums = fg_smem + 8 * FG_M * (FG_N + 4);
+  float *sums = fg_smem + 9 * FG_TILE_FLOATS;
   if (want_sum) sums[tid] = rs;
   __syncthreads();
-  if (p.c_vec) dg_finish<FG_N, 8, 4, 1>(p, fg_smem, 1, 0, FG_M, m0, n0);
-  else dg_finish<FG_N, 8, 1, 4>(p, fg_smem, 1, 0, FG_M, m0, n0);
-  if (want_sum && tid < FG_M && m0 + tid < p.M) {
-    float v = 0.f;
+  if constexpr (!CUT) {
+    if (p.c_vec) dg_finish<FG_N, 8, 4, 1>(p, fg_smem, 1, 0, FG_M, m0, n0);
+    else dg_finish<FG_N, 8, 1, 4>(p, fg_smem, 1, 0, FG_M, m0, n0);
+    if (want_sum && tid < FG_M && m0 + tid < p.M) {
+      float v = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) v += sums[w * 32 + tid];
-    p.row_sum[m0 + tid] += v;
+      for (int w = 0; w < 8; ++w) v += sums[w * 32 + tid];
+      p.row_sum[m0 + tid] += v;
+    }
+  } else {
+    float *tot = fg_smem + 8 * FG_TILE_FLOATS;
+    {
+      const int at = (tid >> 3) * (FG_N + 4) + (tid & 7) * 4;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int w = 0; w < 8; ++w) add4(v, *reinterpret_cast<const float4 *>(fg_smem + w * FG_TILE_FLOATS + at));
+      *reinterpret_cast<float4 *>(tot + at) = v;
+    }
+    if (want_sum && tid < FG_M) {
+      float v = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) v += sums[w * 32 + tid];
+      sums[8 * FG_M + tid] = v;
+    }
+    ptx::cluster_sync_all();
+    const int my_rows = FG_M / static_cast<int>(S), first = static_cast<int>(rank) * my_rows;
+    if (p.c_vec) dg_finish<FG_N, 1, 4, 1>(p, tot, S, first, my_rows, m0, n0);
+    else dg_finish<FG_N, 1, 1, 4>(p, tot, S, first, my_rows, m0, n0);
+    if (want_sum && tid < my_rows && m0 + first + tid < p.M) {
+      float v = 0.f;
+      for (uint32_t q = 0; q < S; ++q) {
+        float x;
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(ptx::map_to_cta(ptx::smem_u32(sums + 8 * FG_M + first + tid), q)) : "memory");
+        v += x;
+      }
+      p.row_sum[m0 + first + tid] += v;
+    }
+    ptx::cluster_sync_all();   // a peer may still be reading this CTA's tile
   }
 }
 
@@ -600,26 +645,46 @@ static bool epilogue_is_vector(const Epilogue &e, long long N) {
   return (bits & 15) == 0 && ((N | e.ldc | e.ld_addend | e.ld_aux | e.seg_off[0] | e.seg_off[1] | e.seg_off[2] | e.seg_off[3]) & 3) == 0;
 }
 
-template <bool AT, bool BT, int MAX>
-static int launch_fma(Context &ctx, const DirectGroup<MAX> &g, int tiles) {
-  auto kernel = fma_gemm_kernel<AT, BT, MAX>;
+template <bool AT, bool BT, int MAX, bool CUT>
+static int launch_fma_cut(Context &ctx, const DirectGroup<MAX> &g, int tiles, int cluster) {
+  auto kernel = fma_gemm_kernel<AT, BT, MAX, CUT>;
   static std::once_flag flags[64];
   static bool ok[64] = {};
   if (ctx.device < 0 || ctx.device >= 64) return MYEA_E_CUDA;
   std::call_once(flags[ctx.device], [&] { ok[ctx.device] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FG_SMEM) == cudaSuccess; });
   if (!ok[ctx.device]) return MYEA_E_CUDA;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(tiles * cluster));
+  cfg.blockDim = dim3(DG_THREADS);
+  cfg.dynamicSmemBytes = FG_SMEM;
+  cfg.stream = ctx.stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = (ctx.dependent_launch && !ctx.profiling) ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CUT ? 2 : 1;
   ctx.begin(TC_GEMM);
-  const cudaError_t err = launch_dependent(ctx, kernel, dim3(static_cast<unsigned>(tiles)), dim3(DG_THREADS), FG_SMEM, g);
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, g);
   ctx.end(TC_GEMM);
   return err == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
 
-// One tile per SM at most: two of these CTAs take all registers of an SM, so that the next launch cannot set itself up beside
-// them (a 256 x 1024 x 10 product alone took 3.4 us instead of 4.6, and the training step around it 5 us more).  Then the walk over
-// K decides: about 2.6 us and 11 ns per K, where the tensor-core tile takes 5.2 us at K = 64, 6.8 at 256 and 8.5 at 512, and 3 us
-// more where its operands' rows are not 16-byte aligned.  Measured (us, FMAs / tensor cores): 128 x 256 x 64 3.5 / 5.3,
-// 128 x 256 x 256 5.4 / 6.8, 256 x 512 x 256 5.6 / 6.9, 384^3 8.0 / 7.8; unaligned 203 x 333 x 75 4.1 / 9.7, 203 x 333 x 333 8.2 / 9.7.
-static bool fma_suits(const DirectItem *items, int n) {
+template <bool AT, bool BT, int MAX>
+static int launch_fma(Context &ctx, const DirectGroup<MAX> &g, int tiles, int cluster) {
+  return cluster > 1 ? launch_fma_cut<AT, BT, MAX, true>(ctx, g, tiles, cluster) : launch_fma_cut<AT, BT, MAX, false>(ctx, g, tiles, 1);
+}
+
+// How many CTAs share the K range of a 32 x 32 tile, 0: tensor-core tiles instead.  One CTA per SM at most: two of them take all
+// registers of an SM, so that the next launch cannot set itself up beside them (a 256 x 1024 x 10 product alone took 3.4 us instead
+// of 4.6, and the training step around it 5 us more).  Estimates (us) from these measurements of FMAs with 1 / 2 / 4 / 8 CTAs and of
+// tensor-core tiles: 128 x 256 x 64 3.4 / 4.6 / 4.8 / 5.7, 5.5; 128 x 256 x 256 5.2 / 5.5 / 5.4 / 6.0, 6.8; 64 x 512 x 512 8.4 / 6.7 / 6.2 /
+// 6.4, 8.0; 256 x 10 x 1024 15.2 / 10.2 / 7.3 / 6.5, 11.5; 32 x 64 x 4096 54 / 30 / 17 / 10, 17; 384^3 8.0, 7.8; rows that are not
+// 16-byte aligned: 203 x 333 x 75 4.1, 9.8.
+static int fma_cluster(const DirectItem *items, int n) {
   long long tiles = 0, longest = 0;
   bool aligned = true;
   for (int i = 0; i < n; ++i) {
@@ -628,7 +693,14 @@ static bool fma_suits(const DirectItem *items, int n) {
     for (const Operand *o : {&items[i].A, &items[i].B})
       aligned = aligned && (reinterpret_cast<uintptr_t>(o->ptr) & 15) == 0 && ((o->stride_k != 1 ? o->stride_k : o->stride_r) & 3) == 0;
   }
-  return tiles <= 148 && longest <= (aligned ? 280 : 360);
+  const double K = static_cast<double>(longest);
+  double best = 5.0 + 0.006 * std::min(K, 1024.0) + 0.002 * std::max(0.0, K - 1024.0) + (aligned ? 0.0 : 2.0) - 0.5;
+  int cluster = 0;
+  for (int S = 1; S <= 8 && tiles * S <= 148; S *= 2) {
+    const double t = 2.6 + 0.011 * K / S + (S > 1 ? 2.2 : 0.0) + (S == 8 ? 0.5 : 0.0);
+    if (t < best) { best = t; cluster = S; }
+  }
+  return cluster;
 }
 
 template <int MAX>
@@ -637,7 +709,7 @@ static int direct_gemm_launch(Context &ctx, const DirectItem *items, int n) {
   g.count = n;
   int tiles = 0, min_steps = 1 << 30;
   const bool at = items[0].A.stride_k != 1, bt = items[0].B.stride_k != 1;
-  const bool fma = fma_suits(items, n);
+  const int fma = fma_cluster(items, n);
   const int tile_m = fma ? FG_M : DG_M, tile_n = fma ? FG_N : DG_N;
   for (int i = 0; i < n; ++i) {
     const DirectItem &it = items[i];
@@ -660,8 +732,8 @@ static int direct_gemm_launch(Context &ctx, const DirectItem *items, int n) {
     ctx.gemm_flops += 2.0 * p.M * p.N * static_cast<double>(p.K);
   }
   if (fma) {
-    if (at) return bt ? launch_fma<true, true>(ctx, g, tiles) : launch_fma<true, false>(ctx, g, tiles);
-    return bt ? launch_fma<false, true>(ctx, g, tiles) : launch_fma<false, false>(ctx, g, tiles);
+    if (at) return bt ? launch_fma<true, true>(ctx, g, tiles, fma) : launch_fma<true, false>(ctx, g, tiles, fma);
+    return bt ? launch_fma<false, true>(ctx, g, tiles, fma) : launch_fma<false, false>(ctx, g, tiles, fma);
   }
   // K is cut in up to four while the grid stays within one CTA per SM and every CTA keeps two stages.  Measured (us per
   // launch, cut 1 / 2 / 4 / 8): 128 x 256 x 256 9.6 / 8.0 / 6.6 / 7.2, 203 x 333 x 333 18.6 / 13.6 / 9.8 / 11.3, 512^3 15.7 / 11.2

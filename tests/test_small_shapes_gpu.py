@@ -128,3 +128,20 @@ def test_contraction_with_fmas(M, N, K, columns):
     a, b = np.ascontiguousarray(A.T if columns & (1 << 17) else A), np.ascontiguousarray(B.T if columns & (1 << 18) else B)
     assert lib.myea_b200_gemm_nt(0, columns, M, N, K, a.ctypes.data, b.ctypes.data, out.ctypes.data, 1, None, 0) == 0
     assert rel_err(out, want) < 5e-6
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 10, 1024), (33, 7, 1025), (1, 1, 600), (40, 31, 4099), (1, 1000, 1000), (64, 512, 512), (65, 129, 515)])
+def test_contraction_with_fmas_over_a_cluster(M, N, K):
+    """few tiles and a long K: cut over 2, 4 and 8 CTAs, the last share shorter or empty"""
+    lib = capi.load()
+    rng = np.random.default_rng(M + N + K)
+    A, B = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
+    out = rng.standard_normal((M, N), dtype=np.float32)
+    want = A.astype(np.float64) @ B.astype(np.float64).T + out
+    assert lib.myea_b200_gemm_nt(0, 0, M, N, K, A.ctypes.data, B.ctypes.data, out.ctypes.data, 1, None, 0) == 0
+    assert rel_err(out, want) < 5e-6
+
+
+@pytest.mark.parametrize("widths,B", [((20, 30, 10), 640), ((5, 33, 40, 3), 1027)])   # weight derivatives with a long K: bias sums over a cluster
+def test_derivatives_over_long_batches(widths, B):
+    _step(_mlp(widths, B, capi.AF_TANH))
