@@ -332,9 +332,9 @@ int softmax_forward(Context &ctx, const float *z, float *out, long long rows, lo
 int norm_backward(Context &ctx, const float *z, const float *delta_af, float *delta_out, long long rows, long long H,
                   const NormParams &np, const SumHook *hook = nullptr, int fused_chunks = 0, const HalfPanels *sink = nullptr);
 // delta = f'(pre,y) * (y - desired); loss / accuracy accumulators (double[2] + uint64) on the device
-int output_error(Context &ctx, const float *pre, const float *y, const float *desired, float *delta, long long rows,
-                 long long H, uint32_t af, uint32_t loss, uint32_t accuracy, float accuracy_variance, double *d_acc,
-                 unsigned long long *d_count);
+// softmax: y has not been made yet (the epoch loop, which runs the two one after the other, leaves it to this kernel)
+int output_error(Context &ctx, const float *pre, float *y, const float *desired, float *delta, long long rows, long long H, uint32_t af, uint32_t loss,
+                 uint32_t accuracy, float accuracy_variance, double *d_acc, unsigned long long *d_count, bool softmax = false);
 // out[j] (+)= sum_rows in[r][j]
 int column_sum(Context &ctx, const float *in, long long rows, long long H, float *out, int accumulate, float *partial,
                int chunks);

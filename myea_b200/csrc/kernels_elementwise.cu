@@ -539,12 +539,8 @@ __device__ __forceinline__ float block_reduce_sum(float v, float *sh) {
   return r;
 }
 
-__global__ void __launch_bounds__(128) softmax_forward_kernel(const float *__restrict__ z, float *__restrict__ out, long long H) {
-  __shared__ float sh[4];
-  grid_dependency_wait();
-  grid_dependency_release();
-  const float *zr = z + blockIdx.x * H;
-  float *orow = out + blockIdx.x * H;
+// one row by the 128 threads of a block
+__device__ __forceinline__ void softmax_row(const float *zr, float *orow, long long H, float *sh) {
   float mx = -3.402823466e+38f;
   for (long long j = threadIdx.x; j < H; j += blockDim.x) mx = fmaxf(mx, zr[j]);
   mx = block_reduce_max(mx, sh);
@@ -557,6 +553,12 @@ __global__ void __launch_bounds__(128) softmax_forward_kernel(const float *__res
   s = block_reduce_sum(s, sh);
   const float inv = 1.0f / s;
   for (long long j = threadIdx.x; j < H; j += blockDim.x) orow[j] *= inv;
+}
+__global__ void __launch_bounds__(128) softmax_forward_kernel(const float *__restrict__ z, float *__restrict__ out, long long H) {
+  __shared__ float sh[4];
+  grid_dependency_wait();
+  grid_dependency_release();
+  softmax_row(z + blockIdx.x * H, out + blockIdx.x * H, H, sh);
 }
 
 // (z or y null: the derivative does not read it)
@@ -781,7 +783,9 @@ int norm_backward(Context &ctx, const float *z, const float *delta_af, float *de
 // loss type only selects what is added to the loss accumulator.  One block per row.
 // d_acc[0] += loss terms, d_acc[1] += accuracy hits, d_count[0] += number of loss terms.
 // ---------------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) output_error_kernel(const float *__restrict__ pre, const float *__restrict__ y,
+// SOFTMAX: y is made here first, from the summations, as softmax_forward_kernel makes it (a thread reads back what it wrote)
+template <bool SOFTMAX>
+__global__ void __launch_bounds__(128) output_error_kernel(const float *__restrict__ pre, float *y,
                                                            const float *__restrict__ desired, float *__restrict__ delta, long long H,
                                                            uint32_t af, uint32_t loss, uint32_t accuracy, float accuracy_variance,
                                                            double *d_acc, unsigned long long *d_count) {
@@ -790,6 +794,7 @@ __global__ void __launch_bounds__(128) output_error_kernel(const float *__restri
   __shared__ float shv[4];
   grid_dependency_wait();
   grid_dependency_release();
+  if constexpr (SOFTMAX) softmax_row(pre + blockIdx.x * H, y + blockIdx.x * H, H, sh);
   const long long base = blockIdx.x * H;
   float loss_sum = 0.f, hits = 0.f;
   // arg max of the prediction (the LAST maximum wins: the reference compares with >=) and first desired == 1
@@ -842,11 +847,11 @@ __global__ void __launch_bounds__(128) output_error_kernel(const float *__restri
   }
 }
 
-int output_error(Context &ctx, const float *pre, const float *y, const float *desired, float *delta, long long rows, long long H,
-                 uint32_t af, uint32_t loss, uint32_t accuracy, float accuracy_variance, double *d_acc, unsigned long long *d_count) {
+int output_error(Context &ctx, const float *pre, float *y, const float *desired, float *delta, long long rows, long long H, uint32_t af, uint32_t loss,
+                 uint32_t accuracy, float accuracy_variance, double *d_acc, unsigned long long *d_count, bool softmax) {
   ctx.begin(TC_ELEMENTWISE);
-  launch_dependent(ctx, output_error_kernel, dim3(static_cast<unsigned>(rows)), dim3(128), 0, pre, y, desired, delta, H, af, loss, accuracy, accuracy_variance,
-                   d_acc, d_count);
+  launch_dependent(ctx, softmax ? output_error_kernel<true> : output_error_kernel<false>, dim3(static_cast<unsigned>(rows)), dim3(128), 0, pre, y, desired, delta, H, af,
+                   loss, accuracy, accuracy_variance, d_acc, d_count);
   ctx.end(TC_ELEMENTWISE);
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }

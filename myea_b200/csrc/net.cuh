@@ -105,6 +105,8 @@ struct myea_b200_net {
   bool full_pitch = false; // recurrent (T > 1 or an LSTM layer): buffers keep the allocated B as the row pitch of a time step
   long long pitch() const { return full_pitch ? B : active_B; }  // rows per time step the kernels of the step in flight run over
   bool any_norm = false;
+  bool defer_softmax = false, softmax_pending = false;  // epoch loop: the output layer's softmax is left to the error kernel
+  bool desired_unmarked = false;  // the targets' buffer was last read by a kernel that no event stands behind
   // flat buffers, [P] (norm averages: [total_norm_units])
   float *params = nullptr, *grads = nullptr, *m1 = nullptr, *m2 = nullptr, *m2hat = nullptr, *prev_delta = nullptr,
         *mask_reg = nullptr;
