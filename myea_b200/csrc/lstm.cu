@@ -259,6 +259,9 @@ int lstm_create(myea_b200_net *net, LayerPlan &L) {
   P->zoneout = L.desc.type_dropout == MYEA_DROPOUT_ZONEOUT;
   if (cpb != 1) return lstm_blocks_create(net, L, P);
   const long long rows = net->T * net->B, C = P->C;
+  const bool tensor = net->ctx.gemm_engine == 0;
+  const bool in_panels = tensor && !direct_gemm_suits(net->ctx, rows, 4 * C, L.n_in);
+  const bool dw_panels = tensor && !direct_gemm_suits(net->ctx, 4 * C, std::max(L.n_in, C), rows);
   // biases: the reference stores first_bias_connection_index already shifted by the number of cells and then reads
   // [bz | bi | bf | bo] from it, so bo overlaps the next layer's bias slots.  Reproduced for the unidirectional layer;
   // the bidirectional layer (no usable reference) uses its true, unshifted block, one [bz|bi|bf|bo] run per direction.
@@ -271,7 +274,10 @@ int lstm_create(myea_b200_net *net, LayerPlan &L) {
       net->ctx.error = "LSTM output-gate bias would run past the parameter buffer (the next layer must be at least as wide as the LSTM layer)";
       return MYEA_E_INVALID;
     }
-    LRC(lalloc(net, &D.gates_in, rows * 4 * C));
+    // the input projections are dead after the forward walk, the gate errors' panels are made after the backward walk: one
+    // buffer for both (of 268 MB at 1024 cells, 64 steps and 256 rows; mapping and clearing memory is most of what a handle costs)
+    LRC(lalloc(net, &D.gates_in, in_panels || dw_panels ? std::max(static_cast<size_t>(rows * 4 * C), half_panel_floats(rows, 4 * C)) : static_cast<size_t>(rows * 4 * C)));
+    if (in_panels || dw_panels) P->dg_all_mem[d] = D.gates_in;
     LRC(lalloc(net, &D.act, rows * 4 * C));
     LRC(lalloc(net, &D.cstate, rows * C));
     LRC(lalloc(net, &D.cact, rows * C));
@@ -292,7 +298,6 @@ int lstm_create(myea_b200_net *net, LayerPlan &L) {
   size_t need = static_cast<size_t>(P->dirs) * 4 * C * std::max<long long>(L.n_in, C);  // gathered weights
   LRC(lstm_persistent_plan(net, L));
   LRC(lstm_resident_plan(net, L));
-  const bool tensor = net->ctx.gemm_engine == 0;
   if (tensor && P->resident == nullptr && lstm_persistent_ready(P)) {
     LRC(lalloc(net, &P->peep_compact, static_cast<size_t>(P->dirs) * 3 * C));
     const long long a_rows = (net->B + 127) / 128 * 128;
@@ -318,12 +323,9 @@ int lstm_create(myea_b200_net *net, LayerPlan &L) {
       for (int d = 0; d < P->dirs; ++d) LRC(lalloc(net, &P->w_rec_mem[d], static_cast<size_t>(4 * C * C)));
     }
   }
-  const bool in_panels = tensor && !direct_gemm_suits(net->ctx, rows, 4 * C, L.n_in);
-  const bool dw_panels = tensor && !direct_gemm_suits(net->ctx, 4 * C, std::max(L.n_in, C), rows);
   if (in_panels || dw_panels) LRC(lalloc(net, &P->x_mem, half_panel_floats(rows, L.n_in)));
   for (int d = 0; d < P->dirs; ++d) {
     if (in_panels) LRC(lalloc(net, &P->w_in_mem[d], half_panel_floats(4 * C, L.n_in)));
-    if (in_panels || dw_panels) LRC(lalloc(net, &P->dg_all_mem[d], half_panel_floats(rows, 4 * C)));
     if (dw_panels) LRC(lalloc(net, &P->h_shift_mem[d], half_panel_floats(rows, C)));
   }
   net->scratch.floats = std::max(net->scratch.floats, need + 256);
