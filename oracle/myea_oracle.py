@@ -261,6 +261,7 @@ class OracleNet:
     def __init__(self, desc, opt, threads=1, dtype=np.float32):
         self.desc, self.opt, self.dt = desc, opt, dtype
         self.T, self.B = int(desc.number_recurrent_depth), int(desc.batch_size)
+        self.active_B = self.B   # samples of the batch in flight
         self.layers, self.P, self.W, self.n_bias, self.n_norm = build_index_map(desc)
         z = lambda k: np.zeros(k, dtype)
         self.buf = {capi.BUF_PARAMETERS: z(self.P), capi.BUF_DERIVATIVES: z(self.P), capi.BUF_FIRST_MOMENT: z(self.P),
@@ -316,12 +317,12 @@ class OracleNet:
         return float(self.loss_sum), int(self.n_loss), float(self.acc_sum)
 
     def outputs(self, l):
-        return np.asarray(self.layers[l].values, np.float32).reshape(self.T, self.B, -1)
+        return np.asarray(self.layers[l].values, np.float32).reshape(self.T, self.active_B, -1)
 
     def errors(self, l):
         L = self.layers[l]
         e = L.dh if L.type == capi.LAYER_LSTM else L.errors
-        return np.asarray(e, np.float32).reshape(self.T, self.B, -1)
+        return np.asarray(e, np.float32).reshape(self.T, self.active_B, -1)
 
     def _p(self):
         return self.buf[capi.BUF_PARAMETERS]
@@ -558,7 +559,7 @@ class OracleNet:
 
     def forward(self, X, training=True, batch=None):
         self.training = training
-        self.active_B = int(batch or self.B)   # Forward_Pass(batch_size_received, ...): any batch up to the allocated one (T = 1)
+        self.active_B = int(batch or self.B)   # Forward_Pass(batch_size_received, ...): any batch up to the allocated one
         X = np.asarray(X, self.dt).reshape(self.T * self.active_B, -1)
         self.layers[0].values = X
         n = len(self.layers)
@@ -594,9 +595,9 @@ class OracleNet:
             L = self.layers[len(self.layers) - k]
             if k > 1:
                 Y = self.layers[k - 1].values
-        Y = np.asarray(Y, dt).reshape(self.T * getattr(self, "active_B", self.B), -1)
+        Y = np.asarray(Y, dt).reshape(self.T * self.active_B, -1)
         t0 = min(int(self.desc.number_time_delays), self.T) if self.T > 1 else 0
-        skip = t0 * getattr(self, "active_B", self.B)
+        skip = t0 * self.active_B
         y, t, pre = L.values[skip:], Y[skip:], L.pre[skip:]
         diff = y - t
         af = int(L.d.type_activation_function)

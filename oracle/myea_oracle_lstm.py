@@ -79,7 +79,7 @@ class _Views:
 def forward(net, l, x):
     L = net.layers[l]
     dt = net.dt
-    T, B = net.T, net.B
+    T, B = net.T, net.active_B
     dirs = 2 if L.d.use_bidirectional else 1
     x = x.reshape(T, B, -1)
     L.st, L.views = [], []
@@ -132,7 +132,7 @@ def backward(net, l):
     The zoneout masks are ignored, as in the reference."""
     L = net.layers[l]
     dt = net.dt
-    T, B = net.T, net.B
+    T, B = net.T, net.active_B
     dirs = 2 if L.d.use_bidirectional else 1
     dh_all = np.array(L.dh, dt).reshape(T, B, -1)
     L.dg = []
@@ -174,7 +174,7 @@ def backward(net, l):
 def error_to_input(net, l):
     """error arriving on the outputs of the layer feeding LSTM layer l: sum over gates and directions of dg W_in"""
     L = net.layers[l]
-    T, B = net.T, net.B
+    T, B = net.T, net.active_B
     dirs = 2 if L.d.use_bidirectional else 1
     p = net._p()
     out = 0
@@ -189,7 +189,7 @@ def error_to_input(net, l):
 def update_derivative_weight(net, l):
     L = net.layers[l]
     dt = net.dt
-    T, B = net.T, net.B
+    T, B = net.T, net.active_B
     dirs = 2 if L.d.use_bidirectional else 1
     x = L.x.reshape(T * B, -1)
     G = net._g()

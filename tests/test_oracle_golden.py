@@ -7,6 +7,7 @@ import pytest
 
 import cases
 from conftest import rel_err
+from myea_b200 import capi
 from oracle import myea_oracle, ref
 
 TOL = 5e-5   # float32 summation-order noise between numpy and the reference's scalar loops (the adaptive optimizers amplify it)
@@ -91,3 +92,21 @@ def test_reference_openmp_equals_loop():
     a.close(); b.close()
     assert rel_err(ob["grad0"], oa["grad0"]) < 1e-5
     assert rel_err(ob["param1"], oa["param1"]) < 1e-5
+
+
+@pytest.mark.parametrize("name", ["mlp_relu_gd", "lstm1_all_steps_adam", "lstm2_zoneout_clip", "recurrent_fc_batch_renorm", "lstm_two_cells_per_block"])
+def test_short_batch_is_the_step_of_a_smaller_network(name):
+    """a batch below the allocated one: the same step as on a network whose batch size it is"""
+    wl = cases.CASES[name]()
+    small = cases.CASES[name]()
+    b = wl.B - wl.B // 3
+    small.desc.batch_size = b
+    X, Y = wl.batch()
+    out = []
+    for w, kw in ((wl, {"batch": b}), (small, {})):
+        net = myea_oracle.OracleNet(w.desc, w.opt)
+        w.materialize(net)
+        net.reset_loss()
+        net.forward(X[:, :b], **kw); net.compute_error(Y[:, :b]); net.backward(); net.update_derivative_weight()
+        out.append((net.buf[capi.BUF_DERIVATIVES], net.outputs(len(w.layers) - 1), net.loss()))
+    assert b < wl.B and np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1]) and out[0][2] == out[1][2]
