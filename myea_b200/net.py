@@ -111,8 +111,17 @@ class Net:
         self._ck(self.lib.myea_b200_set_pre_training_level(self.h, int(level)), "set_pre_training_level")
 
     def set_shakedrop(self, layer, mask, alpha, beta):
+        """mask[B]; alpha, beta [B, units of the layer], or [B, units of the block] where the block is narrower than its shortcut"""
         m = np.ascontiguousarray(mask, dtype=np.uint8).ravel()
-        a, b = _f32(alpha), _f32(beta)
+        units = int(self.layer_index(layer).number_outputs)
+
+        def rows(a):
+            a = _f32(a).reshape(m.size, -1)
+            if a.shape[1] > units:
+                raise ValueError("ShakeDrop coefficients of %d columns for a layer of %d units" % (a.shape[1], units))
+            return np.ascontiguousarray(np.pad(a, ((0, 0), (0, units - a.shape[1]))))   # (the library reads [B, units])
+
+        a, b = rows(alpha), rows(beta)
         self._ck(self.lib.myea_b200_set_shakedrop(self.h, layer, m.ctypes.data, a.ctypes.data, b.ctypes.data, m.size), "set_shakedrop")
 
     def dataset_set(self, X, Y):
