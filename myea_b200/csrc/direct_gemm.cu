@@ -678,20 +678,22 @@ static int launch_fma(Context &ctx, const DirectGroup<MAX> &g, int tiles, int cl
   return cluster > 1 ? launch_fma_cut<AT, BT, MAX, true>(ctx, g, tiles, cluster) : launch_fma_cut<AT, BT, MAX, false>(ctx, g, tiles, 1);
 }
 
+static long long operand_pitch(const Operand &o, bool columns) { return columns ? o.stride_k : o.stride_r; }
+
 // How many CTAs share the K range of a 32 x 32 tile, 0: tensor-core tiles instead.  One CTA per SM at most: two of them take all
 // registers of an SM, so that the next launch cannot set itself up beside them (a 256 x 1024 x 10 product alone took 3.4 us instead
 // of 4.6, and the training step around it 5 us more).  Estimates (us) from these measurements of FMAs with 1 / 2 / 4 / 8 CTAs and of
 // tensor-core tiles: 128 x 256 x 64 3.4 / 4.6 / 4.8 / 5.7, 5.5; 128 x 256 x 256 5.2 / 5.5 / 5.4 / 6.0, 6.8; 64 x 512 x 512 8.4 / 6.7 / 6.2 /
 // 6.4, 8.0; 256 x 10 x 1024 15.2 / 10.2 / 7.3 / 6.5, 11.5; 32 x 64 x 4096 54 / 30 / 17 / 10, 17; 384^3 8.0, 7.8; rows that are not
 // 16-byte aligned: 203 x 333 x 75 4.1, 9.8.
-static int fma_cluster(const DirectItem *items, int n) {
+static int fma_cluster(const DirectItem *items, int n, bool at, bool bt) {
   long long tiles = 0, longest = 0;
   bool aligned = true;
   for (int i = 0; i < n; ++i) {
     tiles += (items[i].A.rows + FG_M - 1) / FG_M * ((items[i].B.rows + FG_N - 1) / FG_N);
     longest = std::max(longest, items[i].A.k);
-    for (const Operand *o : {&items[i].A, &items[i].B})
-      aligned = aligned && (reinterpret_cast<uintptr_t>(o->ptr) & 15) == 0 && ((o->stride_k != 1 ? o->stride_k : o->stride_r) & 3) == 0;
+    aligned = aligned && ((reinterpret_cast<uintptr_t>(items[i].A.ptr) | reinterpret_cast<uintptr_t>(items[i].B.ptr)) & 15) == 0 &&
+              ((operand_pitch(items[i].A, at) | operand_pitch(items[i].B, bt)) & 3) == 0;
   }
   const double K = static_cast<double>(longest);
   double best = 5.0 + 0.006 * std::min(K, 1024.0) + 0.002 * std::max(0.0, K - 1024.0) + (aligned ? 0.0 : 2.0) - 0.5;
@@ -703,21 +705,40 @@ static int fma_cluster(const DirectItem *items, int n) {
   return cluster;
 }
 
+// How the operands of a launch are read: through their columns (rows contiguous, pitch stride_k) or their rows (K contiguous,
+// pitch stride_r).  All items share the choice, and an operand of a single row or a single K can be read either way whatever
+// its strides say: the errors of a layer of one unit are a column of pitch 1, which beside wider layers is read as theirs are.
+static bool reads_columns(const Operand &o) { return o.stride_r == 1 || o.rows == 1; }
+static bool reads_rows(const Operand &o) { return o.stride_k == 1 || o.k == 1; }
+static bool choose_reading(const DirectItem *items, int n, Operand DirectItem::*which, bool columns, bool *out) {
+  bool all_columns = true, all_rows = true;
+  for (int i = 0; i < n; ++i) {
+    const Operand &o = items[i].*which;
+    columns = columns || o.stride_k != 1;
+    all_columns = all_columns && reads_columns(o);
+    all_rows = all_rows && reads_rows(o);
+  }
+  *out = columns && all_columns;
+  return *out || all_rows;
+}
+
 template <int MAX>
 static int direct_gemm_launch(Context &ctx, const DirectItem *items, int n) {
   DirectGroup<MAX> g;
   g.count = n;
   int tiles = 0, min_steps = 1 << 30;
-  const bool at = items[0].A.stride_k != 1, bt = items[0].B.stride_k != 1;
-  const int fma = fma_cluster(items, n);
+  bool at, bt, sums = false;
+  for (int i = 0; i < n; ++i) sums = sums || items[i].row_sum != nullptr;   // these are taken from operands read through their columns
+  if (!choose_reading(items, n, &DirectItem::A, sums, &at) || !choose_reading(items, n, &DirectItem::B, false, &bt)) return MYEA_E_INVALID;
+  const int fma = fma_cluster(items, n, at, bt);
   const int tile_m = fma ? FG_M : DG_M, tile_n = fma ? FG_N : DG_N;
   for (int i = 0; i < n; ++i) {
     const DirectItem &it = items[i];
     DirectProblem &p = g.p[i];
-    if (it.A.k != it.B.k || it.A.rows <= 0 || it.B.rows <= 0 || it.A.k <= 0 || (it.A.stride_k != 1) != at || (it.B.stride_k != 1) != bt) return MYEA_E_INVALID;
+    if (it.A.k != it.B.k || it.A.rows <= 0 || it.B.rows <= 0 || it.A.k <= 0) return MYEA_E_INVALID;
     p.a = it.A.ptr; p.b = it.B.ptr;
-    p.lda = at ? it.A.stride_k : it.A.stride_r;
-    p.ldb = bt ? it.B.stride_k : it.B.stride_r;
+    p.lda = operand_pitch(it.A, at);
+    p.ldb = operand_pitch(it.B, bt);
     p.M = static_cast<int>(it.A.rows); p.N = static_cast<int>(it.B.rows); p.K = static_cast<int>(it.A.k);
     p.a_vec = (reinterpret_cast<uintptr_t>(p.a) & 15) == 0 && (p.lda & 3) == 0;
     p.b_vec = (reinterpret_cast<uintptr_t>(p.b) & 15) == 0 && (p.ldb & 3) == 0;
@@ -745,7 +766,7 @@ static int direct_gemm_launch(Context &ctx, const DirectItem *items, int n) {
   return bt ? launch_direct<false, true>(ctx, g, tiles, cluster) : launch_direct<false, false>(ctx, g, tiles, cluster);
 }
 
-// Items of one call share the orientation of A and of B.
+// Items of one call are read alike: all A through their rows or all through their columns, and all B.
 int direct_gemm(Context &ctx, const DirectItem *items, int count) {
   for (int first = 0; first < count; first += DG_MAX_ITEMS) {
     const int n = std::min(DG_MAX_ITEMS, count - first);

@@ -145,3 +145,18 @@ def test_contraction_with_fmas_over_a_cluster(M, N, K):
 @pytest.mark.parametrize("widths,B", [((20, 30, 10), 640), ((5, 33, 40, 3), 1027)])   # weight derivatives with a long K: bias sums over a cluster
 def test_derivatives_over_long_batches(widths, B):
     _step(_mlp(widths, B, capi.AF_TANH))
+
+
+@pytest.mark.parametrize("widths", [(1, 1), (5, 7, 1), (1, 6, 4), (3, 1, 2), (9, 1, 1, 1, 5), (1, 40, 70, 1)])   # layers of one unit beside wider ones, one input
+@pytest.mark.parametrize("B,norm", [(1, capi.NORM_NONE), (65, capi.NORM_NONE), (65, capi.NORM_BN)])
+def test_layers_of_one_unit(widths, B, norm):
+    _step(_mlp(widths, B, capi.AF_TANH, norm))
+
+
+@pytest.mark.parametrize("n_in,H,out", [(1, 8, 8), (1, 37, 40), (4, 1, 1), (4, 1, 6), (1, 1, 1)])   # univariate series, layers of one cell
+@pytest.mark.parametrize("T,B", [(1, 4), (5, 1), (4, 9)])
+@pytest.mark.parametrize("bidirectional", [False, True])
+def test_lstm_of_one_input_or_one_cell(n_in, H, out, T, B, bidirectional):
+    layers = [capi.fc(n_in), capi.lstm(H, bidirectional=bidirectional), capi.fc(out, capi.AF_LINEAR)]
+    _step(workloads.Workload("narrow lstm", capi.net(layers, B, T=T, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE),
+                             capi.opt(capi.OPT_GD, gd_lr=0.01 / B, momentum=0.9), n_in, out, False, layers))
