@@ -111,8 +111,10 @@ template <typename F>
 __global__ void __launch_bounds__(HP_THREADS, 2) half_produce_kernel(const F f, const HalfPanels p) {
   grid_dependency_wait();
   grid_dependency_release();
-  const long long c = blockIdx.x * static_cast<long long>(HP_BLOCK) + (threadIdx.x & 15) * 8;
-  const long long r0 = blockIdx.y * static_cast<long long>(HP_BLOCK) + (threadIdx.x >> 4);
+  // (one dimension: the row blocks of a tensor of many million rows are more than the others hold)
+  const unsigned across = static_cast<unsigned>((p.C + HP_BLOCK - 1) / HP_BLOCK), by = blockIdx.x / across, bx = blockIdx.x - by * across;
+  const long long c = bx * static_cast<long long>(HP_BLOCK) + (threadIdx.x & 15) * 8;
+  const long long r0 = by * static_cast<long long>(HP_BLOCK) + (threadIdx.x >> 4);
   const int n = static_cast<int>(max(0ll, min(8ll, p.C - c)));
   typename F::Cols cols;
   f.columns(cols, c, n);
@@ -130,7 +132,7 @@ __global__ void __launch_bounds__(HP_THREADS, 2) half_produce_kernel(const F f, 
 #pragma unroll
   for (int i = 0; i < HP_ROWS; ++i) m = amax8(v[i], m);
   const int e = half_block_exponent(m);
-  if (threadIdx.x == 0) p.exps[blockIdx.y * p.exp_r + blockIdx.x * p.exp_c] = e;
+  if (threadIdx.x == 0) p.exps[by * p.exp_r + bx * p.exp_c] = e;
   if (c >= p.pitch) return;
   const float scale = pow2(-e);
 #pragma unroll
@@ -143,7 +145,7 @@ __global__ void __launch_bounds__(HP_THREADS, 2) half_produce_kernel(const F f, 
 }
 template <typename F>
 inline cudaError_t half_produce(const Context &ctx, const F &f, const HalfPanels &p) {
-  const dim3 grid(static_cast<unsigned>((p.C + HP_BLOCK - 1) / HP_BLOCK), static_cast<unsigned>((p.R + HP_BLOCK - 1) / HP_BLOCK));
+  const dim3 grid(static_cast<unsigned>(((p.C + HP_BLOCK - 1) / HP_BLOCK) * ((p.R + HP_BLOCK - 1) / HP_BLOCK)));
   return launch_dependent(ctx, half_produce_kernel<F>, grid, dim3(HP_THREADS), 0, f, p);
 }
 

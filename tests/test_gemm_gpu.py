@@ -6,6 +6,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
+from conftest import rel_err
 from myea_b200 import capi
 
 pytestmark = pytest.mark.gpu
@@ -103,3 +104,15 @@ def test_fused_activation_derivative_epilogue(tile, shape):
 def test_invalid_arguments():
     lib = capi.load()
     assert lib.myea_b200_gemm_nt(0, 0, 0, 4, 4, None, None, None, 0, None, 0) == -1
+
+
+def test_operand_panels_of_many_million_rows():
+    """more row blocks than the second dimension of a grid holds (65535 of 128 rows)"""
+    lib = capi.load()
+    M, N, K = 65536 * 128 + 1, 5, 16
+    rng = np.random.default_rng(0)
+    A, B = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
+    out = np.zeros((M, N), np.float32)
+    assert lib.myea_b200_gemm_nt(0, 0, M, N, K, A.ctypes.data, B.ctypes.data, out.ctypes.data, 0, None, 0) == 0
+    for rows in (slice(0, 1000), slice(M // 2, M // 2 + 1000), slice(M - 1000, M)):
+        assert rel_err(out[rows], A[rows].astype(np.float64) @ B.astype(np.float64).T) < 5e-6
