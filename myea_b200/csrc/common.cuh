@@ -236,23 +236,27 @@ size_t gemm_scratch_floats(long long M, long long N, long long K);
 bool epilogue_takes_stats(const Context &ctx, const Epilogue &e, long long N);
 // Launches split kernels + the tensor-core kernel (engine 0) or the FP32 FMA kernel (engine 1) on ctx.stream.
 int gemm_nt(Context &ctx, const Operand &A, const Operand &B, const Epilogue &epi, const GemmScratch &scratch);
-// A tensor [R][C] as two half-precision arrays and an exponent per block of 128 x 128 (half_panels.cuh)
-struct HalfPanels {
-  uint16_t *h0 = nullptr, *h1 = nullptr;
-  long long R = 0, C = 0, pitch = 0;   // pitch in elements, a multiple of 64
-  int *exps = nullptr;                 // block (r / 128, c / 128) at exps[(r / 128) * exp_r + (c / 128) * exp_c]
-  long long exp_r = 0, exp_c = 0;      // both 0: one exponent for the whole tensor
+// A tensor [R][C] as two half-precision arrays and powers of two, for either reading of it (half_panels.cuh)
+struct HalfReading {
+  uint16_t *h0 = nullptr, *h1 = nullptr;   // null: the panels of this reading are not made
+  uint16_t *scale = nullptr;               // upper half of the float 2^(e - 14): rows [C / 128][row], columns [R / 128][column]
+  long long pitch = 0;                     // of scale, a multiple of 128
 };
-// An operand of a contraction: rows x k elements of a tensor from (row0, k0) on, read through the tensor's rows (K along C)
-// or through its columns (K along R).  Where the tensor has an exponent per block, row0 and k0 are multiples of 128.
+struct HalfPanels {
+  long long R = 0, C = 0, pitch = 0;   // pitch in elements, a multiple of 64
+  HalfReading rows, cols;              // read through its rows (K along C) / through its columns (K along R)
+};
+// An operand of a contraction: rows x k elements, the rows (or the columns) of a tensor
 struct HalfOperand {
   HalfPanels p;
   bool cols = false;
-  long long row0 = 0, k0 = 0, rows = 0, k = 0;
+  long long rows = 0, k = 0;
+  const HalfReading &reading() const { return cols ? p.cols : p.rows; }
 };
-// floats of memory the panels of an [R][C] tensor take, and where they lie in it (256-byte aligned)
-size_t half_panel_floats(long long R, long long C);
-HalfPanels half_panels_at(float *mem, long long R, long long C);
+// floats of memory the panels of an [R][C] tensor take for the given readings, and where they lie in it (256-byte aligned)
+enum { HALF_ROWS = 1, HALF_COLS = 2, HALF_BOTH = 3 };
+size_t half_panel_floats(long long R, long long C, int readings);
+HalfPanels half_panels_at(float *mem, long long R, long long C, int readings);
 // Splits `src` (pitch stride) into panels.  seg_rows != 0: row r of the tensor is row r % seg_rows of the array that starts
 // at src + seg_off[r / seg_rows] (the four gate matrices inside an LSTM layer's parameter blocks).
 struct RowSegments {

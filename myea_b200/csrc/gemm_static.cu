@@ -35,7 +35,7 @@ constexpr int kMaxDevices = 64;
 
 // (the panels of the largest problems that fit the documented limit are a few hundred floats longer: block exponents and
 // alignment)
-static __device__ __align__(256) float g_static_scratch[kStaticScratchFloats + (size_t(64) << 10)];
+static __device__ __align__(256) float g_static_scratch[kStaticScratchFloats + (size_t(128) << 10)];
 static __device__ __align__(256) int g_static_status[64];
 
 struct StaticSetup {
@@ -116,7 +116,7 @@ extern "C" int myea_b200_gemm_nt_static(int device, uint64_t M, uint64_t N, uint
   e.C = device_C;
   e.ldc = static_cast<long long>(N);
   e.accumulate = accumulate;
-  GemmScratch gs{su.scratch, kStaticScratchFloats + (size_t(64) << 10)};
+  GemmScratch gs{su.scratch, kStaticScratchFloats + (size_t(128) << 10)};
   int rc = gemm_nt(ctx, a, b, e, gs);
   if (rc != MYEA_OK) {
     say(error_message, error_capacity, "gemm_nt_static: kernel launch failed");

@@ -7,8 +7,9 @@
 // Update_Derivative_Weight__FC (…Update_Derivative_Weight__OpenMP.cpp:178-216), and the LSTM gate products.
 //
 // Operands come as half panels (half_panels.cuh): x = (h0 + h1) * 2^e.  Per 16 of K three tcgen05.mma kind::f16
-// (h1*h0, h0*h1, h0*h0) accumulate in fp32 in tensor memory.  Exponents belong to blocks of 128 x 128, and an accumulator
-// holds 128 of K: the drain multiplies it by the one power of two of its pair of blocks while it adds it to the running sum.
+// (h1*h0, h0*h1, h0*h0) accumulate in fp32 in tensor memory.  An exponent belongs to one row of an operand and 128 of K, and an
+// accumulator holds 128 of K: the drain multiplies it by the powers of two of its row and column while it adds it to the running
+// sum.
 //
 // One kernel, persistent: a CTA pair (cta_group::2) computes 256 x BN output tiles (BN = 256; 128 where N <= 128), each
 // CTA 128 rows.  384 threads in three warpgroups:
@@ -69,13 +70,28 @@ struct WideWork {
 };
 constexpr int HG_REGION_FLOATS = 32 * 128;  // one drain warp's share of a 256 x 256 tile: 32 rows x 128 columns
 
-// exponents of an operand as the kernel walks them: block b along its rows, chunk c along K
-struct ExpView {
-  const int *p;
-  long long step_row, step_k;
-  int last_row, last_k;   // blocks past the tensor repeat the last one
-  __device__ __forceinline__ int at(int b, int c) const { return p[min(b, last_row) * step_row + min(c, last_k) * step_k]; }
+// powers of two of an operand as the kernel walks them: chunk c of K, block b of 128 of its rows
+struct ScaleView {
+  const uint16_t *p;
+  long long step_k;
+  int last;   // blocks past the tensor repeat the last one
+  __device__ __forceinline__ const uint16_t *block(int b) const { return p + static_cast<long long>(min(b, last)) * HP_BLOCK; }
 };
+
+// two neighbouring columns in packed arithmetic (half the instructions): sum += product * column's power of two * row's
+__device__ __forceinline__ void scaled_add2(float &s0, float &s1, uint32_t r0, uint32_t r1, uint32_t columns, uint64_t row) {
+  asm("{\n"
+      ".reg .b64 r, c, s;\n"
+      "mov.b64 r, {%2, %3};\n"
+      "mov.b64 c, {%4, %5};\n"
+      "mov.b64 s, {%0, %1};\n"
+      "mul.rn.f32x2 r, r, c;\n"
+      "fma.rn.f32x2 s, r, %6, s;\n"
+      "mov.b64 {%0, %1}, s;\n"
+      "}\n"
+      : "+f"(s0), "+f"(s1)
+      : "r"(r0), "r"(r1), "r"(columns << 16), "r"(columns & 0xffff0000u), "l"(row));
+}
 
 __device__ __forceinline__ void wide_tile_coords(const WideWork &w, int t, int &tm, int &tn) {
   const int per_band = HG_BAND * w.tiles_n;
@@ -140,7 +156,7 @@ __device__ __forceinline__ void half_load_operand(uint8_t *dst0, uint8_t *dst1, 
 template <int BN, bool A_COLS, bool B_COLS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(HG_THREADS, 1)
 half_gemm_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_constant__ CUtensorMap tm_a1, const __grid_constant__ CUtensorMap tm_b0,
-                 const __grid_constant__ CUtensorMap tm_b1, const ExpView exp_a, const ExpView exp_b, const GemmDims dims, const WideWork work,
+                 const __grid_constant__ CUtensorMap tm_b1, const ScaleView scale_a, const ScaleView scale_b, const GemmDims dims, const WideWork work,
                  const Epilogue epi, const int variant, int *error_flag) {
   using S = HalfSmem<BN>;
   constexpr int STAGES = HG_STAGES, TMEM_COLS = 2 * BN, HALF_N = BN / 2;
@@ -276,13 +292,22 @@ half_gemm_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_constan
     while (ok && seg.next()) {
       int tm, tn;
       wide_tile_coords(work, seg.tile, tm, tn);
-      const int block_a = tm * 2 + static_cast<int>(cta_rank), block_b = (tn * BN + half * HALF_N) / HP_BLOCK;
+      const uint16_t *pa = scale_a.block(tm * 2 + static_cast<int>(cta_rank)) + q * 32 + lane;
+      const uint16_t *pb = scale_b.block((tn * BN + half * HALF_N) / HP_BLOCK) + (half * HALF_N) % HP_BLOCK;
       float sum[HALF_N];
 #pragma unroll
       for (int j = 0; j < HALF_N; ++j) sum[j] = 0.f;
       for (int c = seg.c0; c < seg.c1; ++c, ++g) {
         const uint32_t b = g & 1u;
-        const int e = exp_a.at(block_a, c) + exp_b.at(block_b, c);
+        // Powers of two of this lane's row and of the columns (32 of them ahead of the products they belong to).  The column's
+        // comes first, times 2^-14 as it is kept, and the row's times 2^14 after it, so that the step between leaves the range
+        // of fp32 only for columns beyond 2^118.
+        const uint32_t row_bits = (static_cast<uint32_t>(pa[c * scale_a.step_k]) << 16) + (28u << 23);
+        const uint64_t sa = static_cast<uint64_t>(row_bits) << 32 | row_bits;
+        const uint4 *sb = reinterpret_cast<const uint4 *>(pb + c * scale_b.step_k);
+        uint4 next[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) next[i] = sb[i];
         if (!ptx::mbar_wait_or_abort(&acc_full_bar[b], (g >> 1) & 1u, abort_flag)) {
           ok = false;
           if (lane == 0) atomicCAS(error_flag, 0, 303);
@@ -290,20 +315,20 @@ half_gemm_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_constan
         }
         ptx::tc_fence_after();
         const uint32_t tsrc = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + b * static_cast<uint32_t>(BN) + static_cast<uint32_t>(half * HALF_N);
-        // 2^e in two factors, so that neither leaves the range of fp32 where their product with the sum does not
-        const int e1 = max(-126, min(127, e)), e2 = max(-126, min(127, e - e1));
-        const float s1 = pow2(e1), s2 = pow2(e2);
 #pragma unroll
         for (int jc = 0; jc < HALF_N / 32; ++jc) {
           uint32_t r[32];
           ptx::tmem_ld_32x32(tsrc + static_cast<uint32_t>(jc * 32), r);
+          uint32_t w[16];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            w[4 * i] = next[i].x; w[4 * i + 1] = next[i].y; w[4 * i + 2] = next[i].z; w[4 * i + 3] = next[i].w;
+            if (jc + 1 < HALF_N / 32) next[i] = sb[4 * (jc + 1) + i];
+          }
           ptx::tmem_ld_wait();
-          if (e2 == 0) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) sum[jc * 32 + j] = fmaf(__uint_as_float(r[j]), s1, sum[jc * 32 + j]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) sum[jc * 32 + j] = fmaf(__uint_as_float(r[j]) * s2, s1, sum[jc * 32 + j]);
+          for (int j = 0; j < 32; j += 2) {
+            scaled_add2(sum[jc * 32 + j], sum[jc * 32 + j + 1], r[j], r[j + 1], w[j / 2], sa);
           }
         }
         // this warp's reads of the buffer are complete: hand it back to the MMA issuer
@@ -485,37 +510,47 @@ bool make_half_map(CUtensorMap *map, const HalfOperand &o, const uint16_t *h, in
   if (fn == nullptr) return false;
   const cuuint64_t pitch = static_cast<cuuint64_t>(o.p.pitch) * 2;
   cuuint32_t estr[3] = {1, 1, 1};
+  if (h == nullptr) return false;   // (the panels of this reading were not made)
   if (!o.cols) {
     cuuint64_t gdim[2] = {static_cast<cuuint64_t>(o.k), static_cast<cuuint64_t>(o.rows)};
     cuuint64_t gstride[1] = {pitch};
     cuuint32_t box[2] = {HG_BK, static_cast<cuuint32_t>(box_rows)};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<uint16_t *>(h + o.row0 * o.p.pitch + o.k0), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<uint16_t *>(h), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   }
   // 64 operand rows (128 bytes) x K x chunks of 64 rows: a box lands chunk after chunk, each chunk 64 K rows of 128 bytes
   cuuint64_t gdim[3] = {64, static_cast<cuuint64_t>(o.k), static_cast<cuuint64_t>((o.rows + 63) / 64)};
   cuuint64_t gstride[2] = {pitch, 128};
   cuuint32_t box[3] = {64, HG_BK, static_cast<cuuint32_t>(box_rows / 64)};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<uint16_t *>(h + o.k0 * o.p.pitch + o.row0), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<uint16_t *>(h), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 static inline long long round_up(long long x, long long m) { return (x + m - 1) / m * m; }
-static size_t exp_count(long long R, long long C) { return static_cast<size_t>((R + HP_BLOCK - 1) / HP_BLOCK) * static_cast<size_t>((C + HP_BLOCK - 1) / HP_BLOCK); }
-
-size_t half_panel_floats(long long R, long long C) {
-  return static_cast<size_t>(R * round_up(C, 64)) + static_cast<size_t>(round_up(static_cast<long long>(exp_count(R, C)), 64)) + 128;
+static size_t scale_floats(long long R, long long C) {   // of the panels read through R rows
+  return static_cast<size_t>(round_up(R, HP_BLOCK) / 2) * static_cast<size_t>((C + HP_BLOCK - 1) / HP_BLOCK);
 }
 
-HalfPanels half_panels_at(float *mem, long long R, long long C) {
+size_t half_panel_floats(long long R, long long C, int readings) {
+  size_t n = 64;   // alignment of the base
+  if (readings & HALF_ROWS) n += static_cast<size_t>(R * round_up(C, 64)) + scale_floats(R, C);
+  if (readings & HALF_COLS) n += static_cast<size_t>(R * round_up(C, 64)) + scale_floats(C, R);
+  return n;
+}
+
+HalfPanels half_panels_at(float *mem, long long R, long long C, int readings) {
   HalfPanels p;
   p.R = R; p.C = C; p.pitch = round_up(C, 64);
   mem = reinterpret_cast<float *>((reinterpret_cast<uintptr_t>(mem) + 255) & ~static_cast<uintptr_t>(255));
-  p.h0 = reinterpret_cast<uint16_t *>(mem);
-  p.h1 = p.h0 + R * p.pitch;   // (R * pitch is a multiple of 64: both arrays start on 128-byte boundaries)
-  p.exps = reinterpret_cast<int *>(p.h1 + R * p.pitch);
-  p.exp_r = (C + HP_BLOCK - 1) / HP_BLOCK;
-  p.exp_c = 1;
+  auto place = [&](HalfReading &to, long long rows, long long k) {   // (every part is a multiple of 64 floats or, an array of halves, of 32)
+    to.h0 = reinterpret_cast<uint16_t *>(mem);
+    to.h1 = to.h0 + R * p.pitch;
+    to.scale = to.h1 + R * p.pitch;
+    to.pitch = round_up(rows, HP_BLOCK);
+    mem += R * p.pitch + static_cast<long long>(scale_floats(rows, k));
+  };
+  if (readings & HALF_ROWS) place(p.rows, R, C);
+  if (readings & HALF_COLS) place(p.cols, C, R);
   return p;
 }
 
@@ -531,7 +566,7 @@ HalfOperand half_cols(const HalfPanels &p) {
 }
 
 int half_split(Context &ctx, const float *src, long long stride, const HalfPanels &p, const RowSegments *seg) {
-  if (src == nullptr || p.h0 == nullptr || p.R <= 0 || p.C <= 0) return MYEA_E_INVALID;
+  if (src == nullptr || (p.rows.h0 == nullptr && p.cols.h0 == nullptr) || p.R <= 0 || p.C <= 0) return MYEA_E_INVALID;
   SplitSource f;
   f.src = src;
   f.stride = stride;
@@ -599,17 +634,11 @@ static int launch_half(Context &ctx, const HalfOperand &A, const HalfOperand &B,
   });
   if (G <= 0) return MYEA_E_CUDA;
   CUtensorMap maps[4];
-  if (!make_half_map(&maps[0], A, A.p.h0, 128) || !make_half_map(&maps[1], A, A.p.h1, 128) || !make_half_map(&maps[2], B, B.p.h0, BN / 2) ||
-      !make_half_map(&maps[3], B, B.p.h1, BN / 2))
+  if (!make_half_map(&maps[0], A, A.reading().h0, 128) || !make_half_map(&maps[1], A, A.reading().h1, 128) ||
+      !make_half_map(&maps[2], B, B.reading().h0, BN / 2) || !make_half_map(&maps[3], B, B.reading().h1, BN / 2))
     return MYEA_E_CUDA;
-  auto exps = [](const HalfOperand &o) {
-    ExpView v;
-    v.step_row = o.cols ? o.p.exp_c : o.p.exp_r;
-    v.step_k = o.cols ? o.p.exp_r : o.p.exp_c;
-    v.p = o.p.exps + o.row0 / HP_BLOCK * v.step_row + o.k0 / HP_BLOCK * v.step_k;
-    v.last_row = static_cast<int>((o.rows - 1) / HP_BLOCK);
-    v.last_k = static_cast<int>((o.k - 1) / HP_BLOCK);
-    return v;
+  auto scales = [](const HalfOperand &o) {
+    return ScaleView{o.reading().scale, o.reading().pitch, static_cast<int>((o.rows - 1) / HP_BLOCK)};
   };
   const int num_kb = (dims.K + HG_BK - 1) / HG_BK;
   const int num_chunks = (num_kb + HG_KC - 1) / HG_KC;
@@ -641,7 +670,7 @@ static int launch_half(Context &ctx, const HalfOperand &A, const HalfOperand &B,
       grid_clusters = work.dp_tiles > 0 ? G : used;
     }
   }
-  launch_dependent(ctx, kernel, dim3(static_cast<unsigned>(2 * grid_clusters)), dim3(HG_THREADS), S::TOTAL, maps[0], maps[1], maps[2], maps[3], exps(A), exps(B), dims,
+  launch_dependent(ctx, kernel, dim3(static_cast<unsigned>(2 * grid_clusters)), dim3(HG_THREADS), S::TOTAL, maps[0], maps[1], maps[2], maps[3], scales(A), scales(B), dims,
                    work, epi, epilogue_variant(epi), ctx.d_error_flag);
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
@@ -649,13 +678,8 @@ static int launch_half(Context &ctx, const HalfOperand &A, const HalfOperand &B,
 int half_gemm(Context &ctx, const HalfOperand &A, const HalfOperand &B, const Epilogue &epi) {
   const long long M = A.rows, N = B.rows, K = A.k;
   if (B.k != K || M <= 0 || N <= 0 || K <= 0) return MYEA_E_INVALID;
-  for (const HalfOperand *o : {&A, &B}) {
-    const long long r_end = o->row0 + o->rows, k_end = o->k0 + o->k;
-    if (o->row0 < 0 || o->k0 < 0 || r_end > (o->cols ? o->p.C : o->p.R) || k_end > (o->cols ? o->p.R : o->p.C)) return MYEA_E_INVALID;
-    const bool uniform = o->p.exp_r == 0 && o->p.exp_c == 0;
-    if (!uniform && ((o->row0 | o->k0) & (HP_BLOCK - 1)) != 0) return MYEA_E_INVALID;
-    if (((o->cols ? o->row0 : o->k0) & 7) != 0) return MYEA_E_INVALID;   // 16-byte TMA base
-  }
+  for (const HalfOperand *o : {&A, &B})
+    if (o->rows > (o->cols ? o->p.C : o->p.R) || K > (o->cols ? o->p.R : o->p.C) || o->reading().h0 == nullptr) return MYEA_E_INVALID;
   if (!derivative_is_fused(epi.deriv_af)) {
     if (epi.accumulate || epi.seg_rows != 0 || epi.stats_kind != 0 || epi.ldc != N || epi.ld_aux != N) return MYEA_E_UNSUPPORTED;
     Epilogue plain = epi;
@@ -681,7 +705,8 @@ int half_gemm(Context &ctx, const HalfOperand &A, const HalfOperand &B, const Ep
 
 size_t gemm_scratch_floats(long long M, long long N, long long K) {
   // whichever index of an operand is contiguous in memory
-  return std::max(half_panel_floats(M, K), half_panel_floats(K, M)) + std::max(half_panel_floats(N, K), half_panel_floats(K, N));
+  return std::max(half_panel_floats(M, K, HALF_ROWS), half_panel_floats(K, M, HALF_COLS)) +
+         std::max(half_panel_floats(N, K, HALF_ROWS), half_panel_floats(K, N, HALF_COLS));
 }
 
 int gemm_nt(Context &ctx, const Operand &A, const Operand &B, const Epilogue &epi, const GemmScratch &scratch) {
@@ -699,14 +724,14 @@ int gemm_nt(Context &ctx, const Operand &A, const Operand &B, const Epilogue &ep
     const DirectItem item{A, B, epi, nullptr};
     return direct_gemm(ctx, &item, 1);
   }
-  auto need = [](const Operand &o) { return o.stride_k != 1 ? half_panel_floats(o.k, o.rows) : half_panel_floats(o.rows, o.k); };
+  auto need = [](const Operand &o) { return o.stride_k != 1 ? half_panel_floats(o.k, o.rows, HALF_COLS) : half_panel_floats(o.rows, o.k, HALF_ROWS); };
   if (scratch.base == nullptr || scratch.floats < need(A) + need(B)) return MYEA_E_INVALID;
   float *mem = scratch.base;
   HalfOperand ops[2];
   for (int i = 0; i < 2; ++i) {
     const Operand &o = i == 0 ? A : B;
     const bool cols = o.stride_k != 1;   // the operand's rows are contiguous: split as it lies, read through its columns
-    const HalfPanels p = cols ? half_panels_at(mem, o.k, o.rows) : half_panels_at(mem, o.rows, o.k);
+    const HalfPanels p = cols ? half_panels_at(mem, o.k, o.rows, HALF_COLS) : half_panels_at(mem, o.rows, o.k, HALF_ROWS);
     const int rc = half_split(ctx, o.ptr, cols ? o.stride_k : o.stride_r, p);
     if (rc != MYEA_OK) return rc;
     ops[i] = cols ? half_cols(p) : half_rows(p);

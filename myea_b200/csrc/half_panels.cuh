@@ -1,14 +1,19 @@
-// Operand panels of the dense contractions: an fp32 tensor as the sum of two half-precision arrays times a power of two.
+// Operand panels of the dense contractions: an fp32 tensor as the sum of two half-precision arrays times powers of two.
 //
 //   x = (h0 + h1) * 2^e        h0 = x * 2^-e rounded to half, h1 = what is left of x * 2^-e rounded to half
 //
-// Two halves carry 22 significant bits.  e is chosen per block of 128 x 128 elements so that the block's largest magnitude
-// lands in [2^14, 2^15): an element of magnitude a in a block whose largest is m is off by at most max(2^-22 a, 2^-39 m) -
-// half keeps 22 bits down to 2^-17 of the block's largest and then a fixed step of 2^-39 of it.  A product is
-// h1_a*h0_b + h0_a*h1_b + h0_a*h0_b, three half instructions per 16 of K; the dropped h1_a*h1_b is 2^-22 of it.
-// (Before: a TF32 array and, per reading, a bf16 cross-term array - 12 bytes per element for a tensor that is read through
-// rows and columns, two instructions per 8 of K, products off by up to 2^-17.)  The same two arrays serve both operand
-// roles and both readings, through their rows (K contiguous) and through their columns.
+// A contraction reads a tensor through its rows (K along the columns) or through its columns (K along the rows), and its
+// results along the other index are independent of each other: a sample with huge inputs, a unit with tiny errors must not
+// touch its neighbours.  So the exponent belongs to ONE row (column) and 128 of K, and a tensor that is read both ways has
+// two sets, one per reading (4 bytes per element and set).  e puts the largest finite magnitude m of these 128 elements
+// into [2^14, 2^15): an element of magnitude a is off by at most max(2^-22 a, 2^-39 m, 2^-127) - two halves carry 22 bits
+// down to 2^-17 of m and then a fixed step.  Infinities and NaN stay what they are and reach the results of their own row and
+// column only.  A product is h1_a*h0_b + h0_a*h1_b + h0_a*h0_b, three half instructions per 16 of K; the dropped h1_a*h1_b is
+// 2^-22 of it.
+// (With one exponent per block of 128 x 128 and one set for both readings an infinity turned every other row of its block
+// into zeros, and rows or columns below 2^-22 of the block's largest lost digits that a TF32 + bf16 split keeps.  The second set
+// costs 4 bytes written per element: activation of 4096 x 4096 47 -> 58 us, update of 138 M
+// weights 699 -> 764 us, the training step around them 3 % longer.)
 #pragma once
 
 #include <cuda_fp16.h>
@@ -19,14 +24,17 @@ namespace myea {
 
 constexpr int HP_BLOCK = 128;   // rows and columns of a block with one exponent
 
-// exponent for a block whose largest magnitude is amax
+// exponent for a row or column whose largest finite magnitude is amax; the scales 2^-e and 2^(e - 14) have to be normal floats
 __device__ __forceinline__ int half_exponent(float amax) {
   const int E = static_cast<int>((__float_as_uint(amax) >> 23) & 0xFFu);
   if (amax == 0.f) return 0;
-  return max(E - 127 - 14, -126);   // (the scale 2^-e has to be a normal float)
+  return max(E - 127 - 14, -112);
 }
 // 2^n for -126 <= n <= 127
 __device__ __forceinline__ float pow2(int n) { return __uint_as_float(static_cast<uint32_t>(n + 127) << 23); }
+
+// the power of two as it is kept beside the panels: the upper half of the float 2^(e - 14) (see half_gemm.cu)
+__device__ __forceinline__ uint16_t half_scale_bits(int e) { return static_cast<uint16_t>((e - 14 + 127) << 7); }
 
 __device__ __forceinline__ uint32_t half2_bits(float a, float b) {   // a in the lower half
   uint32_t r;
@@ -49,41 +57,104 @@ __device__ __forceinline__ void half_split8(const float (&v)[8], uint4 &h0, uint
 }
 
 // A block of 512 threads holds a 128 x 128 block of the tensor: thread = 8 columns (tid % 16) of rows tid / 16 + 32 i.
-// half_block_finish: the block's exponent from every thread's largest magnitude (all threads of the block call it).
 constexpr int HP_THREADS = 512;
 constexpr int HP_ROWS = HP_BLOCK * 16 / HP_THREADS;   // rows per thread
-template <int THREADS = HP_THREADS>
-__device__ __forceinline__ int half_block_exponent(float amax) {
-  __shared__ float sh[THREADS / 32];
+__device__ __forceinline__ float finite_abs(float x) {
+  x = fabsf(x);
+  return x <= 3.402823466e+38f ? x : 0.f;
+}
+// largest finite magnitudes of a thread's rows and columns -> of the whole rows (16 lanes share them)
+__device__ __forceinline__ void half_row_maxima(const float (&v)[HP_ROWS][8], float (&m)[HP_ROWS]) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = amax;
+  for (int i = 0; i < HP_ROWS; ++i) {
+    m[i] = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m[i] = fmaxf(m[i], finite_abs(v[i][j]));
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], o));
+  }
+}
+// ... and of the block's columns, over the 32 threads that share them (all threads of the block call it)
+__device__ __forceinline__ void half_column_maxima(const float (&v)[HP_ROWS][8], float (&m)[8]) {
+  __shared__ float4 part[HP_THREADS / 32][HP_BLOCK / 4];
+  __shared__ float whole[HP_BLOCK];
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    m[j] = 0.f;
+#pragma unroll
+    for (int i = 0; i < HP_ROWS; ++i) m[j] = fmaxf(m[j], finite_abs(v[i][j]));
+    m[j] = fmaxf(m[j], __shfl_xor_sync(0xffffffffu, m[j], 16));
+  }
+  if (lane < 16) {
+    part[threadIdx.x >> 5][2 * lane] = make_float4(m[0], m[1], m[2], m[3]);
+    part[threadIdx.x >> 5][2 * lane + 1] = make_float4(m[4], m[5], m[6], m[7]);
+  }
+  __syncthreads();
+  if (threadIdx.x < HP_BLOCK) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < HP_THREADS / 32; ++w) t = fmaxf(t, reinterpret_cast<const float *>(part[w])[threadIdx.x]);
+    whole[threadIdx.x] = t;
+  }
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < THREADS / 32; ++w) amax = fmaxf(amax, sh[w]);
-  return half_exponent(amax);
+  for (int j = 0; j < 8; ++j) m[j] = whole[(threadIdx.x & 15) * 8 + j];
 }
-__device__ __forceinline__ float amax8(const float (&v)[8], float m) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j) m = fmaxf(m, fabsf(v[j]));
-  return m;
-}
-// elements (r, c .. c + 7); c + 8 <= pitch, columns past the tensor's width are zeros
-__device__ __forceinline__ void half_store8(const HalfPanels &p, long long r, long long c, const float (&v)[8], float scale) {
-  float s[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) s[j] = v[j] * scale;
+// elements (r, c .. c + 7), already times 2^-e; c + 8 <= pitch, columns past the tensor's width are zeros
+__device__ __forceinline__ void half_store8(const HalfPanels &p, const HalfReading &to, long long r, long long c, const float (&s)[8]) {
   uint4 h0, h1;
   half_split8(s, h0, h1);
-  *reinterpret_cast<uint4 *>(p.h0 + r * p.pitch + c) = h0;
-  *reinterpret_cast<uint4 *>(p.h1 + r * p.pitch + c) = h1;
+  *reinterpret_cast<uint4 *>(to.h0 + r * p.pitch + c) = h0;
+  *reinterpret_cast<uint4 *>(to.h1 + r * p.pitch + c) = h1;
+}
+// A block of the tensor, held by its 512 threads (zeros past the tensor's edges), into the panels of every reading that p has
+__device__ __forceinline__ void half_store_block(const HalfPanels &p, long long by, long long bx, const float (&v)[HP_ROWS][8]) {
+  const long long c = bx * HP_BLOCK + (threadIdx.x & 15) * 8, r0 = by * HP_BLOCK + (threadIdx.x >> 4);
+  if (p.rows.h0 != nullptr) {
+    float m[HP_ROWS];
+    half_row_maxima(v, m);
+#pragma unroll
+    for (int i = 0; i < HP_ROWS; ++i) {
+      const long long r = r0 + HP_THREADS / 16 * i;
+      const int e = half_exponent(m[i]);
+      if ((threadIdx.x & 15) == 0) p.rows.scale[bx * p.rows.pitch + r] = half_scale_bits(e);
+      const float f = pow2(-e);
+      float s[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s[j] = v[i][j] * f;
+      if (r < p.R && c < p.pitch) half_store8(p, p.rows, r, c, s);
+    }
+  }
+  if (p.cols.h0 != nullptr) {
+    float m[8];
+    half_column_maxima(v, m);
+    uint32_t bits[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int e = half_exponent(m[j]);
+      bits[j] = half_scale_bits(e);
+      m[j] = pow2(-e);
+    }
+    if (threadIdx.x < 16)
+      *reinterpret_cast<uint4 *>(p.cols.scale + by * p.cols.pitch + c) =
+          make_uint4(bits[0] | bits[1] << 16, bits[2] | bits[3] << 16, bits[4] | bits[5] << 16, bits[6] | bits[7] << 16);
+#pragma unroll
+    for (int i = 0; i < HP_ROWS; ++i) {
+      const long long r = r0 + HP_THREADS / 16 * i;
+      float s[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s[j] = v[i][j] * m[j];
+      if (r < p.R && c < p.pitch) half_store8(p, p.cols, r, c, s);
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------------------------------------
 // A producer computes an fp32 tensor and leaves it both as an array and as panels for the contractions that read it next:
-// one block of 128 x 128 per CTA, read once, its largest magnitude found in registers, everything written once.  Bound by HBM
-// at 4096 x 4096 (26 us for the 128 MB of a split) and by the chain load - maximum - store of the one block an SM gets at 512 rows:
-// 512 threads of 4 rows (activation of 512 x 4096 11.3 us, with 256 threads of 8 rows 13.1).
+// one block of 128 x 128 per CTA, read once, the largest magnitudes of its rows and columns found on chip, everything written
+// once.  Bound by HBM at 4096 x 4096 (34 us for the 201 MB of a split for both readings) and by the chain load - maximum - store
+// of the one block an SM gets at 512 rows: 512 threads of 4 rows (activation of 512 x 4096 12.5 us).
 // F: struct Cols; columns(Cols &, c, n): what belongs to this thread's columns c .. c + n - 1; row(cols, r, c, n, v): the
 // values of row r (zeros in v[n] ..); keep(r, c, n, v): stores the fp32 result (may do nothing).
 // ---------------------------------------------------------------------------------------------------------
@@ -107,22 +178,17 @@ __device__ __forceinline__ void st8(float *p, const float (&d)[8], int n, bool v
   }
 }
 
+// block (by, bx) of the tensor: this thread's share of its values, zeros past the tensor's edges
 template <typename F>
-__global__ void __launch_bounds__(HP_THREADS, 2) half_produce_kernel(const F f, const HalfPanels p) {
-  grid_dependency_wait();
-  grid_dependency_release();
-  // (one dimension: the row blocks of a tensor of many million rows are more than the others hold)
-  const unsigned across = static_cast<unsigned>((p.C + HP_BLOCK - 1) / HP_BLOCK), by = blockIdx.x / across, bx = blockIdx.x - by * across;
-  const long long c = bx * static_cast<long long>(HP_BLOCK) + (threadIdx.x & 15) * 8;
-  const long long r0 = by * static_cast<long long>(HP_BLOCK) + (threadIdx.x >> 4);
-  const int n = static_cast<int>(max(0ll, min(8ll, p.C - c)));
+__device__ __forceinline__ void half_load_block(const F &f, long long R, long long C, long long by, long long bx, float (&v)[HP_ROWS][8]) {
+  const long long c = bx * HP_BLOCK + (threadIdx.x & 15) * 8, r0 = by * HP_BLOCK + (threadIdx.x >> 4);
+  const int n = static_cast<int>(max(0ll, min(8ll, C - c)));
   typename F::Cols cols;
   f.columns(cols, c, n);
-  float v[HP_ROWS][8], m = 0.f;
 #pragma unroll
   for (int i = 0; i < HP_ROWS; ++i) {
     const long long r = r0 + HP_THREADS / 16 * i;
-    if (r < p.R) {
+    if (r < R) {
       f.row(cols, r, c, n, v[i]);
     } else {
 #pragma unroll
@@ -130,23 +196,32 @@ __global__ void __launch_bounds__(HP_THREADS, 2) half_produce_kernel(const F f, 
     }
   }
 #pragma unroll
-  for (int i = 0; i < HP_ROWS; ++i) m = amax8(v[i], m);
-  const int e = half_block_exponent(m);
-  if (threadIdx.x == 0) p.exps[by * p.exp_r + bx * p.exp_c] = e;
-  if (c >= p.pitch) return;
-  const float scale = pow2(-e);
-#pragma unroll
   for (int i = 0; i < HP_ROWS; ++i) {
     const long long r = r0 + HP_THREADS / 16 * i;
-    if (r >= p.R) continue;
-    f.keep(r, c, n, v[i]);
-    half_store8(p, r, c, v[i], scale);
+    if (r < R) f.keep(r, c, n, v[i]);
   }
+}
+__device__ __forceinline__ void half_block_of(long long C, unsigned block, unsigned &by, unsigned &bx) {
+  // (one dimension: the row blocks of a tensor of many million rows are more than the others hold)
+  const unsigned across = static_cast<unsigned>((C + HP_BLOCK - 1) / HP_BLOCK);
+  by = block / across;
+  bx = block - by * across;
+}
+inline unsigned half_blocks(long long R, long long C) { return static_cast<unsigned>(((C + HP_BLOCK - 1) / HP_BLOCK) * ((R + HP_BLOCK - 1) / HP_BLOCK)); }
+
+template <typename F>
+__global__ void __launch_bounds__(HP_THREADS, 2) half_produce_kernel(const F f, const HalfPanels p) {
+  grid_dependency_wait();
+  grid_dependency_release();
+  unsigned by, bx;
+  half_block_of(p.C, blockIdx.x, by, bx);
+  float v[HP_ROWS][8];
+  half_load_block(f, p.R, p.C, by, bx, v);
+  half_store_block(p, by, bx, v);
 }
 template <typename F>
 inline cudaError_t half_produce(const Context &ctx, const F &f, const HalfPanels &p) {
-  const dim3 grid(static_cast<unsigned>(((p.C + HP_BLOCK - 1) / HP_BLOCK) * ((p.R + HP_BLOCK - 1) / HP_BLOCK)));
-  return launch_dependent(ctx, half_produce_kernel<F>, grid, dim3(HP_THREADS), 0, f, p);
+  return launch_dependent(ctx, half_produce_kernel<F>, dim3(half_blocks(p.R, p.C)), dim3(HP_THREADS), 0, f, p);
 }
 
 }  // namespace myea

@@ -246,6 +246,9 @@ static int lalloc(myea_b200_net *net, T **p, size_t count) {
 
 #define LRC(expr) do { int rc__ = (expr); if (rc__ != MYEA_OK) return rc__; } while (0)
 
+// memory for panels of a tensor that are made for one reading at a time
+static size_t one_reading_floats(long long R, long long C) { return std::max(half_panel_floats(R, C, HALF_ROWS), half_panel_floats(R, C, HALF_COLS)); }
+
 int lstm_create(myea_b200_net *net, LayerPlan &L) {
   const long long cpb = std::max<long long>(1, static_cast<long long>(L.desc.unit_parameters[1]));
   LstmPlan *P = new LstmPlan();
@@ -276,7 +279,7 @@ int lstm_create(myea_b200_net *net, LayerPlan &L) {
     }
     // the input projections are dead after the forward walk, the gate errors' panels are made after the backward walk: one
     // buffer for both (of 268 MB at 1024 cells, 64 steps and 256 rows; mapping and clearing memory is most of what a handle costs)
-    LRC(lalloc(net, &D.gates_in, in_panels || dw_panels ? std::max(static_cast<size_t>(rows * 4 * C), half_panel_floats(rows, 4 * C)) : static_cast<size_t>(rows * 4 * C)));
+    LRC(lalloc(net, &D.gates_in, in_panels || dw_panels ? std::max(static_cast<size_t>(rows * 4 * C), one_reading_floats(rows, 4 * C)) : static_cast<size_t>(rows * 4 * C)));
     if (in_panels || dw_panels) P->dg_all_mem[d] = D.gates_in;
     LRC(lalloc(net, &D.act, rows * 4 * C));
     LRC(lalloc(net, &D.cstate, rows * C));
@@ -302,31 +305,37 @@ int lstm_create(myea_b200_net *net, LayerPlan &L) {
     LRC(lalloc(net, &P->peep_compact, static_cast<size_t>(P->dirs) * 3 * C));
     const long long a_rows = (net->B + 127) / 128 * 128;
     float *mem = nullptr;
-    LRC(lalloc(net, &mem, half_panel_floats(2 * a_rows, C)));       // zero: rows past the batch stay zero for ever
-    P->h_pan = half_panels_at(mem, 2 * a_rows, C);
-    LRC(lalloc(net, &mem, half_panel_floats(2 * a_rows, P->G)));
-    P->dg_pan = half_panels_at(mem, 2 * a_rows, P->G);
-    LRC(lalloc(net, &P->dg_exps, static_cast<size_t>(2 * (a_rows / 128) * (P->G / 64))));
+    LRC(lalloc(net, &mem, half_panel_floats(2 * a_rows, C, HALF_ROWS)));       // zero: rows past the batch stay zero for ever
+    P->h_pan = half_panels_at(mem, 2 * a_rows, C, HALF_ROWS);
+    LRC(lalloc(net, &mem, half_panel_floats(2 * a_rows, P->G, HALF_ROWS)));
+    P->dg_pan = half_panels_at(mem, 2 * a_rows, P->G, HALF_ROWS);
+    LRC(lalloc(net, &P->dg_scale, static_cast<size_t>(2 * a_rows * (P->G / 64))));
+    LRC(lalloc(net, &P->w_rec_max, static_cast<size_t>(P->G + C)));
     for (int d = 0; d < P->dirs; ++d) {
-      LRC(lalloc(net, &P->w_rec_mem[d], half_panel_floats(P->G, C)));
-      P->w_rec[d] = half_panels_at(P->w_rec_mem[d], P->G, C);
+      LRC(lalloc(net, &P->w_rec_mem[d], half_panel_floats(P->G, C, HALF_BOTH)));
+      P->w_rec[d] = half_panels_at(P->w_rec_mem[d], P->G, C, HALF_BOTH);
+      LRC(lalloc(net, &P->w_rec_scale[d], static_cast<size_t>(P->G + C)));
     }
   } else if (P->resident == nullptr) {
     LRC(lalloc(net, &P->s_rec, net->B * 4 * C));
     if (tensor && !direct_gemm_suits(net->ctx, net->B, 4 * C, C)) {
       for (int d = 0; d < P->dirs; ++d) {
-        LRC(lalloc(net, &P->w_rec_mem[d], half_panel_floats(4 * C, C)));
-        P->w_rec[d] = half_panels_at(P->w_rec_mem[d], 4 * C, C);
+        LRC(lalloc(net, &P->w_rec_mem[d], half_panel_floats(4 * C, C, HALF_BOTH)));
+        P->w_rec[d] = half_panels_at(P->w_rec_mem[d], 4 * C, C, HALF_BOTH);
       }
-      LRC(lalloc(net, &P->step_mem, half_panel_floats(net->B, 4 * C)));
+      LRC(lalloc(net, &P->step_mem, half_panel_floats(net->B, 4 * C, HALF_ROWS)));
     } else {
       for (int d = 0; d < P->dirs; ++d) LRC(lalloc(net, &P->w_rec_mem[d], static_cast<size_t>(4 * C * C)));
     }
   }
-  if (in_panels || dw_panels) LRC(lalloc(net, &P->x_mem, half_panel_floats(rows, L.n_in)));
+  if (in_panels || dw_panels) LRC(lalloc(net, &P->x_mem, one_reading_floats(rows, L.n_in)));
+  const int w_in_readings = L.input_layer > 0 ? HALF_BOTH : HALF_ROWS;   // (the network's inputs receive no error)
   for (int d = 0; d < P->dirs; ++d) {
-    if (in_panels) LRC(lalloc(net, &P->w_in_mem[d], half_panel_floats(4 * C, L.n_in)));
-    if (dw_panels) LRC(lalloc(net, &P->h_shift_mem[d], half_panel_floats(rows, C)));
+    if (in_panels) {
+      LRC(lalloc(net, &P->w_in_mem[d], half_panel_floats(4 * C, L.n_in, w_in_readings)));
+      P->w_in[d] = half_panels_at(P->w_in_mem[d], 4 * C, L.n_in, w_in_readings);
+    }
+    if (dw_panels) LRC(lalloc(net, &P->h_shift_mem[d], half_panel_floats(rows, C, HALF_COLS)));
   }
   net->scratch.floats = std::max(net->scratch.floats, need + 256);
   return MYEA_OK;
@@ -390,6 +399,62 @@ struct GroupedGateRows {
   }
   __device__ __forceinline__ void keep(long long, long long, int, const float (&)[8]) const {}
 };
+// Panels of the recurrent weights for the walk: a row (column) has ONE power of two for all of its K, so the walk, which finishes
+// every sum once per step, multiplies by it once instead of stage by stage.  The largest magnitudes take a pass of their own
+// (maxima: [G] of the rows, then [C] of the columns); both passes run when the weights have changed, 10 + 13 us for 1024 cells.
+__global__ void __launch_bounds__(HP_THREADS, 2) weight_extents_kernel(const GroupedGateRows f, long long R, long long C, unsigned int *maxima) {
+  grid_dependency_wait();
+  grid_dependency_release();
+  unsigned by, bx;
+  half_block_of(C, blockIdx.x, by, bx);
+  float v[HP_ROWS][8], m[HP_ROWS], mc[8];
+  half_load_block(f, R, C, by, bx, v);
+  half_row_maxima(v, m);
+  half_column_maxima(v, mc);
+#pragma unroll
+  for (int i = 0; i < HP_ROWS; ++i) {
+    const long long r = by * static_cast<long long>(HP_BLOCK) + (threadIdx.x >> 4) + HP_THREADS / 16 * i;
+    if ((threadIdx.x & 15) == 0 && r < R) atomicMax(maxima + r, __float_as_uint(m[i]));   // (magnitudes order like their bits)
+  }
+  if (threadIdx.x < 16) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const long long c = bx * static_cast<long long>(HP_BLOCK) + threadIdx.x * 8 + j;
+      if (c < C) atomicMax(maxima + R + c, __float_as_uint(mc[j]));
+    }
+  }
+}
+__global__ void __launch_bounds__(HP_THREADS, 2) weight_panels_kernel(const GroupedGateRows f, const HalfPanels p, const unsigned int *maxima, float *scale) {
+  grid_dependency_wait();
+  grid_dependency_release();
+  unsigned by, bx;
+  half_block_of(p.C, blockIdx.x, by, bx);
+  float v[HP_ROWS][8], fc[8];
+  half_load_block(f, p.R, p.C, by, bx, v);
+  const long long c = bx * static_cast<long long>(HP_BLOCK) + (threadIdx.x & 15) * 8;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int e = c + j < p.C ? half_exponent(__uint_as_float(maxima[p.R + c + j])) : 0;
+    fc[j] = pow2(-e);
+    if (by == 0 && threadIdx.x < 16 && c + j < p.C) scale[p.R + c + j] = pow2(e);
+  }
+#pragma unroll
+  for (int i = 0; i < HP_ROWS; ++i) {
+    const long long r = by * static_cast<long long>(HP_BLOCK) + (threadIdx.x >> 4) + HP_THREADS / 16 * i;
+    if (r >= p.R) continue;
+    const int e = half_exponent(__uint_as_float(maxima[r]));
+    if (bx == 0 && (threadIdx.x & 15) == 0) scale[r] = pow2(e);
+    if (c >= p.pitch) continue;
+    const float fr = pow2(-e);
+    float s[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s[j] = v[i][j] * fr;
+    half_store8(p, p.rows, r, c, s);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s[j] = v[i][j] * fc[j];
+    half_store8(p, p.cols, r, c, s);
+  }
+}
 // rows of `src` shifted by `shift` rows, zeros where there is none
 struct ShiftedRows {
   const float *src;
@@ -413,11 +478,12 @@ static bool vec8(const float *p, long long a, long long b = 0) { return ((reinte
 // ---------------------------------------------------------------------------------------------------------
 // forward
 // ---------------------------------------------------------------------------------------------------------
-static int prepare_input(myea_b200_net *net, LstmPlan *P, const float *input, long long rows, long long n_in) {
-  if (P->x_src == input) return MYEA_OK;
-  P->x = half_panels_at(P->x_mem, rows, n_in);
+static int prepare_input(myea_b200_net *net, LstmPlan *P, const float *input, long long rows, long long n_in, int reading) {
+  if (P->x_src == input && P->x_reading == reading) return MYEA_OK;
+  P->x = half_panels_at(P->x_mem, rows, n_in, reading);
   LRC(half_split(net->ctx, input, n_in, P->x));
   P->x_src = input;
+  P->x_reading = reading;
   return MYEA_OK;
 }
 
@@ -428,7 +494,7 @@ int lstm_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long
   const long long T = net->T, B = net->B, rows = T * B, C = P->C, ldh = L.n_out;
   const BlockOffsets off = block_offsets(n_in, C);
   P->x_src = nullptr;
-  P->dg_all_valid[0] = P->dg_all_valid[1] = false;
+  P->dg_all_reading[0] = P->dg_all_reading[1] = 0;
   // input projection of all steps: gates_in = x W_in^T + b, columns [z | i | f | o]
   if (P->w_in_mem[0] == nullptr) {  // the four gates (of both directions) in one launch, straight from the blocks
     DirectItem items[8];
@@ -448,14 +514,13 @@ int lstm_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long
       for (int i = 0; i < n; ++i) LRC(gemm_nt(ctx, items[i].A, items[i].B, items[i].epi, net->scratch));
     }
   } else {
-    LRC(prepare_input(net, P, input, rows, n_in));
+    LRC(prepare_input(net, P, input, rows, n_in, HALF_ROWS));
     for (int d = 0; d < P->dirs; ++d) {
       if (!L.w_fresh) {
         RowSegments seg;
         seg.seg_rows = C;
         seg.seg_off[0] = off.z_in;
         for (int g = 0; g < 3; ++g) seg.seg_off[g + 1] = off.in[g];
-        P->w_in[d] = half_panels_at(P->w_in_mem[d], 4 * C, n_in);
         LRC(half_split(ctx, net->params + P->d[d].w_base, P->stride, P->w_in[d], &seg));
       }
       Epilogue e;
@@ -481,9 +546,12 @@ int lstm_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long
       lstm_gather_peepholes_kernel<<<static_cast<unsigned>((C + 255) / 256), 256, 0, ctx.stream>>>(w + off.peep, P->stride, C, P->peep_compact + static_cast<size_t>(d) * 3 * C);
       ctx.end(TC_RECURRENT);
       ctx.begin(TC_SPLIT);
-      GroupedGateRows src{w, P->stride, {rec[0], rec[1], rec[2], rec[3]}, C, vec8(w, P->stride, rec[0] | rec[1] | rec[2] | rec[3])};
-      half_produce(ctx, src, P->w_rec[d]);
-      ctx.end(TC_SPLIT);
+      const GroupedGateRows src{w, P->stride, {rec[0], rec[1], rec[2], rec[3]}, C, vec8(w, P->stride, rec[0] | rec[1] | rec[2] | rec[3])};
+      const dim3 grid(half_blocks(P->G, C)), block(HP_THREADS);
+      if (cudaMemsetAsync(P->w_rec_max, 0, static_cast<size_t>(P->G + C) * sizeof(unsigned int), ctx.stream) != cudaSuccess) return MYEA_E_CUDA;
+      launch_dependent(ctx, weight_extents_kernel, grid, block, 0, src, P->G, C, P->w_rec_max);
+      launch_dependent(ctx, weight_panels_kernel, grid, block, 0, src, P->w_rec[d], static_cast<const unsigned int *>(P->w_rec_max), P->w_rec_scale[d]);
+      ctx.end(TC_SPLIT, 2);
       LRC(lstm_persistent_forward(net, L, d, zone));
     }
     return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
@@ -516,7 +584,7 @@ int lstm_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long
         er.C = P->s_rec;
         er.ldc = 4 * C;
         if (P->step_mem != nullptr) {
-          const HalfPanels ph = half_panels_at(P->step_mem, B, C);
+          const HalfPanels ph = half_panels_at(P->step_mem, B, C, HALF_ROWS);
           LRC(half_split(ctx, h_prev, ldh, ph));
           LRC(half_gemm(ctx, half_rows(ph), half_rows(P->w_rec[d]), er));
         } else {
@@ -553,7 +621,7 @@ int lstm_backward(myea_b200_net *net, LayerPlan &L) {
   Context &ctx = net->ctx;
   const long long T = net->T, B = net->B, C = P->C, ldh = L.n_out, n_in = P->n_in;
   const BlockOffsets off = block_offsets(n_in, C);
-  P->dg_all_valid[0] = P->dg_all_valid[1] = false;
+  P->dg_all_reading[0] = P->dg_all_reading[1] = 0;
   if (P->resident != nullptr) {
     const long long rec[4] = {off.z_rec, off.rec[0], off.rec[1], off.rec[2]};
     return lstm_resident_run(net, L, 2, false, rec, off.peep);
@@ -576,7 +644,7 @@ int lstm_backward(myea_b200_net *net, LayerPlan &L) {
         e.ldc = ldh;
         e.accumulate = 1;
         if (P->step_mem != nullptr) {
-          const HalfPanels pd = half_panels_at(P->step_mem, B, 4 * C);
+          const HalfPanels pd = half_panels_at(P->step_mem, B, 4 * C, HALF_ROWS);
           LRC(half_split(ctx, dg, 4 * C, pd));
           LRC(half_gemm(ctx, half_rows(pd), half_cols(P->w_rec[d]), e));
         } else {
@@ -606,12 +674,13 @@ int lstm_backward(myea_b200_net *net, LayerPlan &L) {
 }
 
 // the gate errors of all steps as panels: read through their rows by the error to the layer below, through their columns by
-// the weight derivatives
-static int prepare_gate_errors(myea_b200_net *net, LstmPlan *P, int d, long long rows) {
-  if (P->dg_all_valid[d]) return MYEA_OK;
-  P->dg_all[d] = half_panels_at(P->dg_all_mem[d], rows, 4 * P->C);
+// the weight derivatives.  One after the other in the same memory: both at once would double the largest buffer of a layer, and
+// clearing it is most of what creating a handle costs; the second pass over the gate errors is 0.5 % of a step.
+static int prepare_gate_errors(myea_b200_net *net, LstmPlan *P, int d, long long rows, int reading) {
+  if (P->dg_all_reading[d] == reading) return MYEA_OK;
+  P->dg_all[d] = half_panels_at(P->dg_all_mem[d], rows, 4 * P->C, reading);
   LRC(half_split(net->ctx, P->d[d].dgates, 4 * P->C, P->dg_all[d]));
-  P->dg_all_valid[d] = true;
+  P->dg_all_reading[d] = reading;
   return MYEA_OK;
 }
 
@@ -645,7 +714,7 @@ int lstm_backward_to_input(myea_b200_net *net, LayerPlan &L, float *prev_deriv, 
       if (ctx.gemm_engine == 0) LRC(direct_gemm(ctx, &it, 1));
       else LRC(gemm_nt(ctx, it.A, it.B, e, GemmScratch{}));
     } else {
-      LRC(prepare_gate_errors(net, P, d, rows));
+      LRC(prepare_gate_errors(net, P, d, rows, HALF_ROWS));
       LRC(half_gemm(ctx, half_rows(P->dg_all[d]), half_cols(P->w_in[d]), e));
     }
   }
@@ -695,8 +764,8 @@ int lstm_update_derivative_weight(myea_b200_net *net, LayerPlan &L, const float 
       }
     } else {
       // the four gates in one contraction: row g*C + c of the product lands in block c at gate g's offset
-      LRC(prepare_input(net, P, input, rows, n_in));
-      LRC(prepare_gate_errors(net, P, d, rows));
+      LRC(prepare_input(net, P, input, rows, n_in, HALF_COLS));
+      LRC(prepare_gate_errors(net, P, d, rows, HALF_COLS));
       Epilogue e;
       e.C = gw;
       e.ldc = P->stride;
@@ -707,7 +776,7 @@ int lstm_update_derivative_weight(myea_b200_net *net, LayerPlan &L, const float 
       LRC(half_gemm(ctx, half_cols(P->dg_all[d]), half_cols(P->x), e));
       if (T > 1) {
         // recurrent weights over all rows too: the outputs shifted by one step, zeros at the direction's first step
-        const HalfPanels hs = half_panels_at(P->h_shift_mem[d], rows, C);
+        const HalfPanels hs = half_panels_at(P->h_shift_mem[d], rows, C, HALF_COLS);
         ctx.begin(TC_SPLIT);
         half_produce(ctx, ShiftedRows{L.values + d * C, ldh, shift, rows, vec8(L.values, ldh, C)}, hs);
         ctx.end(TC_SPLIT);

@@ -32,17 +32,23 @@ struct LstmPlan {
   // earlier in the direction [T*B, C] (zeros at its first step).
   float *x_mem = nullptr, *w_in_mem[2] = {nullptr, nullptr}, *dg_all_mem[2] = {nullptr, nullptr}, *h_shift_mem[2] = {nullptr, nullptr};
   HalfPanels x, w_in[2], dg_all[2];
-  const float *x_src = nullptr;   // the array the x panels were made from in this step
-  bool dg_all_valid[2] = {false, false};
+  // x and dg_all hold the panels of one reading at a time: through rows for the products on the way forward and back, through
+  // columns for the weight derivatives behind them
+  const float *x_src = nullptr;   // the array the x panels were made from in this step, and their reading
+  int x_reading = 0;
+  int dg_all_reading[2] = {0, 0};   // 0: not made in this step
   // Recurrent weights as panels: for the persistent walk [G, C] with the gate rows in the order (group of 16 cells, gate,
-  // cell), G = 64 * ceil(C / 16); for the walk by launches [4C, C] gate after gate, or (small products) gathered in fp32.
+  // cell), G = 64 * ceil(C / 16), and one power of two for ALL of K (w_rec_scale: [G] of the rows, [C] of the columns; the walk
+  // multiplies by it once per step); for the walk by launches [4C, C] gate after gate, or (small products) gathered in fp32.
   long long G = 0;
   float *w_rec_mem[2] = {nullptr, nullptr};
   HalfPanels w_rec[2];
+  float *w_rec_scale[2] = {nullptr, nullptr};
+  unsigned int *w_rec_max = nullptr;   // [G + C] largest magnitudes on the way to the scales
   // Ping-pong operand panels of the persistent walk, both buffers in one tensor of 2 * a_rows rows (a_rows: the batch rounded up to
-  // 128): h [.., C] with a fixed exponent, gate errors [.., G] with exponents [2][rows / 128][G / 64]
+  // 128): h [.., C] with a fixed exponent, gate errors [.., G] with powers of two [2][rows / 128][G / 64][128 rows]
   HalfPanels h_pan, dg_pan;
-  int *dg_exps = nullptr;
+  uint16_t *dg_scale = nullptr;
   float *step_mem = nullptr;   // walk by launches: panels of one step's operand
   LstmPersistent *persist = nullptr;
   LstmResident *resident = nullptr;  // the walk with resident weights (lstm_resident.cu), where it is the faster one

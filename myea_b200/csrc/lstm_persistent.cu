@@ -12,14 +12,14 @@
 //             a layer of 1024 cells needs), so that every SM streams a small share of the recurrent weights per step
 //             (they do not fit shared memory; they stay in L2)
 //   operands  half panels (half_panels.cuh): 4 bytes per element.  The gate rows of the weights are ordered (group of 16
-//             cells, gate, cell), one tensor for both passes: forward reads its rows, backward its columns.  h is at most 1 in
-//             magnitude and has a fixed exponent; the gate errors have one exponent per 128 batch rows and group of 16 cells -
-//             the 64 of K that one CTA produces and that one stage of a later step consumes
+//             cells, gate, cell): forward reads the tensor's rows, backward its columns, each with one power of two for all of
+//             their K.  h is at most 1 in magnitude and has a fixed exponent; the gate errors have one exponent per batch row and
+//             group of 16 cells - the 64 of K that one CTA produces and that one stage of a later step consumes
 //   warp 0    TMA producer: waits until the operand panels of the previous step are complete (step barrier), then
 //             loads its K slice of the step's operand (h of step s-1, or the gate errors of step s-1 of the walk) and
 //             of the recurrent weights, 64 of K per stage
 //   warp 1    one lane issues tcgen05.mma (h1*h0 + h0*h1 + h0*h0 per 16 of K) into a ring of accumulators in tensor memory
-//   warps 4-11 take the partial sums out of tensor memory, times the power of two of their operands' exponents, and exchange
+//   warps 4-11 take the partial sums out of tensor memory, backward times the power of two of their batch row, and exchange
 //             them inside the cluster: every thread pushes the columns that other CTAs finish into those CTAs' shared
 //             memory (st.async: the receiver's barrier counts the bytes, the sender waits for nothing) and keeps its own; the sums are added in slice order (bitwise
 //             repeatable).  Each thread then finishes 8 cells of one batch row: gates, peepholes, cell state, zoneout keep
@@ -68,7 +68,9 @@ template <int KIND> struct PsSmem {
   static constexpr int RECV_OFFSET = STAGES * STAGE_BYTES;
   static constexpr int RECV_BYTES = (PsShape<KIND>::SPLIT - 1) * 128 * (BN / PsShape<KIND>::SPLIT) * 4;  // one slot per peer
   static constexpr int BAR_OFFSET = RECV_OFFSET + RECV_BYTES;
-  static constexpr int TOTAL = BAR_OFFSET + 512 + 1024;                // barriers, peepholes, slack to align the base
+  static constexpr int SCALE_OFFSET = BAR_OFFSET + 512;                // powers of two of the columns this CTA finishes
+  static constexpr int MAX_OFFSET = SCALE_OFFSET + BN / PsShape<KIND>::SPLIT * 4;   // backward: largest gate errors, [2 halves][128 rows]
+  static constexpr int TOTAL = MAX_OFFSET + (KIND == 2 ? 2 * 128 * 4 : 0) + 1024;   // slack to align the base
   // Accumulators in tensor memory, used as a ring: the exchange warps read one while the tensor core fills the next ones.
   // Two sets: h0 * h0 and the cross products.
   static constexpr int TMEM_COLS = 512;
@@ -89,9 +91,8 @@ struct LstmSeq {
   long long a_rows = 0;         // rows of one of the two operand-panel buffers (a multiple of 128)
   long long kpa = 0;            // pitch of the operand panels
   uint16_t *a0 = nullptr, *a1 = nullptr;      // [2][a_rows][kpa]: step s reads buffer (s-1)&1 and writes buffer s&1
-  int *a_exp = nullptr;                       // backward: [2][tiles_m][num_kb] exponents of the gate errors
-  const int *w_exp = nullptr;                 // exponents of the weights, [gate rows / 128][cells / 128]
-  long long w_exp_pitch = 0;
+  uint16_t *a_scale = nullptr;                // backward: [2][tiles_m][num_kb][128] powers of two of the gate errors' rows
+  const float *w_scale = nullptr;             // powers of two of the weights: of the gate rows forward, of the cells backward
   const float *peep = nullptr;                // [3][C]
   const float *gates_in = nullptr;            // [T*B, 4C]
   float *act = nullptr, *cstate = nullptr, *cact = nullptr;
@@ -182,7 +183,8 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
   uint64_t *step_go = red_ready + 1;         // the producer has passed the step barrier
   uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(step_go + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
-  int *amax_s = reinterpret_cast<int *>(tmem_holder + 2);                  // backward: largest gate error of each warp (bits of a float)
+  float *scale_s = reinterpret_cast<float *>(smem + SM::SCALE_OFFSET);
+  float *max_s = reinterpret_cast<float *>(smem + SM::MAX_OFFSET);
   float *peep_s = reinterpret_cast<float *>(smem + SM::BAR_OFFSET + 320);  // [3][16] peepholes of this CTA's cells
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -337,6 +339,9 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
         const long long cell = cta_cell0 + (i & 15);
         peep_s[i] = cell < q.C ? q.peep[static_cast<long long>(i >> 4) * q.C + cell] : 0.f;
       }
+      // so do the powers of two of the columns it finishes (forward with the fixed one of h)
+      const long long col = static_cast<long long>(n0) + static_cast<long long>(rank) * W + i;
+      if (i < W) scale_s[i] = KIND == 1 ? (cta_cell0 < q.C ? q.w_scale[col] * pow2(LSTM_H_EXPONENT) : 0.f) : (col < q.C ? q.w_scale[col] : 0.f);
       ptx::named_barrier_sync(1, PS_EPI_THREADS);
     }
     using In = typename std::conditional<KIND == 1, LstmForwardIn, LstmBackwardIn>::type;
@@ -357,16 +362,15 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
         else lstm_backward_store_array8(pp, out, b, cell0, k);
       }
     };
-    // power of two of the product of accumulator c's operands; asked for one accumulator ahead
-    auto exponent_of = [&](int step, int c) {
-      const int kb = kb0 + c;
-      if constexpr (KIND == 1) return LSTM_H_EXPONENT + __ldg(q.w_exp + tile_n * q.w_exp_pitch + (kb >> 1));
-      else return __ldcg(q.a_exp + (static_cast<long long>((step - 1) & 1) * q.tiles_m + tile_m) * q.num_kb + kb) + __ldg(q.w_exp + (kb >> 1) * q.w_exp_pitch + (tile_n >> 1));
+    // backward: power of two of this thread's row in accumulator c; asked for one accumulator ahead
+    auto row_scale = [&](int step, int c) {
+      const uint16_t *at = q.a_scale + ((static_cast<long long>((step - 1) & 1) * q.tiles_m + tile_m) * q.num_kb + kb0 + c) * 128 + row;
+      return (static_cast<uint32_t>(__ldcg(at)) << 16) + (14u << 23);
     };
     for (int s = 0; s < q.T; ++s) {
       bool ok = true;
       const LstmStep p = step_view<KIND>(q, s);
-      int e_next = 0;
+      uint32_t next_scale = 0;
       In in;
       if (active) {
         // what the cell needs from global memory goes out before any wait; what this thread computed itself in the step
@@ -386,7 +390,7 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
         // operand stream: all at once, the 128 CTAs' stores kept its first copies waiting (4 of a forward step's 30 kcycles), and
         // stored while the step barrier is in flight they slowed the barrier down
         if (!ptx::mbar_wait_or_abort(step_go, static_cast<uint32_t>(s - 1) & 1u, abort_flag)) ok = false;
-        if (ok && my_kb > 0) e_next = exponent_of(s, 0);
+        if (KIND == 2 && ok && my_kb > 0) next_scale = row_scale(s, 0);
       }
       float rec[HW];
 #pragma unroll
@@ -403,12 +407,10 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
           for (int j = 0; j < HW; ++j) part[dd][j] = 0.f;
         for (int c = 0; c < my_kb; ++c, ++n) {
           const uint32_t a = n % ACCS;
-          const int e = e_next;
-          if (c + 1 < my_kb) e_next = exponent_of(s, c + 1);
+          const float sa = __uint_as_float(next_scale);
+          if (KIND == 2 && c + 1 < my_kb) next_scale = row_scale(s, c + 1);
           if (!ptx::mbar_wait_or_abort(&done_bar[n % DONE], (n / DONE) & 1u, abort_flag)) { ok = false; break; }
           ptx::tc_fence_after();
-          const int e1 = max(-126, min(127, e)), e2 = max(-126, min(127, e - e1));
-          const float s1 = pow2(e1), s2 = pow2(e2);
           const uint32_t tq = tmem_base + (static_cast<uint32_t>(qd * 32) << 16) + a * static_cast<uint32_t>(SM::ACC_COLS);
 #pragma unroll
           for (int dd = 1; dd <= S; ++dd) {
@@ -429,7 +431,7 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
                 float v = __uint_as_float(r[j / 8][j % 8]);
                 if constexpr (SETS == 2) v += __uint_as_float(x[j / 8][j % 8]);
                 float &t = part[dd - 1][k0 * 8 + j];
-                t = fmaf(e2 == 0 ? v : v * s2, s1, t);
+                t = KIND == 2 ? fmaf(v, sa, t) : t + v;
               }
             }
           }
@@ -473,6 +475,8 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
               for (int i = 0; i < HW / 4; ++i) { rec[4 * i] += v[i].x; rec[4 * i + 1] += v[i].y; rec[4 * i + 2] += v[i].z; rec[4 * i + 3] += v[i].w; }
             }
           }
+#pragma unroll
+          for (int i = 0; i < HW; ++i) rec[i] *= scale_s[(i >> 3) * 16 + half * 8 + (i & 7)];
         }
       }
       float m = 0.f;   // backward: this thread's largest gate error
@@ -489,22 +493,20 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
           }
         } else if (active) {
           lstm_backward_compute8(in, rec, p.b_c_prev != nullptr, out);
-          m = amax8(out.dz, amax8(out.di, amax8(out.df, amax8(out.d_o, 0.f))));
+#pragma unroll
+          for (int i = 0; i < 8; ++i) m = fmaxf(fmaxf(m, fmaxf(finite_abs(out.dz[i]), finite_abs(out.di[i]))), fmaxf(finite_abs(out.df[i]), finite_abs(out.d_o[i])));
         }
         pending = true;
       }
       if constexpr (KIND == 2) {
         if (p.p_h0 != nullptr) {
-          // one exponent for this CTA's 128 rows x 16 cells x 4 gates (a warp that gave up takes part: the barrier is for all)
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-          if (lane == 0) amax_s[warp - PS_EPI_WARP0] = __float_as_int(m);
+          // one exponent per row for this CTA's 16 cells x 4 gates (a warp that gave up takes part: the barrier is for all)
+          max_s[half * 128 + row] = m;
           ptx::named_barrier_sync(1, PS_EPI_THREADS);
-#pragma unroll
-          for (int w = 0; w < 8; ++w) m = fmaxf(m, __int_as_float(amax_s[w]));
-          const int e = half_exponent(m);
+          const int e = half_exponent(fmaxf(m, max_s[(half ^ 1) * 128 + row]));
           const int group = static_cast<int>(cta_cell0 >> 4);
-          if (warp == PS_EPI_WARP0 && lane == 0 && group < q.num_kb) q.a_exp[(static_cast<long long>(s & 1) * q.tiles_m + tile_m) * q.num_kb + group] = e;
+          if (half == 0 && group < q.num_kb)
+            q.a_scale[((static_cast<long long>(s & 1) * q.tiles_m + tile_m) * q.num_kb + group) * 128 + row] = half_scale_bits(e);
           if (active && ok) lstm_store_gate_panels8(p, out, pow2(-e), b, static_cast<long long>(group) * 64 + half * 8);
         }
       }
@@ -626,12 +628,12 @@ static int launch(myea_b200_net *net, LstmSeq &q, long long K, const HalfPanels 
   Context &ctx = net->ctx;
   // operand panels: both ping-pong buffers in one map (row coordinate = buffer * a_rows + tile row)
   HalfOperand a;
-  a.p.h0 = q.a0; a.p.h1 = q.a1; a.p.R = 2 * q.a_rows; a.p.C = K; a.p.pitch = q.kpa;
+  a.p.R = 2 * q.a_rows; a.p.C = K; a.p.pitch = q.kpa;
   a.rows = a.p.R; a.k = K;
   const HalfOperand b = KIND == 1 ? half_rows(w) : half_cols(w);
   CUtensorMap maps[4];
-  if (!make_half_map(&maps[0], a, a.p.h0, 128) || !make_half_map(&maps[1], a, a.p.h1, 128) || !make_half_map(&maps[2], b, w.h0, PsShape<KIND>::BN) ||
-      !make_half_map(&maps[3], b, w.h1, PsShape<KIND>::BN))
+  if (!make_half_map(&maps[0], a, q.a0, 128) || !make_half_map(&maps[1], a, q.a1, 128) || !make_half_map(&maps[2], b, b.reading().h0, PsShape<KIND>::BN) ||
+      !make_half_map(&maps[3], b, b.reading().h1, PsShape<KIND>::BN))
     return MYEA_E_CUDA;
   if (cudaMemsetAsync(q.sync, 0, (q.tiles_m + 1) * sizeof(unsigned int), ctx.stream) != cudaSuccess) return MYEA_E_CUDA;
   cudaLaunchConfig_t cfg = {};
@@ -660,8 +662,6 @@ static void common_args(myea_b200_net *net, LayerPlan &L, int dir, LstmSeq &q) {
   q.tiles_m = P->persist->tiles_m;
   q.ldh = L.n_out;
   q.a_rows = P->persist->a_rows;
-  q.w_exp = P->w_rec[dir].exps;
-  q.w_exp_pitch = P->w_rec[dir].exp_r;
   q.peep = P->peep_compact + static_cast<size_t>(dir) * 3 * P->C;
   q.sync = P->persist->sync;
   q.error_flag = net->ctx.d_error_flag;
@@ -678,7 +678,8 @@ int lstm_persistent_forward(myea_b200_net *net, LayerPlan &L, int dir, bool zone
   q.num_kb = static_cast<int>((P->C + PS_BK - 1) / PS_BK);
   q.kb_per = (q.num_kb + q.split - 1) / q.split;
   q.kpa = P->h_pan.pitch;
-  q.a0 = P->h_pan.h0; q.a1 = P->h_pan.h1;
+  q.a0 = P->h_pan.rows.h0; q.a1 = P->h_pan.rows.h1;
+  q.w_scale = P->w_rec_scale[dir];
   q.gates_in = D.gates_in; q.act = D.act; q.cstate = D.cstate; q.cact = D.cact;
   q.values = L.values + dir * P->C;
   q.zone_state = zoneout ? D.zone_state : nullptr;
@@ -697,8 +698,9 @@ int lstm_persistent_backward(myea_b200_net *net, LayerPlan &L, int dir) {
   q.num_kb = static_cast<int>(P->G / PS_BK);
   q.kb_per = (q.num_kb + q.split - 1) / q.split;
   q.kpa = P->dg_pan.pitch;
-  q.a0 = P->dg_pan.h0; q.a1 = P->dg_pan.h1;
-  q.a_exp = P->dg_exps;
+  q.a0 = P->dg_pan.rows.h0; q.a1 = P->dg_pan.rows.h1;
+  q.a_scale = P->dg_scale;
+  q.w_scale = P->w_rec_scale[dir] + P->G;
   q.act = D.act; q.cstate = D.cstate; q.cact = D.cact;
   q.deriv = L.deriv + dir * P->C;
   q.dgates = D.dgates; q.dcstate = D.dcstate;

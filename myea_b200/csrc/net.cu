@@ -292,10 +292,15 @@ static int allocate_buffers(myea_b200_net *net) {
       else L.errors = L.deriv;
       if (net->ctx.gemm_engine == 0 && !direct_gemm_suits(net->ctx, rows, L.n_out, L.n_in)) {
         L.shared_panels = true;
-        RC(dev_alloc(net, &L.in_panel_mem, half_panel_floats(rows, L.n_in), false));
-        RC(dev_alloc(net, &L.w_panel_mem, half_panel_floats(L.n_out, L.n_in), false));
-        RC(dev_alloc(net, &L.d_panel_mem, half_panel_floats(rows, L.n_out), false));
-        L.w_pan = half_panels_at(L.w_panel_mem, L.n_out, L.n_in);
+        // (no error is propagated below the first layer: its weights are not read through their columns, its errors not
+        // through their rows)
+        const bool propagates = L.input_layer > 0;
+        L.w_readings = propagates ? HALF_BOTH : HALF_ROWS;
+        L.d_readings = propagates ? HALF_BOTH : HALF_COLS;
+        RC(dev_alloc(net, &L.in_panel_mem, half_panel_floats(rows, L.n_in, HALF_BOTH), false));
+        RC(dev_alloc(net, &L.w_panel_mem, half_panel_floats(L.n_out, L.n_in, L.w_readings), false));
+        RC(dev_alloc(net, &L.d_panel_mem, half_panel_floats(rows, L.n_out, L.d_readings), false));
+        L.w_pan = half_panels_at(L.w_panel_mem, L.n_out, L.n_in, L.w_readings);
       }
       scratch = std::max(scratch, gemm_scratch_floats(rows, L.n_out, L.n_in));   // forward
       scratch = std::max(scratch, gemm_scratch_floats(rows, L.n_in, L.n_out));   // backward data
@@ -562,9 +567,12 @@ static int fc_prepare_weights(myea_b200_net *net, LayerPlan &L) {
   return MYEA_OK;
 }
 
+// forward reads a layer's input through its rows, the weight derivative through its columns
+static int input_readings(const myea_b200_net *net) { return net->training ? HALF_BOTH : HALF_ROWS; }
+
 HalfPanels *fc_input_sink(myea_b200_net *net, LayerPlan &L, const float *input, long long rows) {
   if (L.type != MYEA_LAYER_FULLY_CONNECTED || !fc_uses_shared_panels(net, L, rows)) return nullptr;
-  L.in_pan = half_panels_at(L.in_panel_mem, rows, L.n_in);
+  L.in_pan = half_panels_at(L.in_panel_mem, rows, L.n_in, input_readings(net));
   L.in_ready_src = input;
   L.in_ready_rows = rows;
   return &L.in_pan;
@@ -572,7 +580,7 @@ HalfPanels *fc_input_sink(myea_b200_net *net, LayerPlan &L, const float *input, 
 
 HalfPanels *fc_error_sink(myea_b200_net *net, LayerPlan &L, long long rows) {
   if (!L.shared_panels || !L.in_valid || !fc_uses_shared_panels(net, L, rows)) return nullptr;
-  L.d_pan = half_panels_at(L.d_panel_mem, rows, L.n_out);
+  L.d_pan = half_panels_at(L.d_panel_mem, rows, L.n_out, L.d_readings);
   L.d_valid = true;
   return &L.d_pan;
 }
@@ -584,7 +592,7 @@ int fc_product_forward(myea_b200_net *net, LayerPlan &L, const float *input, lon
   if (fc_uses_shared_panels(net, L, rows)) {
     const bool tr = net->training;
     if (!(L.in_ready_src == input && L.in_ready_rows == rows)) {  // else the kernel that produced `input` has written these panels already
-      L.in_pan = half_panels_at(L.in_panel_mem, rows, L.n_in);
+      L.in_pan = half_panels_at(L.in_panel_mem, rows, L.n_in, input_readings(net));
       RC(half_split(net->ctx, input, L.n_in, L.in_pan));
     }
     L.in_ready_src = nullptr;
@@ -610,9 +618,9 @@ static bool fc_runs_direct(const myea_b200_net *net, const LayerPlan &L, long lo
 }
 
 int fc_product_backward(myea_b200_net *net, LayerPlan &N, long long rows, const Epilogue &e) {
-  if (N.shared_panels && N.w_valid) {
+  if (N.shared_panels && N.w_valid && N.d_readings == HALF_BOTH) {
     if (!N.d_valid) {  // (the kernel that produced N's errors may have written them already)
-      N.d_pan = half_panels_at(N.d_panel_mem, rows, N.n_out);
+      N.d_pan = half_panels_at(N.d_panel_mem, rows, N.n_out, N.d_readings);
       RC(half_split(net->ctx, N.errors, N.n_out, N.d_pan));
     }
     N.d_valid = true;
@@ -1235,7 +1243,7 @@ int fc_update_derivative_weight(myea_b200_net *net, LayerPlan &L, const float *i
   }
   if (L.shared_panels && L.in_valid && input == L.in_src) {
     if (!L.d_valid) {  // no error propagation below this layer (first hidden layer)
-      L.d_pan = half_panels_at(L.d_panel_mem, rows, L.n_out);
+      L.d_pan = half_panels_at(L.d_panel_mem, rows, L.n_out, L.d_readings);
       RC(half_split(net->ctx, L.errors, L.n_out, L.d_pan));
     }
     RC(half_gemm(net->ctx, half_cols(L.d_pan), half_cols(L.in_pan), e));

@@ -36,11 +36,12 @@ struct LayerPlan {
   uint8_t *shake_mask = nullptr;      // [B]
   float *shake_alpha = nullptr, *shake_beta = nullptr;  // [B, n_out]
   long long norm_unit_offset = 0;     // units of earlier layers in the normalized-unit run
-  // Operand panels shared by the three contractions of a large fully connected layer: one set per tensor and step serves
-  // both of its readings.  input: forward (rows) and dW (columns); weights: forward (rows) and error propagation (columns);
-  // errors: error propagation (rows) and dW (columns).
+  // Operand panels shared by the three contractions of a large fully connected layer, made once per tensor and step.
+  // input: forward (rows) and dW (columns); weights: forward (rows) and error propagation (columns); errors: error
+  // propagation (rows) and dW (columns).
   bool shared_panels = false;
   float *in_panel_mem = nullptr, *w_panel_mem = nullptr, *d_panel_mem = nullptr;
+  int w_readings = 0, d_readings = 0;
   HalfPanels in_pan, w_pan, d_pan;  // as of the step in flight (a short batch has fewer rows)
   bool in_valid = false, w_valid = false, d_valid = false;
   bool w_fresh = false;   // the weight panels (of an LSTM layer: all that its forward pass lays out from its weights) match the parameters

@@ -135,15 +135,14 @@ int optimizer_update(Context &ctx, const OptLaunch &o, const OptArrays &a, size_
 }
 
 // The update of weights that contractions read as operand panels: a CTA updates a block of 128 x 128 weights, keeps the new
-// values, finds their exponent and writes the panels of the next step along, which otherwise cost a pass of their own over the
-// weights (4 bytes read and 4 written per weight); the derivatives are not zeroed (4 bytes less), the next accumulation
+// values, finds the exponents of their rows and columns and writes the panels of the next step along, which otherwise cost a pass
+// of their own over the weights (4 bytes read and 8 written per weight); the derivatives are not zeroed (4 bytes less), the next accumulation
 // overwrites them instead of adding to them (4 bytes less again).  Bound by HBM, so by loads in flight: a thread has 8 elements
 // of all arrays on the way, 1024 threads per SM; the new weights wait in shared memory (64 KB) because in registers they leave
-// room for half the threads (134 M weights, Adam: 686 us, 6.26 TB/s, where update and splits were 720 + 200 us; with the
-// weights in registers and 512 threads per SM 1770 us).
+// room for half the threads (138 M weights, Adam: 764 us, 36 bytes per weight at 6.5 TB/s; with the weights in registers and 512
+// threads per SM 1770 us at 32 bytes per weight).
 constexpr int OPT_LAYERS = 32;
-constexpr int OPT_THREADS = 512;
-constexpr int OPT_ROWS = HP_BLOCK * 16 / OPT_THREADS;   // rows per thread: 8 columns of rows tid / 16 + 32 i
+constexpr int OPT_THREADS = HP_THREADS, OPT_ROWS = HP_ROWS;   // 8 columns of rows tid / 16 + 32 i
 constexpr int OPT_SMEM = HP_BLOCK * HP_BLOCK * 4;
 struct OptPanelTable {
   OptPanelLayer l[OPT_LAYERS];
@@ -163,7 +162,6 @@ __global__ void __launch_bounds__(OPT_THREADS, 2) optimizer_panels_kernel(const 
   const int across = static_cast<int>((p.C + HP_BLOCK - 1) / HP_BLOCK), by = block / across, bx = block - by * across;
   const long long c = bx * static_cast<long long>(HP_BLOCK) + (threadIdx.x & 15) * 8;
   const long long r0 = by * static_cast<long long>(HP_BLOCK) + (threadIdx.x >> 4);
-  float amax = 0.f;
 #pragma unroll 1
   for (int i = 0; i < OPT_ROWS; ++i) {
     const long long r = r0 + OPT_THREADS / 16 * i;
@@ -183,22 +181,17 @@ __global__ void __launch_bounds__(OPT_THREADS, 2) optimizer_panels_kernel(const 
       if (adam_like) { st8(a.m + at, m, 8, true); st8(a.v + at, v, 8, true); }
       if (HAS_VHAT) st8(a.vhat + at, vh, 8, true);
       if (HAS_PREV) st8(a.prev + at, pv, 8, true);
-      amax = amax8(w, amax);
     }
     kept[(2 * i) * OPT_THREADS + threadIdx.x] = make_float4(w[0], w[1], w[2], w[3]);
     kept[(2 * i + 1) * OPT_THREADS + threadIdx.x] = make_float4(w[4], w[5], w[6], w[7]);
   }
-  const int e = half_block_exponent<OPT_THREADS>(amax);
-  if (threadIdx.x == 0) p.exps[by * p.exp_r + bx * p.exp_c] = e;
-  if (c >= p.pitch) return;
-  const float s = pow2(-e);
+  float v[OPT_ROWS][8];
 #pragma unroll
   for (int i = 0; i < OPT_ROWS; ++i) {
-    const long long r = r0 + OPT_THREADS / 16 * i;
     const float4 x = kept[(2 * i) * OPT_THREADS + threadIdx.x], y = kept[(2 * i + 1) * OPT_THREADS + threadIdx.x];
-    const float w[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-    if (r < p.R) half_store8(p, r, c, w, s);
+    v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w; v[i][4] = y.x; v[i][5] = y.y; v[i][6] = y.z; v[i][7] = y.w;
   }
+  half_store_block(p, by, bx, v);
 }
 template <bool HAS_VHAT, bool HAS_PREV>
 static int launch_optimizer_panels(Context &ctx, int blocks, const OptLaunch &o, const OptArrays &a, const OptPanelTable &t) {

@@ -160,3 +160,64 @@ def test_lstm_of_one_input_or_one_cell(n_in, H, out, T, B, bidirectional):
     layers = [capi.fc(n_in), capi.lstm(H, bidirectional=bidirectional), capi.fc(out, capi.AF_LINEAR)]
     _step(workloads.Workload("narrow lstm", capi.net(layers, B, T=T, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE),
                              capi.opt(capi.OPT_GD, gd_lr=0.01 / B, momentum=0.9), n_in, out, False, layers))
+
+
+@pytest.mark.parametrize("spread_of", ["samples", "features"])
+def test_panels_of_a_step_with_units_of_different_magnitude(spread_of):
+    """samples or features, and units, spread over 2^+-18 (the largest weight derivative is 2^120 then) on a network whose products
+    read operand panels: outputs, errors, weight derivatives and the outputs behind an update, each against float64 at its own
+    scale (|row| |column| of the operands)"""
+    n_in, H, n_out, B = 1000, 1096, 904, 700
+    rng = np.random.default_rng(11)
+    spread = lambda *shape: 2.0 ** rng.uniform(-18, 18, shape)
+    layers = [capi.fc(n_in), capi.fc(H, capi.AF_LINEAR), capi.fc(n_out, capi.AF_LINEAR)]
+    desc, opt = capi.net(layers, B, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE), capi.opt(capi.OPT_GD, gd_lr=2.0 ** -60)
+    X = (rng.standard_normal((1, B, n_in)) * (spread(B, 1) if spread_of == "samples" else spread(n_in))).astype(np.float32)
+    W1 = (rng.standard_normal((H, n_in)) * spread(H, 1)).astype(np.float32)
+    W2 = (rng.standard_normal((n_out, H)) * spread(n_out, 1)).astype(np.float32)
+    gpu = Net(desc, opt)
+    p = np.zeros(gpu.P, np.float32)
+    at = [int(gpu.layer_index(l).first_connection_index) for l in (1, 2)]
+    p[at[0]:at[0] + W1.size], p[at[1]:at[1] + W2.size] = W1.ravel(), W2.ravel()
+    gpu.set(capi.BUF_PARAMETERS, p)
+    gpu.forward(X); gpu.compute_error(np.zeros((1, B, n_out), np.float32)); gpu.backward(); gpu.update_derivative_weight()
+    norm = lambda a, axis: np.linalg.norm(a, axis=axis)
+
+    def check(got, a, b, bias=0.0):   # got = a b^T + bias, all in float64
+        scale = norm(a, 1)[:, None] * norm(b, 1)[None, :] + np.abs(bias)
+        assert (np.abs(got - a @ b.T - bias) / scale).max() < 5e-6
+
+    # every product against float64 on the operands the GPU itself computed
+    f64 = lambda a: np.asarray(a, np.float64)
+    x, h, y, g = f64(X[0]), f64(gpu.outputs(1)).reshape(B, H), f64(gpu.outputs(2)).reshape(B, n_out), f64(gpu.get(capi.BUF_DERIVATIVES))
+    check(h, x, f64(W1)); check(y, h, f64(W2))
+    check(g[at[1]:at[1] + W2.size].reshape(n_out, H), y.T, h.T)
+    d1 = f64(gpu.errors(1)).reshape(B, H)
+    check(d1, y, f64(W2).T)
+    check(g[at[0]:at[0] + W1.size].reshape(H, n_in), d1.T, x.T)
+    gpu.update_parameter()
+    q = gpu.get(capi.BUF_PARAMETERS)
+    gpu.forward(X, training=False)
+    bias = int(gpu.layer_index(1).first_bias_connection_index)
+    check(f64(gpu.outputs(1)).reshape(B, H), x, f64(q[at[0]:at[0] + W1.size]).reshape(H, n_in), f64(q[bias:bias + H]))
+    gpu.synchronize()
+    gpu.close()
+
+
+@pytest.mark.parametrize("bidirectional", [False, True])
+def test_lstm_errors_of_samples_of_different_magnitude(bidirectional):
+    """the tensor-core walk back through time: samples whose errors lie 2^36 apart, each against float64 at its own scale (fp32
+    gates and three steps of products leave about 1e-6)"""
+    H, B, T = (1024, 136, 4) if not bidirectional else (512, 300, 3)
+    layers = [capi.fc(9), capi.lstm(H, bidirectional=bidirectional), capi.fc(H, capi.AF_LINEAR)]
+    wl = workloads.Workload("samples", capi.net(layers, B, T=T, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE), capi.opt(capi.OPT_GD, gd_lr=1e-6), 9, H, False, layers)
+    gpu, cpu = Net(wl.desc, wl.opt), myea_oracle.OracleNet(wl.desc, wl.opt, dtype=np.float64)
+    X, Y = wl.batch(5)
+    Y = (Y + 1.0) * (2.0 ** np.random.default_rng(1).uniform(0, 36, (1, B, 1))).astype(np.float32)
+    for net in (gpu, cpu):
+        wl.materialize(net)
+        net.forward(X); net.compute_error(Y); net.backward()
+    got, want = np.asarray(gpu.errors(1), np.float64), np.asarray(cpu.layers[1].dh, np.float64).reshape(T, B, -1)
+    assert (np.linalg.norm(got - want, axis=2) / np.linalg.norm(want, axis=2)).max() < 1e-5
+    gpu.synchronize()
+    gpu.close()
