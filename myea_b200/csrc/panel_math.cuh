@@ -91,7 +91,8 @@ __device__ __forceinline__ void lstm_forward_compute8(const LstmForwardIn &in, c
     o.h[i] = hh;
   }
 }
-// h is at most 1 in magnitude: its panels have one fixed exponent
+// h is at most 1 in magnitude and known to 2^-24 of that (tanh_cell is a difference from 1): its panels have one fixed exponent and a
+// step of 2^-39
 constexpr int LSTM_H_EXPONENT = -14;
 // what the NEXT step's contraction reads: h as operand panels
 __device__ __forceinline__ void lstm_store_h_panels8(const LstmStep &p, const float (&h)[8], long long b, long long c0) {
