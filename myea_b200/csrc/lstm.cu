@@ -13,12 +13,14 @@
 // Zoneout (forward only, as in the reference): where the state mask is false c = c_prev (0 at the first step), where
 // the output mask is false h = h_prev (0 at the first step); the backward pass ignores the masks.
 //
-// Mapping to the GPU: the four gate matrices stay in the reference's interleaved per-block parameter layout and are read
-// through strided operands into fused K-major panels ([4C, in], [4C, C] and their transposes), so the input projection
-// of all T steps is ONE tensor-core contraction [T*B, in] x [in, 4C], each recurrent step is one [B, C] x [C, 4C]
-// contraction plus one fused cell kernel (gate nonlinearities, peepholes, cell-state recurrence, zoneout select), each
-// BPTT step is one [B, 4C] x [4C, C] contraction accumulated into the output error plus one fused cell-backward kernel,
-// and the weight derivatives are contractions over K = T*B.  Bias and peephole derivatives are column reductions.
+// Mapping to the GPU: the four gate matrices stay in the reference's interleaved per-block parameter layout.  The input
+// projection of all T steps is ONE contraction [T*B, in] x [in, 4C] and the weight derivatives are contractions over K = T*B, for
+// small products straight from the blocks (one launch for all gates), for large ones from operand panels (half_panels.cuh) that
+// are split out of them.  The recurrent part is serial: one launch walks all steps of a layer where the weights fit shared
+// memory (lstm_resident.cu) or the tiles of a step fit the chip (lstm_persistent.cu); else a [B, C] x [C, 4C] contraction and a
+// fused cell kernel (gate nonlinearities, peepholes, cell-state recurrence, zoneout select) per step, and on the way back a
+// [B, 4C] x [4C, C] contraction accumulated into the output error and a fused cell-backward kernel.  Bias and peephole
+// derivatives are column reductions.
 #include "half_panels.cuh"
 #include "lstm.cuh"
 #include "panel_math.cuh"
@@ -301,27 +303,33 @@ int lstm_create(myea_b200_net *net, LayerPlan &L) {
   size_t need = static_cast<size_t>(P->dirs) * 4 * C * std::max<long long>(L.n_in, C);  // gathered weights
   LRC(lstm_persistent_plan(net, L));
   LRC(lstm_resident_plan(net, L));
-  if (tensor && P->resident == nullptr && lstm_persistent_ready(P)) {
+  const bool walks[2] = {!P->resident_pass[0], !P->resident_pass[1]};   // passes that read the weights from what is laid out here
+  const int w_readings = (walks[0] ? HALF_ROWS : 0) | (walks[1] ? HALF_COLS : 0);
+  if (tensor && w_readings != 0 && lstm_persistent_ready(P)) {
     LRC(lalloc(net, &P->peep_compact, static_cast<size_t>(P->dirs) * 3 * C));
     const long long a_rows = (net->B + 127) / 128 * 128;
     float *mem = nullptr;
-    LRC(lalloc(net, &mem, half_panel_floats(2 * a_rows, C, HALF_ROWS)));       // zero: rows past the batch stay zero for ever
-    P->h_pan = half_panels_at(mem, 2 * a_rows, C, HALF_ROWS);
-    LRC(lalloc(net, &mem, half_panel_floats(2 * a_rows, P->G, HALF_ROWS)));
-    P->dg_pan = half_panels_at(mem, 2 * a_rows, P->G, HALF_ROWS);
-    LRC(lalloc(net, &P->dg_scale, static_cast<size_t>(2 * a_rows * (P->G / 64))));
+    if (walks[0]) {
+      LRC(lalloc(net, &mem, half_panel_floats(2 * a_rows, C, HALF_ROWS)));       // zero: rows past the batch stay zero for ever
+      P->h_pan = half_panels_at(mem, 2 * a_rows, C, HALF_ROWS);
+    }
+    if (walks[1]) {
+      LRC(lalloc(net, &mem, half_panel_floats(2 * a_rows, P->G, HALF_ROWS)));
+      P->dg_pan = half_panels_at(mem, 2 * a_rows, P->G, HALF_ROWS);
+      LRC(lalloc(net, &P->dg_scale, static_cast<size_t>(2 * a_rows * (P->G / 64))));
+    }
     LRC(lalloc(net, &P->w_rec_max, static_cast<size_t>(P->G + C)));
     for (int d = 0; d < P->dirs; ++d) {
-      LRC(lalloc(net, &P->w_rec_mem[d], half_panel_floats(P->G, C, HALF_BOTH)));
-      P->w_rec[d] = half_panels_at(P->w_rec_mem[d], P->G, C, HALF_BOTH);
+      LRC(lalloc(net, &P->w_rec_mem[d], half_panel_floats(P->G, C, w_readings)));
+      P->w_rec[d] = half_panels_at(P->w_rec_mem[d], P->G, C, w_readings);
       LRC(lalloc(net, &P->w_rec_scale[d], static_cast<size_t>(P->G + C)));
     }
-  } else if (P->resident == nullptr) {
-    LRC(lalloc(net, &P->s_rec, net->B * 4 * C));
+  } else if (w_readings != 0) {
+    if (walks[0]) LRC(lalloc(net, &P->s_rec, net->B * 4 * C));
     if (tensor && !direct_gemm_suits(net->ctx, net->B, 4 * C, C)) {
       for (int d = 0; d < P->dirs; ++d) {
-        LRC(lalloc(net, &P->w_rec_mem[d], half_panel_floats(4 * C, C, HALF_BOTH)));
-        P->w_rec[d] = half_panels_at(P->w_rec_mem[d], 4 * C, C, HALF_BOTH);
+        LRC(lalloc(net, &P->w_rec_mem[d], half_panel_floats(4 * C, C, w_readings)));
+        P->w_rec[d] = half_panels_at(P->w_rec_mem[d], 4 * C, C, w_readings);
       }
       LRC(lalloc(net, &P->step_mem, half_panel_floats(net->B, 4 * C, HALF_ROWS)));
     } else {
@@ -449,10 +457,10 @@ __global__ void __launch_bounds__(HP_THREADS, 2) weight_panels_kernel(const Grou
     float s[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) s[j] = v[i][j] * fr;
-    half_store8(p, p.rows, r, c, s);
+    if (p.rows.h0 != nullptr) half_store8(p, p.rows, r, c, s);
 #pragma unroll
     for (int j = 0; j < 8; ++j) s[j] = v[i][j] * fc[j];
-    half_store8(p, p.cols, r, c, s);
+    if (p.cols.h0 != nullptr) half_store8(p, p.cols, r, c, s);
   }
 }
 // rows of `src` shifted by `shift` rows, zeros where there is none
@@ -485,6 +493,41 @@ static int prepare_input(myea_b200_net *net, LstmPlan *P, const float *input, lo
   P->x_src = input;
   P->x_reading = reading;
   return MYEA_OK;
+}
+
+// the recurrent weights as the walks that do not keep them resident read them; made by the first of them after the parameters
+// have changed
+static int lay_out_recurrent_weights(myea_b200_net *net, LstmPlan *P, const BlockOffsets &off) {
+  if (P->w_rec_fresh) return MYEA_OK;
+  Context &ctx = net->ctx;
+  const long long C = P->C, rec[4] = {off.z_rec, off.rec[0], off.rec[1], off.rec[2]};
+  for (int d = 0; d < P->dirs; ++d) {
+    const float *w = net->params + P->d[d].w_base;
+    if (lstm_persistent_ready(P)) {
+      ctx.begin(TC_RECURRENT);
+      lstm_gather_peepholes_kernel<<<static_cast<unsigned>((C + 255) / 256), 256, 0, ctx.stream>>>(w + off.peep, P->stride, C, P->peep_compact + static_cast<size_t>(d) * 3 * C);
+      ctx.end(TC_RECURRENT);
+      ctx.begin(TC_SPLIT);
+      const GroupedGateRows src{w, P->stride, {rec[0], rec[1], rec[2], rec[3]}, C, vec8(w, P->stride, rec[0] | rec[1] | rec[2] | rec[3])};
+      const dim3 grid(half_blocks(P->G, C)), block(HP_THREADS);
+      if (cudaMemsetAsync(P->w_rec_max, 0, static_cast<size_t>(P->G + C) * sizeof(unsigned int), ctx.stream) != cudaSuccess) return MYEA_E_CUDA;
+      launch_dependent(ctx, weight_extents_kernel, grid, block, 0, src, P->G, C, P->w_rec_max);
+      launch_dependent(ctx, weight_panels_kernel, grid, block, 0, src, P->w_rec[d], static_cast<const unsigned int *>(P->w_rec_max), P->w_rec_scale[d]);
+      ctx.end(TC_SPLIT, 2);
+    } else if (P->step_mem != nullptr) {
+      RowSegments seg;
+      seg.seg_rows = C;
+      for (int g = 0; g < 4; ++g) seg.seg_off[g] = rec[g];
+      LRC(half_split(ctx, w, P->stride, P->w_rec[d], &seg));
+    } else {
+      ctx.begin(TC_RECURRENT);
+      lstm_gather_weights_kernel<<<static_cast<unsigned>(std::min<long long>((4 * C * C + 255) / 256, 148 * 8)), 256, 0, ctx.stream>>>(w, nullptr, P->stride, rec[0], rec[1], C, C,
+                                                                                                                                   P->w_rec_mem[d]);
+      ctx.end(TC_RECURRENT);
+    }
+  }
+  P->w_rec_fresh = true;
+  return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
 
 int lstm_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long n_in) {
@@ -531,47 +574,21 @@ int lstm_forward(myea_b200_net *net, LayerPlan &L, const float *input, long long
     }
   }
   const bool zone = P->zoneout && net->training;
-  const long long rec[4] = {off.z_rec, off.rec[0], off.rec[1], off.rec[2]};
-  const bool fresh = L.w_fresh;
-  L.w_fresh = true;   // (what is laid out from the weights below stays until the parameters change)
-  if (P->resident != nullptr) return lstm_resident_run(net, L, 1, zone, rec, off.peep);
+  if (!L.w_fresh) P->w_rec_fresh = false;
+  L.w_fresh = true;   // (what is laid out from the weights stays until the parameters change)
+  if (P->resident_pass[0]) {
+    const long long rec[4] = {off.z_rec, off.rec[0], off.rec[1], off.rec[2]};
+    return lstm_resident_run(net, L, 1, zone, rec, off.peep);
+  }
+  LRC(lay_out_recurrent_weights(net, P, off));
   if (lstm_persistent_ready(P)) {
-    for (int d = 0; d < P->dirs; ++d) {
-      if (fresh) {
-        LRC(lstm_persistent_forward(net, L, d, zone));
-        continue;
-      }
-      const float *w = net->params + P->d[d].w_base;
-      ctx.begin(TC_RECURRENT);
-      lstm_gather_peepholes_kernel<<<static_cast<unsigned>((C + 255) / 256), 256, 0, ctx.stream>>>(w + off.peep, P->stride, C, P->peep_compact + static_cast<size_t>(d) * 3 * C);
-      ctx.end(TC_RECURRENT);
-      ctx.begin(TC_SPLIT);
-      const GroupedGateRows src{w, P->stride, {rec[0], rec[1], rec[2], rec[3]}, C, vec8(w, P->stride, rec[0] | rec[1] | rec[2] | rec[3])};
-      const dim3 grid(half_blocks(P->G, C)), block(HP_THREADS);
-      if (cudaMemsetAsync(P->w_rec_max, 0, static_cast<size_t>(P->G + C) * sizeof(unsigned int), ctx.stream) != cudaSuccess) return MYEA_E_CUDA;
-      launch_dependent(ctx, weight_extents_kernel, grid, block, 0, src, P->G, C, P->w_rec_max);
-      launch_dependent(ctx, weight_panels_kernel, grid, block, 0, src, P->w_rec[d], static_cast<const unsigned int *>(P->w_rec_max), P->w_rec_scale[d]);
-      ctx.end(TC_SPLIT, 2);
-      LRC(lstm_persistent_forward(net, L, d, zone));
-    }
-    return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
+    for (int d = 0; d < P->dirs; ++d) LRC(lstm_persistent_forward(net, L, d, zone));
+    return MYEA_OK;
   }
   // the walk by launches: per step the recurrent product and the cell kernel
   for (int d = 0; d < P->dirs; ++d) {
     LstmDir &D = P->d[d];
     const float *w = net->params + D.w_base;
-    if (fresh) {
-    } else if (P->step_mem != nullptr) {
-      RowSegments seg;
-      seg.seg_rows = C;
-      for (int g = 0; g < 4; ++g) seg.seg_off[g] = rec[g];
-      LRC(half_split(ctx, w, P->stride, P->w_rec[d], &seg));
-    } else {
-      ctx.begin(TC_RECURRENT);
-      lstm_gather_weights_kernel<<<static_cast<unsigned>(std::min<long long>((4 * C * C + 255) / 256, 148 * 8)), 256, 0, ctx.stream>>>(w, nullptr, P->stride, rec[0], rec[1], C, C,
-                                                                                                                                   P->w_rec_mem[d]);
-      ctx.end(TC_RECURRENT);
-    }
     for (long long s = 0; s < T; ++s) {
       const long long t = d == 0 ? s : T - 1 - s;
       const long long tp = d == 0 ? t - 1 : t + 1;
@@ -622,10 +639,11 @@ int lstm_backward(myea_b200_net *net, LayerPlan &L) {
   const long long T = net->T, B = net->B, C = P->C, ldh = L.n_out, n_in = P->n_in;
   const BlockOffsets off = block_offsets(n_in, C);
   P->dg_all_reading[0] = P->dg_all_reading[1] = 0;
-  if (P->resident != nullptr) {
+  if (P->resident_pass[1]) {
     const long long rec[4] = {off.z_rec, off.rec[0], off.rec[1], off.rec[2]};
     return lstm_resident_run(net, L, 2, false, rec, off.peep);
   }
+  LRC(lay_out_recurrent_weights(net, P, off));
   for (int d = 0; d < P->dirs; ++d) {
     LstmDir &D = P->d[d];
     if (lstm_persistent_ready(P)) {

@@ -51,7 +51,9 @@ struct LstmPlan {
   uint16_t *dg_scale = nullptr;
   float *step_mem = nullptr;   // walk by launches: panels of one step's operand
   LstmPersistent *persist = nullptr;
-  LstmResident *resident = nullptr;  // the walk with resident weights (lstm_resident.cu), where it is the faster one
+  LstmResident *resident = nullptr;  // the walk with resident weights (lstm_resident.cu)
+  bool resident_pass[2] = {false, false};   // whether the forward / backward pass takes it
+  bool w_rec_fresh = false;                 // the recurrent weights as the other walks read them match the parameters
   // blocks of several cells (lstm_blocks.cu): K blocks of cpb cells per direction, gate rows of G = C + 3K columns
   // [z (C) | i (K) | f (K) | o (K)], weights gathered into dense matrices for the pass and their derivatives scattered back
   long long K = 0, cpb = 1;
@@ -81,7 +83,7 @@ int lstm_persistent_forward(myea_b200_net *net, LayerPlan &L, int dir, bool zone
 int lstm_persistent_backward(myea_b200_net *net, LayerPlan &L, int dir);
 
 // The walk for small batches and narrow or odd layers: all time steps (and both directions) in one launch, recurrent weights
-// in shared memory, read from the parameter buffer itself.  Set by lstm_resident_plan where it is estimated to be faster.
+// in shared memory, read from the parameter buffer itself.  lstm_resident_plan decides which passes take it.
 int lstm_resident_plan(myea_b200_net *net, LayerPlan &L);
 void lstm_resident_destroy(LstmPlan *P);
 int lstm_resident_run(myea_b200_net *net, LayerPlan &L, int kind, bool zoneout, const long long rec[4], long long peep);

@@ -370,32 +370,69 @@ static bool resident_shape(int kind, long long B, long long C, int dirs, int sms
   return true;
 }
 
+// Which walk a pass takes.  The three are measured per time step and direction (us; weights loaded, T = 72 against T = 8):
+//                     forward                            backward
+//   cells x rows      resident  tensor  launches         resident  tensor  launches
+//   128 x 32             3.2      6.5                       3.6      6.7
+//   256 x 256            8.7     10.5                       9.8     12.9
+//   301 x 512           31.8               27.7            31.7               32.3
+//   512 x 32             5.9      8.9                       8.9     10.6
+//   512 x 64             8.7      9.5                      15.3     11.7
+//   512 x 128           14.4     11.4                      28.8     15.4
+//   601 x 128           29.8               24.0            45.1               25.0
+//   768 x 16             7.5     10.3                      12.5     12.2
+//   768 x 32            11.9     10.5                      23.3     13.1
+//   1001 x 4             5.0               20.3             9.1               21.7
+//   1001 x 32           19.9               24.6            54.6               34.6
+//   1024 x 4             4.9     11.7                       9.3     14.9
+//   1024 x 16            9.5     11.7                      28.0     14.6
+//   1024 x 32           16.4     11.8                      53.4     15.4
+//   1024 x 256         113.8     14.7                     414.6     20.8
+// Backward K is four times as long and only a quarter as wide, so the two passes cross at different sizes and are chosen by
+// themselves (all walks leave the same arrays).  The estimates below are within 20 % of these times; resident_shape counts
+// wavefronts and instructions and comes out 1.6 (forward) and 1.45 times (backward) below the clock.
+static double resident_walk_us(int kind, double clocks) { return (kind == 1 ? 1.6 : 1.45) * clocks / 1900.0; }
+static double other_walk_us(const LstmPlan *P, int kind, long long B) {   // per direction: one after the other
+  const double C = static_cast<double>(P->C), rows = static_cast<double>(std::min<long long>(B, 128)) / 128.0, more = B > 128 ? 0.5 : 0.0;
+  if (lstm_persistent_ready(P)) return kind == 1 ? 6.2 + 5.5 * C / 1024.0 + 2.7 * rows + more : 5.0 + 9.6 * C / 1024.0 + 5.6 * rows + more;
+  const double products = static_cast<double>(B) * 4.0 * C * C;   // straight from fp32 or, from 600 Mi on, from panels
+  return 5.5 + 0.0148 * C + products * 2e-6 / (products <= 629145600.0 ? 36.0 : 75.0);
+}
+
 int lstm_resident_plan(myea_b200_net *net, LayerPlan &L) {
   LstmPlan *P = L.lstm;
   P->resident = nullptr;
+  P->resident_pass[0] = P->resident_pass[1] = false;
   if (net->ctx.gemm_engine != 0 || P->cpb != 1 || P->C > 1400) return MYEA_OK;
   int sms = 0, coop = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, net->ctx.device) != cudaSuccess ||
       cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, net->ctx.device) != cudaSuccess || !coop)
     return MYEA_OK;
-  LstmResident best;
-  double best_clocks = 1e30;
+  // best shape of either pass by itself, and of both with the same groups (where both are taken: the estimates of neighbouring
+  // shapes are closer together than they are to the clock)
+  LstmResident best, both;
+  double best_clocks[2] = {1e30, 1e30}, sum_clocks = 1e30;
   for (int G = 1; G * P->dirs <= sms; ++G) {
     LstmResident r;
-    double cf = 0, cb = 0;
-    if (!resident_shape(1, net->B, P->C, P->dirs, sms, G, &r.f, &r.smem_f, &cf) || !resident_shape(2, net->B, P->C, P->dirs, sms, G, &r.b, &r.smem_b, &cb)) continue;
-    if (cf + cb < best_clocks) { best_clocks = cf + cb; best = r; }
+    double c[2] = {1e30, 1e30};
+    const bool fits[2] = {resident_shape(1, net->B, P->C, P->dirs, sms, G, &r.f, &r.smem_f, &c[0]), resident_shape(2, net->B, P->C, P->dirs, sms, G, &r.b, &r.smem_b, &c[1])};
+    if (fits[0] && c[0] < best_clocks[0]) { best_clocks[0] = c[0]; best.f = r.f; best.smem_f = r.smem_f; }
+    if (fits[1] && c[1] < best_clocks[1]) { best_clocks[1] = c[1]; best.b = r.b; best.smem_b = r.smem_b; }
+    if (fits[0] && fits[1] && c[0] + c[1] < sum_clocks) { sum_clocks = c[0] + c[1]; both = r; }
   }
-  if (best_clocks > 1e29) return MYEA_OK;
-  // What the layer would run otherwise, per step forward + backward: the tensor-core walk (22 + 31 us at 1024 cells and 256
-  // rows, mostly the stream of the weights; both directions one after the other), or the launches of the per-step path.
-  const double clock = 1900.0;  // per us
-  const double other = (lstm_persistent_ready(P) ? 14.0 + 39.0 * static_cast<double>(P->C) / 1024.0 : 60.0 + 20.0 * static_cast<double>(P->C) / 1024.0) * P->dirs * clock;
-  if (best_clocks > other) return MYEA_OK;
+  for (int k = 0; k < 2; ++k)
+    P->resident_pass[k] = best_clocks[k] < 1e29 && resident_walk_us(k + 1, best_clocks[k]) < other_walk_us(P, k + 1, net->B) * P->dirs;
+  if (P->resident_pass[0] && P->resident_pass[1] && sum_clocks < 1e29) best = both;
+  if (!P->resident_pass[0] && !P->resident_pass[1]) return MYEA_OK;
   for (auto kernel : {lstm_resident_kernel<1>, lstm_resident_kernel<2>})
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LR_SMEM_MAX) != cudaSuccess) { cudaGetLastError(); return MYEA_OK; }
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LR_SMEM_MAX) != cudaSuccess) {
+      cudaGetLastError();
+      P->resident_pass[0] = P->resident_pass[1] = false;
+      return MYEA_OK;
+    }
   LstmResident *r = new LstmResident(best);
   P->resident = r;
+  // (a pass that is not taken here has groups, K and Rp of its best shape or of none: both only size the buffers)
   const int counters = P->dirs * std::max(r->f.groups, r->b.groups);
   void *p = nullptr;
   const size_t ex_floats = 2 * static_cast<size_t>(P->dirs) * std::max(static_cast<size_t>(r->f.groups) * r->f.K * r->f.Rp, static_cast<size_t>(r->b.groups) * r->b.K * r->b.Rp);

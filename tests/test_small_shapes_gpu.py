@@ -221,3 +221,31 @@ def test_lstm_errors_of_samples_of_different_magnitude(bidirectional):
     assert (np.linalg.norm(got - want, axis=2) / np.linalg.norm(want, axis=2)).max() < 1e-5
     gpu.synchronize()
     gpu.close()
+
+
+@pytest.mark.parametrize("n_in,H,T,B,bidirectional,zoneout", [
+    (8, 1024, 3, 16, False, 0.2), (8, 512, 3, 64, True, 0.1), (8, 1024, 2, 40, False, 0.0),   # resident forward and tensor-core backward, both tensor-core
+    (8, 1001, 3, 32, False, 0.2), (8, 601, 3, 128, True, 0.0)])                                # the same against the walk by launches
+def test_lstm_passes_on_different_walks(n_in, H, T, B, bidirectional, zoneout):
+    """every pass of a layer takes the walk that is estimated to be the fastest; two steps and an inference pass with new weights"""
+    layers = [capi.fc(n_in), capi.lstm(H, bidirectional=bidirectional, dropout=capi.DROP_ZONEOUT if zoneout else capi.DROP_NONE, p=(zoneout, zoneout, 0.0)),
+              capi.fc(H, capi.AF_LINEAR)]
+    wl = workloads.Workload("walks", capi.net(layers, B, T=T, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE),
+                            capi.opt(capi.OPT_GD, gd_lr=0.01 / B, momentum=0.9), n_in, H, False, layers)
+    gpu, cpu = Net(wl.desc, wl.opt), myea_oracle.OracleNet(wl.desc, wl.opt)
+    X, Y = wl.batch(5)
+    out = []
+    for net in (gpu, cpu):
+        wl.materialize(net)
+        got = []
+        for step in range(2):
+            net.reset_loss(); net.forward(X); net.compute_error(Y); net.backward(); net.update_derivative_weight()
+            got += [net.outputs(1), net.errors(1), net.get(capi.BUF_DERIVATIVES)]
+            net.update_parameter()
+            got.append(net.get(capi.BUF_PARAMETERS))
+        net.forward(X, training=False)
+        out.append(got + [net.outputs(1)])
+    gpu.synchronize()
+    gpu.close()
+    for got, want in zip(*out):
+        assert rel_err(got, want) < TOL
