@@ -362,14 +362,14 @@ int myea_b200_gemm_nt(int device, int engine, uint64_t M, uint64_t N, uint64_t K
 /* No counterpart in the reference.  The same contraction for callers that cannot allocate device memory in the call
  * path (a host that reserved all GPU memory up front, a tick-driven trading loop that cannot absorb cudaMalloc's
  * device-wide synchronisation or its failure): C[M,N] (+)= A[M,K] * B[N,K]^T with A, B, C DEVICE pointers owned by
- * the caller and the operand-panel scratch in a fixed array of a little over 32 MiB inside the library image, so the call performs no
+ * the caller and the operand-panel scratch in a fixed array of MYEA_STATIC_SCRATCH_BYTES inside the library image, so the call performs no
  * cudaMalloc / cudaFree.  Limit: 2*(M+N)*round_up(K,32)+64 floats <= 8 Mi floats, else MYEA_E_INVALID with a message in
  * error_message (optional, error_capacity bytes).  Every GPU that loads the library holds the array until exit.  All
  * calls share it: calls that overlap on the GPU race and must be serialised by the caller.  The first call on a
  * device looks up the array's device address.  The call is synchronous (it returns after the stream is idle and has
  * read a status word back), so never make it on a stream that is being captured.  It makes `device` current for its
  * own work and restores the caller's current device before returning. */
-#define MYEA_STATIC_SCRATCH_BYTES (32u << 20)
+#define MYEA_STATIC_SCRATCH_BYTES ((32u << 20) + (512u << 10))
 int myea_b200_gemm_nt_static(int device, uint64_t M, uint64_t N, uint64_t K, const float *device_A, const float *device_B,
                              float *device_C, int accumulate, void *stream, char *error_message, size_t error_capacity);
 

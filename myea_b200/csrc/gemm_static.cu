@@ -8,10 +8,11 @@
 // scratch in a fixed array that is part of the loaded library image, so the call path contains no cudaMalloc,
 // cudaFree or allocating library routine at all.  Inputs and output stay the caller's (device pointers).
 //
-// Cost: every GPU that loads the library holds the array (MYEA_STATIC_SCRATCH_BYTES = 32 MiB, plus a 256-byte status
+// Cost: every GPU that loads the library holds the array (MYEA_STATIC_SCRATCH_BYTES = 32.5 MiB, plus a 256-byte status
 // word) until the process exits, whether or not this entry point is ever called.
-// Limit: the hi/lo K-major panels of both operands must fit: 2 * (M + N) * round_up(K, 32) + 64 floats <= 8 Mi floats;
-// larger problems are refused with MYEA_E_INVALID and a message, never truncated.
+// Limit: 2 * (M + N) * round_up(K, 32) + 64 floats <= 8 Mi floats; larger problems are refused with MYEA_E_INVALID and a
+// message, never truncated.  The operand panels (half_panels.cuh) take (M + N) * round_up(K, 64) floats, which is never more than
+// that limit, and their powers of two a half per row and 128 of K: the last half MiB of the array.
 // Sharing: all calls on a device use the same array, which keeps whatever the previous call left in it.  Nothing in
 // it has to start at zero except the status word, which each call clears first: a call writes every element of the panels
 // it reads, and the tensor maps the kernel loads through end where the operands end (the hardware fills the rest of a
@@ -30,12 +31,11 @@
 
 namespace {
 
-constexpr size_t kStaticScratchFloats = size_t(8) << 20;  // 32 MiB
+constexpr size_t kLimitFloats = size_t(8) << 20;
+constexpr size_t kStaticScratchFloats = MYEA_STATIC_SCRATCH_BYTES / sizeof(float);
 constexpr int kMaxDevices = 64;
 
-// (the panels of the largest problems that fit the documented limit are a few hundred floats longer: block exponents and
-// alignment)
-static __device__ __align__(256) float g_static_scratch[kStaticScratchFloats + (size_t(128) << 10)];
+static __device__ __align__(256) float g_static_scratch[kStaticScratchFloats];
 static __device__ __align__(256) int g_static_status[64];
 
 struct StaticSetup {
@@ -65,12 +65,12 @@ extern "C" int myea_b200_gemm_nt_static(int device, uint64_t M, uint64_t N, uint
     return MYEA_E_INVALID;
   }
   const size_t need = 2 * (M + N) * ((K + 31) / 32 * 32) + 64;
-  if (M > (1u << 30) || N > (1u << 30) || K > (1u << 30) || need > kStaticScratchFloats) {
+  if (M > (1u << 30) || N > (1u << 30) || K > (1u << 30) || need > kLimitFloats) {
     char msg[200];
     snprintf(msg, sizeof(msg),
              "gemm_nt_static: problem too large for the fixed scratch: 2*(M+N)*round_up(K,32)+64 = %zu floats, limit %zu "
              "(32 MiB); use a handle-based call instead",
-             need, kStaticScratchFloats);
+             need, kLimitFloats);
     say(error_message, error_capacity, msg);
     return MYEA_E_INVALID;
   }
@@ -116,7 +116,7 @@ extern "C" int myea_b200_gemm_nt_static(int device, uint64_t M, uint64_t N, uint
   e.C = device_C;
   e.ldc = static_cast<long long>(N);
   e.accumulate = accumulate;
-  GemmScratch gs{su.scratch, kStaticScratchFloats + (size_t(128) << 10)};
+  GemmScratch gs{su.scratch, kStaticScratchFloats};
   int rc = gemm_nt(ctx, a, b, e, gs);
   if (rc != MYEA_OK) {
     say(error_message, error_capacity, "gemm_nt_static: kernel launch failed");

@@ -65,6 +65,23 @@ def test_static_scratch_reaches_the_wide_kernel_and_allocates_nothing():
     assert torch.cuda.current_device() == 0
 
 
+def test_static_scratch_holds_the_largest_problem_it_accepts():
+    """M + N = 131071 at K = 32 is one row short of the documented limit; panels and powers of two fill the array"""
+    torch = pytest.importorskip("torch")
+    lib = capi.load()
+    M, N, K = 129000, 2071, 32
+    g = torch.Generator(device="cuda").manual_seed(5)
+    A, B = torch.randn(M, K, device="cuda", generator=g), torch.randn(N, K, device="cuda", generator=g)
+    out = torch.zeros(M, N, device="cuda")
+    torch.cuda.synchronize()
+    msg = C.create_string_buffer(256)
+    assert lib.myea_b200_gemm_nt_static(0, M, N, K, A.data_ptr(), B.data_ptr(), out.data_ptr(), 0, None, msg, 256) == 0, msg.value
+    for rows in (slice(0, 300), slice(M - 300, M)):
+        want = A[rows].double() @ B.double().T
+        assert float((out[rows].double() - want).abs().max() / want.abs().max()) < TOL
+    assert lib.myea_b200_gemm_nt_static(0, M + 1, N, K, A.data_ptr(), B.data_ptr(), out.data_ptr(), 0, None, msg, 256) == -1
+
+
 def test_static_scratch_refuses_oversized_problems():
     torch = pytest.importorskip("torch")
     lib = capi.load()
