@@ -815,4 +815,35 @@ int lstm_update_derivative_weight(myea_b200_net *net, LayerPlan &L, const float 
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
 
+// how far reciprocal_from_one is from the correctly rounded reciprocal over `count` floats from the bit pattern `first` on
+__global__ void __launch_bounds__(256) reciprocal_check_kernel(unsigned int first, unsigned int count, unsigned long long *different, unsigned int *most) {
+  unsigned long long n = 0;
+  unsigned int worst = 0;
+  for (unsigned int i = blockIdx.x * 256u + threadIdx.x; i < count; i += gridDim.x * 256u) {
+    const float d = __uint_as_float(first + i);
+    const int ulps = abs(__float_as_int(reciprocal_from_one(d)) - __float_as_int(__frcp_rn(d)));
+    n += ulps != 0;
+    worst = max(worst, static_cast<unsigned int>(ulps));
+  }
+  if (n != 0) atomicAdd(different, n);
+  atomicMax(most, worst);
+}
+
 }  // namespace myea
+
+// Diagnostic (not part of the training interface): over the floats with bit patterns first .. first + count - 1 (positive), how many
+// reciprocals of the LSTM cells differ from the correctly rounded ones, and by how many units in the last place at most.
+extern "C" int myea_b200_reciprocal_check(int device, uint32_t first, uint32_t count, uint64_t *different, uint32_t *most) {
+  if (different == nullptr || most == nullptr || first > 0x7f800000u || count > 0x7f800000u - first) return MYEA_E_INVALID;
+  if (cudaSetDevice(device) != cudaSuccess) return MYEA_E_CUDA;
+  unsigned long long *out = nullptr;   // [0] count, [1] maximum
+  if (cudaMalloc(&out, 2 * sizeof(*out)) != cudaSuccess) return MYEA_E_CUDA;
+  unsigned long long got[2] = {0, 0};
+  const bool ok = cudaMemset(out, 0, sizeof(got)) == cudaSuccess &&
+                  (myea::reciprocal_check_kernel<<<148 * 8, 256>>>(first, count, out, reinterpret_cast<unsigned int *>(out + 1)), cudaGetLastError() == cudaSuccess) &&
+                  cudaMemcpy(got, out, sizeof(got), cudaMemcpyDeviceToHost) == cudaSuccess;
+  cudaFree(out);
+  *different = got[0];
+  *most = static_cast<uint32_t>(got[1]);
+  return ok ? MYEA_OK : MYEA_E_CUDA;
+}

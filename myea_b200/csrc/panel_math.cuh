@@ -27,9 +27,10 @@ __device__ __forceinline__ void store32(float *p, const float (&d)[8]) {
                "f"(d[7])
                : "memory");
 }
-// 1 / d for d in [1, inf]: the hardware's approximation and one Newton-Raphson step in fused arithmetic, which rounds the
-// result correctly (P. Markstein, IA-64 and Elementary Functions, 2000) as the division does, without its branch: the eight
-// cells of a thread interleave.  Past 2^126 the approximation stands (0: the division gives at most 1.2e-38 there).
+// 1 / d for d in [1, inf], without a branch, so that the eight cells of a thread interleave: the hardware's approximation and one
+// Newton-Raphson step in fused arithmetic (P. Markstein, IA-64 and Elementary Functions, 2000).  The theorem there does not cover
+// every d: tests/test_small_shapes_gpu.py compares all of [1, 2^126) with __frcp_rn, and none of the 1056964608 differs.
+// Past 2^126 the approximation stands (0 where the reciprocal is at most 1.2e-38).
 __device__ __forceinline__ float reciprocal_from_one(float d) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));

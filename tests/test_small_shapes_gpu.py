@@ -249,3 +249,12 @@ def test_lstm_passes_on_different_walks(n_in, H, T, B, bidirectional, zoneout):
     gpu.close()
     for got, want in zip(*out):
         assert rel_err(got, want) < TOL
+
+
+def test_reciprocal_of_the_lstm_cells_against_the_correctly_rounded_one():
+    """every float of [1, 2^126) against CUDA's __frcp_rn"""
+    lib = capi.load()
+    one, end = 0x3F800000, 0x7E800000
+    different, most = C.c_uint64(), C.c_uint32()
+    assert lib.myea_b200_reciprocal_check(0, one, end - one, C.byref(different), C.byref(most)) == 0
+    assert different.value == 0 and most.value == 0
