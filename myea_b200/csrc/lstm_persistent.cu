@@ -29,7 +29,8 @@
 //   step barrier: every CTA of a row of tiles counts itself in on a global counter when its results of step s are
 //             written; producers poll it before they load step s + 1.  Every wait in the kernel is bounded (about a
 //             second of SM clock): a wait that runs out sets the handle's error flag and an abort word that makes all
-//             other waits give up, the CTAs meet at their final barriers, free tensor memory and return.
+//             other waits give up, the CTAs wait (bounded as well) until every copy into their shared memory and every product
+//             has landed, meet at their final barriers, free tensor memory and return.
 // The launch needs all its CTAs resident at once (they wait for each other): lstm_persistent_plan checks the tile count
 // against cudaOccupancyMaxActiveClusters and the layer falls back to one launch pair per step otherwise.
 #include "half_panels.cuh"
@@ -101,6 +102,8 @@ struct LstmSeq {
   float *deriv = nullptr;                     // error on the outputs, this direction's columns, pitch ldh
   float *dgates = nullptr, *dcstate = nullptr;
   unsigned int *sync = nullptr;               // [tiles_m] step counters, then one abort word
+  long long wait_cycles = 1ll << 31;          // limit of the wait at a step barrier
+  int stall_step = 0;                         // tests only: the step whose barrier is never reached (0: none)
   int *error_flag = nullptr;
 };
 
@@ -152,11 +155,12 @@ __device__ __forceinline__ void red_release_gpu_add(unsigned int *p, unsigned in
 
 // Bounded wait for a step counter; gives up when any CTA has raised the abort word or after about a second.  The counter is
 // polled alone (the abort word every 64 looks: a second round trip per look delayed every step by half of it).
-__device__ __forceinline__ bool wait_step_counter(const unsigned int *counter, unsigned int target, const unsigned int *abort_word, volatile int *abort_flag) {
+__device__ __forceinline__ bool wait_step_counter(const unsigned int *counter, unsigned int target, const unsigned int *abort_word, volatile int *abort_flag,
+                                                  long long limit) {
   if (*abort_flag) return false;
   const long long t0 = clock64();
   for (int look = 0; ld_relaxed_gpu(counter) < target; ++look) {
-    if ((look & 63) == 63 && (ld_relaxed_gpu(abort_word) != 0u || clock64() - t0 > (1ll << 31))) {
+    if ((look & 63) == 63 && (ld_relaxed_gpu(abort_word) != 0u || clock64() - t0 > limit)) {
       *abort_flag = 1;
       return false;
     }
@@ -181,8 +185,11 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
   uint64_t *acc_empty = done_bar + DONE;     // [ACCS] the 8 exchange warps have read the accumulator
   uint64_t *red_ready = acc_empty + ACCS;    // the peers' partial sums for this CTA have landed
   uint64_t *step_go = red_ready + 1;         // the producer has passed the step barrier
-  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(step_go + 1);
+  uint64_t *drained = step_go + 1;           // a wait has given up: the products issued so far are done
+  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(drained + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
+  uint32_t *left_early = tmem_holder + 2;    // a wait of this cluster has given up
+  uint32_t *pushed_s = tmem_holder + 3, *armed_s = tmem_holder + 4;   // threads' pushes, and steps whose pushes were expected, in all
   float *scale_s = reinterpret_cast<float *>(smem + SM::SCALE_OFFSET);
   float *max_s = reinterpret_cast<float *>(smem + SM::MAX_OFFSET);
   float *peep_s = reinterpret_cast<float *>(smem + SM::BAR_OFFSET + 320);  // [3][16] peepholes of this CTA's cells
@@ -204,7 +211,9 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
     for (int a = 0; a < ACCS; ++a) ptx::mbar_init(&acc_empty[a], 8);
     ptx::mbar_init(red_ready, 1);
     ptx::mbar_init(step_go, 1);
+    ptx::mbar_init(drained, 1);
     *abort_flag = 0;
+    *left_early = *pushed_s = *armed_s = 0;
     ptx::fence_barrier_init();
     ptx::fence_proxy_async();
   }
@@ -246,17 +255,21 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
       for (int s = 1; s < q.T && ok; ++s) {
         // the weights of the step's first stages do not depend on the step before: they are on their way before the barrier
         const int ahead = min(STAGES, my_kb);
-        for (int i = 0; i < ahead; ++i) {
-          const uint32_t u = issued + static_cast<uint32_t>(i);
+        int loaded = 0;
+        for (; loaded < ahead; ++loaded) {
+          const uint32_t u = issued + static_cast<uint32_t>(loaded);
           if (!wait_free(u)) { ok = false; break; }
           ptx::mbar_arrive_expect_tx(&full_bar[u % STAGES], SM::STAGE_BYTES);
-          load_b(u, kb0 + i);
+          load_b(u, kb0 + loaded);
         }
-        if (!ok || !wait_step_counter(counter, per_step * static_cast<unsigned int>(s), abort_word, abort_flag)) { ok = false; break; }
+        if (ok) ok = wait_step_counter(counter, per_step * static_cast<unsigned int>(s) + (s == q.stall_step ? 1u : 0u), abort_word, abort_flag, q.wait_cycles);
         ptx::fence_proxy_async_global();  // the other CTAs wrote them with ordinary stores; TMA reads through the async proxy
         const int a_row = ((s - 1) & 1) * static_cast<int>(q.a_rows) + m0;
-        for (int i = 0; i < ahead; ++i) load_a(issued + static_cast<uint32_t>(i), kb0 + i, a_row);
-        issued += static_cast<uint32_t>(ahead);
+        // (after a wait that gave up as well, whatever lies there: the barriers of the weights on their way complete, so that the
+        // exit below can wait for them)
+        for (int i = 0; i < loaded; ++i) load_a(issued + static_cast<uint32_t>(i), kb0 + i, a_row);
+        issued += static_cast<uint32_t>(loaded);
+        if (!ok) break;
         // only now may the other warps store the arrays of the step before: their stores would keep these copies waiting
         ptx::mbar_arrive_local(step_go);
         for (int kb = kb0 + ahead; kb < kb1; ++kb, ++issued) {
@@ -352,6 +365,7 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
     for (int i = 0; i < 8; ++i) fn[i] = 0.f;
     bool pending = false;
     uint32_t n = 0;        // accumulators read so far
+    uint32_t pushed = 0, armed = 0;   // steps whose partial sums this thread has pushed / expects from the peers
     constexpr int ARRAYS = KIND == 1 ? LSTM_FORWARD_ARRAYS : LSTM_BACKWARD_ARRAYS;
     auto store_arrays = [&](int step, int first, int last) {
       const LstmStep pp = step_view<KIND>(q, step);
@@ -455,7 +469,11 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
               ptx::st_async_f4(dst + (static_cast<uint32_t>((half * (HW / 4) + i) ^ swz) << 4),
                                make_float4(part[dd - 1][4 * i], part[dd - 1][4 * i + 1], part[dd - 1][4 * i + 2], part[dd - 1][4 * i + 3]), bar);
           }
-          if (warp == PS_EPI_WARP0 && lane == 0) ptx::mbar_arrive_expect_tx(red_ready, static_cast<uint32_t>(SM::RECV_BYTES));
+          ++pushed;
+          if (warp == PS_EPI_WARP0 && lane == 0) {
+            ptx::mbar_arrive_expect_tx(red_ready, static_cast<uint32_t>(SM::RECV_BYTES));
+            ++armed;
+          }
           if (!ptx::mbar_wait_cluster_or_abort(red_ready, static_cast<uint32_t>(s - 1) & 1u, abort_flag)) ok = false;
         }
         if (ok) {
@@ -524,6 +542,8 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
       if (warp == PS_EPI_WARP0 && lane == 0) red_release_gpu_add(counter, 1u);
     }
     if (pending && active) store_arrays(q.T - 1, 0, ARRAYS);
+    atomicAdd(pushed_s, pushed);
+    if (warp == PS_EPI_WARP0 && lane == 0) *armed_s = armed;
   } else {
     ptx::reg_release<40>();  // warps 2-3: no role, but the whole warpgroup has to give its registers back
   }
@@ -535,19 +555,40 @@ lstm_persistent_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_c
       if (!ptx::mbar_wait(&full_bar[i % STAGES], (i / STAGES) & 1u)) break;
     }
   }
-  // A wait has given up: copies whose barriers will never complete - weights of a step that did not begin, partial sums that
-  // nobody waits for - may be on their way into this CTA's shared memory.  They land within microseconds; half a millisecond
-  // passes before the CTA goes on to its end.
-  if (*abort_flag != 0) {
-    const long long t0 = clock64();
-    while (clock64() - t0 < (1ll << 20)) {
-    }
-  }
   // peers may still be pushing into this CTA's receive slots or signalling its barriers: the cluster stays together until
   // everybody is here
   ptx::tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag != 0) {
+    for (int d = 0; d < S; ++d) ptx::st_cluster_u32(ptx::map_to_cta(ptx::smem_u32(left_early), static_cast<uint32_t>(d)), 1u);
+  }
   ptx::cluster_sync_all();
+  // A wait of the cluster has given up (every CTA of it sees that here): products may still be reading shared memory, and partial
+  // sums whose step nobody finished may be on their way into the receive slots.  The first have a barrier of their own.  The
+  // second are counted by red_ready: it is told which bytes will never come, or to expect those that nobody had asked for, and
+  // then completes when the last one has landed.  A peer is at most one step ahead (it has passed the step barrier of the step
+  // before, where this CTA counted itself in with that step's sums complete), so one phase is all that can be open.
+  if (*reinterpret_cast<volatile uint32_t *>(left_early) != 0u) {
+    if (warp == 1 && lane == 0) {
+      ptx::tc_commit(drained);
+      ptx::mbar_wait(drained, 0);
+    }
+    if (threadIdx.x == PS_EPI_WARP0 * 32) {
+      uint32_t threads = 0;
+      for (int d = 0; d < S; ++d)
+        if (d != static_cast<int>(rank)) threads += ptx::ld_cluster_u32(ptx::map_to_cta(ptx::smem_u32(pushed_s), static_cast<uint32_t>(d)));
+      const uint32_t sent = threads * (W / 2 * 4), expected = *armed_s * static_cast<uint32_t>(SM::RECV_BYTES);
+      uint32_t phases = *armed_s;
+      if (sent < expected) ptx::mbar_complete_tx(red_ready, expected - sent);
+      if (sent > expected) {
+        ptx::mbar_arrive_expect_tx(red_ready, sent - expected);
+        ++phases;
+      }
+      if (phases > 0) ptx::mbar_wait(red_ready, (phases - 1u) & 1u);
+    }
+    __syncthreads();
+    ptx::cluster_sync_all();
+  }
   if (warp == 1) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem_base, SM::TMEM_COLS);
@@ -562,6 +603,8 @@ struct LstmPersistent {
   int tiles_m = 0;
   long long a_rows = 0;
   unsigned int *sync = nullptr;  // [tiles_m + 1]
+  int stall_step = 0;            // see LstmSeq
+  long long wait_cycles = 1ll << 31;
 };
 
 template <int KIND>
@@ -664,6 +707,8 @@ static void common_args(myea_b200_net *net, LayerPlan &L, int dir, LstmSeq &q) {
   q.a_rows = P->persist->a_rows;
   q.peep = P->peep_compact + static_cast<size_t>(dir) * 3 * P->C;
   q.sync = P->persist->sync;
+  q.stall_step = P->persist->stall_step;
+  q.wait_cycles = P->persist->wait_cycles;
   q.error_flag = net->ctx.d_error_flag;
 }
 
@@ -716,4 +761,18 @@ extern "C" int myea_b200_lstm_resident_clusters(int device, int *forward_pairs, 
   if (forward_pairs) *forward_pairs = myea::resident_clusters<1>(device);
   if (backward_quads) *backward_quads = myea::resident_clusters<2>(device);
   return MYEA_OK;
+}
+
+// For tests: the barrier in front of step `step` (1 to T - 1; 0: none) of every tensor-core walk of this handle is never reached, and
+// the wait there gives up after `cycles` SM clocks.  MYEA_E_UNSUPPORTED when no layer has such a walk.
+extern "C" int myea_b200_lstm_stall(myea_handle net, int step, uint64_t cycles) {
+  if (net == nullptr || step < 0 || cycles > (1ull << 31)) return MYEA_E_INVALID;
+  int found = 0;
+  for (auto &L : net->layers) {
+    if (L.lstm == nullptr || !myea::lstm_persistent_ready(L.lstm)) continue;
+    L.lstm->persist->stall_step = step;
+    L.lstm->persist->wait_cycles = static_cast<long long>(cycles);
+    ++found;
+  }
+  return found > 0 ? MYEA_OK : MYEA_E_UNSUPPORTED;
 }

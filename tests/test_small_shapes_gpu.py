@@ -258,3 +258,30 @@ def test_reciprocal_of_the_lstm_cells_against_the_correctly_rounded_one():
     different, most = C.c_uint64(), C.c_uint32()
     assert lib.myea_b200_reciprocal_check(0, one, end - one, C.byref(different), C.byref(most)) == 0
     assert different.value == 0 and most.value == 0
+
+
+@pytest.mark.parametrize("backward", [False, True])
+def test_a_step_barrier_that_is_never_reached_ends_in_an_error_status(backward):
+    """the tensor-core walk whose wait gives up (after half a millisecond here; its other waits after a second): every copy and
+    product in flight is waited for, the status is an error, and the GPU goes on - a new handle computes what the first one did"""
+    H, B, T = 1024, 136, 4
+    layers = [capi.fc(9), capi.lstm(H), capi.fc(H, capi.AF_LINEAR)]
+    wl = workloads.Workload("stall", capi.net(layers, B, T=T, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE), capi.opt(capi.OPT_GD, gd_lr=1e-6), 9, H, False, layers)
+    X, Y = wl.batch(5)
+    out = []
+    for stall in (0, 2, 0):
+        net = Net(wl.desc, wl.opt)
+        wl.materialize(net)
+        if not backward:
+            assert net.lib.myea_b200_lstm_stall(net.h, stall, C.c_uint64(1 << 20)) == 0
+        net.forward(X)
+        if backward:
+            net.compute_error(Y)
+            assert net.lib.myea_b200_lstm_stall(net.h, stall, C.c_uint64(1 << 20)) == 0
+            net.backward()
+        rc = net.lib.myea_b200_synchronize(net.h)
+        assert rc == (0 if stall == 0 else -3), net.lib.myea_b200_last_error(net.h)
+        if stall == 0:
+            out.append(net.errors(1) if backward else net.outputs(1))
+        net.close()
+    assert np.array_equal(out[0], out[1])
