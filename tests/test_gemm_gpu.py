@@ -1,6 +1,7 @@
-"""GPU tests of the dense contraction alone (myea_b200_gemm_nt): split-precision tcgen05 against a float64 product.
-Shapes cover single tiles, ragged edges in all three dimensions (TMA zero fill, guarded epilogue), K tails that are
-not a multiple of the 32-float stage, accumulate mode, long K, and the FP32 FMA engine."""
+"""GPU tests of the dense contraction alone (myea_b200_gemm_nt) against a float64 product: the kernel that the size chooses
+(FMA tiles, tensor-core tiles from fp32), and operand panels forced by bits 8..16 of `engine` - single tiles, ragged edges in
+all three dimensions (TMA zero fill, guarded epilogue), K tails that are not a multiple of a stage, accumulate mode, long K,
+rows of different magnitude - and the FP32 FMA engine."""
 import ctypes as C
 
 import numpy as np
@@ -33,10 +34,20 @@ def _gemm(M, N, K, engine=0, accumulate=0, seed=0, positive=False, return_out=Fa
     return (err, out) if return_out else err
 
 
-@pytest.mark.parametrize("shape", [(128, 128, 32), (128, 256, 64), (1, 1, 1), (5, 3, 7), (100, 10, 256), (129, 130, 33),
-                                   (300, 520, 100), (256, 64, 128), (512, 512, 512), (127, 1000, 2048)])
+SHAPES = [(128, 128, 32), (128, 256, 64), (1, 1, 1), (5, 3, 7), (100, 10, 256), (129, 130, 33), (300, 520, 100), (256, 64, 128), (512, 512, 512),
+          (127, 1000, 2048)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
 def test_tcgen05_matches_float64(shape):
+    """as the size chooses: (300, 520, 100), (512, 512, 512) and (127, 1000, 2048) run on tensor-core tiles, the others on FMA tiles"""
     assert _gemm(*shape) < 2e-5
+
+
+@pytest.mark.parametrize("shape", SHAPES + [(257, 129, 65), (255, 385, 129), (1, 300, 191), (513, 1, 64)])
+def test_operand_panels_match_float64(shape):
+    assert _gemm(*shape, engine=TILE_WIDE) < 2e-5
+    assert _gemm(*shape, engine=TILE_WIDE, accumulate=1) < 2e-5
 
 
 @pytest.mark.parametrize("shape", [(64, 64, 16), (5, 3, 7), (300, 520, 100)])

@@ -1,7 +1,8 @@
 """GPU tests of the paths small and middle networks take, at the edges of their tiles: contractions straight from fp32
-operands (128 x 64 tiles, 32 of K per stage, K cut over 1, 2, 4 or 8 CTAs), the one-launch normalization of short batches
-(8 columns per block, 4 to 32 rows per thread) and the LSTM walk with resident weights (groups of 1 to many CTAs, chunks of
-exchange data), against float64 products and the numpy restatement."""
+operands (32 x 32 FMA tiles; 128 x 64 tensor-core tiles, 32 of K per stage, K cut over 1, 2, 4 or 8 CTAs), the one-launch
+normalization of short batches (8 columns per block, 4 to 32 rows per thread), the LSTM walks (resident weights: groups of 1
+to many CTAs, chunks of exchange data; which pass takes which), widths of one, and the updates and products that leave or read
+operand panels - against float64 products and the numpy restatement."""
 import ctypes as C
 
 import numpy as np
@@ -16,6 +17,7 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-4
 
 
+# (the size chooses: (64, 640, 2048) runs on tensor-core tiles, the others on FMA tiles)
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (1, 64, 7), (3, 65, 31), (127, 63, 32), (128, 64, 33), (129, 65, 64), (130, 130, 257), (257, 10, 1000), (64, 640, 2048),
                                    (5, 4, 4099)])
 @pytest.mark.parametrize("accumulate", [0, 1])
@@ -119,7 +121,7 @@ def test_update_writes_operand_panels(widths, B, opt):
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (31, 33, 3), (32, 32, 4), (33, 65, 255), (64, 96, 256), (65, 31, 257), (128, 256, 280), (100, 37, 360), (96, 128, 281), (90, 50, 361)])
 @pytest.mark.parametrize("columns", [0, 1 << 18, 3 << 17])   # both operands by rows, B by columns, both by columns
 def test_contraction_with_fmas(M, N, K, columns):
-    """the 32 x 32 FMA tile and the sizes where the tensor-core tile takes over"""
+    """the 32 x 32 FMA tile at the edges of its rows, columns and the 256 of K it holds at a time"""
     lib = capi.load()
     rng = np.random.default_rng(M + N + K)
     A, B = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
@@ -127,6 +129,24 @@ def test_contraction_with_fmas(M, N, K, columns):
     want = A.astype(np.float64) @ B.astype(np.float64).T + out
     a, b = np.ascontiguousarray(A.T if columns & (1 << 17) else A), np.ascontiguousarray(B.T if columns & (1 << 18) else B)
     assert lib.myea_b200_gemm_nt(0, columns, M, N, K, a.ctypes.data, b.ctypes.data, out.ctypes.data, 1, None, 0) == 0
+    assert rel_err(out, want) < 5e-6
+
+
+@pytest.mark.parametrize("M,N,K", [(257, 640, 64), (300, 520, 7), (385, 449, 31), (1, 4800, 33), (129, 1250, 65), (4801, 1, 40), (415, 417, 1000), (513, 321, 32),
+                                   (128, 1216, 4100)])
+@pytest.mark.parametrize("columns", [0, 1 << 17, 1 << 18, 3 << 17])   # which operands are read through their columns
+@pytest.mark.parametrize("accumulate", [0, 1])
+def test_contraction_on_tensor_core_tiles_from_fp32(M, N, K, columns, accumulate):
+    """more than 148 tiles of 32 x 32, which is where the 128 x 64 tensor-core tile takes over: edges of its rows, columns and the
+    32 of K of a stage, pitches that are not 16-byte aligned, K cut over a cluster"""
+    lib = capi.load()
+    assert -(-M // 32) * -(-N // 32) > 148
+    rng = np.random.default_rng(M + N + K)
+    A, B = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
+    out = rng.standard_normal((M, N), dtype=np.float32)
+    want = A.astype(np.float64) @ B.astype(np.float64).T + (out if accumulate else 0)
+    a, b = np.ascontiguousarray(A.T if columns & (1 << 17) else A), np.ascontiguousarray(B.T if columns & (1 << 18) else B)
+    assert lib.myea_b200_gemm_nt(0, columns, M, N, K, a.ctypes.data, b.ctypes.data, out.ctypes.data, accumulate, None, 0) == 0
     assert rel_err(out, want) < 5e-6
 
 
