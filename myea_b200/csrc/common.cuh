@@ -130,6 +130,8 @@ __host__ __device__ __forceinline__ float af_fire(uint32_t af, float z) {
     default: return z;  // linear
   }
 }
+// out of line, for kernels that carry the common functions themselves
+inline __device__ __noinline__ float af_fire_rare(uint32_t af, float z) { return af_fire(af, z); }
 
 // Activation_Function_Derive (Neural_Network.cpp:3157-3199) at steepness 1.  The threshold functions and the stepwise
 // Gaussian are not in that switch: its default branch hands back the VALUE, and so does this one.  ISRU / ISRLU divide the
@@ -178,10 +180,6 @@ __host__ __device__ __forceinline__ bool af_derive_reads_value(uint32_t af) {
 // ---------------------------------------------------------------------------------------------------------
 // Dense contraction  C[M,N] (+)= A[M,K] * B[N,K]^T  with a fused epilogue.
 // ---------------------------------------------------------------------------------------------------------
-// The reference's sigmoid / tanh of the LSTM gates (Activation_Functions.hpp:40, :45)
-__host__ __device__ inline float sigmoid_ref(float x) { return 1.0f / (1.0f + expf(-x)); }
-__host__ __device__ inline float tanh_ref(float x) { return 2.0f / (1.0f + expf(-2.0f * x)) - 1.0f; }
-
 struct Epilogue {
   float *C = nullptr;
   long long ldc = 0;

@@ -19,7 +19,7 @@
 //   sums      three rotating accumulators for hi*hi and one for the cross terms
 #include "common.cuh"
 #include "gemm_epilogue.cuh"
-#include "panel_math.cuh"
+#include "half_panels.cuh"
 #include "tcgen05.cuh"
 
 #include <algorithm>
@@ -89,7 +89,7 @@ struct DgReader {
 #pragma unroll
         for (int j = 0; j < 8; ++j, q += ld) v[j] = *q;
       } else if (vec) {
-        load8(v, p);
+        ld8(v, p, 8, true);
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = p[j];
@@ -132,8 +132,6 @@ __device__ __forceinline__ void dg_store8(uint8_t *hi, uint8_t *cross, uint32_t 
   *reinterpret_cast<uint4 *>(cross + at) = make_uint4(x[0], x[1], x[2], x[3]);
   *reinterpret_cast<uint4 *>(cross + (at ^ 16u)) = make_uint4(x[4], x[5], x[6], x[7]);
 }
-
-static __device__ __noinline__ float af_fire_rare(uint32_t af, float z) { return af_fire(af, z); }
 
 // What this CTA finishes of its tile: rows [first, first + count), summed over the CTAs of the cluster in rank order, through
 // the epilogue.  A thread keeps VEC adjacent columns and takes NB rows at a time, all their loads before the first use: with
@@ -639,10 +637,7 @@ static int launch_direct(Context &ctx, const DirectGroup<MAX> &g, int tiles, int
 }
 
 static bool epilogue_is_vector(const Epilogue &e, long long N) {
-  const uintptr_t bits = reinterpret_cast<uintptr_t>(e.C) | reinterpret_cast<uintptr_t>(e.bias) | reinterpret_cast<uintptr_t>(e.addend) |
-                         reinterpret_cast<uintptr_t>(e.aux_pre) | reinterpret_cast<uintptr_t>(e.aux_y) | reinterpret_cast<uintptr_t>(e.col_scale) |
-                         reinterpret_cast<uintptr_t>(e.col_shift) | reinterpret_cast<uintptr_t>(e.act_out);
-  return (bits & 15) == 0 && ((N | e.ldc | e.ld_addend | e.ld_aux | e.seg_off[0] | e.seg_off[1] | e.seg_off[2] | e.seg_off[3]) & 3) == 0;
+  return epilogue_vector_ok(e) && (reinterpret_cast<uintptr_t>(e.act_out) & 15) == 0 && (N & 3) == 0;
 }
 
 template <bool AT, bool BT, int MAX, bool CUT>

@@ -432,7 +432,6 @@ __device__ __forceinline__ void act_rows(float (&v)[NR], float cs, float ch, boo
     v[i] = keep ? y * scale : 0.f;
   }
 }
-static __device__ __noinline__ float af_fire_rare(uint32_t af, float z) { return af_fire(af, z); }
 template <int NR>
 __device__ __forceinline__ void act_rows_any(uint32_t af, float (&v)[NR], float cs, float ch, bool keep, float scale) {
   switch (af) {

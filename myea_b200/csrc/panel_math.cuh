@@ -7,14 +7,6 @@
 
 namespace myea {
 
-__device__ __forceinline__ void load8(float (&d)[8], const float *p) {
-  const float4 a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(p + 4);
-  d[0] = a.x; d[1] = a.y; d[2] = a.z; d[3] = a.w; d[4] = b.x; d[5] = b.y; d[6] = b.z; d[7] = b.w;
-}
-__device__ __forceinline__ void store8(float *p, const float (&d)[8]) {
-  *reinterpret_cast<float4 *>(p) = make_float4(d[0], d[1], d[2], d[3]);
-  *reinterpret_cast<float4 *>(p + 4) = make_float4(d[4], d[5], d[6], d[7]);
-}
 // 32 aligned bytes in one access
 __device__ __forceinline__ void load32(float (&d)[8], const float *p) {
   asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -37,7 +29,7 @@ __device__ __forceinline__ float reciprocal_from_one(float d) {
   const float n = fmaf(r, fmaf(-d, r, 1.0f), r);
   return d < 8.507059e37f ? n : r;
 }
-// the gates' functions as common.cuh has them: 1 / (1 + e^-x), 2 / (1 + e^-2x) - 1
+// the gates' functions as the reference has them (Activation_Functions.hpp:40, :45): 1 / (1 + e^-x), 2 / (1 + e^-2x) - 1
 __device__ __forceinline__ float sigmoid_cell(float x) { return reciprocal_from_one(1.0f + expf(-x)); }
 __device__ __forceinline__ float tanh_cell(float x) { return 2.0f * reciprocal_from_one(1.0f + expf(-2.0f * x)) - 1.0f; }
 
