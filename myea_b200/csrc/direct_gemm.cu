@@ -12,7 +12,7 @@
 //             (1, 2, 4 or 8) until the grid fills the chip; partial tiles meet in distributed shared memory and are added
 //             in rank order (bitwise repeatable)
 //   stage     every thread splits 24 elements: 8 consecutive K of three rows, fetched into registers while the stage before
-//             is converted.  hi (TF32) and the cross-term group (bf16, see panel_math.cuh) go into K-major tiles with the
+//             is converted.  hi (TF32) and the cross-term group (bf16, see split_group) go into K-major tiles with the
 //             128-byte swizzle; one thread then issues the eight tcgen05.mma of the stage.  (Warp-level mma.sync was
 //             built first: 512^3 took 12 us instead of 17 with panels; its TF32 rate on this chip is below what the
 //             precision needs - three TF32 products run no faster than plain FMAs.)
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(DG_THREADS, 2) direct_gemm_kernel(const __grid
 
 // ---------------------------------------------------------------------------------------------------------
 // The smallest products with plain FMAs.  A tensor-core tile pays for tensor memory, barriers, conversion, a cluster and its
-// exchange before anything else: 128 x 256 x 256 takes it 6.8 us (here 5.4), of which the products are a tenth.  Here a CTA owns
+// exchange before anything else: 128 x 256 x 256 takes it 6.8 us (here 5.2), of which the products are a tenth.  Here a CTA owns
 // 32 x 32 outputs, fetches both operands' rows for up to 256 of K at once (16 loads of 16 bytes per thread in flight: one trip
 // to L2), and its 8 warps walk interleaved groups of four K each with 4 x 8 sums per lane; the 8 partial tiles are added in warp
 // order in shared memory (bitwise repeatable).  Bound by latency, then by shared-memory reads and FMA issue (11 ns per K): a long K of
