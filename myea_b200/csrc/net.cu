@@ -952,9 +952,11 @@ static int compute_error_impl(myea_b200_net *net, uint64_t batch, const float *s
   LayerPlan &L = net->layers.back();
   const long long pitch = pitch_rows(net), rows = net->T * pitch;
   if (kind == cudaMemcpyDefault) {
-  } else if (kind == cudaMemcpyHostToDevice && rows * L.n_out * static_cast<long long>(sizeof(float)) > (256 << 10)) {
+  } else if (kind == cudaMemcpyHostToDevice) {
     // host targets: copy beside the forward pass still in flight on the main stream (the last use of d_desired by an
-    // error kernel is behind ev_desired_free), and let the main stream wait for the copy only now
+    // error kernel is behind ev_desired_free), and let the main stream wait for the copy only now.  Whatever their size: a step of
+    // a 64-256-256-n network on 256 rows takes 48 / 56 / 145 us with 16 / 256 / 4096 KB of targets and 54 / 72 / 188 us with the copy
+    // on the main stream, and 65 / 69 / 177 against 74 / 78 / 203 us when the loss is read after every step.
     if (net->desired_unmarked) CK(cudaEventRecord(net->ev_desired_free, net->ctx.stream));
     net->desired_unmarked = false;
     CK(cudaStreamWaitEvent(net->copy_stream, net->ev_desired_free, 0));

@@ -152,3 +152,37 @@ def test_bad_requests_are_refused_not_mangled():
     x = np.zeros((wl.desc.number_recurrent_depth, wl.B + 1, wl.n_in), np.float32)
     assert gpu.lib.myea_b200_forward(gpu.h, wl.B + 1, x.ctypes.data, 1) == -1                # batch above the allocated one
     gpu.close()
+
+
+def test_targets_from_host_device_and_dataset_in_turn():
+    """the targets' buffer is filled on a stream of its own, on the main stream or by the epoch loop's gather: whatever the turn, the
+    same steps give the same parameters"""
+    torch = pytest.importorskip("torch")
+    layers = [capi.fc(24), capi.fc(96, capi.AF_TANH), capi.fc(200, capi.AF_LINEAR)]
+    B, steps = 64, 12
+    desc, opt = capi.net(layers, B, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE), capi.opt(capi.OPT_GD, gd_lr=1e-3 / B, momentum=0.9)
+    rng = np.random.default_rng(3)
+    X, Y = rng.standard_normal((steps, B, 24)).astype(np.float32), rng.standard_normal((steps, B, 200)).astype(np.float32)
+    p0 = None
+    out = []
+    for turn in ("h", "d", "e", "hd", "dh", "he", "deh", "hhed"):
+        net = Net(desc, opt)
+        p0 = rng.uniform(-0.2, 0.2, net.P).astype(np.float32) if p0 is None else p0
+        net.set(capi.BUF_PARAMETERS, p0)
+        net.dataset_set(X.reshape(steps * B, -1), Y.reshape(steps * B, -1))
+        host = [(torch.from_numpy(x).pin_memory(), torch.from_numpy(y).pin_memory()) for x, y in zip(X, Y)]
+        device = [(x.cuda(), y.cuda()) for x, y in host]
+        torch.cuda.synchronize()
+        for k in range(steps):
+            how = turn[k % len(turn)]
+            if how == "e":
+                net.train_epoch(np.arange(k * B, (k + 1) * B), B)
+                continue
+            (x, y), lib = (host if how == "h" else device)[k], net.lib
+            forward, error = (lib.myea_b200_forward, lib.myea_b200_compute_error) if how == "h" else (lib.myea_b200_forward_device, lib.myea_b200_compute_error_device)
+            for rc in (forward(net.h, B, x.data_ptr(), 1), error(net.h, B, y.data_ptr()), lib.myea_b200_backward(net.h, B), lib.myea_b200_update_derivative_weight(net.h, B),
+                       lib.myea_b200_update_parameter(net.h, B, B * steps, C.byref(opt))):
+                assert rc == 0
+        out.append(net.get(capi.BUF_PARAMETERS))
+        net.close()
+    assert all(np.array_equal(out[0], p) for p in out[1:])
