@@ -1114,6 +1114,7 @@ extern "C" int myea_b200_backward(myea_handle net, uint64_t batch) {
   if (!net->training) return fail(net, MYEA_E_INVALID, "can not back propagate in inference mode");
   CK(cudaSetDevice(net->ctx.device));
   RC(comm_gather_join(net));
+  for (auto &L : net->layers) L.d_valid = false;   // (panels of the errors of an earlier backward pass on the same forward pass)
   const long long rows = step_rows_total(net);
   const int n = static_cast<int>(net->layers.size());
   if (net->pre_training_level != 0) {  // the decoded layer's error reaches the coded layer and stops there

@@ -305,3 +305,21 @@ def test_a_step_barrier_that_is_never_reached_ends_in_an_error_status(backward):
             out.append(net.errors(1) if backward else net.outputs(1))
         net.close()
     assert np.array_equal(out[0], out[1])
+
+
+def test_a_second_backward_pass_does_not_read_the_errors_of_the_first():
+    """compute_error and backward twice on one forward pass, with other targets, on layers that read operand panels"""
+    layers = [capi.fc(1000), capi.fc(904, capi.AF_TANH), capi.fc(1096, capi.AF_TANH), capi.fc(1000, capi.AF_LINEAR)]
+    wl = workloads.Workload("twice", capi.net(layers, 700, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE), capi.opt(capi.OPT_GD, gd_lr=1e-6), 1000, 1000, False, layers)
+    X, Y = wl.batch(5)
+    out = []
+    for targets in ((Y,), (Y + 1.0, Y)):
+        net = Net(wl.desc, wl.opt)
+        wl.materialize(net)
+        net.forward(X)
+        for t in targets:
+            net.compute_error(t.astype(np.float32)); net.backward()
+        net.update_derivative_weight()
+        out.append(net.get(capi.BUF_DERIVATIVES))
+        net.close()
+    assert np.array_equal(out[0], out[1])
