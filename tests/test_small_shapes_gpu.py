@@ -1,7 +1,7 @@
 """GPU tests of the paths small and middle networks take, at the edges of their tiles: contractions straight from fp32
 operands (32 x 32 FMA tiles; 128 x 64 tensor-core tiles, 32 of K per stage, K cut over 1, 2, 4 or 8 CTAs), the one-launch
 normalization of short batches (8 columns per block, 4 to 32 rows per thread), the LSTM walks (resident weights: groups of 1
-to many CTAs, chunks of exchange data; which pass takes which), widths of one, and the updates and products that leave or read
+to many CTAs, clusters, chunks of exchange data; which pass takes which), widths of one, and the updates and products that leave or read
 operand panels - against float64 products and the numpy restatement."""
 import ctypes as C
 
@@ -68,6 +68,13 @@ def test_plain_networks(widths, B, af):
 @pytest.mark.parametrize("norm", [capi.NORM_BN, capi.NORM_BRN])
 def test_normalized_short_batches(B, norm):
     _step(_mlp((9, 37, 16, 3), B, capi.AF_SIGMOID, norm, capi.DROP_BERNOULLI_INVERTED))
+
+
+# the resident walk on clusters: one to three steps (the barriers' first phases), rows and cells that do not divide
+@pytest.mark.parametrize("n_in,H,T,B,bidirectional,zoneout", [
+    (5, 150, 1, 50, False, 0.0), (5, 150, 2, 50, False, 0.1), (5, 203, 3, 61, False, 0.0), (5, 129, 7, 30, True, 0.2), (5, 300, 4, 5, False, 0.1), (5, 90, 5, 256, True, 0.0)])
+def test_lstm_walk_on_clusters(n_in, H, T, B, bidirectional, zoneout):
+    test_lstm_with_resident_weights(n_in, H, T, B, bidirectional, zoneout)
 
 
 @pytest.mark.parametrize("n_in,H,T,B,bidirectional,zoneout", [
