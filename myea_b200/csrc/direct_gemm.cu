@@ -599,6 +599,330 @@ __global__ void __launch_bounds__(DG_THREADS, 2) fma_gemm_kernel(const __grid_co
 }
 
 // ---------------------------------------------------------------------------------------------------------
+// Products whose tiles of 32 x 32 leave most of the chip idle, with plain FMAs on tiles of 16 x 16: four times as many CTAs, a
+// quarter of the multiplying each, and twice the operand traffic, which comes from L2.  What remains is latency: all loads of up to
+// 256 of K (two chunks) are in flight together whatever the alignment, the third and later chunks travel while one is multiplied,
+// and what the epilogue reads is on its way beside them.  (128 x 256 x 256 4.0 us in a chain of launches where 32 x 32 takes 6.2; 203 x
+// 333 x 333, rows that are not aligned, 6.8 and 10; a launch without work 3.)  The 8 warps walk interleaved groups of four K and
+// their partial tiles are added in warp order (bitwise repeatable).
+// ---------------------------------------------------------------------------------------------------------
+constexpr int SG_TILE = 16, SG_K = 128, SG_PITCH = SG_K + 4;   // K of a chunk, pitch of an operand's rows in shared memory
+constexpr int SG_SMEM = 2 * 2 * SG_TILE * SG_PITCH * 4;          // two chunks; the partial tiles and row sums lie over them
+static_assert(SG_SMEM >= (8 * SG_TILE * (SG_TILE + 4) + 8 * SG_TILE) * 4, "the partial tiles lie over the operands");
+
+// The epilogue of a tile: rows [first, first + count), summed by `sum(row, column, v)` and taken through the
+// epilogue.  A thread keeps VEC adjacent columns and takes NB rows at a time.  What the epilogue reads from memory for the first NB
+// of them is on its way before `work`, which computes the partial tiles and ends with them visible to every thread: behind it this
+// part was latency after latency and took longer than the products (29 of 31 us at K = 10).
+// TN: columns of the tile.
+template <int TN, int VEC, int NB, typename Work, typename Sum>
+__device__ __forceinline__ void sg_finish(const DirectProblem &p, int first, int count, int m0, int n0, Work work, Sum sum) {
+  constexpr int LANES = TN / VEC, STEP = DG_THREADS / LANES;
+  using Vec = float[VEC];
+  const Epilogue &e = p.epi;
+  const int c = (static_cast<int>(threadIdx.x) % LANES) * VEC, n = n0 + c;
+  auto load = [](Vec &d, const float *src) {
+    if constexpr (VEC == 4) { const float4 t = *reinterpret_cast<const float4 *>(src); d[0] = t.x; d[1] = t.y; d[2] = t.z; d[3] = t.w; }
+    else d[0] = *src;
+  };
+  auto store = [](float *dst, const Vec &d) {
+    if constexpr (VEC == 4) *reinterpret_cast<float4 *>(dst) = make_float4(d[0], d[1], d[2], d[3]);
+    else *dst = d[0];
+  };
+  const bool in = n < p.N;
+  const bool affine = e.deriv_af != 0u && e.aux_pre != nullptr && e.col_scale != nullptr;
+  Vec bias = {}, factor = {};
+  if (in && e.bias != nullptr) load(bias, e.bias + n);
+  if (in && e.act_out != nullptr) {
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) factor[k] = (e.act_mask != nullptr && e.act_mask[n + k] == 0) ? 0.f : e.act_scale;
+  }
+  const int end = in ? min(first + count, p.M - m0) : first;
+  Vec add[NB], slope[NB], old[NB];   // bias and addend, activation derivative, what lies in C
+  auto fetch = [&](int r0) {
+    Vec pre[NB], y[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const long long m = m0 + min(r0 + b * STEP, end - 1);   // rows past the end repeat the last one and are not stored
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) add[b][k] = 0.f;
+      if (e.addend != nullptr) load(add[b], e.addend + m * e.ld_addend + n);
+      if (e.deriv_af != 0u && e.aux_pre != nullptr) load(pre[b], e.aux_pre + m * e.ld_aux + n);
+      if (e.deriv_af != 0u && e.aux_y != nullptr) load(y[b], e.aux_y + m * e.ld_aux + n);
+      if (e.accumulate) load(old[b], e.C + c_row(e, m) + n);
+    }
+    if (e.deriv_af != 0u) {
+      Vec cs, ch = {};
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) cs[k] = 1.f;
+      if (affine) { load(cs, e.col_scale + n); load(ch, e.col_shift + n); }
+      auto derive = [&](auto f) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+          for (int k = 0; k < VEC; ++k) slope[b][k] = f(e.aux_pre != nullptr ? pre[b][k] * cs[k] + ch[k] : 0.f, e.aux_y != nullptr ? y[b][k] : 0.f);
+      };
+      switch (e.deriv_af) {
+        case MYEA_AF_TANH: derive([](float z, float w) { return af_derive(MYEA_AF_TANH, z, w); }); break;
+        case MYEA_AF_RELU: derive([](float z, float w) { return af_derive(MYEA_AF_RELU, z, w); }); break;
+        default: { const uint32_t af = e.deriv_af; derive([af](float z, float w) { return af_derive_rare(af, z, w); }); break; }
+      }
+    }
+  };
+  int r0 = first + static_cast<int>(threadIdx.x) / LANES;
+  if (r0 < end) fetch(r0);
+  work();
+#pragma unroll 1
+  while (r0 < end) {
+    Vec v[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) v[b][k] = 0.f;
+      sum(min(r0 + b * STEP, end - 1), c, v[b]);
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) {
+        v[b][k] += bias[k];
+        if (e.addend != nullptr) v[b][k] += add[b][k];
+        if (e.deriv_af != 0u) v[b][k] *= slope[b][k];
+        if (e.accumulate) v[b][k] += old[b][k];
+      }
+      if (r0 + b * STEP < end) store(e.C + c_row(e, m0 + r0 + b * STEP) + n, v[b]);
+    }
+    if (e.act_out != nullptr) {
+      auto fire = [&](auto f) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+          for (int k = 0; k < VEC; ++k) { const float t = f(v[b][k]); v[b][k] = factor[k] != 0.f ? t * factor[k] : 0.f; }
+      };
+      switch (e.act_af) {
+        case MYEA_AF_TANH: fire([](float z) { return af_fire(MYEA_AF_TANH, z); }); break;
+        case MYEA_AF_RELU: fire([](float z) { return af_fire(MYEA_AF_RELU, z); }); break;
+        case MYEA_AF_LINEAR: fire([](float z) { return z; }); break;
+        default: { const uint32_t af = e.act_af; fire([af](float z) { return af_fire_rare(af, z); }); break; }
+      }
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+        if (r0 + b * STEP < end) store(e.act_out + c_row(e, m0 + r0 + b * STEP) + n, v[b]);
+    }
+    r0 += NB * STEP;
+    if (r0 < end) fetch(r0);
+  }
+}
+
+// One operand's share of a chunk of K on its way from memory through a thread's registers into shared memory: all loads of a chunk
+// are in flight together, whatever the alignment.  Rows row0 .. row0 + ROWS - 1 (past `rows`: the last one again), K elements
+// k0 .. k0 + kc - 1 (zeros up to a multiple of 4).
+template <bool T, int ROWS>
+struct SgOperand {
+  static constexpr int N = ROWS / 8;   // 16-byte pieces per thread
+  const float *src;
+  long long ld;
+  int row0, rows;
+  bool vec;
+  struct Set { float4 v[N]; int shift[N]; };
+
+  __device__ __forceinline__ bool wide() const { return vec && row0 + ROWS <= rows; }
+  __device__ __forceinline__ void load(Set &x, int k0, int kc) const {
+    const int tid = static_cast<int>(threadIdx.x);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (T) {
+      if (wide()) {   // lanes take consecutive 16 bytes along the rows
+        constexpr int L = ROWS / 4;
+        const float *q = src + static_cast<long long>(k0) * ld + row0 + (tid % L) * 4;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          const int k = tid / L + i * (DG_THREADS / L);
+          x.v[i] = k < kc ? *reinterpret_cast<const float4 *>(q + k * ld) : zero;
+        }
+      } else {
+        const float *q = src + static_cast<long long>(k0) * ld + min(row0 + tid % ROWS, rows - 1);
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          float e[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int k = tid / ROWS + (4 * i + j) * (DG_THREADS / ROWS);
+            e[j] = k < kc ? q[k * ld] : 0.f;
+          }
+          x.v[i] = make_float4(e[0], e[1], e[2], e[3]);
+        }
+      }
+    } else {
+      // a warp takes a row, its lanes consecutive 16 bytes; a row that does not start on such a boundary is read from the boundary
+      // before it, and store() moves the elements to their places
+      const int warp = tid >> 5, lane = tid & 31;
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const float *q = src + static_cast<long long>(min(row0 + warp + 8 * i, rows - 1)) * ld + k0;
+        x.shift[i] = static_cast<int>(reinterpret_cast<uintptr_t>(q) >> 2) & 3;
+        const int k = 4 * lane - x.shift[i];
+        if (k >= 0 && k + 4 <= kc) {
+          x.v[i] = *reinterpret_cast<const float4 *>(q + k);
+        } else {
+          x.v[i].x = k >= 0 && k < kc ? q[k] : 0.f;
+          x.v[i].y = k + 1 >= 0 && k + 1 < kc ? q[k + 1] : 0.f;
+          x.v[i].z = k + 2 >= 0 && k + 2 < kc ? q[k + 2] : 0.f;
+          x.v[i].w = k + 3 < kc ? q[k + 3] : 0.f;   // (the shift is 3 at most)
+        }
+      }
+    }
+  }
+  __device__ __forceinline__ void store(const Set &x, float *s, int kc) const {
+    const int tid = static_cast<int>(threadIdx.x), kz = (kc + 3) & ~3;
+    if constexpr (T) {
+      if (wide()) {
+        constexpr int L = ROWS / 4;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          const int k = tid / L + i * (DG_THREADS / L);
+          if (k < kz) *reinterpret_cast<float4 *>(s + k * ROWS + (tid % L) * 4) = x.v[i];
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          const float e[4] = {x.v[i].x, x.v[i].y, x.v[i].z, x.v[i].w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int k = tid / ROWS + (4 * i + j) * (DG_THREADS / ROWS);
+            if (k < kz) s[k * ROWS + tid % ROWS] = e[j];
+          }
+        }
+      }
+    } else {
+      const int warp = tid >> 5, lane = tid & 31;
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        float4 v = x.v[i];
+        if (!vec) {
+          const float a = __shfl_down_sync(0xffffffffu, v.x, 1), b = __shfl_down_sync(0xffffffffu, v.y, 1), c = __shfl_down_sync(0xffffffffu, v.z, 1);
+          if (x.shift[i] == 1) v = make_float4(v.y, v.z, v.w, a);
+          else if (x.shift[i] == 2) v = make_float4(v.z, v.w, a, b);
+          else if (x.shift[i] == 3) v = make_float4(v.w, a, b, c);
+        }
+        if (4 * lane < kz) *reinterpret_cast<float4 *>(s + (warp + 8 * i) * SG_PITCH + 4 * lane) = v;
+      }
+    }
+  }
+};
+
+template <bool AT, bool BT, int MAX>
+__global__ void __launch_bounds__(DG_THREADS, 2) small_gemm_kernel(const __grid_constant__ DirectGroup<MAX> g, const int chunk) {
+  constexpr int TM = SG_TILE, TN = SG_TILE, RG = 4, CG = 8, TILE = TM * (TN + 4), BUFFER = (TM + TN) * SG_PITCH;
+  extern __shared__ __align__(16) float sg_smem[];
+  const int tile = static_cast<int>(blockIdx.x);
+  int pi = 0;
+#pragma unroll 1
+  while (pi + 1 < g.count && tile >= g.p[pi + 1].first_tile) ++pi;
+  const DirectProblem &p = g.p[pi];
+  const int tl = tile - p.first_tile;
+  const int tm = tl / p.tiles_n, tn = tl - tm * p.tiles_n;
+  const int m0 = tm * TM, n0 = tn * TN;
+  const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31;
+  const int rg = lane / CG, cg = lane % CG;   // rows rg + 4 i or 4 rg + i, columns cg + 8 j or 2 cg + j
+  const bool want_sum = AT && p.row_sum != nullptr && tn == 0;
+  const int chunks = (p.K + chunk - 1) / chunk;
+  float *sums = sg_smem + 8 * TILE;
+  const SgOperand<AT, TM> oa{p.a, p.lda, m0, p.M, p.a_vec != 0};
+  const SgOperand<BT, TN> ob{p.b, p.ldb, n0, p.N, p.b_vec != 0};
+  typename SgOperand<AT, TM>::Set a_in[2];
+  typename SgOperand<BT, TN>::Set b_in[2];
+  grid_dependency_wait();
+  grid_dependency_release();
+  auto length = [&](int c) { return min(chunk, p.K - c * chunk); };
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    if (j < chunks) {
+      oa.load(a_in[j], j * chunk, length(j));
+      ob.load(b_in[j], j * chunk, length(j));
+    }
+  auto work = [&]() {
+    float acc[4][2] = {};
+    float rs = 0.f;
+#pragma unroll 1
+    for (int c0 = 0; c0 < chunks; c0 += 2) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int c = c0 + j;
+        if (c >= chunks) break;
+        const int kc = length(c);
+        float *sa = sg_smem + j * BUFFER, *sb = sa + TM * SG_PITCH;
+        oa.store(a_in[j], sa, kc);
+        ob.store(b_in[j], sb, kc);
+        __syncthreads();   // (what lay in this buffer had been multiplied by everybody before the last of these)
+        if (c + 2 < chunks) {
+          oa.load(a_in[j], (c + 2) * chunk, length(c + 2));
+          ob.load(b_in[j], (c + 2) * chunk, length(c + 2));
+        }
+        if (want_sum && lane < TM)
+          for (int k = warp; k < kc; k += 8) rs += sa[k * TM + lane];
+#pragma unroll 2
+        for (int k = warp * 4; k < kc; k += 32) {
+          float a[4][4], b[4][2];   // [row][k], [k][column]
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float4 t = *reinterpret_cast<const float4 *>(AT ? sa + (k + i) * TM + rg * 4 : sa + (rg + RG * i) * SG_PITCH + k);
+            if (AT) { a[0][i] = t.x; a[1][i] = t.y; a[2][i] = t.z; a[3][i] = t.w; }
+            else { a[i][0] = t.x; a[i][1] = t.y; a[i][2] = t.z; a[i][3] = t.w; }
+          }
+          if constexpr (BT) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float2 t = *reinterpret_cast<const float2 *>(sb + (k + i) * TN + cg * 2);
+              b[i][0] = t.x; b[i][1] = t.y;
+            }
+          } else {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              const float4 t = *reinterpret_cast<const float4 *>(sb + (cg + CG * q) * SG_PITCH + k);
+              b[0][q] = t.x; b[1][q] = t.y; b[2][q] = t.z; b[3][q] = t.w;
+            }
+          }
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+              for (int q = 0; q < 2; ++q) acc[i][q] = fmaf(a[i][kk], b[kk][q], acc[i][q]);
+        }
+      }
+    }
+    __syncthreads();   // the operands have been read: the partial tiles take their place
+    float *part = sg_smem + warp * TILE;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float *d = part + (AT ? rg * 4 + i : rg + RG * i) * (TN + 4);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) d[BT ? cg * 2 + q : cg + CG * q] = acc[i][q];
+    }
+    if (want_sum && lane < TM) sums[warp * TM + lane] = rs;
+    __syncthreads();
+  };
+  auto sum = [&](int r, int c, auto &v) {
+    constexpr int VEC = sizeof(v) / sizeof(float);
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      const float *t = sg_smem + w * TILE + r * (TN + 4) + c;
+      if constexpr (VEC == 4) {
+        const float4 x = *reinterpret_cast<const float4 *>(t);
+        v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+      } else {
+        v[0] += *t;
+      }
+    }
+  };
+  if (p.c_vec) sg_finish<TN, 4, 1>(p, 0, TM, m0, n0, work, sum);
+  else sg_finish<TN, 1, 1>(p, 0, TM, m0, n0, work, sum);
+  if (want_sum && tid < TM && m0 + tid < p.M) {
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) v += sums[w * TM + tid];
+    p.row_sum[m0 + tid] += v;
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------------------
 // Up to 600 M multiply-adds.  Measured against the panel kernels with their splits (us): 512^3 9.0 / 16.0, 256 x 1024 x 1024 12.1 /
@@ -673,31 +997,57 @@ static int launch_fma(Context &ctx, const DirectGroup<MAX> &g, int tiles, int cl
   return cluster > 1 ? launch_fma_cut<AT, BT, MAX, true>(ctx, g, tiles, cluster) : launch_fma_cut<AT, BT, MAX, false>(ctx, g, tiles, 1);
 }
 
+template <bool AT, bool BT, int MAX>
+static int launch_small(Context &ctx, const DirectGroup<MAX> &g, int tiles) {
+  int chunk = SG_K;
+  for (int i = 0; i < g.count; ++i)
+    if ((!AT && !g.p[i].a_vec) || (!BT && !g.p[i].b_vec)) chunk = SG_K - 4;   // (a row that is read from the boundary before it takes one lane more)
+  ctx.begin(TC_GEMM);
+  const cudaError_t err = launch_dependent(ctx, small_gemm_kernel<AT, BT, MAX>, dim3(static_cast<unsigned>(tiles)), dim3(DG_THREADS), SG_SMEM, g, chunk);
+  ctx.end(TC_GEMM);
+  return err == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
+}
+
 static long long operand_pitch(const Operand &o, bool columns) { return columns ? o.stride_k : o.stride_r; }
 
-// How many CTAs share the K range of a 32 x 32 tile, 0: tensor-core tiles instead.  One CTA per SM at most: two of them take all
+// How many CTAs share the K range of a 32 x 32 tile, or tensor-core tiles instead.  One CTA per SM at most: two of them take all
 // registers of an SM, so that the next launch cannot set itself up beside them (a 256 x 1024 x 10 product alone took 3.4 us instead
 // of 4.6, and the training step around it 5 us more).  Estimates (us) from these measurements of FMAs with 1 / 2 / 4 / 8 CTAs and of
 // tensor-core tiles: 128 x 256 x 64 3.4 / 4.6 / 4.8 / 5.7, 5.5; 128 x 256 x 256 5.2 / 5.5 / 5.4 / 6.0, 6.8; 64 x 512 x 512 8.4 / 6.7 / 6.2 /
 // 6.4, 8.0; 256 x 10 x 1024 15.2 / 10.2 / 7.3 / 6.5, 11.5; 32 x 64 x 4096 54 / 30 / 17 / 10, 17; 384^3 8.0, 7.8; rows that are not
 // 16-byte aligned: 203 x 333 x 75 4.1, 9.8.
-static int fma_cluster(const DirectItem *items, int n, bool at, bool bt) {
-  long long tiles = 0, longest = 0;
+// Tiles of 16 x 16 (cluster 0, tile 16) where they are up to two CTAs per SM.  Estimates from these measurements, beside the others':
+// 128 x 256 x 64 3.4, 128 x 256 x 256 4.0, 64 x 512 x 512 5.0, 256 x 256 x 512 6.6 (256 tiles), 256 x 10 x 1024 8.4, 32 x 64 x 4096 26; not aligned:
+// 203 x 333 x 75 3.4, 203 x 333 x 333 6.8 (273 tiles), 161 x 150 x 2000 read through its columns 20.6.
+struct FmaPlan {
+  int tile = 0, cluster = 1;   // tile 0: tensor-core tiles
+};
+static FmaPlan fma_plan(const DirectItem *items, int n, bool at, bool bt) {
+  auto tiles_of = [&](long long t) {
+    long long tiles = 0;
+    for (int i = 0; i < n; ++i) tiles += (items[i].A.rows + t - 1) / t * ((items[i].B.rows + t - 1) / t);
+    return tiles;
+  };
+  long long longest = 0;
   bool aligned = true;
   for (int i = 0; i < n; ++i) {
-    tiles += (items[i].A.rows + FG_M - 1) / FG_M * ((items[i].B.rows + FG_N - 1) / FG_N);
     longest = std::max(longest, items[i].A.k);
     aligned = aligned && ((reinterpret_cast<uintptr_t>(items[i].A.ptr) | reinterpret_cast<uintptr_t>(items[i].B.ptr)) & 15) == 0 &&
               ((operand_pitch(items[i].A, at) | operand_pitch(items[i].B, bt)) & 3) == 0;
   }
   const double K = static_cast<double>(longest);
   double best = 5.0 + 0.006 * std::min(K, 1024.0) + 0.002 * std::max(0.0, K - 1024.0) + (aligned ? 0.0 : 2.0) - 0.5;
-  int cluster = 0;
-  for (int S = 1; S <= 8 && tiles * S <= 148; S *= 2) {
+  FmaPlan plan;
+  const long long t32 = tiles_of(FG_M), t16 = tiles_of(SG_TILE);
+  for (int S = 1; S <= 8 && t32 * S <= 148; S *= 2) {
     const double t = 2.6 + 0.011 * K / S + (S > 1 ? 2.2 : 0.0) + (S == 8 ? 0.5 : 0.0);
-    if (t < best) { best = t; cluster = S; }
+    if (t < best) { best = t; plan.tile = FG_M; plan.cluster = S; }
   }
-  return cluster;
+  if (t16 <= 296 && 2.4 + 0.0055 * K * (t16 > 148 ? 1.6 : 1.0) * (aligned ? 1.0 : 1.5) < best) {
+    plan.tile = SG_TILE;
+    plan.cluster = 1;
+  }
+  return plan;
 }
 
 // How the operands of a launch are read: through their columns (rows contiguous, pitch stride_k) or their rows (K contiguous,
@@ -725,8 +1075,8 @@ static int direct_gemm_launch(Context &ctx, const DirectItem *items, int n) {
   bool at, bt, sums = false;
   for (int i = 0; i < n; ++i) sums = sums || items[i].row_sum != nullptr;   // these are taken from operands read through their columns
   if (!choose_reading(items, n, &DirectItem::A, sums, &at) || !choose_reading(items, n, &DirectItem::B, false, &bt)) return MYEA_E_INVALID;
-  const int fma = fma_cluster(items, n, at, bt);
-  const int tile_m = fma ? FG_M : DG_M, tile_n = fma ? FG_N : DG_N;
+  const FmaPlan fma = fma_plan(items, n, at, bt);
+  const int tile_m = fma.tile ? fma.tile : DG_M, tile_n = fma.tile ? fma.tile : DG_N;
   for (int i = 0; i < n; ++i) {
     const DirectItem &it = items[i];
     DirectProblem &p = g.p[i];
@@ -747,9 +1097,13 @@ static int direct_gemm_launch(Context &ctx, const DirectItem *items, int n) {
     min_steps = std::min(min_steps, (p.K + BK - 1) / BK);
     ctx.gemm_flops += 2.0 * p.M * p.N * static_cast<double>(p.K);
   }
-  if (fma) {
-    if (at) return bt ? launch_fma<true, true>(ctx, g, tiles, fma) : launch_fma<true, false>(ctx, g, tiles, fma);
-    return bt ? launch_fma<false, true>(ctx, g, tiles, fma) : launch_fma<false, false>(ctx, g, tiles, fma);
+  if (fma.tile == SG_TILE) {
+    if (at) return bt ? launch_small<true, true>(ctx, g, tiles) : launch_small<true, false>(ctx, g, tiles);
+    return bt ? launch_small<false, true>(ctx, g, tiles) : launch_small<false, false>(ctx, g, tiles);
+  }
+  if (fma.tile) {
+    if (at) return bt ? launch_fma<true, true>(ctx, g, tiles, fma.cluster) : launch_fma<true, false>(ctx, g, tiles, fma.cluster);
+    return bt ? launch_fma<false, true>(ctx, g, tiles, fma.cluster) : launch_fma<false, false>(ctx, g, tiles, fma.cluster);
   }
   // K is cut in up to four while the grid stays within one CTA per SM and every CTA keeps two stages.  Measured (us per
   // launch, cut 1 / 2 / 4 / 8): 128 x 256 x 256 9.6 / 8.0 / 6.6 / 7.2, 203 x 333 x 333 18.6 / 13.6 / 9.8 / 11.3, 512^3 15.7 / 11.2

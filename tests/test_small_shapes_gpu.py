@@ -1,5 +1,5 @@
 """GPU tests of the paths small and middle networks take, at the edges of their tiles: contractions straight from fp32
-operands (32 x 32 FMA tiles; 128 x 64 tensor-core tiles, 32 of K per stage, K cut over 1, 2, 4 or 8 CTAs), the one-launch
+operands (16 x 16 and 32 x 32 FMA tiles; 128 x 64 tensor-core tiles, 32 of K per stage, K cut over 1, 2, 4 or 8 CTAs), the one-launch
 normalization of short batches (8 columns per block, 4 to 32 rows per thread), the LSTM walks (resident weights: groups of 1
 to many CTAs, clusters, chunks of exchange data; which pass takes which), widths of one, and the updates and products that leave or read
 operand panels - against float64 products and the numpy restatement."""
@@ -29,6 +29,20 @@ def test_contraction_from_fp32_operands(M, N, K, accumulate):
     want = A.astype(np.float64) @ B.astype(np.float64).T + (out if accumulate else 0)
     assert lib.myea_b200_gemm_nt(0, 0, M, N, K, A.ctypes.data, B.ctypes.data, out.ctypes.data, accumulate, None, 0) == 0
     assert rel_err(out, want) < 5e-6
+
+
+# edges of the chunks of K (128, 124 where rows start off 16-byte boundaries) and of the 16 x 16 tiles, through rows and columns
+@pytest.mark.parametrize("K", [1, 3, 8, 123, 124, 125, 128, 129, 249, 256, 257, 333, 513])
+@pytest.mark.parametrize("M,N", [(1, 1), (17, 33), (203, 333), (128, 256)])
+@pytest.mark.parametrize("engine", [0, 1 << 17, 1 << 18, 3 << 17])
+def test_contraction_from_fp32_operands_over_k(M, N, K, engine):
+    lib = capi.load()
+    rng = np.random.default_rng(M + N + K)
+    A, B = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
+    out = np.zeros((M, N), np.float32)
+    a, b = np.ascontiguousarray(A.T) if engine & (1 << 17) else A, np.ascontiguousarray(B.T) if engine & (1 << 18) else B
+    assert lib.myea_b200_gemm_nt(0, engine, M, N, K, a.ctypes.data, b.ctypes.data, out.ctypes.data, 0, None, 0) == 0
+    assert rel_err(out, A.astype(np.float64) @ B.astype(np.float64).T) < 5e-6
 
 
 def _step(wl, seed=5, rows=None):
