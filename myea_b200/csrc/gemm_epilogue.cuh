@@ -106,15 +106,23 @@ __device__ __forceinline__ void epilogue_block32(const Epilogue &e, float *tr, c
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const float4 bias = e.bias != nullptr ? ld4(e.bias + n) : zero;
   const float4 cs = affine ? ld4(e.col_scale + n) : make_float4(1.f, 1.f, 1.f, 1.f), ch = affine ? ld4(e.col_shift + n) : zero;
+  // rows rsub + 4 i of the block; one pointer per array and a step between its rows (in segments every row has a place of its own)
+  const int rows = static_cast<int>(min(32ll, static_cast<long long>(M) - row0));
+  const long long first = row0 + rsub;
+  const bool segments = e.seg_rows != 0;
+  float *const c_first = e.C + first * e.ldc + n;
+  const long long c_step = 4 * e.ldc;
+  auto place = [&](int i) { return segments ? e.C + c_row(e, first + 4 * i) + n : c_first + i * c_step; };
   float4 add[ADD ? 8 : 1], pre[PRE ? 8 : 1], y[Y ? 8 : 1], old[ACC ? 8 : 1];
+  const float *const add_first = ADD ? e.addend + first * e.ld_addend + n : nullptr, *const pre_first = PRE ? e.aux_pre + first * e.ld_aux + n : nullptr,
+                    *const y_first = Y ? e.aux_y + first * e.ld_aux + n : nullptr;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const long long m = row0 + rsub + 4 * i;
-    const bool in = m < M;
-    if (ADD) add[i] = in ? ld4(e.addend + m * e.ld_addend + n) : zero;
-    if (PRE) pre[i] = in ? ld4(e.aux_pre + m * e.ld_aux + n) : zero;
-    if (Y) y[i] = in ? ld4(e.aux_y + m * e.ld_aux + n) : zero;
-    if (ACC) old[i] = in ? ld4(e.C + c_row(e, m) + n) : zero;
+    const bool in = rsub + 4 * i < rows;
+    if (ADD) add[i] = in ? ld4(add_first + i * (4 * e.ld_addend)) : zero;
+    if (PRE) pre[i] = in ? ld4(pre_first + i * (4 * e.ld_aux)) : zero;
+    if (Y) y[i] = in ? ld4(y_first + i * (4 * e.ld_aux)) : zero;
+    if (ACC) old[i] = in ? ld4(place(i)) : zero;
   }
   // column statistics of this 32 x 32 block: this lane's four columns over its eight rows first
   float4 st0 = zero, st1 = zero;
@@ -122,9 +130,15 @@ __device__ __forceinline__ void epilogue_block32(const Epilogue &e, float *tr, c
   __syncwarp();   // the block before has been read
   stage(tr);
   __syncwarp();
+  constexpr bool AHEAD = ADD + PRE + Y + ACC <= 1;   // (the rows wait in registers where there is room beside the other arrays)
+  float4 v[AHEAD ? 8 : 1];
+  if constexpr (AHEAD) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = *reinterpret_cast<const float4 *>(tr + tr_at(rsub + 4 * i, lane & 7));
+  }
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    float4 x = *reinterpret_cast<const float4 *>(tr + tr_at(rsub + 4 * i, lane & 7));
+    float4 x = AHEAD ? v[i] : *reinterpret_cast<const float4 *>(tr + tr_at(rsub + 4 * i, lane & 7));
     add4(x, bias);
     if (ADD) add4(x, add[i]);
     if (AUX != AUX_NONE) {
@@ -135,10 +149,9 @@ __device__ __forceinline__ void epilogue_block32(const Epilogue &e, float *tr, c
       }
       derive4<AUX>(e.deriv_af, x, z, Y ? y[i] : zero);
     }
-    const long long m = row0 + rsub + 4 * i;
     if (ACC) add4(x, old[i]);
-    if (m < M) {
-      *reinterpret_cast<float4 *>(e.C + c_row(e, m) + n) = x;
+    if (rsub + 4 * i < rows) {
+      *reinterpret_cast<float4 *>(place(i)) = x;
       if (STATS == 1) {
         add4(st0, x);
         st1.x = fmaf(x.x, x.x, st1.x); st1.y = fmaf(x.y, x.y, st1.y); st1.z = fmaf(x.z, x.z, st1.z); st1.w = fmaf(x.w, x.w, st1.w);
@@ -233,6 +246,7 @@ inline int epilogue_variant(const Epilogue &e) {
 // one copy of the code: the block's registers are picked by a uniform switch in front of the staging stores.
 template <int NCOLS>
 __device__ __forceinline__ void epilogue_strip(const Epilogue &e, int variant, float *tr, const float (&sum)[NCOLS], int lane, long long row0, long long col_base, int M, int N) {
+  __builtin_assume(__isShared(tr));   // (its address went through an integer on the way here)
 #pragma unroll 1
   for (int jc = 0; jc < NCOLS / 32; ++jc) {
     const long long col0 = col_base + jc * 32;

@@ -93,6 +93,22 @@ __device__ __forceinline__ void scaled_add2(float &s0, float &s1, uint32_t r0, u
       : "r"(r0), "r"(r1), "r"(columns << 16), "r"(columns & 0xffff0000u), "l"(row));
 }
 
+// What the epilogue will read of one row of a tile, on its way from HBM to L2 while the products are computed: behind the last of
+// them a single-wave contraction otherwise waits for arrays that earlier launches have left there.
+template <int COLS>
+__device__ __forceinline__ void prefetch_epilogue(const Epilogue &e, long long row, long long col, long long M, long long N) {
+  if (row >= M) return;
+  auto line = [](const float *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); };
+#pragma unroll
+  for (int j = 0; j < COLS; j += 32) {
+    if (col + j >= N) break;
+    if (e.aux_pre != nullptr) line(e.aux_pre + row * e.ld_aux + col + j);
+    if (e.aux_y != nullptr) line(e.aux_y + row * e.ld_aux + col + j);
+    if (e.addend != nullptr) line(e.addend + row * e.ld_addend + col + j);
+    if (e.accumulate) line(e.C + c_row(e, row) + col + j);
+  }
+}
+
 __device__ __forceinline__ void wide_tile_coords(const WideWork &w, int t, int &tm, int &tn) {
   const int per_band = HG_BAND * w.tiles_n;
   const int band = t / per_band;
@@ -153,6 +169,12 @@ __device__ __forceinline__ void half_load_operand(uint8_t *dst0, uint8_t *dst1, 
   }
 }
 
+template <bool COLS>
+__device__ __forceinline__ void half_prefetch_operand(const CUtensorMap *m, int kb, int row0) {
+  if (!COLS) asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(m), "r"(kb * HG_BK), "r"(row0) : "memory");
+  else asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(m), "r"(0), "r"(kb * HG_BK), "r"(row0 >> 6) : "memory");
+}
+
 template <int BN, bool A_COLS, bool B_COLS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(HG_THREADS, 1)
 half_gemm_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_constant__ CUtensorMap tm_a1, const __grid_constant__ CUtensorMap tm_b0,
@@ -199,7 +221,21 @@ half_gemm_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_constan
   ptx::cluster_sync_all();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  grid_dependency_wait();     // everything above touched no global memory
+  if (warp == 0 && lane == 0) {
+    // The first stages' rows of B on their way from HBM to L2 while the launch before this one drains (all CTAs at once want 28 MB
+    // before the first product).  A prefetch is no read: what that launch may still write there reaches L2 all the same.
+    WideSegments seg(work, cluster_id, num_clusters, num_chunks);
+    if (seg.next()) {
+      int tm, tn;
+      wide_tile_coords(work, seg.tile, tm, tn);
+      const int nb0 = tn * BN + static_cast<int>(cta_rank) * HALF_N;
+      for (int kb = seg.c0 * HG_KC; kb < min(num_kb, seg.c0 * HG_KC + STAGES); ++kb) {
+        half_prefetch_operand<B_COLS>(&tm_b0, kb, nb0);
+        half_prefetch_operand<B_COLS>(&tm_b1, kb, nb0);
+      }
+    }
+  }
+  grid_dependency_wait();     // everything above read no global memory
   grid_dependency_release();
 
   if (warp == 0) {
@@ -294,6 +330,8 @@ half_gemm_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_constan
       wide_tile_coords(work, seg.tile, tm, tn);
       const uint16_t *pa = scale_a.block(tm * 2 + static_cast<int>(cta_rank)) + q * 32 + lane;
       const uint16_t *pb = scale_b.block((tn * BN + half * HALF_N) / HP_BLOCK) + (half * HALF_N) % HP_BLOCK;
+      prefetch_epilogue<HALF_N>(epi, static_cast<long long>(tm) * 256 + static_cast<long long>(cta_rank) * 128 + q * 32 + lane,
+                                static_cast<long long>(tn) * BN + half * HALF_N, dims.M, dims.N);
       float sum[HALF_N];
 #pragma unroll
       for (int j = 0; j < HALF_N; ++j) sum[j] = 0.f;
@@ -375,12 +413,12 @@ half_gemm_kernel(const __grid_constant__ CUtensorMap tm_a0, const __grid_constan
             if (two && cc == cluster_id) continue;
             const float4 *theirs = slot_of(cc);
 #pragma unroll
-            for (int jb = 0; jb < HALF_N / 4; jb += 8) {
-              float4 v[8];
+            for (int jb = 0; jb < HALF_N / 4; jb += 16) {
+              float4 v[16];
 #pragma unroll
-              for (int j = 0; j < 8; ++j) v[j] = __ldcg(theirs + (jb + j) * 32 + lane);
+              for (int j = 0; j < 16; ++j) v[j] = __ldcg(theirs + (jb + j) * 32 + lane);
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
+              for (int j = 0; j < 16; ++j) {
                 sum[4 * (jb + j)] += v[j].x; sum[4 * (jb + j) + 1] += v[j].y; sum[4 * (jb + j) + 2] += v[j].z; sum[4 * (jb + j) + 3] += v[j].w;
               }
             }
@@ -579,7 +617,7 @@ int half_split(Context &ctx, const float *src, long long stride, const HalfPanel
 }
 
 bool epilogue_takes_stats(const Context &ctx, const Epilogue &e, long long N) {
-  if (ctx.gemm_engine != 0 || (N & 31) != 0 || e.ldc != N || e.seg_rows != 0) return false;
+  if (ctx.gemm_engine != 0 || (N & 31) != 0 || e.ldc != N || e.seg_rows != 0 || !derivative_is_fused(e.deriv_af)) return false;
   if (((reinterpret_cast<uintptr_t>(e.col_stats) | reinterpret_cast<uintptr_t>(e.col_mean)) & 15) != 0) return false;
   const int v = epilogue_variant(e);
   return v == EPI_PLAIN_STATS || v == EPI_PRE_STATS || v == EPI_Y_STATS || v == EPI_BOTH_STATS;
@@ -658,6 +696,15 @@ static int launch_half(Context &ctx, const HalfOperand &A, const HalfOperand &B,
     // partial sums, and past 8 that pass outweighs the shorter K walk
     constexpr int max_split = 8;
     per_cluster = std::max(per_cluster, (num_chunks + max_split - 1) / max_split);
+    // A run that ends inside a tile makes a third contributor and a second set of partial sums (7 - 9 kcycles at the end of a
+    // launch that walks a chunk in 3): where equal shares of a tile are hardly longer, every run is one share of one tile (32
+    // tiles on 74 pairs, 16 chunks instead of 14: 512 x 4096 x 4096 with the splits of its operands 84.7 -> 78.9 us, 2048 x 1024 x 2048 49.8
+    // -> 44.2).
+    const int shares = G / rem;
+    if (work.num_tiles == rem && shares >= 1) {
+      const int share = (num_chunks + shares - 1) / shares;
+      if (share - per_cluster <= 2 && num_chunks % share == 0) per_cluster = share;
+    }
     // splitting a tile costs about the time of two chunks (partial sums through L2, one counter round trip, the second
     // pass of the warp that arrives last): worth it when it takes at least three off the longest cluster
     if (num_chunks - per_cluster >= 3) {
