@@ -341,6 +341,7 @@ int output_error(Context &ctx, const float *pre, float *y, const float *desired,
 int column_sum(Context &ctx, const float *in, long long rows, long long H, float *out, int accumulate, float *partial,
                int chunks);
 int fill_zero(Context &ctx, float *p, size_t n);
+int copy_floats(Context &ctx, float *dst, const float *src, size_t n);   // both on the device
 
 struct OptLaunch {
   uint32_t type = 0;

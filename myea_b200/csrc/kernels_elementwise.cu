@@ -20,6 +20,8 @@ template <int VEC, int KIND>
 __global__ void __launch_bounds__(256) column_reduce_kernel(const float *__restrict__ x, const float *__restrict__ y,
                                                             const float *__restrict__ mean, long long rows, long long H,
                                                             int chunks, float *__restrict__ partial) {
+  grid_dependency_wait();
+  grid_dependency_release();
   __shared__ float s0[8][32 * VEC + 1];
   __shared__ float s1[8][32 * VEC + 1];
   const int cl = threadIdx.x & 31, rl = threadIdx.x >> 5;
@@ -88,10 +90,10 @@ static void launch_column_reduce(Context &ctx, const float *x, const float *y, c
   const bool vec4 = (H % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0) && (y == nullptr || (reinterpret_cast<uintptr_t>(y) & 15) == 0);
   if (vec4) {
     dim3 grid(static_cast<unsigned>((H + 127) / 128), chunks);
-    column_reduce_kernel<4, KIND><<<grid, 256, 0, ctx.stream>>>(x, y, mean, rows, H, chunks, partial);
+    launch_dependent(ctx, column_reduce_kernel<4, KIND>, grid, dim3(256), 0, x, y, mean, rows, H, chunks, partial);
   } else {
     dim3 grid(static_cast<unsigned>((H + 31) / 32), chunks);
-    column_reduce_kernel<1, KIND><<<grid, 256, 0, ctx.stream>>>(x, y, mean, rows, H, chunks, partial);
+    launch_dependent(ctx, column_reduce_kernel<1, KIND>, grid, dim3(256), 0, x, y, mean, rows, H, chunks, partial);
   }
 }
 
@@ -110,7 +112,8 @@ __device__ __forceinline__ void chunk_sums(const float *__restrict__ partial, in
   const int cl = threadIdx.x & 31, rl = threadIdx.x >> 5;
   float a = 0.f, b = 0.f;
   if (j < H) {
-#pragma unroll 4
+    // (16 loads in flight per thread: the way to L2 and back is all there is to this)
+#pragma unroll 8
     for (int c = rl; c < chunks; c += 8) { a += partial[(0ll * chunks + c) * H + j]; b += partial[(1ll * chunks + c) * H + j]; }
   }
   sh[0][rl][cl] = a;
@@ -135,13 +138,23 @@ __global__ void __launch_bounds__(256) chunk_sum_kernel(const float *__restrict_
 
 // statistics, running averages, r / d corrections and affine coefficients of column j from its sum s and sum of squares q
 // (one thread per column: the averages are updated in place)
-__device__ __forceinline__ void norm_stats_of_column(const NormParams &np, long long j, float s, float q, long long rows, int training, float &cs, float &ch) {
+// (what it reads besides the sums is fetched before they are formed)
+struct NormColumn {
+  float mean_avg = 0.f, sigma_avg = 0.f, gamma = 0.f, beta = 0.f;
+};
+__device__ __forceinline__ NormColumn norm_column(const NormParams &np, long long j) {
+  NormColumn c;
+  c.mean_avg = np.mean_avg[j]; c.sigma_avg = np.sigma_avg[j]; c.gamma = np.gamma[j]; c.beta = np.beta[j];
+  return c;
+}
+__device__ __forceinline__ void norm_stats_of_column(const NormParams &np, const NormColumn &c, long long j, float s, float q, long long rows, int training, float &cs,
+                                                     float &ch) {
   float mean, sigma, r = 1.f, d = 0.f;
   if (training) {
     const float scale = 1.0f / static_cast<float>(rows);
     mean = s * scale;
     sigma = sqrtf(q * scale - mean * mean + np.epsilon);
-    float ma = np.mean_avg[j], sa = np.sigma_avg[j];
+    float ma = c.mean_avg, sa = c.sigma_avg;
     ma += np.momentum * (mean - ma);
     sa += np.momentum * (sigma - sa);
     if (np.type == MYEA_NORM_BATCH_RENORMALIZATION) {
@@ -155,10 +168,10 @@ __device__ __forceinline__ void norm_stats_of_column(const NormParams &np, long 
     np.r[j] = r;
     np.d[j] = d;
   } else {
-    mean = np.mean_avg[j];
-    sigma = np.sigma_avg[j];
+    mean = c.mean_avg;
+    sigma = c.sigma_avg;
   }
-  const float g = np.gamma[j], b = np.beta[j];
+  const float g = c.gamma, b = c.beta;
   const float k = r / sigma;
   cs = g * k;
   ch = b + g * (d - mean * k);
@@ -173,11 +186,13 @@ __global__ void __launch_bounds__(256) norm_stats_finalize_kernel(const float *_
   grid_dependency_wait();
   grid_dependency_release();
   const long long j = blockIdx.x * 32ll + (threadIdx.x & 31);
+  NormColumn column;
+  if (threadIdx.x < 32 && j < H) column = norm_column(np, j);
   float s = 0.f, q = 0.f;
   if (training) chunk_sums(partial, chunks, H, j, s, q);
   if (threadIdx.x >= 32 || j >= H) return;
   float cs, ch;
-  norm_stats_of_column(np, j, s, q, rows, training, cs, ch);
+  norm_stats_of_column(np, column, j, s, q, rows, training, cs, ch);
 }
 
 int norm_forward_stats(Context &ctx, const float *z, long long rows, long long H, const NormParams &np, int training,
@@ -231,6 +246,8 @@ __global__ void __launch_bounds__(256) activation_forward_kernel(const float *__
                                                                  long long H, uint32_t af, const float *__restrict__ col_scale,
                                                                  const float *__restrict__ col_shift,
                                                                  const uint8_t *__restrict__ mask, float keep_scale) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const long long hv = H / VEC;
   const long long total = rows * hv;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -269,6 +286,8 @@ __global__ void __launch_bounds__(256) activation_forward_cols_kernel(const floa
                                                                       long long H, const float *__restrict__ col_scale,
                                                                       const float *__restrict__ col_shift, const uint8_t *__restrict__ mask,
                                                                       float keep_scale) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const long long c = (blockIdx.x * 256ll + threadIdx.x) * 4;
   if (c >= H) return;
   const bool affine = col_scale != nullptr;
@@ -400,7 +419,7 @@ int activation_forward(Context &ctx, const float *z, float *out, long long rows,
   const int blocks = static_cast<int>(std::max<long long>(1, std::min<long long>((total + 255) / 256, 148 * 16)));
   if (vec4) {
     const dim3 grid = column_walk_grid(rows, H);
-#define MYEA_AF_CASE(A) case A: activation_forward_cols_kernel<A><<<grid, 256, 0, ctx.stream>>>(z, out, rows, H, col_scale, col_shift, mask, keep_scale); break
+#define MYEA_AF_CASE(A) case A: launch_dependent(ctx, activation_forward_cols_kernel<A>, grid, dim3(256), 0, z, out, rows, H, col_scale, col_shift, mask, keep_scale); break
     switch (af) {
       MYEA_AF_CASE(MYEA_AF_TANH);
       MYEA_AF_CASE(MYEA_AF_SIGMOID);
@@ -408,11 +427,11 @@ int activation_forward(Context &ctx, const float *z, float *out, long long rows,
       MYEA_AF_CASE(MYEA_AF_LEAKY_RELU);
       MYEA_AF_CASE(MYEA_AF_ELU);
       MYEA_AF_CASE(MYEA_AF_SELU);
-      default: activation_forward_kernel<4><<<blocks, 256, 0, ctx.stream>>>(z, out, rows, H, af, col_scale, col_shift, mask, keep_scale); break;
+      default: launch_dependent(ctx, activation_forward_kernel<4>, dim3(blocks), dim3(256), 0, z, out, rows, H, af, col_scale, col_shift, mask, keep_scale); break;
     }
 #undef MYEA_AF_CASE
   } else
-    activation_forward_kernel<1><<<blocks, 256, 0, ctx.stream>>>(z, out, rows, H, af, col_scale, col_shift, mask, keep_scale);
+    launch_dependent(ctx, activation_forward_kernel<1>, dim3(blocks), dim3(256), 0, z, out, rows, H, af, col_scale, col_shift, mask, keep_scale);
   ctx.end(TC_ELEMENTWISE);
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
@@ -475,6 +494,8 @@ __global__ void __launch_bounds__(256) norm_activation_strip_kernel(const float 
   const int rl = threadIdx.x >> 3;
   const long long j = blockIdx.x * 8ll + (threadIdx.x & 7);
   const bool in = j < H;
+  NormColumn column;
+  if (rl == 0 && in) column = norm_column(np, j);
   float v[NR], s = 0.f, q = 0.f;
 #pragma unroll
   for (int i = 0; i < NR; ++i) {
@@ -487,7 +508,7 @@ __global__ void __launch_bounds__(256) norm_activation_strip_kernel(const float 
     strip_sums(s, q);
   }
   __shared__ float coef[2][8];
-  if (rl == 0 && in) norm_stats_of_column(np, j, s, q, rows, training, coef[0][threadIdx.x], coef[1][threadIdx.x]);
+  if (rl == 0 && in) norm_stats_of_column(np, column, j, s, q, rows, training, coef[0][threadIdx.x], coef[1][threadIdx.x]);
   __syncthreads();
   if (!in) return;
   const float cs = coef[0][threadIdx.x & 7], ch = coef[1][threadIdx.x & 7];
@@ -565,6 +586,8 @@ __global__ void __launch_bounds__(128) softmax_forward_kernel(const float *__res
 __global__ void __launch_bounds__(256) activation_backward_kernel(float *__restrict__ d, const float *__restrict__ z, const float *__restrict__ y,
                                                                   long long rows, long long H, uint32_t af, const float *__restrict__ col_scale,
                                                                   const float *__restrict__ col_shift) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const long long total = rows * H;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -580,7 +603,7 @@ int activation_backward(Context &ctx, float *d, const float *z, const float *y, 
   if (rows <= 0 || H <= 0) return MYEA_OK;
   ctx.begin(TC_ELEMENTWISE);
   const int blocks = static_cast<int>(std::max<long long>(1, std::min<long long>((rows * H + 255) / 256, 148 * 16)));
-  activation_backward_kernel<<<blocks, 256, 0, ctx.stream>>>(d, z, y, rows, H, af, col_scale, col_shift);
+  launch_dependent(ctx, activation_backward_kernel, dim3(blocks), dim3(256), 0, d, z, y, rows, H, af, col_scale, col_shift);
   ctx.end(TC_ELEMENTWISE);
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
@@ -603,14 +626,23 @@ int softmax_forward(Context &ctx, const float *z, float *out, long long rows, lo
 // d_mean = -gamma*(r/sigma)*S1, d_sigma = -gamma*(r/sigma^2)*S2, so one reduction pass and one apply pass suffice.
 // r and d are constants of the backward pass, as in the reference.
 // ---------------------------------------------------------------------------------------------------------
+// (what the two read besides the sums is fetched before they are formed)
+struct NormBackwardColumn {
+  float sigma = 1.f, r = 0.f, d = 0.f, gamma = 0.f;
+};
+__device__ __forceinline__ NormBackwardColumn norm_backward_column(const NormParams &np, long long j) {
+  NormBackwardColumn c;
+  c.sigma = np.sigma[j]; c.r = np.r[j]; c.d = np.d[j]; c.gamma = np.gamma[j];
+  return c;
+}
 // d_gamma and d_beta of column j
-__device__ __forceinline__ void norm_backward_parameters(const NormParams &np, long long j, float s1, float s2) {
+__device__ __forceinline__ void norm_backward_parameters(const NormParams &np, const NormBackwardColumn &c, long long j, float s1, float s2) {
   np.d_beta[j] += s1;
-  np.d_gamma[j] += np.r[j] / np.sigma[j] * s2 + np.d[j] * s1;
+  np.d_gamma[j] += c.r / c.sigma * s2 + c.d * s1;
 }
 // error = delta * k0 + (z - mean) * k1 + k2
-__device__ __forceinline__ void norm_backward_coefficients(const NormParams &np, long long j, float s1, float s2, long long rows, float &k0, float &k1, float &k2) {
-  const float sigma = np.sigma[j], r = np.r[j], g = np.gamma[j];
+__device__ __forceinline__ void norm_backward_coefficients(const NormBackwardColumn &c, float s1, float s2, long long rows, float &k0, float &k1, float &k2) {
+  const float sigma = c.sigma, r = c.r, g = c.gamma;
   const float k = r / sigma;
   const float d_mean = -g * k * s1;
   const float d_sigma = -g * (r / (sigma * sigma)) * s2;
@@ -625,18 +657,22 @@ __global__ void __launch_bounds__(256) norm_backward_finalize_kernel(const float
   grid_dependency_wait();
   grid_dependency_release();
   const long long j = blockIdx.x * 32ll + (threadIdx.x & 31);
+  NormBackwardColumn column;
+  if (threadIdx.x < 32 && j < H) column = norm_backward_column(np, j);
   float s1, s2;
   chunk_sums(partial, chunks, H, j, s1, s2);
   if (threadIdx.x >= 32 || j >= H) return;
-  norm_backward_parameters(np, j, s1, s2);
+  norm_backward_parameters(np, column, j, s1, s2);
   if (global != nullptr) { s1 = global[j]; s2 = global[H + j]; }
-  norm_backward_coefficients(np, j, s1, s2, rows, coef[0 * H + j], coef[1 * H + j], coef[2 * H + j]);
+  norm_backward_coefficients(column, s1, s2, rows, coef[0 * H + j], coef[1 * H + j], coef[2 * H + j]);
 }
 
 template <int VEC>
 __global__ void __launch_bounds__(256) norm_backward_apply_kernel(const float *__restrict__ z, const float *__restrict__ delta,
                                                                   float *__restrict__ out, long long rows, long long H,
                                                                   const float *__restrict__ mean, const float *__restrict__ coef) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const long long hv = H / VEC;
   const long long total = rows * hv;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -667,6 +703,8 @@ __global__ void __launch_bounds__(256) norm_backward_apply_kernel(const float *_
 __global__ void __launch_bounds__(256) norm_backward_apply_cols_kernel(const float *__restrict__ z, const float *__restrict__ delta,
                                                                        float *__restrict__ out, long long rows, long long H,
                                                                        const float *__restrict__ mean, const float *__restrict__ coef) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const long long c = (blockIdx.x * 256ll + threadIdx.x) * 4;
   if (c >= H) return;
   const float4 mu = *reinterpret_cast<const float4 *>(mean + c);
@@ -704,6 +742,8 @@ __global__ void __launch_bounds__(256) norm_backward_strip_kernel(const float *_
   const long long j = blockIdx.x * 8ll + (threadIdx.x & 7);
   const bool in = j < H;
   const float mu = in ? np.mean[j] : 0.f;
+  NormBackwardColumn column;
+  if (in) column = norm_backward_column(np, j);
   float x[NR], e[NR], s1 = 0.f, s2 = 0.f;
 #pragma unroll
   for (int i = 0; i < NR; ++i) {
@@ -721,8 +761,8 @@ __global__ void __launch_bounds__(256) norm_backward_strip_kernel(const float *_
   strip_sums(s1, s2);
   if (!in) return;
   float k0, k1, k2;
-  norm_backward_coefficients(np, j, s1, s2, rows, k0, k1, k2);
-  if (rl == 0) norm_backward_parameters(np, j, s1, s2);
+  norm_backward_coefficients(column, s1, s2, rows, k0, k1, k2);
+  if (rl == 0) norm_backward_parameters(np, column, j, s1, s2);
 #pragma unroll
   for (int i = 0; i < NR; ++i) {
     const long long r = rl + 32 * i;
@@ -767,11 +807,11 @@ int norm_backward(Context &ctx, const float *z, const float *delta_af, float *de
   if (sink != nullptr)
     half_produce(ctx, NormBackwardProducer{z, delta_af, delta_out, H, np.mean, coef, vec4}, *sink);
   else if (cols_ok)
-    norm_backward_apply_cols_kernel<<<column_walk_grid(rows, H), 256, 0, ctx.stream>>>(z, delta_af, delta_out, rows, H, np.mean, coef);
+    launch_dependent(ctx, norm_backward_apply_cols_kernel, column_walk_grid(rows, H), dim3(256), 0, z, delta_af, delta_out, rows, H, np.mean, coef);
   else if (vec4)
-    norm_backward_apply_kernel<4><<<blocks, 256, 0, ctx.stream>>>(z, delta_af, delta_out, rows, H, np.mean, coef);
+    launch_dependent(ctx, norm_backward_apply_kernel<4>, dim3(blocks), dim3(256), 0, z, delta_af, delta_out, rows, H, np.mean, coef);
   else
-    norm_backward_apply_kernel<1><<<blocks, 256, 0, ctx.stream>>>(z, delta_af, delta_out, rows, H, np.mean, coef);
+    launch_dependent(ctx, norm_backward_apply_kernel<1>, dim3(blocks), dim3(256), 0, z, delta_af, delta_out, rows, H, np.mean, coef);
   ctx.end(TC_NORM, 3);
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
@@ -860,6 +900,8 @@ int output_error(Context &ctx, const float *pre, float *y, const float *desired,
 // ---------------------------------------------------------------------------------------------------------
 __global__ void column_sum_finalize_kernel(const float *__restrict__ partial, int chunks, long long H, float *__restrict__ out,
                                            int accumulate) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const long long j = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (j >= H) return;
   float s = 0.f;
@@ -872,9 +914,38 @@ int column_sum(Context &ctx, const float *in, long long rows, long long H, float
   ctx.begin(TC_ELEMENTWISE);
   const int chunks = pick_chunks(rows, H, (H % 4 == 0) ? 4 : 1, max_chunks);
   launch_column_reduce<RK_SUM>(ctx, in, nullptr, nullptr, rows, H, chunks, partial);
-  column_sum_finalize_kernel<<<static_cast<unsigned>((H + 255) / 256), 256, 0, ctx.stream>>>(partial, chunks, H, out, accumulate);
+  launch_dependent(ctx, column_sum_finalize_kernel, dim3(static_cast<unsigned>((H + 255) / 256)), dim3(256), 0, partial, chunks, H, out, accumulate);
   ctx.end(TC_ELEMENTWISE, 2);
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
+}
+
+// Batches that a step copies into place: as a kernel the copy starts under the tail of the launch before it and lets the next one
+// start under its own (a copy by the driver waits for the first and holds up the second).
+__global__ void __launch_bounds__(256) copy_kernel(float *__restrict__ dst, const float *__restrict__ src, size_t n, int vec) {
+  grid_dependency_wait();
+  grid_dependency_release();
+  const size_t stride = static_cast<size_t>(gridDim.x) * 256, first = blockIdx.x * static_cast<size_t>(256) + threadIdx.x;
+  const size_t n4 = vec ? n >> 2 : 0;
+  for (size_t i = first; i < n4; i += 4 * stride) {
+    float4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i + k * stride < n4) v[k] = reinterpret_cast<const float4 *>(src)[i + k * stride];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i + k * stride < n4) reinterpret_cast<float4 *>(dst)[i + k * stride] = v[k];
+  }
+  for (size_t i = 4 * n4 + first; i < n; i += stride) dst[i] = src[i];
+}
+
+int copy_floats(Context &ctx, float *dst, const float *src, size_t n) {
+  const int vec = ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0;
+  const size_t per_block = vec ? 256 * 16 : 256 * 4;
+  const int blocks = static_cast<int>(std::max<size_t>(1, std::min<size_t>((n + per_block - 1) / per_block, 148 * 4)));
+  ctx.begin(TC_ELEMENTWISE);
+  const cudaError_t err = launch_dependent(ctx, copy_kernel, dim3(blocks), dim3(256), 0, dst, src, n, vec);
+  ctx.end(TC_ELEMENTWISE);
+  return err == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
 
 int fill_zero(Context &ctx, float *p, size_t n) {

@@ -143,6 +143,8 @@ __global__ void __launch_bounds__(256) lstm_cell_backward_kernel(const CellBwd p
 __global__ void __launch_bounds__(256) lstm_bias_peephole_reduce_kernel(const float *__restrict__ dgates, const float *__restrict__ cstate,
                                                                         long long R, long long C, long long shift, int chunks,
                                                                         float *__restrict__ partial) {
+  grid_dependency_wait();
+  grid_dependency_release();
   __shared__ float sh[7][8][33];
   const int cl = threadIdx.x & 31, rl = threadIdx.x >> 5;
   const long long c = static_cast<long long>(blockIdx.x) * 32 + cl;
@@ -180,16 +182,21 @@ __global__ void __launch_bounds__(256) lstm_bias_peephole_reduce_kernel(const fl
 // 32 cells per block, the chunks of a sum spread over 8 threads per cell
 __global__ void __launch_bounds__(256) lstm_bias_peephole_finalize_kernel(const float *__restrict__ partial, int chunks, long long C, float *d_bias,
                                                                           float *d_peep, long long stride) {
+  grid_dependency_wait();
+  grid_dependency_release();
   __shared__ float sh[7][8][33];
   const int cl = threadIdx.x & 31, rl = threadIdx.x >> 5;
   const long long c = static_cast<long long>(blockIdx.x) * 32 + cl;
+  float sum[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (c < C) {
+#pragma unroll 4
+    for (int ch = rl; ch < chunks; ch += 8) {
 #pragma unroll
-  for (int k = 0; k < 7; ++k) {
-    float t = 0.f;
-    if (c < C)
-      for (int ch = rl; ch < chunks; ch += 8) t += partial[(static_cast<long long>(k) * chunks + ch) * C + c];
-    sh[k][rl][cl] = t;
+      for (int k = 0; k < 7; ++k) sum[k] += partial[(static_cast<long long>(k) * chunks + ch) * C + c];
+    }
   }
+#pragma unroll
+  for (int k = 0; k < 7; ++k) sh[k][rl][cl] = sum[k];
   __syncthreads();
   if (rl != 0 || c >= C) return;
   float t[7];
@@ -212,6 +219,8 @@ __global__ void __launch_bounds__(256) lstm_bias_peephole_finalize_kernel(const 
 
 // peepholes p_i, p_f, p_o of every cell, gathered from the blocks of the parameter buffer into [3][C]
 __global__ void lstm_gather_peepholes_kernel(const float *__restrict__ peep, long long stride, long long C, float *__restrict__ out) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (c >= C) return;
   out[c] = peep[c * stride];
@@ -223,6 +232,8 @@ __global__ void lstm_gather_peepholes_kernel(const float *__restrict__ peep, lon
 // direction; the cell input's row lies at off_z, the three gates' rows at off_gates, one after the other)
 __global__ void __launch_bounds__(256) lstm_gather_weights_kernel(const float *__restrict__ w0, const float *__restrict__ w1, long long stride, long long off_z,
                                                                   long long off_gates, long long width, long long C, float *__restrict__ out) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const long long total = 4 * C * width;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total; i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const long long r = i / width, k = i - r * width, g = r / C, c = r - g * C;
@@ -505,7 +516,7 @@ static int lay_out_recurrent_weights(myea_b200_net *net, LstmPlan *P, const Bloc
     const float *w = net->params + P->d[d].w_base;
     if (lstm_persistent_ready(P)) {
       ctx.begin(TC_RECURRENT);
-      lstm_gather_peepholes_kernel<<<static_cast<unsigned>((C + 255) / 256), 256, 0, ctx.stream>>>(w + off.peep, P->stride, C, P->peep_compact + static_cast<size_t>(d) * 3 * C);
+      launch_dependent(ctx, lstm_gather_peepholes_kernel, dim3(static_cast<unsigned>((C + 255) / 256)), dim3(256), 0, w + off.peep, P->stride, C, P->peep_compact + static_cast<size_t>(d) * 3 * C);
       ctx.end(TC_RECURRENT);
       ctx.begin(TC_SPLIT);
       const GroupedGateRows src{w, P->stride, {rec[0], rec[1], rec[2], rec[3]}, C, vec8(w, P->stride, rec[0] | rec[1] | rec[2] | rec[3])};
@@ -521,7 +532,7 @@ static int lay_out_recurrent_weights(myea_b200_net *net, LstmPlan *P, const Bloc
       LRC(half_split(ctx, w, P->stride, P->w_rec[d], &seg));
     } else {
       ctx.begin(TC_RECURRENT);
-      lstm_gather_weights_kernel<<<static_cast<unsigned>(std::min<long long>((4 * C * C + 255) / 256, 148 * 8)), 256, 0, ctx.stream>>>(w, nullptr, P->stride, rec[0], rec[1], C, C,
+      launch_dependent(ctx, lstm_gather_weights_kernel, dim3(static_cast<unsigned>(std::min<long long>((4 * C * C + 255) / 256, 148 * 8))), dim3(256), 0, w, nullptr, P->stride, rec[0], rec[1], C, C,
                                                                                                                                    P->w_rec_mem[d]);
       ctx.end(TC_RECURRENT);
     }
@@ -715,7 +726,7 @@ int lstm_backward_to_input(myea_b200_net *net, LayerPlan &L, float *prev_deriv, 
   const bool gathered = P->w_in_mem[0] == nullptr;
   if (gathered) {  // the input weights gathered out of the blocks once (their four gate matrices are one K range then)
     ctx.begin(TC_RECURRENT);
-    lstm_gather_weights_kernel<<<static_cast<unsigned>(std::min<long long>((4 * C * n_in + 255) / 256, 148 * 8)), 256, 0, ctx.stream>>>(
+    launch_dependent(ctx, lstm_gather_weights_kernel, dim3(static_cast<unsigned>(std::min<long long>((4 * C * n_in + 255) / 256, 148 * 8))), dim3(256), 0, 
         net->params + P->d[0].w_base, P->dirs > 1 ? net->params + P->d[1].w_base : nullptr, P->stride, off.z_in, off.in[0], n_in, C, net->scratch.base);
     ctx.end(TC_RECURRENT);
   }
@@ -807,8 +818,8 @@ int lstm_update_derivative_weight(myea_b200_net *net, LayerPlan &L, const float 
     const int chunks = static_cast<int>(std::max<long long>(1, std::min<long long>(net->reduce_chunks, rows / 8)));
     ctx.begin(TC_RECURRENT);
     dim3 grid(static_cast<unsigned>((C + 31) / 32), chunks);
-    lstm_bias_peephole_reduce_kernel<<<grid, 256, 0, ctx.stream>>>(D.dgates, D.cstate, rows, C, shift, chunks, P->partial);
-    lstm_bias_peephole_finalize_kernel<<<static_cast<unsigned>((C + 31) / 32), 256, 0, ctx.stream>>>(P->partial, chunks, C, net->grads + D.b_base,
+    launch_dependent(ctx, lstm_bias_peephole_reduce_kernel, grid, dim3(256), 0, D.dgates, D.cstate, rows, C, shift, chunks, P->partial);
+    launch_dependent(ctx, lstm_bias_peephole_finalize_kernel, dim3(static_cast<unsigned>((C + 31) / 32)), dim3(256), 0, P->partial, chunks, C, net->grads + D.b_base,
                                                                                                     gw + off.peep, P->stride);
     ctx.end(TC_RECURRENT, 2);
   }

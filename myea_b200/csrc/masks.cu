@@ -53,6 +53,8 @@ __device__ __forceinline__ float draw_uniform(const DrawStream &s, unsigned long
 // direction of a bidirectional layer ([T][C] on the device) take its elements from the [T][dirs * C] numbering
 __global__ void draw_mask_kernel(uint8_t *__restrict__ out, long long n, float p, uint8_t below, uint8_t other, long long inner,
                                  long long outer_pitch, long long offset, const DrawStream s) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
   const long long e = (i / inner) * outer_pitch + offset + (i % inner);
@@ -64,6 +66,8 @@ __global__ void draw_mask_kernel(uint8_t *__restrict__ out, long long n, float p
 // 2 x 4 Mi elements: 10 us in one launch (one block and one 4-byte store per element took three launches and 43 us).
 __global__ void draw_shakedrop_kernel(float *__restrict__ out_a, float *__restrict__ out_b, long long n, uint32_t stream_a, uint32_t stream_b,
                                       uint8_t *__restrict__ mask, long long rows, float p, const DrawStream s) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   if (i < rows) mask[i] = draw_uniform(s, static_cast<unsigned long long>(i)) < p ? 1 : 0;
   if (4 * i >= n) return;
@@ -98,7 +102,7 @@ extern "C" int myea_b200_generate_masks(myea_handle net, uint64_t seed, uint64_t
       const long long n = net->T * L.n_out;
       s.stream = static_cast<uint32_t>(8 * l + MYEA_MASK_BERNOULLI);
       ctx.begin(TC_ELEMENTWISE);
-      draw_mask_kernel<<<blocks_for(n), 256, 0, ctx.stream>>>(L.mask_bernoulli, n, L.desc.dropout_values[0], 1, 0, n, 0, 0, s);
+      launch_dependent(ctx, draw_mask_kernel, dim3(blocks_for(n)), dim3(256), 0, L.mask_bernoulli, n, L.desc.dropout_values[0], 1, 0, n, 0, 0, s);
       ctx.end(TC_ELEMENTWISE);
     }
     if (L.type == MYEA_LAYER_LSTM && L.desc.type_dropout == MYEA_DROPOUT_ZONEOUT) {
@@ -112,9 +116,9 @@ extern "C" int myea_b200_generate_masks(myea_handle net, uint64_t seed, uint64_t
         const long long n = net->T * cells;
         ctx.begin(TC_ELEMENTWISE);
         s.stream = static_cast<uint32_t>(8 * l + MYEA_MASK_ZONEOUT_STATE);
-        draw_mask_kernel<<<blocks_for(n), 256, 0, ctx.stream>>>(zs, n, ps, 0, 1, cells, dirs * cells, d * cells, s);
+        launch_dependent(ctx, draw_mask_kernel, dim3(blocks_for(n)), dim3(256), 0, zs, n, ps, 0, 1, cells, dirs * cells, d * cells, s);
         s.stream = static_cast<uint32_t>(8 * l + MYEA_MASK_ZONEOUT_OUTPUT);
-        draw_mask_kernel<<<blocks_for(n), 256, 0, ctx.stream>>>(zo, n, po, 0, 1, cells, dirs * cells, d * cells, s);
+        launch_dependent(ctx, draw_mask_kernel, dim3(blocks_for(n)), dim3(256), 0, zo, n, po, 0, 1, cells, dirs * cells, d * cells, s);
         ctx.end(TC_ELEMENTWISE, 2);
       }
     }
@@ -122,7 +126,7 @@ extern "C" int myea_b200_generate_masks(myea_handle net, uint64_t seed, uint64_t
       const long long n = net->B * L.n_out;
       ctx.begin(TC_ELEMENTWISE);
       s.stream = static_cast<uint32_t>(8 * l + MYEA_MASK_SHAKEDROP);
-      draw_shakedrop_kernel<<<blocks_for(std::max((n + 3) / 4, net->B)), 256, 0, ctx.stream>>>(
+      launch_dependent(ctx, draw_shakedrop_kernel, dim3(blocks_for(std::max((n + 3) / 4, net->B))), dim3(256), 0, 
           L.shake_alpha, L.shake_beta, n, static_cast<uint32_t>(8 * l + MYEA_MASK_SHAKEDROP_ALPHA), static_cast<uint32_t>(8 * l + MYEA_MASK_SHAKEDROP_BETA),
           L.shake_mask, net->B, L.desc.dropout_values[0], s);
       ctx.end(TC_ELEMENTWISE);

@@ -785,10 +785,31 @@ static int batch_for_forward(myea_b200_net *net, uint64_t batch) {
 // rows the kernels of the step in flight run over, and the rows per time step among them
 static long long pitch_rows(const myea_b200_net *net) { return net->pitch(); }
 static long long step_rows_total(const myea_b200_net *net) { return net->T * pitch_rows(net); }
+// whether a kernel on this handle's device may read all of [p, p + bytes): what the driver's copy would find out, and refuse, by itself
+static bool readable_here(const myea_b200_net *net, const void *p, size_t bytes) {
+  typedef CUresult (*AddressRange)(CUdeviceptr *, size_t *, CUdeviceptr);
+  static const AddressRange range = [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    return cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &found) == cudaSuccess && found == cudaDriverEntryPointSuccess
+               ? reinterpret_cast<AddressRange>(f) : static_cast<AddressRange>(nullptr);
+  }();
+  cudaPointerAttributes at;
+  if (range == nullptr || cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return false; }
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  const CUdeviceptr q = reinterpret_cast<CUdeviceptr>(p);
+  return at.type == cudaMemoryTypeDevice && at.device == net->ctx.device && range(&base, &size, q) == CUDA_SUCCESS && q >= base && q - base <= size &&
+         bytes <= size - (q - base);
+}
 // host or device block packed [T][active_B][units] -> [T][pitch][units], padding rows zeroed
 static int copy_batch_in(myea_b200_net *net, float *dst, const float *src, long long units, cudaMemcpyKind kind, cudaStream_t stream) {
   const long long pitch = pitch_rows(net), b = net->active_B;
   if (b == pitch) {
+    // (past 4 MB the driver's copy is as fast)
+    const size_t n = static_cast<size_t>(net->T * b * units);
+    if (kind == cudaMemcpyDeviceToDevice && stream == net->ctx.stream && n <= (1u << 20) && readable_here(net, src, n * sizeof(float)))
+      return copy_floats(net->ctx, dst, src, n);
     CK(cudaMemcpyAsync(dst, src, net->T * b * units * sizeof(float), kind, stream));
     return MYEA_OK;
   }

@@ -223,6 +223,8 @@ int optimizer_update_panels(Context &ctx, const OptLaunch &o, const OptArrays &a
 
 // sum of squares of the whole derivative buffer, double accumulation across blocks
 __global__ void __launch_bounds__(256) sum_squares_kernel(const float *__restrict__ g, size_t n, double *out) {
+  grid_dependency_wait();
+  grid_dependency_release();
   __shared__ float sh[8];
   float s = 0.f;
   const size_t n4 = n >> 2;
@@ -245,18 +247,20 @@ int sum_squares(Context &ctx, const float *g, size_t n, double *d_out, bool accu
   ctx.begin(TC_OPTIMIZER);
   if (!accumulate) cudaMemsetAsync(d_out, 0, sizeof(double), ctx.stream);
   const int blocks = static_cast<int>(std::max<size_t>(1, std::min<size_t>(((n >> 2) + 255) / 256, 148 * 8)));
-  sum_squares_kernel<<<blocks, 256, 0, ctx.stream>>>(g, n, d_out);
+  launch_dependent(ctx, sum_squares_kernel, dim3(blocks), dim3(256), 0, g, n, d_out);
   ctx.end(TC_OPTIMIZER);
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
 
 __global__ void clip_scale_kernel(const double *sumsq, float clip, float *scale) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const float norm = sqrtf(static_cast<float>(*sumsq));
   *scale = norm >= clip ? clip / norm : 1.0f;
 }
 
 int clip_scale_from_norm(Context &ctx, const double *d_sumsq, float clip, float *d_scale) {
-  clip_scale_kernel<<<1, 1, 0, ctx.stream>>>(d_sumsq, clip, d_scale);
+  launch_dependent(ctx, clip_scale_kernel, dim3(1), dim3(1), 0, d_sumsq, clip, d_scale);
   ctx.launches += 1;
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }

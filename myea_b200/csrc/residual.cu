@@ -34,6 +34,8 @@ template <int VEC>
 __global__ void __launch_bounds__(256) shakedrop_kernel(const float *__restrict__ x, const float *__restrict__ s, float *__restrict__ out,
                                                         const uint8_t *__restrict__ mask, const float *__restrict__ coef, float scale,
                                                         long long rows, long long H) {
+  grid_dependency_wait();
+  grid_dependency_release();
   const long long hv = H / VEC, total = rows * hv;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -145,8 +147,8 @@ static int launch_shakedrop(Context &ctx, const float *x, const float *s, float 
   }
   const long long total = rows * (vec4 ? H / 4 : H);
   const int blocks = static_cast<int>(std::max<long long>(1, std::min<long long>((total + 255) / 256, 148 * 16)));
-  if (vec4) shakedrop_kernel<4><<<blocks, 256, 0, ctx.stream>>>(x, s, out, mask, coef, scale, rows, H);
-  else shakedrop_kernel<1><<<blocks, 256, 0, ctx.stream>>>(x, s, out, mask, coef, scale, rows, H);
+  if (vec4) launch_dependent(ctx, shakedrop_kernel<4>, dim3(blocks), dim3(256), 0, x, s, out, mask, coef, scale, rows, H);
+  else launch_dependent(ctx, shakedrop_kernel<1>, dim3(blocks), dim3(256), 0, x, s, out, mask, coef, scale, rows, H);
   ctx.end(TC_ELEMENTWISE);
   return cudaGetLastError() == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
