@@ -173,9 +173,24 @@ const float *residual_fc_input(myea_b200_net *net, int r, int k) {
   return k == 1 ? net->layers[net->layers[r].input_layer].values : net->layers[r + k].values;
 }
 
+// Whether the contraction behind `e` (rows x N, K = k) can leave the column sums of its result for normalization `np`: on operand
+// panels, in the vector epilogue.  The number of row blocks it leaves, or 0; e carries them then.
+static int sums_from_product(const myea_b200_net *net, const LayerPlan &L, Epilogue &e, int kind, const NormParams &np, long long rows, long long N, long long k) {
+  if (!L.shared_panels || direct_gemm_suits(net->ctx, rows, N, k)) return 0;
+  Epilogue probe = e;
+  probe.stats_kind = kind;
+  probe.col_stats = np.partial;
+  probe.col_mean = kind == 2 ? np.mean : nullptr;
+  probe.stats_blocks = (rows + 31) / 32;
+  if (probe.stats_blocks > np.chunks || !epilogue_takes_stats(net->ctx, probe, N)) return 0;
+  e = probe;
+  return static_cast<int>(probe.stats_blocks);
+}
+
 int residual_forward(myea_b200_net *net, int r) {
   LayerPlan &R = net->layers[r];
   RRC(residual_check(net, r));
+  int fused_chunks = 0;   // row blocks whose sums the product before has left
   Context &ctx = net->ctx;
   const long long rows = net->pitch();
   const float *x = net->layers[R.input_layer].values;
@@ -191,7 +206,7 @@ int residual_forward(myea_b200_net *net, int r) {
       } else {
         const float *cs = nullptr, *ch = nullptr;
         if (L.has_norm) {
-          RRC(norm_forward_stats(ctx, prev, rows, L.n_in, L.norm, net->training ? 1 : 0, &net->hook));
+          RRC(norm_forward_stats(ctx, prev, rows, L.n_in, L.norm, net->training ? 1 : 0, &net->hook, nullptr, fused_chunks));
           cs = L.norm.col_scale;
           ch = L.norm.col_shift;
         }
@@ -204,6 +219,9 @@ int residual_forward(myea_b200_net *net, int r) {
     e.C = L.summations;
     e.ldc = L.n_out;
     e.bias = L.use_bias ? net->params + L.idx.first_bias_connection_index : nullptr;
+    fused_chunks = 0;
+    if (net->training && k < R.block_depth && net->layers[r + k + 1].has_norm && (net->layers[r + k + 1].shared_panels || !norm_strip_suits(rows, &net->hook)))
+      fused_chunks = sums_from_product(net, L, e, 1, net->layers[r + k + 1].norm, rows, L.n_out, L.n_in);
     RRC(fc_product_forward(net, L, in, rows, e));
   }
   const LayerPlan &last = net->layers[r + R.block_depth];
@@ -220,9 +238,11 @@ int residual_forward(myea_b200_net *net, int r) {
     s = R.summations;
   }
   if (A == W) {
+    // (what reads this block may be another one: its first layer takes the residual layer's input)
     size_t reader = static_cast<size_t>(r + R.block_depth + 1);
-    if (reader < net->layers.size() && net->layers[reader].type == MYEA_LAYER_RESIDUAL) ++reader;
-    const HalfPanels *sink = reader < net->layers.size() && net->layers[reader].input_layer == r ? fc_input_sink(net, net->layers[reader], R.values, rows) : nullptr;
+    const bool reads = reader < net->layers.size() && net->layers[reader].input_layer == r;
+    if (reads && net->layers[reader].type == MYEA_LAYER_RESIDUAL) ++reader;
+    const HalfPanels *sink = reads && reader < net->layers.size() ? fc_input_sink(net, net->layers[reader], R.values, rows) : nullptr;
     return launch_shakedrop(ctx, x, s, R.values, mask, R.shake_alpha, scale, rows, R.n_out, sink);
   }
   const long long pad = residual_padding(A, W);
@@ -272,8 +292,9 @@ int residual_backward(myea_b200_net *net, int r) {
     e.aux_y = L.values;
     e.ld_aux = L.n_in;
     if (L.has_norm) { e.col_scale = L.norm.col_scale; e.col_shift = L.norm.col_shift; }
+    const int chunks = L.has_norm && L.w_valid && L.d_readings == HALF_BOTH ? sums_from_product(net, L, e, 2, L.norm, rows, L.n_in, L.n_out) : 0;
     RRC(fc_product_backward(net, L, rows, e));
-    if (L.has_norm) RRC(norm_backward(ctx, below.summations, L.deriv, below.errors, rows, L.n_in, L.norm, &net->hook, 0, fc_error_sink(net, below, rows)));
+    if (L.has_norm) RRC(norm_backward(ctx, below.summations, L.deriv, below.errors, rows, L.n_in, L.norm, &net->hook, chunks, fc_error_sink(net, below, rows)));
   }
   // the layer feeding the block: skip error + W_1^T delta_1, then its own activation derivative / normalization
   LayerPlan &first = net->layers[r + 1];
