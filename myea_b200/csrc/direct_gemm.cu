@@ -1015,7 +1015,7 @@ static long long operand_pitch(const Operand &o, bool columns) { return columns 
 // of 4.6, and the training step around it 5 us more).  Estimates (us) from these measurements of FMAs with 1 / 2 / 4 / 8 CTAs and of
 // tensor-core tiles: 128 x 256 x 64 3.4 / 4.6 / 4.8 / 5.7, 5.5; 128 x 256 x 256 5.2 / 5.5 / 5.4 / 6.0, 6.8; 64 x 512 x 512 8.4 / 6.7 / 6.2 /
 // 6.4, 8.0; 256 x 10 x 1024 15.2 / 10.2 / 7.3 / 6.5, 11.5; 32 x 64 x 4096 54 / 30 / 17 / 10, 17; 384^3 8.0, 7.8; rows that are not
-// 16-byte aligned: 203 x 333 x 75 4.1, 9.8.
+// 16-byte aligned: 203 x 333 x 75 5.3, 9.8; 203 x 333 x 333 9.5 / 11.5, 9.9; 333 x 333 x 203 6.6 / 8.3, 8.6; 161 x 150 x 2000 33 / 20 / 15 / 13, 12.
 // Tiles of 16 x 16 (cluster 0, tile 16) where they are up to two CTAs per SM.  Estimates from these measurements, beside the others':
 // 128 x 256 x 64 3.4, 128 x 256 x 256 4.0, 64 x 512 x 512 5.0, 256 x 256 x 512 6.6 (256 tiles), 256 x 10 x 1024 8.4, 32 x 64 x 4096 26; not aligned:
 // 203 x 333 x 75 3.4, 203 x 333 x 333 6.8 (273 tiles), 161 x 150 x 2000 read through its columns 20.6.
@@ -1040,7 +1040,7 @@ static FmaPlan fma_plan(const DirectItem *items, int n, bool at, bool bt) {
   FmaPlan plan;
   const long long t32 = tiles_of(FG_M), t16 = tiles_of(SG_TILE);
   for (int S = 1; S <= 8 && t32 * S <= 148; S *= 2) {
-    const double t = 2.6 + 0.011 * K / S + (S > 1 ? 2.2 : 0.0) + (S == 8 ? 0.5 : 0.0);
+    const double t = 2.6 + 0.011 * K / S * (aligned ? 1.0 : 2.0) + (S > 1 ? 2.2 : 0.0) + (S == 8 ? 0.5 : 0.0);
     if (t < best) { best = t; plan.tile = FG_M; plan.cluster = S; }
   }
   if (t16 <= 296 && 2.4 + 0.0055 * K * (t16 > 148 ? 1.6 : 1.0) * (aligned ? 1.0 : 1.5) < best) {
