@@ -1039,11 +1039,14 @@ static FmaPlan fma_plan(const DirectItem *items, int n, bool at, bool bt) {
   double best = 5.0 + 0.006 * std::min(K, 1024.0) + 0.002 * std::max(0.0, K - 1024.0) + (aligned ? 0.0 : 2.0) - 0.5;
   FmaPlan plan;
   const long long t32 = tiles_of(FG_M), t16 = tiles_of(SG_TILE);
+  // (rows off the 16-byte boundaries take tiles of 32 x 32 about twice as long per K.  That decides between the two FMA tiles; against
+  // the tensor-core tiles, which are hardly faster there and less exact, it does not count)
+  double fma = 1e30;
   for (int S = 1; S <= 8 && t32 * S <= 148; S *= 2) {
-    const double t = 2.6 + 0.011 * K / S * (aligned ? 1.0 : 2.0) + (S > 1 ? 2.2 : 0.0) + (S == 8 ? 0.5 : 0.0);
-    if (t < best) { best = t; plan.tile = FG_M; plan.cluster = S; }
+    const double walk = 0.011 * K / S, t = 2.6 + walk + (S > 1 ? 2.2 : 0.0) + (S == 8 ? 0.5 : 0.0);
+    if (t < best) { best = t; fma = t + (aligned ? 0.0 : walk); plan.tile = FG_M; plan.cluster = S; }
   }
-  if (t16 <= 296 && 2.4 + 0.0055 * K * (t16 > 148 ? 1.6 : 1.0) * (aligned ? 1.0 : 1.5) < best) {
+  if (t16 <= 296 && 2.4 + 0.0055 * K * (t16 > 148 ? 1.6 : 1.0) * (aligned ? 1.0 : 1.5) < (plan.tile ? fma : best)) {
     plan.tile = SG_TILE;
     plan.cluster = 1;
   }
