@@ -84,6 +84,13 @@ def test_normalized_short_batches(B, norm):
     _step(_mlp((9, 37, 16, 3), B, capi.AF_SIGMOID, norm, capi.DROP_BERNOULLI_INVERTED))
 
 
+# normalizations and activations that write operand panels: ragged blocks of 128 rows and columns, masked units
+@pytest.mark.parametrize("widths,B", [((1000, 1048, 904, 130), 700), ((512, 1032, 1160, 64), 1025)])
+@pytest.mark.parametrize("norm", [capi.NORM_NONE, capi.NORM_BN, capi.NORM_BRN])
+def test_producers_of_operand_panels(widths, B, norm):
+    _step(_mlp(widths, B, capi.AF_TANH, norm, capi.DROP_BERNOULLI_INVERTED))
+
+
 # the resident walk on clusters: one to three steps (the barriers' first phases), rows and cells that do not divide
 @pytest.mark.parametrize("n_in,H,T,B,bidirectional,zoneout", [
     (5, 150, 1, 50, False, 0.0), (5, 150, 2, 50, False, 0.1), (5, 203, 3, 61, False, 0.0), (5, 129, 7, 30, True, 0.2), (5, 300, 4, 5, False, 0.1), (5, 90, 5, 256, True, 0.0)])
