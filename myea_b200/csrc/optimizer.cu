@@ -140,7 +140,8 @@ int optimizer_update(Context &ctx, const OptLaunch &o, const OptArrays &a, size_
 // overwrites them instead of adding to them (4 bytes less again).  Bound by HBM, so by loads in flight: a thread has 8 elements
 // of all arrays on the way, 1024 threads per SM; the new weights wait in shared memory (64 KB) because in registers they leave
 // room for half the threads (138 M weights, Adam: 764 us, 36 bytes per weight at 6.5 TB/s; with the weights in registers and 512
-// threads per SM 1770 us at 32 bytes per weight).
+// threads per SM 1770 us at 32 bytes per weight).  Behind contractions that hold the chip at its power cap it takes
+// 950 us, with or without its arithmetic, and in proportion without its panels: memory at the clocks that are left.
 constexpr int OPT_LAYERS = 32;
 constexpr int OPT_THREADS = HP_THREADS, OPT_ROWS = HP_ROWS;   // 8 columns of rows tid / 16 + 32 i
 constexpr int OPT_SMEM = HP_BLOCK * HP_BLOCK * 4;
