@@ -785,7 +785,8 @@ static int batch_for_forward(myea_b200_net *net, uint64_t batch) {
 // rows the kernels of the step in flight run over, and the rows per time step among them
 static long long pitch_rows(const myea_b200_net *net) { return net->pitch(); }
 static long long step_rows_total(const myea_b200_net *net) { return net->T * pitch_rows(net); }
-// whether a kernel on this handle's device may read all of [p, p + bytes): what the driver's copy would find out, and refuse, by itself
+// whether a kernel on this handle's device may read all of [p, p + bytes) as floats: what the driver's copy would find out, and refuse,
+// by itself (or would manage: it takes addresses that are no multiple of 4)
 static bool readable_here(const myea_b200_net *net, const void *p, size_t bytes) {
   typedef CUresult (*AddressRange)(CUdeviceptr *, size_t *, CUdeviceptr);
   static const AddressRange range = [] {
@@ -799,7 +800,7 @@ static bool readable_here(const myea_b200_net *net, const void *p, size_t bytes)
   CUdeviceptr base = 0;
   size_t size = 0;
   const CUdeviceptr q = reinterpret_cast<CUdeviceptr>(p);
-  return at.type == cudaMemoryTypeDevice && at.device == net->ctx.device && range(&base, &size, q) == CUDA_SUCCESS && q >= base && q - base <= size &&
+  return q % sizeof(float) == 0 && at.type == cudaMemoryTypeDevice && at.device == net->ctx.device && range(&base, &size, q) == CUDA_SUCCESS && q >= base && q - base <= size &&
          bytes <= size - (q - base);
 }
 // host or device block packed [T][active_B][units] -> [T][pitch][units], padding rows zeroed

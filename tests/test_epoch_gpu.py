@@ -5,6 +5,7 @@ import ctypes as C
 
 import numpy as np
 import pytest
+import torch
 
 import cases
 from conftest import rel_err
@@ -186,3 +187,36 @@ def test_targets_from_host_device_and_dataset_in_turn():
         out.append(net.get(capi.BUF_PARAMETERS))
         net.close()
     assert all(np.array_equal(out[0], p) for p in out[1:])
+
+
+# 0, 4, 8 bytes past a 16-byte boundary: copied by a kernel up to 1 Mi floats (by vectors, by elements), by the driver beyond; 1 and 2 bytes:
+# by the driver whatever the size
+@pytest.mark.parametrize("offset", [0, 4, 8, 1, 2])
+@pytest.mark.parametrize("inputs,B", [(3, 1), (37, 5), (8, 128), (1024, 1024), (1025, 1024)])
+def test_device_batches_at_any_address(inputs, B, offset):
+    layers = [capi.fc(inputs), capi.fc(7, capi.AF_TANH), capi.fc(5, capi.AF_LINEAR)]
+    desc, opt = capi.net(layers, B, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE), capi.opt(capi.OPT_GD, gd_lr=1e-3)
+    gen = torch.Generator().manual_seed(inputs + B)
+    x, y = torch.randn(B * inputs, generator=gen), torch.randn(B * 5, generator=gen)
+    out = []
+    for on_device in (False, True):
+        net = Net(desc, opt)
+        net.set(capi.BUF_PARAMETERS, np.random.default_rng(2).standard_normal(net.P, dtype=np.float32))
+        net.reset_loss()
+        if on_device:
+            def place(a):
+                raw = torch.empty(a.numel() * 4 + 16, dtype=torch.uint8, device="cuda")
+                raw[offset:offset + a.numel() * 4].copy_(a.view(torch.uint8))
+                return raw
+            rx, ry = place(x), place(y)
+            torch.cuda.synchronize()
+            assert rx.data_ptr() % 16 == 0 and ry.data_ptr() % 16 == 0
+            net._ck(net.lib.myea_b200_forward_device(net.h, B, rx.data_ptr() + offset, 1), "forward_device")
+            net._ck(net.lib.myea_b200_compute_error_device(net.h, B, ry.data_ptr() + offset), "compute_error_device")
+        else:
+            net.forward(x.numpy()); net.compute_error(y.numpy())
+        net.backward(); net.update_derivative_weight()
+        out.append((net.loss(), net.outputs(2), net.get(capi.BUF_DERIVATIVES)))
+        net.synchronize(); net.close()
+    assert out[0][0] == pytest.approx(out[1][0], rel=1e-12)   # (the order of its atomic sums varies)
+    assert all(np.array_equal(a, b) for a, b in zip(out[0][1:], out[1][1:]))
