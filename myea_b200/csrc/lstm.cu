@@ -233,7 +233,8 @@ __global__ void lstm_gather_peepholes_kernel(const float *__restrict__ peep, lon
 __global__ void __launch_bounds__(256) lstm_gather_weights_kernel(const float *__restrict__ w0, const float *__restrict__ w1, long long stride, long long off_z,
                                                                   long long off_gates, long long width, long long C, float *__restrict__ out) {
   grid_dependency_wait();
-  grid_dependency_release();
+  // (no early release: in front of a walk by launches the first cells would set themselves up beside these blocks, the product of the
+  // second step beside both, two of its CTAs to an SM, and every later step's like it: 701 cells, 200 rows 35 us per forward step, 52 then)
   const long long total = 4 * C * width;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total; i += static_cast<long long>(gridDim.x) * blockDim.x) {
     const long long r = i / width, k = i - r * width, g = r / C, c = r - g * C;
