@@ -68,8 +68,8 @@ template <int MAX> struct DirectGroup {   // kernel argument: 400 bytes for a si
 
 // One thread's 8 consecutive K elements of one operand row, stage after stage.  T: the rows are contiguous in memory (pitch
 // ld between K steps), a warp's lanes take consecutive rows; else K is contiguous.  Rows past the matrix repeat its last
-// row (what they produce is never stored); K elements past its end are zeros.
-template <bool T>
+// row (what they produce is never stored); K elements past its end are zeros.  WIDE: whole sectors at once where they are aligned.
+template <bool T, bool WIDE>
 struct DgReader {
   const float *p;     // element (row, k)
   long long ld, advance;
@@ -89,7 +89,12 @@ struct DgReader {
 #pragma unroll
         for (int j = 0; j < 8; ++j, q += ld) v[j] = *q;
       } else if (vec) {
-        ld8(v, p, 8, true);
+        if (WIDE) {
+          ld8(v, p, 8, true);
+        } else {
+          const float4 a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(p + 4);
+          v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        }
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = p[j];
@@ -259,7 +264,7 @@ __device__ __forceinline__ void dg_finish(const DirectProblem &p, const float *p
   }
 }
 
-template <bool AT, bool BT, int MAX>
+template <bool AT, bool BT, int MAX, bool WIDE>
 __global__ void __launch_bounds__(DG_THREADS, 2) direct_gemm_kernel(const __grid_constant__ DirectGroup<MAX> g, int *error_flag) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -303,8 +308,8 @@ __global__ void __launch_bounds__(DG_THREADS, 2) direct_gemm_kernel(const __grid
   // two register sets: the loads of stage i + 2 leave when stage i has been stored, so that their way to L2 and back
   // runs beside the conversion of stage i + 1
   float va0[2][8], va1[2][8], vb[2][8];
-  DgReader<AT> ra0(p.a, p.lda, a0, m0, p.M, ag0, s0 * BK, p.K, p.a_vec != 0), ra1(p.a, p.lda, a1, m0, p.M, ag1, s0 * BK, p.K, p.a_vec != 0);
-  DgReader<BT> rb(p.b, p.ldb, b0, n0, p.N, bg, s0 * BK, p.K, p.b_vec != 0);
+  DgReader<AT, WIDE> ra0(p.a, p.lda, a0, m0, p.M, ag0, s0 * BK, p.K, p.a_vec != 0), ra1(p.a, p.lda, a1, m0, p.M, ag1, s0 * BK, p.K, p.a_vec != 0);
+  DgReader<BT, WIDE> rb(p.b, p.ldb, b0, n0, p.N, bg, s0 * BK, p.K, p.b_vec != 0);
   auto fetch = [&](float (&x0)[8], float (&x1)[8], float (&xb)[8]) { ra0.fetch(x0); ra1.fetch(x1); rb.fetch(xb); };
   float rs = 0.f;   // thread: row tid & 127, half of the K groups of every stage
   bool ok = true;
@@ -932,9 +937,9 @@ bool direct_gemm_suits(const Context &ctx, long long M, long long N, long long K
   return ctx.gemm_engine == 0 && ctx.gemm_bn == 0 && M > 0 && N > 0 && K > 0 && M * N * K <= (600ll << 20);
 }
 
-template <bool AT, bool BT, int MAX>
-static int launch_direct(Context &ctx, const DirectGroup<MAX> &g, int tiles, int cluster) {
-  auto kernel = direct_gemm_kernel<AT, BT, MAX>;
+template <bool AT, bool BT, int MAX, bool WIDE>
+static int launch_direct_reading(Context &ctx, const DirectGroup<MAX> &g, int tiles, int cluster) {
+  auto kernel = direct_gemm_kernel<AT, BT, MAX, WIDE>;
   static std::once_flag flags[64];
   static bool ok[64] = {};
   if (ctx.device < 0 || ctx.device >= 64) return MYEA_E_CUDA;
@@ -958,6 +963,24 @@ static int launch_direct(Context &ctx, const DirectGroup<MAX> &g, int tiles, int
   const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, g, ctx.d_error_flag);
   ctx.end(TC_GEMM);
   return err == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
+}
+
+// Accesses of whole sectors where every operand read through its rows allows 16 bytes at least and K is not short.  A kernel that has
+// them beside the element-wise reads of other rows is slower at those (us without / with them: 512 x 709 x 1001 24.5 / 24.8, the second
+// operand through its columns 22.4 / 23.3; 256 x 1024 x 1001 13.6 / 14.1), and of a short K they gain nothing that a step shows (an
+// output layer's 512 x 709 x 64 8.5 / 8.4 by itself, 12 / 17 behind the error).  Aligned rows: 64 x 6000 x 256 9.7 / 9.4, 512 x 709 x
+// 784 17.7 / 17.1.
+template <bool AT, bool BT, int MAX>
+static int launch_direct(Context &ctx, const DirectGroup<MAX> &g, int tiles, int cluster) {
+  bool wide = !(AT && BT);
+  int longest = 0;
+  for (int i = 0; i < g.count; ++i) {
+    wide = wide && (AT || g.p[i].a_vec) && (BT || g.p[i].b_vec);
+    longest = std::max(longest, g.p[i].K);
+  }
+  if constexpr (!(AT && BT))
+    if (wide && longest >= 256) return launch_direct_reading<AT, BT, MAX, true>(ctx, g, tiles, cluster);
+  return launch_direct_reading<AT, BT, MAX, false>(ctx, g, tiles, cluster);
 }
 
 static bool epilogue_is_vector(const Epilogue &e, long long N) {
