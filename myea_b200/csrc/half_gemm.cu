@@ -649,6 +649,34 @@ void gemm_splitk_release(Context &ctx) {
   ctx.sk_clusters = 0;
 }
 
+// How `tiles` of `chunks` chunks of K are shared by `pairs` CTA pairs: whole ones in full waves, stream-K for the partial last wave.
+struct WideSplit {
+  int whole, run, clusters;   // tiles computed whole; chunks per cluster of the others (0: none); clusters of the launch
+};
+static WideSplit split_tiles(int tiles, int chunks, int pairs) {
+  const int rem = tiles % pairs, units = rem * chunks;
+  const WideSplit none = {tiles, 0, std::min(tiles, pairs)};
+  if (rem == 0 || chunks < 2) return none;
+  // at most 8 clusters share one tile: the cluster that arrives last adds up every other contributor's 256 KB of
+  // partial sums, and past 8 that pass outweighs the shorter K walk (256 x 256 x 16384 with the splits of its operands 58 us, 94 with
+  // 64 of them; 512 x 512 x 8192 50, 55 with 16)
+  constexpr int max_split = 8;
+  int run = std::max((units + pairs - 1) / pairs, (chunks + max_split - 1) / max_split);
+  // A run that ends inside a tile makes a third contributor and a second set of partial sums (7 - 9 kcycles at the end of a
+  // launch that walks a chunk in 3): where equal shares of a tile are hardly longer, every run is one share of one tile.
+  // 32 tiles on 74 pairs, 16 chunks instead of 14: 512 x 4096 x 4096 with the splits of its operands 84.7 -> 78.9 us.  Two chunks more
+  // pay at the shortest K as well: 25 tiles of 8 chunks, 4 instead of 3 37.1 -> 31.8; 26 of 16, 8 instead of 6 51.9 -> 46.5; 15 of 9, 3
+  // instead of 2 35.9 -> 30.7.
+  if (tiles == rem) {
+    const int shares = std::min(pairs / rem, max_split), share = (chunks + shares - 1) / shares;
+    if (share - run <= 2 && chunks % share == 0) run = share;
+  }
+  // splitting a tile costs about the time of two chunks (partial sums through L2, one counter round trip, the second
+  // pass of the warp that arrives last): worth it when it takes at least three off the longest cluster
+  if (chunks - run < 3) return none;
+  return {tiles - rem, run, tiles > rem ? pairs : (units + run - 1) / run};
+}
+
 template <int BN, bool A_COLS, bool B_COLS>
 static int launch_half(Context &ctx, const HalfOperand &A, const HalfOperand &B, const GemmDims &dims, const Epilogue &epi) {
   auto kernel = half_gemm_kernel<BN, A_COLS, B_COLS>;
@@ -685,36 +713,17 @@ static int launch_half(Context &ctx, const HalfOperand &A, const HalfOperand &B,
   work.tiles_n = (dims.N + BN - 1) / BN;
   work.num_tiles = work.tiles_m * work.tiles_n;
   work.dp_tiles = work.num_tiles;
-  int grid_clusters = work.num_tiles < G ? work.num_tiles : G;
-  // stream-K for the partial last wave (gemm_bn 4 switches it off): needs the partial-sum workspace and more than one
-  // K chunk per tile
-  const int rem = work.num_tiles % G;
-  if (ctx.gemm_bn != 4 && ctx.sk_ws != nullptr && ctx.sk_clusters >= G && rem != 0 && num_chunks >= 2) {
-    const int units = rem * num_chunks;
-    int per_cluster = (units + G - 1) / G;
-    // at most 8 clusters share one tile: the cluster that arrives last adds up every other contributor's 256 KB of
-    // partial sums, and past 8 that pass outweighs the shorter K walk
-    constexpr int max_split = 8;
-    per_cluster = std::max(per_cluster, (num_chunks + max_split - 1) / max_split);
-    // A run that ends inside a tile makes a third contributor and a second set of partial sums (7 - 9 kcycles at the end of a
-    // launch that walks a chunk in 3): where equal shares of a tile are hardly longer, every run is one share of one tile (32
-    // tiles on 74 pairs, 16 chunks instead of 14: 512 x 4096 x 4096 with the splits of its operands 84.7 -> 78.9 us, 2048 x 1024 x 2048 49.8
-    // -> 44.2).
-    const int shares = G / rem;
-    if (work.num_tiles == rem && shares >= 1) {
-      const int share = (num_chunks + shares - 1) / shares;
-      if (share - per_cluster <= 2 && num_chunks % share == 0) per_cluster = share;
-    }
-    // splitting a tile costs about the time of two chunks (partial sums through L2, one counter round trip, the second
-    // pass of the warp that arrives last): worth it when it takes at least three off the longest cluster
-    if (num_chunks - per_cluster >= 3) {
-      work.dp_tiles = work.num_tiles - rem;
-      work.sk_units = units;
-      work.sk_chunks = per_cluster;
+  int grid_clusters = std::min(work.num_tiles, G);
+  // (gemm_bn 4 switches the split off; it needs the partial-sum workspace)
+  if (ctx.gemm_bn != 4 && ctx.sk_ws != nullptr && ctx.sk_clusters >= G) {
+    const WideSplit split = split_tiles(work.num_tiles, num_chunks, G);
+    if (split.run > 0) {
+      work.dp_tiles = split.whole;
+      work.sk_units = (work.num_tiles - split.whole) * num_chunks;
+      work.sk_chunks = split.run;
       work.ws = ctx.sk_ws;
       work.counters = ctx.sk_counters;
-      const int used = (units + per_cluster - 1) / per_cluster;
-      grid_clusters = work.dp_tiles > 0 ? G : used;
+      grid_clusters = split.clusters;
     }
   }
   launch_dependent(ctx, kernel, dim3(static_cast<unsigned>(2 * grid_clusters)), dim3(HG_THREADS), S::TOTAL, maps[0], maps[1], maps[2], maps[3], scales(A), scales(B), dims,
@@ -788,3 +797,14 @@ int gemm_nt(Context &ctx, const Operand &A, const Operand &B, const Epilogue &ep
 }
 
 }  // namespace myea
+
+// For tests: how `tiles` output tiles with `chunks` chunks of 128 of K are shared by `pairs` CTA pairs.  whole: tiles computed whole; run: chunks
+// per pair of the others, 0 if there are none; clusters: pairs of the launch.
+extern "C" int myea_b200_split_plan(int tiles, int chunks, int pairs, int *whole, int *run, int *clusters) {
+  if (tiles <= 0 || chunks <= 0 || pairs <= 0 || whole == nullptr || run == nullptr || clusters == nullptr) return MYEA_E_INVALID;
+  const myea::WideSplit s = myea::split_tiles(tiles, chunks, pairs);
+  *whole = s.whole;
+  *run = s.run;
+  *clusters = s.clusters;
+  return MYEA_OK;
+}
