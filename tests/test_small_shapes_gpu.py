@@ -45,8 +45,9 @@ def test_contraction_from_fp32_operands_over_k(M, N, K, engine):
     assert rel_err(out, A.astype(np.float64) @ B.astype(np.float64).T) < 5e-6
 
 
-def _step(wl, seed=5, rows=None):
-    """one training step and one inference pass on the GPU and on the restatement"""
+def _step(wl, seed=5, kinks=0.0):
+    """one training step and one inference pass on the GPU and on the restatement; kinks: bound in the 2-norm of the derivatives, and of the
+    outputs behind the update that they make, where single elements may take the other branch of an activation's derivative"""
     gpu, cpu = Net(wl.desc, wl.opt), myea_oracle.OracleNet(wl.desc, wl.opt)
     X, Y = wl.batch(seed)
     for net in (gpu, cpu):
@@ -61,6 +62,9 @@ def _step(wl, seed=5, rows=None):
         out += [(gpu.get(b), cpu.get(b)) for b in (capi.BUF_NORM_MEAN_AVERAGE, capi.BUF_NORM_VARIANCE_AVERAGE)]
     gpu.synchronize()
     gpu.close()
+    if kinks:
+        for got, want in (out.pop(3), out.pop(1)):
+            assert np.linalg.norm(got - want) < kinks * np.linalg.norm(want)
     for got, want in out:
         assert rel_err(got, want) < TOL
 
@@ -89,6 +93,24 @@ def test_normalized_short_batches(B, norm):
 @pytest.mark.parametrize("norm", [capi.NORM_NONE, capi.NORM_BN, capi.NORM_BRN])
 def test_producers_of_operand_panels(widths, B, norm):
     _step(_mlp(widths, B, capi.AF_TANH, norm, capi.DROP_BERNOULLI_INVERTED))
+
+
+# residual blocks whose products run on operand panels (from 600 Mi multiply-adds on): column sums of a normalization from the product
+# before it, forward and backward, and panels of the next block's first layer from the ShakeDrop kernel; rows that are a multiple of 32 and
+# not, and a width that is none, where the sums are taken in a pass of their own
+@pytest.mark.parametrize("H,B", [(1024, 704), (1024, 700), (1000, 700)])
+@pytest.mark.parametrize("norm,af", [(capi.NORM_BN, capi.AF_TANH), (capi.NORM_BRN, capi.AF_TANH), (capi.NORM_BN, capi.AF_ELU), (capi.NORM_BRN, capi.AF_SIGMOID)])
+@pytest.mark.parametrize("depth", [2, 3])
+def test_residual_blocks_on_operand_panels(H, B, norm, af, depth):
+    """The derivative of ELU (as the reference has it) jumps from 0 to 1 at 0: pre-activations within rounding of it, about 2e-6 of
+    B * H * 7 layers or 10 elements, may take either side, and each is sqrt(1 / (B * H)) of its layer's error: 4e-3 in the 2-norm."""
+    assert H * H * B > 600 << 20
+    layers = [capi.fc(40), capi.fc(H, af)]
+    for _ in range(2):
+        layers += [capi.residual(depth, capi.DROP_SHAKEDROP, (0.5, 0.0, 0.0)), capi.fc(H, af)] + [capi.fc(H, af, norm) for _ in range(depth - 1)]
+    layers.append(capi.fc(30, capi.AF_LINEAR))
+    _step(workloads.Workload("blocks on panels", capi.net(layers, B, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE, r_max=3.0, d_max=5.0),
+                             capi.opt(capi.OPT_GD, gd_lr=0.01 / B, momentum=0.9), 40, 30, False, layers), kinks=1e-2 if af == capi.AF_ELU else 0.0)
 
 
 # the resident walk on clusters: one to three steps (the barriers' first phases), rows and cells that do not divide
