@@ -86,6 +86,7 @@ int lstm_persistent_backward(myea_b200_net *net, LayerPlan &L, int dir);
 // in shared memory, read from the parameter buffer itself.  lstm_resident_plan decides which passes take it.
 int lstm_resident_plan(myea_b200_net *net, LayerPlan &L);
 void lstm_resident_destroy(LstmPlan *P);
+bool lstm_resident_stall(LstmPlan *P, int step, long long cycles);
 int lstm_resident_run(myea_b200_net *net, LayerPlan &L, int kind, bool zoneout, const long long rec[4], long long peep);
 
 }  // namespace myea

@@ -763,13 +763,16 @@ extern "C" int myea_b200_lstm_resident_clusters(int device, int *forward_pairs, 
   return MYEA_OK;
 }
 
-// For tests: the barrier in front of step `step` (1 to T - 1; 0: none) of every tensor-core walk of this handle is never reached, and
-// the wait there gives up after `cycles` SM clocks.  MYEA_E_UNSUPPORTED when no layer has such a walk.
+// For tests: the barrier in front of step `step` (1 to T - 1; 0: none) of every walk in one launch of this handle is never reached, and
+// the wait there gives up after `cycles` SM clocks (of a walk with resident weights so does any other wait).  MYEA_E_UNSUPPORTED when no
+// layer has a walk that waits.
 extern "C" int myea_b200_lstm_stall(myea_handle net, int step, uint64_t cycles) {
   if (net == nullptr || step < 0 || cycles > (1ull << 31)) return MYEA_E_INVALID;
   int found = 0;
   for (auto &L : net->layers) {
-    if (L.lstm == nullptr || !myea::lstm_persistent_ready(L.lstm)) continue;
+    if (L.lstm == nullptr) continue;
+    if (myea::lstm_resident_stall(L.lstm, step, static_cast<long long>(cycles))) ++found;
+    if (!myea::lstm_persistent_ready(L.lstm)) continue;
     L.lstm->persist->stall_step = step;
     L.lstm->persist->wait_cycles = static_cast<long long>(cycles);
     ++found;

@@ -54,6 +54,8 @@ struct ResidentArgs {
   unsigned int *sync = nullptr;           // [direction][group] counters, then one abort word
   int sync_count = 0;
   int *error_flag = nullptr;
+  int stall_step = 0;                     // tests only: the step whose wait is never over (0: none); in a cluster for its first CTA
+  long long wait_cycles = 1ll << 31;
 };
 
 __device__ __forceinline__ unsigned int lr_ld_acquire(const unsigned int *p) {
@@ -64,12 +66,12 @@ __device__ __forceinline__ unsigned int lr_ld_acquire(const unsigned int *p) {
 __device__ __forceinline__ void lr_add_release(unsigned int *p) { asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory"); }
 
 // one thread: until the counter has reached `target`
-__device__ __forceinline__ bool lr_wait(const unsigned int *counter, unsigned int target, unsigned int *abort_word) {
+__device__ __forceinline__ bool lr_wait(const unsigned int *counter, unsigned int target, unsigned int *abort_word, long long cycles) {
   if (lr_ld_acquire(counter) >= target) return true;
   const long long t0 = clock64();
   for (int n = 0;; ++n) {
     if (lr_ld_acquire(counter) >= target) return true;
-    if ((n & 63) == 63 && (lr_ld_acquire(abort_word) != 0u || clock64() - t0 > (1ll << 31))) return false;
+    if ((n & 63) == 63 && (lr_ld_acquire(abort_word) != 0u || clock64() - t0 > cycles)) return false;
   }
 }
 
@@ -178,7 +180,7 @@ __device__ __forceinline__ void lr_cell(const LrIn &in, const LrPeepholes &p, co
 template <int KIND, bool CLUSTER>
 __global__ void __launch_bounds__(LR_THREADS, 1) lstm_resident_kernel(const __grid_constant__ ResidentArgs q) {
   extern __shared__ __align__(16) float lr_smem[];
-  __shared__ int s_ok;
+  __shared__ volatile int s_ok[2];             // of even and odd steps: a wait of the next step may give up before every thread has read this step's
   __shared__ uint64_t landed[2];      // CLUSTER: the exchange data of a step is complete in in_s[step & 1]
   __shared__ uint32_t pushed_steps;   // CLUSTER: steps whose results this CTA has pushed
   float *red_s = lr_smem;                                // [KW][RB][NOp]
@@ -231,7 +233,7 @@ __global__ void __launch_bounds__(LR_THREADS, 1) lstm_resident_kernel(const __gr
   if (!CLUSTER && q.G == 1)
     for (int i = tid; i < static_cast<int>(2 * ex_size); i += LR_THREADS) in_s[i] = 0.f;
   if (tid == 0) {
-    s_ok = 1;
+    s_ok[0] = s_ok[1] = 1;
     if constexpr (CLUSTER) {
       ptx::mbar_init(&landed[0], 1);
       ptx::mbar_init(&landed[1], 1);
@@ -335,30 +337,33 @@ __global__ void __launch_bounds__(LR_THREADS, 1) lstm_resident_kernel(const __gr
   }
 
   int s = 0;
+  bool ok = true;
   for (; s < q.T; ++s) {
     const bool has_rec = s > 0;
     if (CLUSTER && has_rec) {
       // (every thread waits by itself; what it reads after a wait that gave up is not used: s_ok below)
       uint64_t *bar = &landed[(s - 1) & 1];
       const uint32_t parity = static_cast<uint32_t>((s - 1) >> 1) & 1u;
-      if (!ptx::mbar_try_wait_acquire_cluster(bar, parity)) {
+      const bool stalled = s == q.stall_step && g == 0;   // (s is 1 at least here)
+      if (stalled || !ptx::mbar_try_wait_acquire_cluster(bar, parity)) {
         const long long t0 = clock64();
-        while (!ptx::mbar_try_wait_acquire_cluster(bar, parity)) {
-          if (clock64() - t0 > (1ll << 31)) {
-            *static_cast<volatile int *>(&s_ok) = 0;
+        while (stalled || !ptx::mbar_try_wait_acquire_cluster(bar, parity)) {
+          if (clock64() - t0 > q.wait_cycles) {
+            s_ok[s & 1] = 0;
             atomicCAS(q.error_flag, 0, 412);
             break;
           }
         }
       }
     } else if (has_rec && q.G > 1) {
-      if (tid == 0 && !lr_wait(counter, static_cast<unsigned int>(q.G) * static_cast<unsigned int>(s), abort_word)) {
-        s_ok = 0;
+      if (tid == 0 && !lr_wait(counter, static_cast<unsigned int>(q.G) * static_cast<unsigned int>(s) + (s == q.stall_step ? 1u : 0u), abort_word, q.wait_cycles)) {
+        s_ok[s & 1] = 0;
         atomicCAS(q.error_flag, 0, 411);
         atomicExch(abort_word, 1u);
       }
       __syncthreads();
-      if (!s_ok) break;
+      ok = s_ok[s & 1] != 0;
+      if (!ok) break;
     }
     const size_t src_at = (s & 1) != 0 ? 0 : ex_odd, dst_at = (s & 1) != 0 ? ex_odd : 0;
     for (int rb = 0; rb < q.Rp; rb += q.RB) {
@@ -410,7 +415,8 @@ __global__ void __launch_bounds__(LR_THREADS, 1) lstm_resident_kernel(const __gr
         else lr_leave_sums<4>(acc, lane, works && col_live, sums_mine, q.NOp);
         __syncthreads();
         if constexpr (CLUSTER) {
-          if (!*static_cast<volatile int *>(&s_ok)) break;
+          ok = s_ok[s & 1] != 0;
+          if (!ok) break;
           if (rb == 0 && tid == 0 && s + 2 < q.T) ptx::mbar_arrive_expect_tx(&landed[(s + 1) & 1], lr_pushed_bytes<KIND>(q));   // of step s + 1
         }
       }
@@ -525,7 +531,7 @@ __global__ void __launch_bounds__(LR_THREADS, 1) lstm_resident_kernel(const __gr
         at.h += dh_step;
       }
     }
-    if (CLUSTER && !*static_cast<volatile int *>(&s_ok)) break;
+    if (CLUSTER && !ok) break;
   }
   if constexpr (CLUSTER) {
     // Nobody leaves while another CTA may push into its shared memory.  All steps done: whatever was sent here has been waited
@@ -556,6 +562,8 @@ struct LstmResident {
   size_t smem_f = 0, smem_b = 0;
   float *ex = nullptr;
   unsigned int *sync = nullptr;
+  int stall_step = 0;     // see ResidentArgs
+  long long wait_cycles = 1ll << 31;
 };
 
 // shape of one kind for G CTAs per group (one cluster or not) where `max_groups` of them run at once; false when it does not fit.
@@ -692,18 +700,27 @@ int lstm_resident_plan(myea_b200_net *net, LayerPlan &L) {
   if (!P->resident_pass[0] && !P->resident_pass[1]) return MYEA_OK;
   LstmResident *r = new LstmResident(best);
   P->resident = r;
-  // (a pass that is not taken here has groups, K and Rp of its best shape or of none: both only size the buffers)
+  // (a pass that is not taken here has groups, K and Rp of its best shape or of none: both only size the buffers, which the two passes
+  // share.  Rows that pad a group are numbers of no use: zeros at first, then what the other pass has left there; no live row reads them)
   const int counters = P->dirs * std::max(r->f.groups, r->b.groups);
   void *p = nullptr;
   const size_t ex_floats = 2 * static_cast<size_t>(P->dirs) * std::max(static_cast<size_t>(r->f.groups) * r->f.K * r->f.Rp, static_cast<size_t>(r->b.groups) * r->b.K * r->b.Rp);
   if (cudaMalloc(&p, ex_floats * sizeof(float)) != cudaSuccess) { net->ctx.error = "cudaMalloc failed (LSTM exchange buffer)"; return MYEA_E_CUDA; }
   net->allocations.push_back(p);
   r->ex = static_cast<float *>(p);
-  if (cudaMemsetAsync(p, 0, ex_floats * sizeof(float), net->ctx.stream) != cudaSuccess) return MYEA_E_CUDA;  // rows that pad a group stay zero
+  if (cudaMemsetAsync(p, 0, ex_floats * sizeof(float), net->ctx.stream) != cudaSuccess) return MYEA_E_CUDA;
   if (cudaMalloc(&p, (counters + 1) * sizeof(unsigned int)) != cudaSuccess) { net->ctx.error = "cudaMalloc failed (LSTM step counters)"; return MYEA_E_CUDA; }
   net->allocations.push_back(p);
   r->sync = static_cast<unsigned int *>(p);
   return MYEA_OK;
+}
+
+// Tests: see myea_b200_lstm_stall.  False where no CTA of this layer's walks waits for another.
+bool lstm_resident_stall(LstmPlan *P, int step, long long cycles) {
+  if (P->resident == nullptr) return false;
+  P->resident->stall_step = step;
+  P->resident->wait_cycles = cycles;
+  return (P->resident_pass[0] && P->resident->f.G > 1) || (P->resident_pass[1] && P->resident->b.G > 1);
 }
 
 void lstm_resident_destroy(LstmPlan *P) {
@@ -736,6 +753,8 @@ int lstm_resident_run(myea_b200_net *net, LayerPlan &L, int kind, bool zoneout, 
   q.sync = r->sync;
   q.sync_count = P->dirs * q.groups;
   q.error_flag = ctx.d_error_flag;
+  q.stall_step = r->stall_step;
+  q.wait_cycles = r->wait_cycles;
   if (q.G > 1 && !q.cluster && cudaMemsetAsync(q.sync, 0, (q.sync_count + 1) * sizeof(unsigned int), ctx.stream) != cudaSuccess) return MYEA_E_CUDA;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(P->dirs * q.groups * q.G));
@@ -767,3 +786,26 @@ int lstm_resident_run(myea_b200_net *net, LayerPlan &L, int kind, bool zoneout, 
 }
 
 }  // namespace myea
+
+// For tests: the walk that pass `kind` (1 forward, 2 backward) of layer `layer` takes.  walk: 0 launches, 1 tensor cores, 2 resident weights; of
+// the latter: CTAs per group, whether they are a cluster, groups per direction, row passes per step, rows per thread, whether a thread keeps one
+// row and cell.
+extern "C" int myea_b200_lstm_walk(myea_handle net, uint32_t layer, int kind, int out[7]) {
+  if (net == nullptr || out == nullptr || layer >= net->layers.size() || (kind != 1 && kind != 2)) return MYEA_E_INVALID;
+  const myea::LstmPlan *P = net->layers[layer].lstm;
+  if (P == nullptr || P->cpb != 1) return MYEA_E_INVALID;
+  for (int i = 0; i < 7; ++i) out[i] = 0;
+  if (!P->resident_pass[kind - 1]) {
+    out[0] = myea::lstm_persistent_ready(P) ? 1 : 0;
+    return MYEA_OK;
+  }
+  const myea::ResidentArgs &q = kind == 1 ? P->resident->f : P->resident->b;
+  out[0] = 2;
+  out[1] = q.G;
+  out[2] = q.cluster ? 1 : 0;
+  out[3] = q.groups;
+  out[4] = (q.Rp + q.RB - 1) / q.RB;
+  out[5] = q.RT;
+  out[6] = q.RB == q.Rp && q.Rp * q.cpc <= myea::LR_THREADS ? 1 : 0;
+  return MYEA_OK;
+}

@@ -330,17 +330,33 @@ def test_reciprocal_of_the_lstm_cells_against_the_correctly_rounded_one():
     assert different.value == 0 and most.value == 0
 
 
+def _walk(net, layer=1):
+    """what the forward and the backward pass of an LSTM layer take: [walk, CTAs per group, cluster, groups, row passes, rows per thread, one cell
+    per thread]; walk 0 launches, 1 tensor cores, 2 resident weights"""
+    out = []
+    for kind in (1, 2):
+        w = (C.c_int * 7)()
+        assert net.lib.myea_b200_lstm_walk(net.h, layer, kind, w) == 0
+        out.append(list(w))
+    return out
+
+
 @pytest.mark.parametrize("backward", [False, True])
-def test_a_step_barrier_that_is_never_reached_ends_in_an_error_status(backward):
-    """the tensor-core walk whose wait gives up (after half a millisecond here; its other waits after a second): every copy and
-    product in flight is waited for, the status is an error, and the GPU goes on - a new handle computes what the first one did"""
-    H, B, T = 1024, 136, 4
-    layers = [capi.fc(9), capi.lstm(H), capi.fc(H, capi.AF_LINEAR)]
+@pytest.mark.parametrize("H,B,bidirectional,walks,stalls", [   # walks: of the forward and the backward pass, whether on clusters
+    (1024, 136, False, ([1, 0], [1, 0]), (2,)), (150, 50, False, ([2, 1], [2, 1]), (1, 2, 3)), (512, 16, False, ([2, 0], [2, 0]), (1, 2, 3)),
+    (150, 256, True, ([2, 1], [2, 0]), (1, 3)), (142, 256, True, ([2, 0], [2, 1]), (1, 3))])   # two row passes; several cells per thread
+def test_a_step_barrier_that_is_never_reached_ends_in_an_error_status(H, B, bidirectional, walks, stalls, backward):
+    """a walk whose wait gives up (after half a millisecond here; the tensor-core walk's other waits after a second), in the first, a middle and
+    the last step: every copy and product in flight is waited for, the status is an error, and the GPU goes on - a new handle
+    computes what the first one did"""
+    T = 4
+    layers = [capi.fc(9), capi.lstm(H, bidirectional=bidirectional), capi.fc(H, capi.AF_LINEAR)]
     wl = workloads.Workload("stall", capi.net(layers, B, T=T, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE), capi.opt(capi.OPT_GD, gd_lr=1e-6), 9, H, False, layers)
     X, Y = wl.batch(5)
     out = []
-    for stall in (0, 2, 0):
+    for stall in (0,) + stalls + (0,):
         net = Net(wl.desc, wl.opt)
+        assert [w[:3:2] for w in _walk(net)] == list(walks)
         wl.materialize(net)
         if not backward:
             assert net.lib.myea_b200_lstm_stall(net.h, stall, C.c_uint64(1 << 20)) == 0
