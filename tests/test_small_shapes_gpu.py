@@ -113,22 +113,46 @@ def test_residual_blocks_on_operand_panels(H, B, norm, af, depth):
                              capi.opt(capi.OPT_GD, gd_lr=0.01 / B, momentum=0.9), 40, 30, False, layers), kinks=1e-2 if af == capi.AF_ELU else 0.0)
 
 
-# the resident walk on clusters: one to three steps (the barriers' first phases), rows and cells that do not divide
-@pytest.mark.parametrize("n_in,H,T,B,bidirectional,zoneout", [
-    (5, 150, 1, 50, False, 0.0), (5, 150, 2, 50, False, 0.1), (5, 203, 3, 61, False, 0.0), (5, 129, 7, 30, True, 0.2), (5, 300, 4, 5, False, 0.1), (5, 90, 5, 256, True, 0.0)])
-def test_lstm_walk_on_clusters(n_in, H, T, B, bidirectional, zoneout):
-    test_lstm_with_resident_weights(n_in, H, T, B, bidirectional, zoneout)
+def _walk(net, layer=1):
+    """what the forward and the backward pass of an LSTM layer take: [walk, CTAs per group, cluster, groups, row passes, rows per thread, one cell
+    per thread]; walk 0 launches, 1 tensor cores, 2 resident weights"""
+    out = []
+    for kind in (1, 2):
+        w = (C.c_int * 7)()
+        assert net.lib.myea_b200_lstm_walk(net.h, layer, kind, w) == 0
+        out.append(list(w))
+    return out
+
+
+# The resident walk on clusters: one to three steps (the barriers' first phases), rows and cells that do not divide; whether the forward and the
+# backward pass runs on one, in how many row passes, with how many rows per thread, and whether a thread keeps one row and cell
+@pytest.mark.parametrize("H,T,B,bidirectional,zoneout,forward,backward", [
+    (150, 1, 50, False, 0.0, (1, 1, 4, 1), (1, 1, 4, 1)), (150, 2, 50, False, 0.1, (1, 1, 4, 1), (1, 1, 4, 1)), (203, 3, 61, False, 0.0, (1, 1, 4, 1), (0, 1, 4, 1)),
+    (129, 7, 30, True, 0.2, (1, 1, 4, 1), (1, 1, 4, 1)), (120, 4, 200, False, 0.1, (1, 1, 4, 1), (1, 1, 4, 1)), (160, 4, 128, True, 0.0, (1, 1, 4, 1), (1, 1, 8, 1)),
+    (150, 5, 256, True, 0.0, (1, 2, 4, 0), (0, 1, 8, 0)), (205, 3, 256, True, 0.1, (1, 2, 4, 0), (0, 1, 8, 0)), (180, 4, 250, True, 0.2, (1, 2, 4, 0), (0, 1, 4, 0)),
+    (142, 4, 256, True, 0.1, (0, 1, 4, 1), (1, 1, 8, 0)), (142, 1, 255, True, 0.0, (0, 1, 4, 1), (1, 1, 8, 0))])
+def test_lstm_walk_on_clusters(H, T, B, bidirectional, zoneout, forward, backward):
+    wl = _one_lstm(5, H, T, B, bidirectional, zoneout)
+    net = Net(wl.desc, wl.opt)
+    walks = _walk(net)
+    net.close()
+    assert [(w[0], w[2], w[4], w[5], w[6]) for w in walks] == [(2,) + forward, (2,) + backward]
+    _step(wl)
+
+
+def _one_lstm(n_in, H, T, B, bidirectional, zoneout):
+    layers = [capi.fc(n_in), capi.lstm(H, bidirectional=bidirectional, dropout=capi.DROP_ZONEOUT if zoneout else capi.DROP_NONE, p=(zoneout, zoneout, 0.0)),
+              capi.fc(H, capi.AF_LINEAR)]
+    return workloads.Workload("lstm edges", capi.net(layers, B, T=T, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE),
+                              capi.opt(capi.OPT_GD, gd_lr=0.01 / B, momentum=0.9), n_in, H, False, layers)
 
 
 @pytest.mark.parametrize("n_in,H,T,B,bidirectional,zoneout", [
     (3, 5, 4, 3, False, 0.0), (7, 32, 3, 5, True, 0.3), (11, 37, 5, 50, False, 0.2), (16, 64, 1, 4, False, 0.0), (20, 107, 3, 9, False, 0.0), (20, 150, 4, 50, True, 0.1),
-    (9, 313, 3, 33, False, 0.0), (12, 512, 3, 70, False, 0.1), (5, 601, 3, 7, True, 0.0), (8, 1100, 2, 3, False, 0.0)])
+    (9, 313, 3, 33, False, 0.0), (12, 512, 3, 70, False, 0.1), (5, 601, 3, 7, True, 0.0), (8, 1100, 2, 3, False, 0.0), (5, 300, 4, 5, False, 0.1),
+    (5, 90, 5, 256, True, 0.0)])
 def test_lstm_with_resident_weights(n_in, H, T, B, bidirectional, zoneout):
-    layers = [capi.fc(n_in), capi.lstm(H, bidirectional=bidirectional, dropout=capi.DROP_ZONEOUT if zoneout else capi.DROP_NONE, p=(zoneout, zoneout, 0.0)),
-              capi.fc(H, capi.AF_LINEAR)]
-    wl = workloads.Workload("lstm edges", capi.net(layers, B, T=T, loss=capi.LOSS_MSE, accuracy=capi.ACC_DISTANCE),
-                            capi.opt(capi.OPT_GD, gd_lr=0.01 / B, momentum=0.9), n_in, H, False, layers)
-    _step(wl)
+    _step(_one_lstm(n_in, H, T, B, bidirectional, zoneout))
 
 
 @pytest.mark.parametrize("widths,B", [((1000, 904, 1100, 130), 700), ((1004, 1000, 1096), 640)])   # multiples of 8 and not, ragged blocks of 128
@@ -328,17 +352,6 @@ def test_reciprocal_of_the_lstm_cells_against_the_correctly_rounded_one():
     different, most = C.c_uint64(), C.c_uint32()
     assert lib.myea_b200_reciprocal_check(0, one, end - one, C.byref(different), C.byref(most)) == 0
     assert different.value == 0 and most.value == 0
-
-
-def _walk(net, layer=1):
-    """what the forward and the backward pass of an LSTM layer take: [walk, CTAs per group, cluster, groups, row passes, rows per thread, one cell
-    per thread]; walk 0 launches, 1 tensor cores, 2 resident weights"""
-    out = []
-    for kind in (1, 2):
-        w = (C.c_int * 7)()
-        assert net.lib.myea_b200_lstm_walk(net.h, layer, kind, w) == 0
-        out.append(list(w))
-    return out
 
 
 @pytest.mark.parametrize("backward", [False, True])
