@@ -1039,7 +1039,7 @@ static long long operand_pitch(const Operand &o, bool columns) { return columns 
 // tensor-core tiles: 128 x 256 x 64 3.4 / 4.6 / 4.8 / 5.7, 5.5; 128 x 256 x 256 5.2 / 5.5 / 5.4 / 6.0, 6.8; 64 x 512 x 512 8.4 / 6.7 / 6.2 /
 // 6.4, 8.0; 256 x 10 x 1024 15.2 / 10.2 / 7.3 / 6.5, 11.5; 32 x 64 x 4096 54 / 30 / 17 / 10, 17; 384^3 8.0, 7.8; rows that are not
 // 16-byte aligned: 203 x 333 x 75 5.3, 9.8; 203 x 333 x 333 9.5 / 11.5, 9.9; 333 x 333 x 203 6.6 / 8.3, 8.6; 161 x 150 x 2000 33 / 20 / 15 / 13, 12.
-// Tiles of 16 x 16 (cluster 0, tile 16) where they are up to two CTAs per SM.  Estimates from these measurements, beside the others':
+// Tiles of 16 x 16 (one CTA each) where they are up to two CTAs per SM.  Estimates from these measurements, beside the others':
 // 128 x 256 x 64 3.4, 128 x 256 x 256 4.0, 64 x 512 x 512 5.0, 256 x 256 x 512 6.6 (256 tiles), 256 x 10 x 1024 8.4, 32 x 64 x 4096 26; not aligned:
 // 203 x 333 x 75 3.4, 203 x 333 x 333 6.8 (273 tiles), 161 x 150 x 2000 read through its columns 20.6.
 struct FmaPlan {
@@ -1093,16 +1093,50 @@ static bool choose_reading(const DirectItem *items, int n, Operand DirectItem::*
   return *out || all_rows;
 }
 
+// How a launch runs: readings of its operands, tile and CTAs per tile
+struct DirectPlan {
+  bool at = false, bt = false;
+  int tile_m = DG_M, tile_n = DG_N, cluster = 1;
+};
+static bool plan_direct(const DirectItem *items, int n, DirectPlan *plan) {
+  bool sums = false;
+  for (int i = 0; i < n; ++i) sums = sums || items[i].row_sum != nullptr;   // these are taken from operands read through their columns
+  if (!choose_reading(items, n, &DirectItem::A, sums, &plan->at) || !choose_reading(items, n, &DirectItem::B, false, &plan->bt)) return false;
+  const FmaPlan fma = fma_plan(items, n, plan->at, plan->bt);
+  if (fma.tile != 0) {
+    plan->tile_m = plan->tile_n = fma.tile;
+    plan->cluster = fma.cluster;
+    return true;
+  }
+  long long tiles = 0, min_steps = 1 << 30;
+  for (int i = 0; i < n; ++i) {
+    tiles += (items[i].A.rows + DG_M - 1) / DG_M * ((items[i].B.rows + DG_N - 1) / DG_N);
+    min_steps = std::min(min_steps, (items[i].A.k + BK - 1) / BK);
+  }
+  // K is cut in up to four while the grid stays within one CTA per SM and every CTA keeps two stages.  Measured (us per
+  // launch, cut 1 / 2 / 4 / 8): 128 x 256 x 256 9.6 / 8.0 / 6.6 / 7.2, 203 x 333 x 333 18.6 / 13.6 / 9.8 / 11.3, 512^3 15.7 / 11.2
+  // / 8.8 / 12.3, 640^3 18.7 / 12.8 / 13.1 / 24.3, 1024 x 1024 x 256 10.1 / 11.1 / 18.0: clusters of eight are placed late, and
+  // pay only for very long walks (64 x 2048 x 2048: 53.0 / 30.1 / 17.8 / 16.6)
+  int &cluster = plan->cluster;
+  while (cluster < (min_steps >= 64 ? 8 : 4) && tiles * cluster * 2 <= (cluster == 4 ? 256 : 148) && min_steps >= cluster * 4) cluster *= 2;
+  return true;
+}
+
+template <bool AT, bool BT, int MAX>
+static int launch_planned(Context &ctx, const DirectGroup<MAX> &g, int tiles, const DirectPlan &plan) {
+  if (plan.tile_m == SG_TILE) return launch_small<AT, BT, MAX>(ctx, g, tiles);
+  if (plan.tile_m == FG_M) return launch_fma<AT, BT, MAX>(ctx, g, tiles, plan.cluster);
+  return launch_direct<AT, BT, MAX>(ctx, g, tiles, plan.cluster);
+}
+
 template <int MAX>
 static int direct_gemm_launch(Context &ctx, const DirectItem *items, int n) {
   DirectGroup<MAX> g;
   g.count = n;
-  int tiles = 0, min_steps = 1 << 30;
-  bool at, bt, sums = false;
-  for (int i = 0; i < n; ++i) sums = sums || items[i].row_sum != nullptr;   // these are taken from operands read through their columns
-  if (!choose_reading(items, n, &DirectItem::A, sums, &at) || !choose_reading(items, n, &DirectItem::B, false, &bt)) return MYEA_E_INVALID;
-  const FmaPlan fma = fma_plan(items, n, at, bt);
-  const int tile_m = fma.tile ? fma.tile : DG_M, tile_n = fma.tile ? fma.tile : DG_N;
+  int tiles = 0;
+  DirectPlan plan;
+  if (!plan_direct(items, n, &plan)) return MYEA_E_INVALID;
+  const bool at = plan.at, bt = plan.bt;
   for (int i = 0; i < n; ++i) {
     const DirectItem &it = items[i];
     DirectProblem &p = g.p[i];
@@ -1114,31 +1148,16 @@ static int direct_gemm_launch(Context &ctx, const DirectItem *items, int n) {
     p.a_vec = (reinterpret_cast<uintptr_t>(p.a) & 15) == 0 && (p.lda & 3) == 0;
     p.b_vec = (reinterpret_cast<uintptr_t>(p.b) & 15) == 0 && (p.ldb & 3) == 0;
     p.c_vec = epilogue_is_vector(it.epi, p.N);
-    p.tiles_n = (p.N + tile_n - 1) / tile_n;
+    p.tiles_n = (p.N + plan.tile_n - 1) / plan.tile_n;
     p.first_tile = tiles;
-    tiles += p.tiles_n * ((p.M + tile_m - 1) / tile_m);
+    tiles += p.tiles_n * ((p.M + plan.tile_m - 1) / plan.tile_m);
     p.row_sum = at ? it.row_sum : nullptr;
     p.epi = it.epi;
     if ((it.row_sum != nullptr && !at) || it.epi.stats_kind != 0) return MYEA_E_INVALID;
-    min_steps = std::min(min_steps, (p.K + BK - 1) / BK);
     ctx.gemm_flops += 2.0 * p.M * p.N * static_cast<double>(p.K);
   }
-  if (fma.tile == SG_TILE) {
-    if (at) return bt ? launch_small<true, true>(ctx, g, tiles) : launch_small<true, false>(ctx, g, tiles);
-    return bt ? launch_small<false, true>(ctx, g, tiles) : launch_small<false, false>(ctx, g, tiles);
-  }
-  if (fma.tile) {
-    if (at) return bt ? launch_fma<true, true>(ctx, g, tiles, fma.cluster) : launch_fma<true, false>(ctx, g, tiles, fma.cluster);
-    return bt ? launch_fma<false, true>(ctx, g, tiles, fma.cluster) : launch_fma<false, false>(ctx, g, tiles, fma.cluster);
-  }
-  // K is cut in up to four while the grid stays within one CTA per SM and every CTA keeps two stages.  Measured (us per
-  // launch, cut 1 / 2 / 4 / 8): 128 x 256 x 256 9.6 / 8.0 / 6.6 / 7.2, 203 x 333 x 333 18.6 / 13.6 / 9.8 / 11.3, 512^3 15.7 / 11.2
-  // / 8.8 / 12.3, 640^3 18.7 / 12.8 / 13.1 / 24.3, 1024 x 1024 x 256 10.1 / 11.1 / 18.0: clusters of eight are placed late, and
-  // pay only for very long walks (64 x 2048 x 2048: 53.0 / 30.1 / 17.8 / 16.6)
-  int cluster = 1;
-  while (cluster < (min_steps >= 64 ? 8 : 4) && tiles * cluster * 2 <= (cluster == 4 ? 256 : 148) && min_steps >= cluster * 4) cluster *= 2;
-  if (at) return bt ? launch_direct<true, true>(ctx, g, tiles, cluster) : launch_direct<true, false>(ctx, g, tiles, cluster);
-  return bt ? launch_direct<false, true>(ctx, g, tiles, cluster) : launch_direct<false, false>(ctx, g, tiles, cluster);
+  if (at) return bt ? launch_planned<true, true>(ctx, g, tiles, plan) : launch_planned<true, false>(ctx, g, tiles, plan);
+  return bt ? launch_planned<false, true>(ctx, g, tiles, plan) : launch_planned<false, false>(ctx, g, tiles, plan);
 }
 
 // Items of one call are read alike: all A through their rows or all through their columns, and all B.
@@ -1152,3 +1171,21 @@ int direct_gemm(Context &ctx, const DirectItem *items, int count) {
 }
 
 }  // namespace myea
+
+// For tests: how a product [M, K] x [N, K]^T of operands that start on 16-byte boundaries runs; columns: bit 0 / 1, A / B is read through its columns.
+// tile: rows of a tile, 16 and 32 with FMAs, 128 on the tensor cores straight from fp32, 256 from operand panels; ctas: that share a tile (0 for panels).
+extern "C" int myea_b200_contraction_plan(uint64_t M, uint64_t N, uint64_t K, int columns, int *tile, int *ctas) {
+  if (M == 0 || N == 0 || K == 0 || tile == nullptr || ctas == nullptr) return MYEA_E_INVALID;
+  const long long m = static_cast<long long>(M), n = static_cast<long long>(N), k = static_cast<long long>(K);
+  *tile = 256;
+  *ctas = 0;
+  if (!myea::direct_gemm_suits(myea::Context(), m, n, k)) return MYEA_OK;
+  myea::DirectItem item;
+  item.A = (columns & 1) != 0 ? myea::Operand{nullptr, m, k, 1, m} : myea::Operand{nullptr, m, k, k, 1};
+  item.B = (columns & 2) != 0 ? myea::Operand{nullptr, n, k, 1, n} : myea::Operand{nullptr, n, k, k, 1};
+  myea::DirectPlan plan;
+  if (!myea::plan_direct(&item, 1, &plan)) return MYEA_E_INVALID;
+  *tile = plan.tile_m;
+  *ctas = plan.cluster;
+  return MYEA_OK;
+}

@@ -17,7 +17,15 @@ pytestmark = pytest.mark.gpu
 TOL = 1e-4
 
 
-# (the size chooses: (64, 640, 2048) runs on tensor-core tiles, the others on FMA tiles)
+def _plan(M, N, K, columns=0):
+    """(rows of a tile, CTAs that share one): 16 and 32 with FMAs, 128 on the tensor cores straight from fp32, 256 from operand panels"""
+    tile, ctas = C.c_int(), C.c_int()
+    assert capi.load().myea_b200_contraction_plan(C.c_uint64(M), C.c_uint64(N), C.c_uint64(K), columns >> 17, C.byref(tile), C.byref(ctas)) == 0
+    return tile.value, ctas.value
+
+
+# (the size chooses: (64, 640, 2048) runs on tensor-core tiles, (257, 10, 1000) and (5, 4, 4099) on FMA tiles of 32 x 32 over clusters, the others on
+# FMA tiles of 16 x 16)
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (1, 64, 7), (3, 65, 31), (127, 63, 32), (128, 64, 33), (129, 65, 64), (130, 130, 257), (257, 10, 1000), (64, 640, 2048),
                                    (5, 4, 4099)])
 @pytest.mark.parametrize("accumulate", [0, 1])
@@ -37,6 +45,7 @@ def test_contraction_from_fp32_operands(M, N, K, accumulate):
 @pytest.mark.parametrize("engine", [0, 1 << 17, 1 << 18, 3 << 17])
 def test_contraction_from_fp32_operands_over_k(M, N, K, engine):
     lib = capi.load()
+    assert _plan(M, N, K, engine) == (16, 1)
     rng = np.random.default_rng(M + N + K)
     A, B = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
     out = np.zeros((M, N), np.float32)
@@ -192,11 +201,15 @@ def test_update_writes_operand_panels(widths, B, opt):
         assert rel_err(got, want) < TOL
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (31, 33, 3), (32, 32, 4), (33, 65, 255), (64, 96, 256), (65, 31, 257), (128, 256, 280), (100, 37, 360), (96, 128, 281), (90, 50, 361)])
+@pytest.mark.parametrize("M,N,K,tile", [
+    (1, 1, 1, 16), (31, 33, 3, 16), (32, 32, 4, 16), (33, 65, 255, 16), (64, 96, 256, 16), (65, 31, 257, 16), (128, 256, 280, 16), (100, 37, 360, 16), (96, 128, 281, 16),
+    (90, 50, 361, 16), (384, 384, 1, 32), (290, 310, 64, 32), (33, 2300, 130, 32), (300, 300, 255, 32), (320, 320, 256, 32), (300, 300, 257, 32), (257, 450, 281, 32),
+    (301, 303, 361, 32)])
 @pytest.mark.parametrize("columns", [0, 1 << 18, 3 << 17])   # both operands by rows, B by columns, both by columns
-def test_contraction_with_fmas(M, N, K, columns):
-    """the 32 x 32 FMA tile at the edges of its rows, columns and the 256 of K it holds at a time"""
+def test_contraction_with_fmas(M, N, K, tile, columns):
+    """the FMA tiles of 16 x 16 and, uncut, of 32 x 32 at the edges of their rows, columns and the 128 and 256 of K that they hold at a time"""
     lib = capi.load()
+    assert _plan(M, N, K, columns) == (tile, 1)
     rng = np.random.default_rng(M + N + K)
     A, B = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
     out = rng.standard_normal((M, N), dtype=np.float32)
@@ -207,14 +220,14 @@ def test_contraction_with_fmas(M, N, K, columns):
 
 
 @pytest.mark.parametrize("M,N,K", [(257, 640, 64), (300, 520, 7), (385, 449, 31), (1, 4800, 33), (129, 1250, 65), (4801, 1, 40), (415, 417, 1000), (513, 321, 32),
-                                   (128, 1216, 4100)])
+                                   (128, 1216, 4036)])
 @pytest.mark.parametrize("columns", [0, 1 << 17, 1 << 18, 3 << 17])   # which operands are read through their columns
 @pytest.mark.parametrize("accumulate", [0, 1])
 def test_contraction_on_tensor_core_tiles_from_fp32(M, N, K, columns, accumulate):
     """more than 148 tiles of 32 x 32, which is where the 128 x 64 tensor-core tile takes over: edges of its rows, columns and the
     32 of K of a stage, pitches that are not 16-byte aligned, K cut over a cluster"""
     lib = capi.load()
-    assert -(-M // 32) * -(-N // 32) > 148
+    assert -(-M // 32) * -(-N // 32) > 148 and _plan(M, N, K, columns)[0] == 128
     rng = np.random.default_rng(M + N + K)
     A, B = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
     out = rng.standard_normal((M, N), dtype=np.float32)
@@ -224,10 +237,13 @@ def test_contraction_on_tensor_core_tiles_from_fp32(M, N, K, columns, accumulate
     assert rel_err(out, want) < 5e-6
 
 
-@pytest.mark.parametrize("M,N,K", [(256, 10, 1024), (33, 7, 1025), (1, 1, 600), (40, 31, 4099), (1, 1000, 1000), (64, 512, 512), (65, 129, 515)])
-def test_contraction_with_fmas_over_a_cluster(M, N, K):
-    """few tiles and a long K: cut over 2, 4 and 8 CTAs, the last share shorter or empty"""
+@pytest.mark.parametrize("M,N,K,plan", [
+    (64, 1024, 1000, (32, 2)), (65, 600, 900, (32, 2)), (1, 1000, 1000, (32, 4)), (700, 12, 1301, (32, 4)), (256, 10, 1024, (32, 8)), (33, 7, 1025, (32, 8)),
+    (40, 31, 4099, (32, 8)), (1, 1, 600, (16, 1)), (64, 512, 512, (16, 1)), (65, 129, 515, (16, 1))])
+def test_contraction_with_fmas_over_a_cluster(M, N, K, plan):
+    """few tiles and a long K: cut over 2, 4 and 8 CTAs, the last share shorter; or, where they are as fast, tiles of 16 x 16"""
     lib = capi.load()
+    assert _plan(M, N, K) == plan
     rng = np.random.default_rng(M + N + K)
     A, B = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
     out = rng.standard_normal((M, N), dtype=np.float32)
