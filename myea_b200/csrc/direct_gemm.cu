@@ -965,21 +965,23 @@ static int launch_direct_reading(Context &ctx, const DirectGroup<MAX> &g, int ti
   return err == cudaSuccess ? MYEA_OK : MYEA_E_CUDA;
 }
 
-// Accesses of whole sectors where every operand read through its rows allows 16 bytes at least and K is not short.  A kernel that has
-// them beside the element-wise reads of other rows is slower at those (us without / with them: 512 x 709 x 1001 24.5 / 24.8, the second
-// operand through its columns 22.4 / 23.3; 256 x 1024 x 1001 13.6 / 14.1), and of a short K they gain nothing that a step shows (an
-// output layer's 512 x 709 x 64 8.5 / 8.4 by itself, 12 / 17 behind the error).  Aligned rows: 64 x 6000 x 256 9.7 / 9.4, 512 x 709 x
-// 784 17.7 / 17.1.
+// Accesses of whole sectors where every operand read through its rows allows 16 bytes at least.  A kernel that has them beside the
+// element-wise reads of other rows is slower at those (us without / with them: 512 x 709 x 1001 24.5 / 24.8, the second operand through
+// its columns 22.4 / 23.3; 256 x 1024 x 1001 13.6 / 14.1).  Aligned rows: 64 x 6000 x 256 9.7 / 9.4, 512 x 709 x 784 17.7 / 17.1.  Of a short
+// K the reading does not matter, and the product takes the kernel that the next one will, which reads its result: two of them in turn
+// fetch their instructions anew (784-1024-1024-10 on 256 rows: 3 us of a step of 165).
 template <bool AT, bool BT, int MAX>
 static int launch_direct(Context &ctx, const DirectGroup<MAX> &g, int tiles, int cluster) {
-  bool wide = !(AT && BT);
-  int longest = 0;
-  for (int i = 0; i < g.count; ++i) {
-    wide = wide && (AT || g.p[i].a_vec) && (BT || g.p[i].b_vec);
-    longest = std::max(longest, g.p[i].K);
+  if constexpr (!(AT && BT)) {
+    bool rows = true, result = true;
+    int longest = 0;
+    for (int i = 0; i < g.count; ++i) {
+      rows = rows && (AT || g.p[i].a_vec) && (BT || g.p[i].b_vec);
+      result = result && g.p[i].c_vec;
+      longest = std::max(longest, g.p[i].K);
+    }
+    if (longest >= 256 ? rows : result) return launch_direct_reading<AT, BT, MAX, true>(ctx, g, tiles, cluster);
   }
-  if constexpr (!(AT && BT))
-    if (wide && longest >= 256) return launch_direct_reading<AT, BT, MAX, true>(ctx, g, tiles, cluster);
   return launch_direct_reading<AT, BT, MAX, false>(ctx, g, tiles, cluster);
 }
 
