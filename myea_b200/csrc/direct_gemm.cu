@@ -138,6 +138,55 @@ __device__ __forceinline__ void dg_store8(uint8_t *hi, uint8_t *cross, uint32_t 
   *reinterpret_cast<uint4 *>(cross + (at ^ 16u)) = make_uint4(x[4], x[5], x[6], x[7]);
 }
 
+// Steps of the epilogue on VEC adjacent columns of NB rows, for dg_finish and sg_finish
+template <int VEC>
+__device__ __forceinline__ void ld_cols(float (&d)[VEC], const float *src) {
+  if constexpr (VEC == 4) { const float4 t = *reinterpret_cast<const float4 *>(src); d[0] = t.x; d[1] = t.y; d[2] = t.z; d[3] = t.w; }
+  else d[0] = *src;
+}
+template <int VEC>
+__device__ __forceinline__ void st_cols(float *dst, const float (&d)[VEC]) {
+  if constexpr (VEC == 4) *reinterpret_cast<float4 *>(dst) = make_float4(d[0], d[1], d[2], d[3]);
+  else *dst = d[0];
+}
+// what dropout leaves of the columns from n on
+template <int VEC>
+__device__ __forceinline__ void dg_factors(const Epilogue &e, int n, float (&factor)[VEC]) {
+#pragma unroll
+  for (int k = 0; k < VEC; ++k) factor[k] = (e.act_mask != nullptr && e.act_mask[n + k] == 0) ? 0.f : e.act_scale;
+}
+// take(row, column, slope): the activation's derivative at each element
+template <int NB, int VEC, typename Take>
+__device__ __forceinline__ void dg_derive(const Epilogue &e, const float (&pre)[NB][VEC], const float (&y)[NB][VEC], const float (&cs)[VEC], const float (&ch)[VEC], Take take) {
+  auto derive = [&](auto f) {
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) take(b, k, f(e.aux_pre != nullptr ? pre[b][k] * cs[k] + ch[k] : 0.f, e.aux_y != nullptr ? y[b][k] : 0.f));
+  };
+  switch (e.deriv_af) {
+    case MYEA_AF_TANH: derive([](float z, float w) { return af_derive(MYEA_AF_TANH, z, w); }); break;
+    case MYEA_AF_RELU: derive([](float z, float w) { return af_derive(MYEA_AF_RELU, z, w); }); break;
+    default: { const uint32_t af = e.deriv_af; derive([af](float z, float w) { return af_derive_rare(af, z, w); }); break; }
+  }
+}
+// activation and dropout in place
+template <int NB, int VEC>
+__device__ __forceinline__ void dg_fire(const Epilogue &e, float (&v)[NB][VEC], const float (&factor)[VEC]) {
+  auto fire = [&](auto f) {
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) { const float t = f(v[b][k]); v[b][k] = factor[k] != 0.f ? t * factor[k] : 0.f; }
+  };
+  switch (e.act_af) {
+    case MYEA_AF_TANH: fire([](float z) { return af_fire(MYEA_AF_TANH, z); }); break;
+    case MYEA_AF_RELU: fire([](float z) { return af_fire(MYEA_AF_RELU, z); }); break;
+    case MYEA_AF_LINEAR: fire([](float z) { return z; }); break;
+    default: { const uint32_t af = e.act_af; fire([af](float z) { return af_fire_rare(af, z); }); break; }
+  }
+}
+
 // What this CTA finishes of its tile: rows [first, first + count), summed over the CTAs of the cluster in rank order, through
 // the epilogue.  A thread keeps VEC adjacent columns and takes NB rows at a time, all their loads before the first use: with
 // a row at a time this part was latency after latency and took longer than the products (29 of 31 us at K = 10).
@@ -149,25 +198,14 @@ __device__ __forceinline__ void dg_finish(const DirectProblem &p, const float *p
   const Epilogue &e = p.epi;
   const int c = (static_cast<int>(threadIdx.x) % LANES) * VEC, n = n0 + c;
   if (n >= p.N) return;
-  auto load = [](Vec &d, const float *src) {
-    if constexpr (VEC == 4) { const float4 t = *reinterpret_cast<const float4 *>(src); d[0] = t.x; d[1] = t.y; d[2] = t.z; d[3] = t.w; }
-    else d[0] = *src;
-  };
-  auto store = [](float *dst, const Vec &d) {
-    if constexpr (VEC == 4) *reinterpret_cast<float4 *>(dst) = make_float4(d[0], d[1], d[2], d[3]);
-    else *dst = d[0];
-  };
   const bool affine = e.deriv_af != 0u && e.aux_pre != nullptr && e.col_scale != nullptr;
   Vec bias = {}, cs, ch = {};
 #pragma unroll
   for (int k = 0; k < VEC; ++k) cs[k] = 1.f;
-  if (e.bias != nullptr) load(bias, e.bias + n);
-  if (affine) { load(cs, e.col_scale + n); load(ch, e.col_shift + n); }
+  if (e.bias != nullptr) ld_cols(bias, e.bias + n);
+  if (affine) { ld_cols(cs, e.col_scale + n); ld_cols(ch, e.col_shift + n); }
   float factor[VEC];
-  if (e.act_out != nullptr) {
-#pragma unroll
-    for (int k = 0; k < VEC; ++k) factor[k] = (e.act_mask != nullptr && e.act_mask[n + k] == 0) ? 0.f : e.act_scale;
-  }
+  if (e.act_out != nullptr) dg_factors<VEC>(e, n, factor);
   const int end = min(first + count, p.M - m0);
 #pragma unroll 1
   for (int r0 = first + static_cast<int>(threadIdx.x) / LANES; r0 < end; r0 += NB * STEP) {
@@ -180,15 +218,15 @@ __device__ __forceinline__ void dg_finish(const DirectProblem &p, const float *p
       dst[b] = e.C + c_row(e, m) + n;
 #pragma unroll
       for (int k = 0; k < VEC; ++k) v[b][k] = 0.f;
-      if (e.addend != nullptr) load(add[b], e.addend + m * e.ld_addend + n);
-      if (e.deriv_af != 0u && e.aux_pre != nullptr) load(pre[b], e.aux_pre + m * e.ld_aux + n);
-      if (e.deriv_af != 0u && e.aux_y != nullptr) load(y[b], e.aux_y + m * e.ld_aux + n);
-      if (e.accumulate) load(old[b], dst[b]);
+      if (e.addend != nullptr) ld_cols(add[b], e.addend + m * e.ld_addend + n);
+      if (e.deriv_af != 0u && e.aux_pre != nullptr) ld_cols(pre[b], e.aux_pre + m * e.ld_aux + n);
+      if (e.deriv_af != 0u && e.aux_y != nullptr) ld_cols(y[b], e.aux_y + m * e.ld_aux + n);
+      if (e.accumulate) ld_cols(old[b], dst[b]);
       if (S == 1) {
 #pragma unroll
         for (int q = 0; q < PARTS; ++q) {
           Vec t;
-          load(t, partial + (q * FG_M + r) * PITCH + c);   // (one part: row r of it)
+          ld_cols(t, partial + (q * FG_M + r) * PITCH + c);   // (one part: row r of it)
 #pragma unroll
           for (int k = 0; k < VEC; ++k) v[b][k] += t[k];
         }
@@ -220,19 +258,7 @@ __device__ __forceinline__ void dg_finish(const DirectProblem &p, const float *p
         if (e.addend != nullptr) v[b][k] += add[b][k];
       }
     }
-    if (e.deriv_af != 0u) {
-      auto derive = [&](auto f) {
-#pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-          for (int k = 0; k < VEC; ++k) v[b][k] *= f(e.aux_pre != nullptr ? pre[b][k] * cs[k] + ch[k] : 0.f, e.aux_y != nullptr ? y[b][k] : 0.f);
-      };
-      switch (e.deriv_af) {
-        case MYEA_AF_TANH: derive([](float z, float w) { return af_derive(MYEA_AF_TANH, z, w); }); break;
-        case MYEA_AF_RELU: derive([](float z, float w) { return af_derive(MYEA_AF_RELU, z, w); }); break;
-        default: { const uint32_t af = e.deriv_af; derive([af](float z, float w) { return af_derive_rare(af, z, w); }); break; }
-      }
-    }
+    if (e.deriv_af != 0u) dg_derive<NB, VEC>(e, pre, y, cs, ch, [&](int b, int k, float slope) { v[b][k] *= slope; });
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
       if (r0 + b * STEP >= end) break;
@@ -240,25 +266,14 @@ __device__ __forceinline__ void dg_finish(const DirectProblem &p, const float *p
 #pragma unroll
         for (int k = 0; k < VEC; ++k) v[b][k] += old[b][k];
       }
-      store(dst[b], v[b]);
+      st_cols(dst[b], v[b]);
     }
     if (e.act_out != nullptr) {
-      auto fire = [&](auto f) {
-#pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-          for (int k = 0; k < VEC; ++k) { const float t = f(v[b][k]); v[b][k] = factor[k] != 0.f ? t * factor[k] : 0.f; }
-      };
-      switch (e.act_af) {
-        case MYEA_AF_TANH: fire([](float z) { return af_fire(MYEA_AF_TANH, z); }); break;
-        case MYEA_AF_RELU: fire([](float z) { return af_fire(MYEA_AF_RELU, z); }); break;
-        case MYEA_AF_LINEAR: fire([](float z) { return z; }); break;
-        default: { const uint32_t af = e.act_af; fire([af](float z) { return af_fire_rare(af, z); }); break; }
-      }
+      dg_fire<NB, VEC>(e, v, factor);
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         if (r0 + b * STEP >= end) break;
-        store(e.act_out + (dst[b] - e.C), v[b]);
+        st_cols(e.act_out + (dst[b] - e.C), v[b]);
       }
     }
   }
@@ -615,104 +630,49 @@ constexpr int SG_TILE = 16, SG_K = 128, SG_PITCH = SG_K + 4;   // K of a chunk, 
 constexpr int SG_SMEM = 2 * 2 * SG_TILE * SG_PITCH * 4;          // two chunks; the partial tiles and row sums lie over them
 static_assert(SG_SMEM >= (8 * SG_TILE * (SG_TILE + 4) + 8 * SG_TILE) * 4, "the partial tiles lie over the operands");
 
-// The epilogue of a tile: rows [first, first + count), summed by `sum(row, column, v)` and taken through the
-// epilogue.  A thread keeps VEC adjacent columns and takes NB rows at a time.  What the epilogue reads from memory for the first NB
-// of them is on its way before `work`, which computes the partial tiles and ends with them visible to every thread: behind it this
-// part was latency after latency and took longer than the products (29 of 31 us at K = 10).
-// TN: columns of the tile.
-template <int TN, int VEC, int NB, typename Work, typename Sum>
-__device__ __forceinline__ void sg_finish(const DirectProblem &p, int first, int count, int m0, int n0, Work work, Sum sum) {
-  constexpr int LANES = TN / VEC, STEP = DG_THREADS / LANES;
+// The epilogue of a tile of 16 x 16: a thread has VEC adjacent columns of one row at most, summed by `sum(row, column, v)`.  What
+// the epilogue reads from memory is on its way before `work`, which computes the partial tiles and ends with them visible to every thread.
+// (dg_finish, where a thread has several rows, in this form is slower by 1 to 3 us: 512 x 709 x 64 8.5 -> 10.7.)
+template <int VEC, typename Work, typename Sum>
+__device__ __forceinline__ void sg_finish(const DirectProblem &p, int m0, int n0, Work work, Sum sum) {
+  constexpr int LANES = SG_TILE / VEC;
   using Vec = float[VEC];
   const Epilogue &e = p.epi;
-  const int c = (static_cast<int>(threadIdx.x) % LANES) * VEC, n = n0 + c;
-  auto load = [](Vec &d, const float *src) {
-    if constexpr (VEC == 4) { const float4 t = *reinterpret_cast<const float4 *>(src); d[0] = t.x; d[1] = t.y; d[2] = t.z; d[3] = t.w; }
-    else d[0] = *src;
-  };
-  auto store = [](float *dst, const Vec &d) {
-    if constexpr (VEC == 4) *reinterpret_cast<float4 *>(dst) = make_float4(d[0], d[1], d[2], d[3]);
-    else *dst = d[0];
-  };
-  const bool in = n < p.N;
-  const bool affine = e.deriv_af != 0u && e.aux_pre != nullptr && e.col_scale != nullptr;
-  Vec bias = {}, factor = {};
-  if (in && e.bias != nullptr) load(bias, e.bias + n);
-  if (in && e.act_out != nullptr) {
-#pragma unroll
-    for (int k = 0; k < VEC; ++k) factor[k] = (e.act_mask != nullptr && e.act_mask[n + k] == 0) ? 0.f : e.act_scale;
-  }
-  const int end = in ? min(first + count, p.M - m0) : first;
-  Vec add[NB], slope[NB], old[NB];   // bias and addend, activation derivative, what lies in C
-  auto fetch = [&](int r0) {
-    Vec pre[NB], y[NB];
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      const long long m = m0 + min(r0 + b * STEP, end - 1);   // rows past the end repeat the last one and are not stored
-#pragma unroll
-      for (int k = 0; k < VEC; ++k) add[b][k] = 0.f;
-      if (e.addend != nullptr) load(add[b], e.addend + m * e.ld_addend + n);
-      if (e.deriv_af != 0u && e.aux_pre != nullptr) load(pre[b], e.aux_pre + m * e.ld_aux + n);
-      if (e.deriv_af != 0u && e.aux_y != nullptr) load(y[b], e.aux_y + m * e.ld_aux + n);
-      if (e.accumulate) load(old[b], e.C + c_row(e, m) + n);
-    }
+  const int c = (static_cast<int>(threadIdx.x) % LANES) * VEC, n = n0 + c, r = static_cast<int>(threadIdx.x) / LANES;
+  const long long m = m0 + r;
+  const bool in = n < p.N && r < SG_TILE && m < p.M;
+  Vec bias = {}, factor = {}, add = {}, slope, old;   // slope: activation derivative; old: what lies in C
+  if (in) {
+    if (e.bias != nullptr) ld_cols(bias, e.bias + n);
+    if (e.act_out != nullptr) dg_factors<VEC>(e, n, factor);
+    if (e.addend != nullptr) ld_cols(add, e.addend + m * e.ld_addend + n);
+    if (e.accumulate) ld_cols(old, e.C + c_row(e, m) + n);
     if (e.deriv_af != 0u) {
+      float pre[1][VEC], y[1][VEC];
       Vec cs, ch = {};
 #pragma unroll
       for (int k = 0; k < VEC; ++k) cs[k] = 1.f;
-      if (affine) { load(cs, e.col_scale + n); load(ch, e.col_shift + n); }
-      auto derive = [&](auto f) {
-#pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-          for (int k = 0; k < VEC; ++k) slope[b][k] = f(e.aux_pre != nullptr ? pre[b][k] * cs[k] + ch[k] : 0.f, e.aux_y != nullptr ? y[b][k] : 0.f);
-      };
-      switch (e.deriv_af) {
-        case MYEA_AF_TANH: derive([](float z, float w) { return af_derive(MYEA_AF_TANH, z, w); }); break;
-        case MYEA_AF_RELU: derive([](float z, float w) { return af_derive(MYEA_AF_RELU, z, w); }); break;
-        default: { const uint32_t af = e.deriv_af; derive([af](float z, float w) { return af_derive_rare(af, z, w); }); break; }
-      }
+      if (e.aux_pre != nullptr) ld_cols(pre[0], e.aux_pre + m * e.ld_aux + n);
+      if (e.aux_y != nullptr) ld_cols(y[0], e.aux_y + m * e.ld_aux + n);
+      if (e.aux_pre != nullptr && e.col_scale != nullptr) { ld_cols(cs, e.col_scale + n); ld_cols(ch, e.col_shift + n); }
+      dg_derive<1, VEC>(e, pre, y, cs, ch, [&](int, int k, float x) { slope[k] = x; });
     }
-  };
-  int r0 = first + static_cast<int>(threadIdx.x) / LANES;
-  if (r0 < end) fetch(r0);
+  }
   work();
-#pragma unroll 1
-  while (r0 < end) {
-    Vec v[NB];
+  if (!in) return;
+  float v[1][VEC] = {};
+  sum(r, c, v[0]);
 #pragma unroll
-    for (int b = 0; b < NB; ++b) {
-#pragma unroll
-      for (int k = 0; k < VEC; ++k) v[b][k] = 0.f;
-      sum(min(r0 + b * STEP, end - 1), c, v[b]);
-#pragma unroll
-      for (int k = 0; k < VEC; ++k) {
-        v[b][k] += bias[k];
-        if (e.addend != nullptr) v[b][k] += add[b][k];
-        if (e.deriv_af != 0u) v[b][k] *= slope[b][k];
-        if (e.accumulate) v[b][k] += old[b][k];
-      }
-      if (r0 + b * STEP < end) store(e.C + c_row(e, m0 + r0 + b * STEP) + n, v[b]);
-    }
-    if (e.act_out != nullptr) {
-      auto fire = [&](auto f) {
-#pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-          for (int k = 0; k < VEC; ++k) { const float t = f(v[b][k]); v[b][k] = factor[k] != 0.f ? t * factor[k] : 0.f; }
-      };
-      switch (e.act_af) {
-        case MYEA_AF_TANH: fire([](float z) { return af_fire(MYEA_AF_TANH, z); }); break;
-        case MYEA_AF_RELU: fire([](float z) { return af_fire(MYEA_AF_RELU, z); }); break;
-        case MYEA_AF_LINEAR: fire([](float z) { return z; }); break;
-        default: { const uint32_t af = e.act_af; fire([af](float z) { return af_fire_rare(af, z); }); break; }
-      }
-#pragma unroll
-      for (int b = 0; b < NB; ++b)
-        if (r0 + b * STEP < end) store(e.act_out + c_row(e, m0 + r0 + b * STEP) + n, v[b]);
-    }
-    r0 += NB * STEP;
-    if (r0 < end) fetch(r0);
+  for (int k = 0; k < VEC; ++k) {
+    v[0][k] += bias[k];
+    if (e.addend != nullptr) v[0][k] += add[k];
+    if (e.deriv_af != 0u) v[0][k] *= slope[k];
+    if (e.accumulate) v[0][k] += old[k];
+  }
+  st_cols(e.C + c_row(e, m) + n, v[0]);
+  if (e.act_out != nullptr) {
+    dg_fire<1, VEC>(e, v, factor);
+    st_cols(e.act_out + c_row(e, m) + n, v[0]);
   }
 }
 
@@ -917,8 +877,8 @@ __global__ void __launch_bounds__(DG_THREADS, 2) small_gemm_kernel(const __grid_
       }
     }
   };
-  if (p.c_vec) sg_finish<TN, 4, 1>(p, 0, TM, m0, n0, work, sum);
-  else sg_finish<TN, 1, 1>(p, 0, TM, m0, n0, work, sum);
+  if (p.c_vec) sg_finish<4>(p, m0, n0, work, sum);
+  else sg_finish<1>(p, m0, n0, work, sum);
   if (want_sum && tid < TM && m0 + tid < p.M) {
     float v = 0.f;
 #pragma unroll
