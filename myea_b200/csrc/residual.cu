@@ -35,10 +35,10 @@ __global__ void __launch_bounds__(256) shakedrop_kernel(const float *__restrict_
                                                         const uint8_t *__restrict__ mask, const float *__restrict__ coef, float scale,
                                                         long long rows, long long H) {
   grid_dependency_wait();
-  // The product that follows sets itself up early where this kernel has a block per SM at most (512 units, 256 rows, four blocks of
-  // layers, four steps: 1.27 -> 1.24 ms).  Beside several blocks to an SM its CTAs are set two to an SM, and it starts behind the last block
-  // instead (473 units, 224 rows, five blocks, eight steps: 3.58 -> 3.23 ms).
-  if (gridDim.x <= 148) grid_dependency_release();
+  // The product that follows sets itself up early where this kernel has two blocks per SM at most (four blocks of layers, four steps: 512
+  // units, 256 rows 1.27 -> 1.24 ms; 800 units, 224 rows, 175 blocks here, 1.868 -> 1.853).  Beside more of them its CTAs are set two to an
+  // SM, and it starts behind the last block instead (473 units, 224 rows, 414 blocks, early 1.52 ms, late 1.39).
+  if (gridDim.x <= 296) grid_dependency_release();
   const long long hv = H / VEC, total = rows * hv;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
